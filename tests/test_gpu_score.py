@@ -1,0 +1,46 @@
+"""Target probabilities of config.json families (prefill with targets): the device kernel against softmax in float64 over the same pass's logits."""
+import numpy as np
+import pytest
+
+import bolovik_oracle as O
+from xalm_b200 import capi
+from xalm_b200.model import Model
+
+pytestmark = pytest.mark.gpu
+
+
+def small_model(vocab, chunk, max_tokens=96):
+    cfg = O.make_config(vocab=vocab, width=64, layers=[O.attention_layer(4, 2, 16, 16, mlp=O.dense(64))], groups=2)
+    capi.tune("seq_chunk", chunk)
+    m = Model.from_json(cfg, O.random_weights(cfg, vocab)).cuda(max_tokens=max_tokens)
+    capi.tune("seq_chunk", 256)
+    return m
+
+
+# below one value per thread, 16-byte rows with and without a remainder of the unrolled loop, rows that cannot be read 16 bytes at a time
+@pytest.mark.parametrize("vocab", [3, 500, 2048, 8192 + 4 * 513, 10007])
+@pytest.mark.parametrize("fetch", [False, True])
+def test_target_probabilities_over_several_passes(vocab, fetch):
+    rng = np.random.default_rng(vocab)
+    m, n = small_model(vocab, 32), 75
+    toks, targets = rng.integers(0, vocab, n), rng.integers(0, vocab, n)
+    lg = m.prefill(toks, 0, want_logits=2).astype(np.float64)
+    m.release()
+    got_lg, got = m.prefill(toks, 0, want_logits=2, targets=targets, fetch_logits=fetch)
+    assert got_lg is None or np.array_equal(got_lg, lg.astype(np.float32))
+    e = np.exp(lg - lg.max(1, keepdims=True))
+    want = e[np.arange(n), targets] / e.sum(1)
+    # exp in fp32 on differences below 32: 2^-23 * 32 / 2 from rounding the difference, and as much from the sums of up to 10^4 terms in parts
+    assert np.abs(got / want - 1).max() < 1e-5
+    m.close()
+
+
+def test_a_target_out_of_range_is_refused_after_the_rows_before_it():
+    m, n = small_model(100, 32), 40
+    toks = np.arange(n) % 100
+    targets = toks.copy()
+    targets[35] = 100
+    with pytest.raises(capi.XalmError, match="target 100 out of range"):
+        m.prefill(toks, 0, want_logits=2, targets=targets, fetch_logits=False)
+    assert m.info("position") == n
+    m.close()

@@ -43,6 +43,7 @@
 #include "frag_layout.cuh"
 #include "act_ops.cuh"
 #include "prefill.h"
+#include "target_prob.cuh"
 
 namespace xalm {
 
@@ -761,31 +762,6 @@ __global__ void __launch_bounds__(128) rmsnorm_rows_kernel(const float* __restri
 		}
 		for (int j = threadIdx.x * 8 + MAXC * 1024; j < dim; j += 1024)
 			emit(j, *reinterpret_cast<const float4*>(xr + j), *reinterpret_cast<const float4*>(xr + j + 4));
-	}
-}
-
-// Sampler::sample_prob (sampler.cpp:18-33) per row: softmax(logits)[target], the FLT_MIN-seeded max included
-__global__ void target_prob_kernel(const float* __restrict__ logits, int vocab, const int* __restrict__ targets, float* __restrict__ probs) {
-	__shared__ float red[32];
-	const float* l = logits + (size_t) blockIdx.x * vocab;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-	float mx = FLT_MIN;
-	for (int i = threadIdx.x; i < vocab; i += blockDim.x) mx = fmaxf(mx, l[i]);
-	mx = warp_max(mx);
-	if (lane == 0) red[warp] = mx;
-	__syncthreads();
-	mx = red[0];
-	for (int i = 1; i < nw; i++) mx = fmaxf(mx, red[i]);
-	__syncthreads();
-	float sum = 0.f;
-	for (int i = threadIdx.x; i < vocab; i += blockDim.x) sum += expf(l[i] - mx);
-	sum = warp_sum(sum);
-	if (lane == 0) red[warp] = sum;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		float tot = 0.f;
-		for (int i = 0; i < nw; i++) tot += red[i];
-		probs[blockIdx.x] = expf(l[targets[blockIdx.x]] - mx) / tot;
 	}
 }
 
@@ -1687,8 +1663,8 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 			for (int i = 0; i < T; i++)
 				if (targets[i] < 0 || targets[i] >= c.vocab_size) return set_error(XALM_ERR_INVALID, "prefill: target %d out of range", targets[i]);
 			XALM_CUDA_CHECK(cudaMemcpyAsync(sc.targets.p, targets, (size_t) T * 4, cudaMemcpyHostToDevice, s));
-			target_prob_kernel<<<T, 256, 0, s>>>(reinterpret_cast<const float*>(sc.logits.p), c.vocab_size, reinterpret_cast<const int*>(sc.targets.p),
-			                                     reinterpret_cast<float*>(sc.probs.p));
+			target_prob_kernel<<<T, TARGET_PROB_THREADS, 0, s>>>(reinterpret_cast<const float*>(sc.logits.p), c.vocab_size, FLT_MIN,
+			                                                     reinterpret_cast<const int*>(sc.targets.p), reinterpret_cast<float*>(sc.probs.p));
 			launches++;
 			XALM_CUDA_CHECK(cudaMemcpyAsync(probs_host, sc.probs.p, (size_t) T * 4, cudaMemcpyDeviceToHost, s));
 		}
