@@ -1974,6 +1974,14 @@ static inline int swa_pick_tq(int H, int G, int d, int dv, int rows) {
 	return 0;
 }
 
+// swa_one.cu: steps of one to four tokens whose heads do not mix.  Takes a.n_splits > 0
+int launch_swa_one(const SwaArgs& a, int rows, bool cache_f32, cudaStream_t s);
+// It reads the cache 16 bytes at a time and holds a head's channels in registers: whole 8-channel pieces, at most 768 of them
+static inline bool swa_one_ok(const SwaArgs& a, int rows) {
+	return rows <= 4 && !a.talk && a.G > 0 && a.H % a.G == 0 && ((a.d | a.dv | a.ldk | a.ldv) & 7) == 0 && ((a.ldq | a.q_off) & 3) == 0 && std::max(a.d, a.dv) <= 768 && a.G * (long long) a.H <= 65535 &&
+	       ((reinterpret_cast<uintptr_t>(a.kc) | reinterpret_cast<uintptr_t>(a.vc) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
+}
+
 // rows: tokens of the step; cache_f32: element type of the ring.  With n_splits > 1 the merge kernel follows.  Returns the number of
 // launches through *launches (1 or 2) when it is given.
 static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s, int* launches = nullptr) {
@@ -2008,6 +2016,21 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 		}
 	}
 	const int tq = swa_pick_tq(a.H, a.G, a.d, a.dv, rows);
+	if (swa_one_ok(a, rows)) {
+		if (a.n_splits <= 0) { // a cluster of eight CTAs takes up to 4096 keys; beyond that, more clusters and a join
+			long long reach = a.window < 0x7fffffff ? a.window : a.ring;
+			if (a.mask_chunk > 0) reach = std::min<long long>(reach, a.mask_chunk);
+			const long long want = (std::min<long long>(reach, a.ring) + a.keep_first + 4095) / 4096;
+			a.n_splits = (a.part_o && a.part_ml) ? (int) std::max<long long>(1, std::min<long long>(want, a.part_cap / std::max(1, rows))) : 1;
+		}
+		if (launches) *launches = a.n_splits > 1 ? 2 : 1;
+		XALM_TRY(launch_swa_one(a, rows, cache_f32, s));
+		if (a.n_splits > 1) {
+			swa_merge_kernel<<<dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s>>>(a);
+			XALM_TRY(launch_check("swa_merge"));
+		}
+		return XALM_OK;
+	}
 	if (a.n_splits <= 0) { // enough CTAs for two waves, at least two key blocks each
 		const int qblocks = tq ? (rows + tq - 1) / tq : rows;
 		long long reach = a.window < 0x7fffffff ? a.window : a.ring;
