@@ -1,0 +1,47 @@
+"""Products of one token with bf16 weights (four columns per warp, slices of K over warps): columns that do not fill a warp's four, lengths around a lane's
+pieces and around the slices, every epilogue that pairs columns, the chosen experts' products."""
+import numpy as np
+import pytest
+
+from xalm_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+def bf16(a):
+    return (np.ascontiguousarray(a, np.float32).view(np.uint32) + 0x8000 & 0xFFFF0000).view(np.float32)
+
+
+def bound(K):
+    """fp32 sums of K products of order K^-1/2 in K / 256 steps per lane and a tree: far below sqrt(K) roundings of values of order one."""
+    return 2.0 ** -23 * (K ** 0.5 + 8) * 4
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 4, 7, 33, 2500])
+@pytest.mark.parametrize("K", [8, 248, 256, 264, 512, 1000, 2048, 4104])
+def test_plain_and_paired_columns(N, K):
+    rng = np.random.default_rng(N * K)
+    x, w, u = rng.standard_normal((1, K)).astype(np.float32), bf16(rng.standard_normal((N, K)) / K ** 0.5), bf16(rng.standard_normal((N, K)) / K ** 0.5)
+    z, y = x.astype(np.float64) @ w.T, x.astype(np.float64) @ u.T
+    mul = rng.standard_normal((1, N)).astype(np.float32)
+    got = capi.rows_act(x, w, act=0, cap=20.0, mul=mul, w_bf16=True)
+    assert np.abs(got - 20 * np.tanh(z / 20) / (1 + np.exp(-mul))).max() < bound(K)
+    got = capi.glu_rows(x, w, u, 7.0, w_bf16=True)
+    g = np.minimum(z, 7.0)
+    assert np.abs(got - g / (1 + np.exp(-1.702 * g)) * (np.clip(y, -7, 7) + 1)).max() < 4 * bound(K)
+
+
+@pytest.mark.parametrize("T,K,ff", [(1, 64, 24), (1, 1032, 40), (3, 256, 6), (2, 2048, 130)])
+def test_chosen_experts(T, K, ff):
+    rng = np.random.default_rng(K + ff)
+    E, top = 6, 2
+    h = rng.standard_normal((T, K)).astype(np.float32)
+    wr = bf16(rng.standard_normal((E, K)) * 3 / K ** 0.5)
+    wg, wu, wd = (bf16(rng.standard_normal(s) / s[2] ** 0.5) for s in ((E, ff, K), (E, ff, K), (E, K, ff)))
+    idx, wgt, out = capi.moe_ffn(h, wr, wg, wu, wd, top, w_bf16=True)
+    for t in range(T):
+        for r in range(top):
+            e, x = idx[t, r], h[t].astype(np.float64)
+            g = wg[e].astype(np.float64) @ x
+            want = wd[e].astype(np.float64) @ (g / (1 + np.exp(-g)) * (wu[e].astype(np.float64) @ x))
+            assert np.abs(out[t, r] - want).max() < 4 * bound(K) + 4 * bound(ff)

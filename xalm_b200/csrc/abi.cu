@@ -7,6 +7,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <map>
 #include <string>
 #include <vector>
@@ -83,6 +84,26 @@ int tune(const char* k) {
 	return tuning()[k];
 }
 
+
+// ---------------------------------------------------------------------------------------------------------
+// programmatic dependent launches (common.cuh)
+// ---------------------------------------------------------------------------------------------------------
+static std::vector<cudaStream_t>& blocked_streams() { // a few at most: a model's two streams, each asked about soon after
+	static thread_local std::vector<cudaStream_t> b;
+	return b;
+}
+void pdl_block(cudaStream_t s) {
+	std::vector<cudaStream_t>& b = blocked_streams();
+	if (std::find(b.begin(), b.end(), s) == b.end()) b.push_back(s);
+}
+bool pdl_next(cudaStream_t s) {
+	if (!s || !tune("pdl")) return false;
+	std::vector<cudaStream_t>& b = blocked_streams();
+	const auto it = std::find(b.begin(), b.end(), s);
+	if (it == b.end()) return true;
+	b.erase(it);
+	return false;
+}
 
 // ---------------------------------------------------------------------------------------------------------
 // family registry

@@ -65,6 +65,32 @@ __device__ __forceinline__ float4 ld_act4(const float* p) { return *reinterpret_
 // ---- programmatic dependent launch (sm_90+): let the next kernel's prologue overlap this kernel's tail ----
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+// The head of a kernel of a one-token step: its inputs are complete from here on, and the next kernel may take its place on the SMs.  In this order only
+// one kernel is ahead of the running one: with the other, a whole chain of waiting products took the SMs from the step's other branch.
+__device__ __forceinline__ void pdl_enter() {
+	pdl_wait();
+	pdl_launch_dependents();
+}
+// Whether the next kernel launched on `s` may overlap the one before it: true unless pdl_block(s) was called since the last such question (a copy, an
+// event from another stream or another caller's work lies between).  Per thread; the NULL stream never overlaps.  abi.cu.
+bool pdl_next(cudaStream_t s);
+void pdl_block(cudaStream_t s);
+// A launch of a step of `rows` tokens.  One-token steps run their kernels as programmatic dependents: a kernel's launch and its first instructions
+// (for the products also its first weights) overlap the kernel before it, about 1 us of each of a step's 20 to 40 launches.
+template <typename... P, typename... A>
+inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int rows, A... args) {
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = s;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = rows == 1 && pdl_next(s) ? 1 : 0;
+	return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // ---- L2 prefetch of a slice of the NEXT kernel's first bytes (cp.async.bulk.prefetch.L2): CTA `cta` of `n_ctas` takes its share ----
 __device__ __forceinline__ void l2_prefetch_slice(const uint8_t* ptr, unsigned long long bytes, int cta, int n_ctas) {

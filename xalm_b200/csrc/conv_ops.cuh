@@ -49,6 +49,7 @@ struct NormConvArgs {
 constexpr int NORM_CONV_SPAN = NORM_CONV_ROWS + CONV_MAX_TAPS; // most rows a CTA touches
 template <int TAPS>
 __global__ void __launch_bounds__(256) norm_conv_kernel(NormConvArgs a) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	constexpr int M = TAPS ? TAPS : CONV_MAX_TAPS + 1, SPAN = NORM_CONV_ROWS + M - 1;
 	const int W = a.width, taps = TAPS ? TAPS : a.taps, keep = taps - 1, rd = blockIdx.y, gs = W / a.groups, c0 = blockIdx.z * gs;
@@ -138,15 +139,16 @@ static inline int launch_norm_conv(const NormConvArgs& a, int rows, cudaStream_t
 	const int gs = a.width / a.groups, nt = gs >= 256 ? 256 : gs >= 128 ? 128 : 64;
 	const dim3 grid(blocks, a.readers, a.groups);
 	const size_t smem = norm_conv_smem(a.width, a.taps, a.groups);
-	if (a.taps == 1) norm_conv_kernel<1><<<grid, nt, smem, s>>>(a);
-	else if (a.taps == 2) norm_conv_kernel<2><<<grid, nt, smem, s>>>(a);
-	else if (a.taps == 3) norm_conv_kernel<3><<<grid, nt, smem, s>>>(a);
-	else if (a.taps == 4) norm_conv_kernel<4><<<grid, nt, smem, s>>>(a);
-	else norm_conv_kernel<0><<<grid, nt, smem, s>>>(a);
+	if (a.taps == 1) launch_step(norm_conv_kernel<1>, grid, nt, smem, s, rows, a);
+	else if (a.taps == 2) launch_step(norm_conv_kernel<2>, grid, nt, smem, s, rows, a);
+	else if (a.taps == 3) launch_step(norm_conv_kernel<3>, grid, nt, smem, s, rows, a);
+	else if (a.taps == 4) launch_step(norm_conv_kernel<4>, grid, nt, smem, s, rows, a);
+	else launch_step(norm_conv_kernel<0>, grid, nt, smem, s, rows, a);
 	XALM_TRY(launch_check("norm_conv"));
 	if (launches) *launches = 1;
 	if (blocks > 1 && a.taps > 1) {
 		XALM_CUDA_CHECK(cudaMemcpyAsync(a.hist[0], a.stage[0], (size_t) a.readers * (a.taps - 1) * a.width * 4, cudaMemcpyDeviceToDevice, s));
+		pdl_block(s);
 		if (launches) *launches = 2;
 	}
 	return XALM_OK;
@@ -167,6 +169,7 @@ struct ShortConvArgs {
 
 // grid (ceil(C / 128), ceil(T / SHORT_CONV_ROWS)), 128 threads: a thread per channel, the window of its last inputs in registers
 static __global__ void short_conv_kernel(ShortConvArgs a) {
+	pdl_enter();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x, taps = a.taps, keep = taps - 1;
 	const int n = a.step->n, r0 = blockIdx.y * SHORT_CONV_ROWS, r1 = min(n, r0 + SHORT_CONV_ROWS);
 	if (c >= a.C || r0 >= n) return;
@@ -198,11 +201,12 @@ static __global__ void short_conv_kernel(ShortConvArgs a) {
 static inline int launch_short_conv(const ShortConvArgs& a, int rows, cudaStream_t s, int* launches = nullptr) {
 	if (a.taps < 1 || a.taps > CONV_MAX_TAPS) return set_error(XALM_ERR_UNSUPPORTED, "short convolution: %d taps (1 to %d)", a.taps, CONV_MAX_TAPS);
 	const int blocks = (rows + SHORT_CONV_ROWS - 1) / SHORT_CONV_ROWS;
-	short_conv_kernel<<<dim3((a.C + 127) / 128, blocks), 128, 0, s>>>(a);
+	launch_step(short_conv_kernel, dim3((a.C + 127) / 128, blocks), 128, 0, s, rows, a);
 	XALM_TRY(launch_check("short_conv"));
 	if (launches) *launches = 1;
 	if (blocks > 1 && a.taps > 1) {
 		XALM_CUDA_CHECK(cudaMemcpyAsync(a.hist, a.stage, (size_t) (a.taps - 1) * a.C * 4, cudaMemcpyDeviceToDevice, s));
+		pdl_block(s);
 		if (launches) *launches = 2;
 	}
 	return XALM_OK;

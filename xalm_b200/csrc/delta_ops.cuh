@@ -44,6 +44,7 @@ struct DeltaArgs {
 // grid (tokens, 2 G + H): a CTA convolves one head — a q head, a k head (both scaled to unit length afterwards) or a v head; the CTA of
 // the first head also computes the token's write strengths and decays
 static __global__ void delta_prep_kernel(DeltaArgs a) {
+	pdl_enter();
 	__shared__ float red[33];
 	const int t = blockIdx.x, unit = blockIdx.y, tid = threadIdx.x, nth = blockDim.x;
 	if (t >= a.step->n) return;
@@ -108,6 +109,7 @@ __device__ __forceinline__ void delta_cp4(float* dst, const float* src) {
 
 template <int DS, int NS>
 __global__ void __launch_bounds__(512) delta_rule_kernel(DeltaArgs a) {
+	pdl_enter();
 	extern __shared__ __align__(16) float sm[];
 	const int h = blockIdx.x, tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
 	const int d = a.d, dv = a.dv, dp = DS > 0 ? DS * NS : ((d + 3) & ~3), hk = h / (a.H / a.G);
@@ -287,11 +289,11 @@ static inline int delta_prepare(int d, int dv) { // outside a stream capture
 // rows: tokens of the step (host-side bound); two launches
 static inline int launch_delta(const DeltaArgs& a, int rows, cudaStream_t s) {
 	if (a.H % a.G || a.taps < 1 || !delta_ok(a.d, a.dv)) return set_error(XALM_ERR_UNSUPPORTED, "delta rule: heads %d / %d, state %d x %d", a.H, a.G, a.d, a.dv);
-	delta_prep_kernel<<<dim3(rows, 2 * a.G + a.H), 128, 0, s>>>(a);
+	launch_step(delta_prep_kernel, dim3(rows, 2 * a.G + a.H), 128, 0, s, rows, a);
 	XALM_TRY(launch_check("delta_prep"));
 	const DeltaShape z = delta_shape(a.d, a.dv);
 	const size_t smem = delta_rule_smem(a.d, a.dv);
-#define XALM_DELTA_LAUNCH(DS_, NS_) delta_rule_kernel<DS_, NS_><<<a.H, z.threads, smem, s>>>(a)
+#define XALM_DELTA_LAUNCH(DS_, NS_) launch_step(delta_rule_kernel<DS_, NS_>, a.H, z.threads, smem, s, rows, a)
 	XALM_DELTA_DISPATCH(z, XALM_DELTA_LAUNCH);
 #undef XALM_DELTA_LAUNCH
 	return launch_check("delta_rule");

@@ -224,7 +224,7 @@ int enqueue_retention(Du* m, const Layer& L, int n, int* nl) {
 	ha.decay = L.decay; ha.k_scale = 1.f / sqrtf((float) d);
 	ha.norm_plain = 1; ha.eps = m->eps;
 	ha.gate = m->proj; ha.ldg = m->proj_ld; ha.g_off = L.off_g;
-	ha.state = L.state; ha.step = m->d_step; ha.out = m->att; ha.max_rows = m->chunk;
+	ha.state = L.state; ha.step = m->d_step; ha.out = m->att; ha.max_rows = m->chunk; ha.rows = n;
 	XALM_TRY(launch_hgrn2(ha, s));
 	(*nl)++;
 	return XALM_OK;
@@ -275,7 +275,10 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 			XALM_TRY(rows_product(m, m->hn, W, L.w_up, &L.t_up, n, L.ff, W, ea, nl));
 			XALM_TRY(rows_product(m, m->ffh, L.ff, L.w_down, &L.t_down, n, W, L.ff, residual_epi(m), nl));
 		} else if (L.ff_kind == FF_MOE) XALM_TRY(enqueue_experts(m, L, n, nl));
-		if (m->keep_layers) XALM_CUDA_CHECK(cudaMemcpyAsync(m->layer_sums + li * hs, m->x, (size_t) n * W * 4, cudaMemcpyDeviceToDevice, s));
+		if (m->keep_layers) {
+			XALM_CUDA_CHECK(cudaMemcpyAsync(m->layer_sums + li * hs, m->x, (size_t) n * W * 4, cudaMemcpyDeviceToDevice, s));
+			pdl_block(s);
+		}
 	}
 	if (want) {
 		const int rows = want == 2 ? n : 1, first = want == 2 ? 0 : n - 1;

@@ -287,7 +287,7 @@ int enqueue_gla(Kb* m, const Layer& L, const Run& R, int n, const Fork& fk, int*
 	ha.keyed = 1; ha.qk_rep = 1; ha.q_scale = 1.f / sqrtf((float) d);
 	ha.norm_w = L.head_norm; ha.eps = m->eps;
 	ha.gate = m->proj; ha.ldg = m->proj_ld; ha.g_off = L.off_g;
-	ha.state = R.state; ha.step = m->d_step; ha.out = m->att; ha.max_rows = m->chunk;
+	ha.state = R.state; ha.step = m->d_step; ha.out = m->att; ha.max_rows = m->chunk; ha.rows = n;
 	XALM_TRY(fk.open());
 	XALM_TRY(launch_hgrn2(ha, fk.side()));
 	(*nl)++;
@@ -319,7 +319,7 @@ int enqueue_parallel(Kb* m, const Layer& L, const Run& R, int n, const Fork& fk,
 	ha.H = L.sH; ha.d = L.sN; ha.dv = L.sP;
 	ha.keyed = 2; ha.qk_rep = L.sH / L.sG; ha.dt_off = L.off_dt; ha.dt_bias = L.dt_bias; ha.A_log = L.A_log; ha.skip = L.D;
 	ha.eps = m->eps;
-	ha.state = R.state; ha.step = m->d_step; ha.out = m->yssd; ha.max_rows = m->chunk;
+	ha.state = R.state; ha.step = m->d_step; ha.out = m->yssd; ha.max_rows = m->chunk; ha.rows = n;
 	XALM_TRY(launch_hgrn2(ha, side));
 	(*nl)++;
 	GroupNormArgs g;
@@ -406,7 +406,10 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 		} else if (L.ff_kind == FF_MOE) XALM_TRY(enqueue_experts(m, L, n, nl));
 		XALM_TRY(fk.join());
 		XALM_TRY(rows_product(m, m->att, L.k_o, L.w_o, &L.t_o, n, W, L.k_o, residual_epi(m), nl));
-		if (m->keep_layers) XALM_CUDA_CHECK(cudaMemcpyAsync(m->layer_sums + ri * hs, m->x, (size_t) n * W * 4, cudaMemcpyDeviceToDevice, s));
+		if (m->keep_layers) {
+			XALM_CUDA_CHECK(cudaMemcpyAsync(m->layer_sums + ri * hs, m->x, (size_t) n * W * 4, cudaMemcpyDeviceToDevice, s));
+			pdl_block(s);
+		}
 	}
 	if (want) {
 		const int rows = want == 2 ? n : 1, first = want == 2 ? 0 : n - 1;

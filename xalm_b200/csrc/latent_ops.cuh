@@ -39,6 +39,7 @@ struct LatentPostArgs {
 
 // one CTA per token; shared memory: 33 floats
 static __global__ void latent_post_kernel(LatentPostArgs a) {
+	pdl_enter();
 	__shared__ float red[33];
 	const int t = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
 	if (t >= a.step->n) return;
@@ -78,7 +79,7 @@ static __global__ void latent_post_kernel(LatentPostArgs a) {
 static inline int launch_latent_post(const LatentPostArgs& a, int rows, cudaStream_t s) {
 	if (a.rot % 2 || (a.rot && !a.freq)) return set_error(XALM_ERR_INVALID, "latent_post: %d rotated columns", a.rot);
 	const int widest = std::max(a.q_rank, a.kv_rank);
-	latent_post_kernel<<<rows, widest >= 512 ? 256 : widest >= 128 ? 128 : 64, 0, s>>>(a);
+	launch_step(latent_post_kernel, rows, widest >= 512 ? 256 : widest >= 128 ? 128 : 64, 0, s, rows, a);
 	return launch_check("latent_post");
 }
 
@@ -93,6 +94,7 @@ struct RopeHeadsArgs {
 };
 // grid (tokens, ceil(heads / 8)), 256 threads: a warp per head
 static __global__ void rope_heads_kernel(RopeHeadsArgs a) {
+	pdl_enter();
 	const int t = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	if (t >= a.step->n || h >= a.heads) return;
 	const float pos = (float) (a.step->pos0 + t);
@@ -111,7 +113,7 @@ static __global__ void rope_heads_kernel(RopeHeadsArgs a) {
 }
 static inline int launch_rope_heads(const RopeHeadsArgs& a, int rows, cudaStream_t s) {
 	if (a.rot_half < 0 || 2 * a.rot_half > a.n || (a.rot_half && !a.freq)) return set_error(XALM_ERR_INVALID, "rope_heads: %d pairs in a head of %d", a.rot_half, a.n);
-	rope_heads_kernel<<<dim3(rows, (a.heads + 7) / 8), 256, 0, s>>>(a);
+	launch_step(rope_heads_kernel, dim3(rows, (a.heads + 7) / 8), 256, 0, s, rows, a);
 	return launch_check("rope_heads");
 }
 

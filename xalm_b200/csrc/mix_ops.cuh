@@ -88,6 +88,7 @@ struct SeqStep {
 template <typename WT>
 __global__ void embed_streams_kernel(const WT* __restrict__ table, const int* __restrict__ tokens, int width, int S, size_t stream_stride,
                                      float* __restrict__ xs, float scale = 1.f, const WT* __restrict__ positions = nullptr, const SeqStep* step = nullptr) {
+	pdl_enter();
 	const int t = blockIdx.x;
 	const WT* row = table + (size_t) tokens[t] * width;
 	const WT* prow = positions ? positions + (size_t) (step->pos0 + t) * width : nullptr;
@@ -117,6 +118,7 @@ struct EmbedPairArgs {
 };
 template <typename WT>
 __global__ void embed_pair_kernel(EmbedPairArgs a) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	float* u = sm;
 	float* rinv = sm + a.width;
@@ -157,6 +159,7 @@ __global__ void embed_pair_kernel(EmbedPairArgs a) {
 template <int SS>
 __global__ void hc_norm_kernel(const float* __restrict__ xs, int S, size_t stream_stride, const float* __restrict__ a, const float* __restrict__ w,
                                int one_plus, float eps, int width, float* __restrict__ h, float* __restrict__ sum_out) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	float* u = sm;            // width
 	float* red = sm + width;  // 33
@@ -214,6 +217,7 @@ __global__ void hc_norm_kernel(const float* __restrict__ xs, int S, size_t strea
 // between the two sums, so the deviations are taken from the finished mean.  Loads four columns per thread ahead, as hc_norm_kernel.
 static __global__ void layer_norm_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, const float* __restrict__ b, float eps, int width,
                                          float* __restrict__ h) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	float* u = sm;            // width
 	float* red = sm + width;  // 33
@@ -502,6 +506,100 @@ __global__ void __launch_bounds__(256) rows_matvec_kernel(const float* __restric
 	}
 }
 
+// ---- the same for one token and bf16 weights: a warp (or KS warps, each a slice of K) per FOUR output columns ------------------------------------
+// Bound: memory.  Four columns share each read of the activations, two 256-channel pieces of all four (256 bytes per lane) are in flight, and the first
+// two pieces are requested before the kernel waits for its predecessor.  Measured back to back in a graph, buffers beyond L2, two columns per warp
+// without the early request before: 28672 x 4096 47.9 -> 40.1 us (5.9 TB/s), 4096 x 14336 24.6 -> 18.5, 6144 x 4096 13.1 -> 10.2, 4096 x 4096
+// 9.0 -> 6.9, 32000 x 1024 17.0 -> 13.0, 2048 x 2048 3.8 -> 3.2.  Deeper pieces, eight columns or a persistent grid were slower.
+constexpr int RS_COLS = 4, RS_DEPTH = 2;
+__device__ __forceinline__ uint4 ld_stream16(const void* p) { // weights: read once
+	uint4 r;
+	asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+	return r;
+}
+__device__ __forceinline__ float dot8_bf16(float acc, const uint4& r, const float4& x0, const float4& x1) {
+	acc = fmaf(__uint_as_float(r.x << 16), x0.x, acc);
+	acc = fmaf(__uint_as_float(r.x & 0xffff0000u), x0.y, acc);
+	acc = fmaf(__uint_as_float(r.y << 16), x0.z, acc);
+	acc = fmaf(__uint_as_float(r.y & 0xffff0000u), x0.w, acc);
+	acc = fmaf(__uint_as_float(r.z << 16), x1.x, acc);
+	acc = fmaf(__uint_as_float(r.z & 0xffff0000u), x1.y, acc);
+	acc = fmaf(__uint_as_float(r.w << 16), x1.z, acc);
+	return fmaf(__uint_as_float(r.w & 0xffff0000u), x1.w, acc);
+}
+// columns c0 .. c0 + 3 of W (N, K) times A over the warp's slice of K: every lane gets the four sums.  ready() is called once the first weights are requested.
+template <int KS, typename Ready>
+__device__ __forceinline__ void rows_stream_dot(const __nv_bfloat16* W, const float* A, int c0, int N, int K, int ks, int lane, float (&acc)[RS_COLS], Ready ready) {
+	const __nv_bfloat16* w[RS_COLS];
+#pragma unroll
+	for (int c = 0; c < RS_COLS; c++) w[c] = W + (size_t) min(c0 + c, N - 1) * K;
+	constexpr int STEP = 256 * KS;
+	const int k0 = (ks * 32 + lane) * 8;
+	uint4 r[RS_DEPTH][RS_COLS];
+#pragma unroll
+	for (int i = 0; i < RS_DEPTH; i++)
+		if (k0 + i * STEP < K)
+#pragma unroll
+			for (int c = 0; c < RS_COLS; c++) r[i][c] = ld_stream16(w[c] + k0 + i * STEP);
+	ready();
+	for (int kb = k0; kb < K; kb += RS_DEPTH * STEP)
+#pragma unroll
+		for (int i = 0; i < RS_DEPTH; i++) {
+			const int k = kb + i * STEP;
+			if (k < K) {
+				const float4 x0 = *reinterpret_cast<const float4*>(A + k), x1 = *reinterpret_cast<const float4*>(A + k + 4);
+#pragma unroll
+				for (int c = 0; c < RS_COLS; c++) acc[c] = dot8_bf16(acc[c], r[i][c], x0, x1);
+				if (k + RS_DEPTH * STEP < K)
+#pragma unroll
+					for (int c = 0; c < RS_COLS; c++) r[i][c] = ld_stream16(w[c] + k + RS_DEPTH * STEP);
+			}
+		}
+#pragma unroll
+	for (int c = 0; c < RS_COLS; c++) acc[c] = warp_sum(acc[c]);
+}
+// the slices of K joined (red: 8 x RS_COLS floats of shared memory) and the epilogue of row `row`, a lane per column (per pair of them for the GLU).
+// Every thread of the CTA calls it.
+template <int KS>
+__device__ __forceinline__ void rows_stream_finish(const RowsEpi& e, int row, int c0, int N, int warp, int lane, int ks, const float (&acc)[RS_COLS], float (*red)[RS_COLS]) {
+	float v = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
+	if (KS > 1) {
+		if (lane < RS_COLS) red[warp][lane] = v;
+		__syncthreads();
+		if (ks == 0 && lane < RS_COLS)
+#pragma unroll
+			for (int j = 1; j < KS; j++) v += red[warp + j][lane];
+	}
+	if (ks) return;
+	const float next = __shfl_down_sync(0xffffffffu, v, 1);
+	if (lane >= RS_COLS || c0 + lane >= N) return;
+	if (e.kind == EPI_GLU) {
+		if (!(lane & 1) && c0 + lane + 1 < N) epi_apply(e, row, c0 + lane, N, v, next);
+	} else epi_apply(e, row, c0 + lane, N, v, 0.f);
+}
+// warps per four columns: enough CTAs for two per SM, each slice of K at least 256 long
+static inline int rows_stream_ks(int N, int K, int batch) {
+	const long long sets = (N + RS_COLS - 1) / RS_COLS;
+	int ks = 1;
+	while (ks < 8 && (sets * ks + 7) / 8 * batch < 296 && K >= 512 * ks) ks *= 2;
+	return ks;
+}
+template <int KS>
+__global__ void __launch_bounds__(256) rows_stream_kernel(const float* __restrict__ A, const __nv_bfloat16* __restrict__ W, int N, int K, RowsEpi e) {
+	__shared__ float red[8][RS_COLS];
+	if (blockIdx.z) { // one product of a batch
+		A += (size_t) blockIdx.z * e.batch_a;
+		W += (size_t) blockIdx.z * e.batch_w;
+		e.out += (size_t) blockIdx.z * e.batch_o;
+		if (e.mul) e.mul += (size_t) blockIdx.z * e.batch_o;
+	}
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ks = warp % KS, c0 = (blockIdx.x * (8 / KS) + warp / KS) * RS_COLS;
+	float acc[RS_COLS] = {};
+	if (c0 < N) rows_stream_dot<KS>(W, A, c0, N, K, ks, lane, acc, [] { pdl_enter(); });
+	else pdl_enter();
+	rows_stream_finish<KS>(e, 0, c0, N, warp, lane, ks, acc, red);
+}
+
 // ---- sliding-window softmax attention with score mixing across heads -------------------------------------------------------------
 struct SwaArgs {
 	const float* q;    // (T, ldq): head h at columns q_off + h * d
@@ -625,6 +723,7 @@ __device__ __forceinline__ void swa_merge_rows(const SwaArgs& a, int t_first, in
 }
 // grid (rows, ceil(H dv / 128)), 128 threads: a thread per output value, so that a one-token step's join is spread over many SMs
 static __global__ void swa_merge_kernel(SwaArgs a) {
+	pdl_enter();
 	const int hc = blockIdx.y * blockDim.x + threadIdx.x;
 	if (hc < a.H * a.dv) swa_merge_one(a, blockIdx.x, hc);
 }
@@ -1141,6 +1240,7 @@ __global__ void __launch_bounds__(256) swa_tile_kernel(SwaArgs a) {
 
 // ---- gated linear recurrence (HGRN2) --------------------------------------------------------------------------------------------
 struct Hgrn2Args {
+	int rows; // tokens of this launch where the host knows them, else 0
 	const float* proj; // (T, ld): per head h, q at q_off + h * d, forget pre-activation at f_off + h * d, v at v_off + h * dv
 	int ld, q_off, f_off, v_off;
 	int H, d, dv;
@@ -1289,6 +1389,7 @@ __device__ __forceinline__ float warp_sum_transposed32(float (&v)[32], int lane)
 
 template <int DPL, int KEYED>
 __global__ void hgrn2_cols_kernel(Hgrn2Args a) {
+	pdl_enter();
 	namespace cg = cooperative_groups;
 	cg::cluster_group cluster = cg::this_cluster();
 	extern __shared__ float sm[];
@@ -1458,6 +1559,7 @@ struct NextRead {
 template <int SS>
 __global__ void dual_norm_hc_kernel(const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ wa, const float* __restrict__ wb,
                                     float eps, int width, RowsEpi e, NextRead next) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	__shared__ float hm[MAX_STREAMS * MAX_STREAMS], ho[MAX_STREAMS], an[MAX_STREAMS];
 	float* red = sm;      // 33
@@ -1557,7 +1659,15 @@ static inline int norm_threads(int width) { return width >= 1024 ? 256 : width >
 // out(T,N) = A(T,K) . W(N,K)^T with epilogue e, IEEE fp32 arithmetic; W is bf16 or fp32
 // batch > 1: that many products in one launch, operands and output advancing by e.batch_a / batch_w / batch_o per product
 static inline int launch_rows(const float* A, int lda, const void* W, bool w_bf16, int T, int N, int K, const RowsEpi& e, cudaStream_t s, int batch = 1) {
-	if (T <= 4) {
+	if (T == 1 && w_bf16 && K % 8 == 0 && (e.batch_a % 4 == 0 && e.batch_w % 8 == 0) && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A)) & 15) == 0) {
+		const int ks = rows_stream_ks(N, K, batch), sets = (N + RS_COLS - 1) / RS_COLS;
+		const dim3 grid((sets * ks + 7) / 8, 1, batch);
+		const __nv_bfloat16* w = (const __nv_bfloat16*) W;
+		if (ks == 1) launch_step(rows_stream_kernel<1>, grid, 256, 0, s, T, A, w, N, K, e);
+		else if (ks == 2) launch_step(rows_stream_kernel<2>, grid, 256, 0, s, T, A, w, N, K, e);
+		else if (ks == 4) launch_step(rows_stream_kernel<4>, grid, 256, 0, s, T, A, w, N, K, e);
+		else launch_step(rows_stream_kernel<8>, grid, 256, 0, s, T, A, w, N, K, e);
+	} else if (T <= 4) {
 		const int pairs = (N + 1) / 2;
 		int ks = 1; // warps per column pair: enough CTAs for two per SM, each slice of K at least 256 long
 		while (ks < 8 && (pairs * ks + 7) / 8 * batch < 296 && K >= 512 * ks) ks *= 2;
@@ -1570,8 +1680,7 @@ static inline int launch_rows(const float* A, int lda, const void* W, bool w_bf1
 		else rows_matvec_kernel<WT_, TB_, 8><<<grid, 256, 0, s>>>(A, lda, (const WT_*) W, T, N, K, e);                               \
 	} while (0)
 		if (w_bf16) {
-			if (T == 1) XALM_ROWS_MATVEC(__nv_bfloat16, 1);
-			else XALM_ROWS_MATVEC(__nv_bfloat16, 4);
+			XALM_ROWS_MATVEC(__nv_bfloat16, 4);
 		} else {
 			if (T == 1) XALM_ROWS_MATVEC(float, 1);
 			else XALM_ROWS_MATVEC(float, 4);
@@ -1648,6 +1757,7 @@ struct GroupNormArgs {
 	int ld_out = 0;                // elements between rows of x_out (0: width): the result may be a run of columns of a wider buffer
 };
 static __global__ void group_norm_residual_kernel(GroupNormArgs a) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	float* u = sm;               // width
 	float* rinv = sm + a.width;  // groups
@@ -1733,7 +1843,7 @@ static inline int group_norm_prepare(int width, int groups) {
 }
 static inline int launch_group_norm(const GroupNormArgs& a, int rows, cudaStream_t s) {
 	if (a.groups <= 0 || a.width % a.groups) return set_error(XALM_ERR_INVALID, "group norm: %d groups do not divide a row of %d", a.groups, a.width);
-	group_norm_residual_kernel<<<rows, norm_threads(a.width), group_norm_smem(a.width, a.groups), s>>>(a);
+	launch_step(group_norm_residual_kernel, rows, norm_threads(a.width), group_norm_smem(a.width, a.groups), s, rows, a);
 	return launch_check("group_norm_residual");
 }
 
@@ -1766,6 +1876,7 @@ struct QkvPostArgs {
 	const SeqStep* step;
 };
 static __global__ void qkv_post_kernel(QkvPostArgs a) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 	const int unit = blockIdx.y * nw + warp;
@@ -1821,6 +1932,7 @@ static __global__ void qkv_post_kernel(QkvPostArgs a) {
 // grid (rows, parts), 256 threads; shared memory: 2 * rot_half + 33 floats.  Every CTA sums the squares of whole rows (of the rows its share needs) and
 // finishes its share of the (entry, entry) pairs, so that a one-token step spreads over several CTAs; that needs q_out apart from proj.
 static __global__ void qkv_rows_post_kernel(QkvPostArgs a) {
+	pdl_enter();
 	extern __shared__ float sm[];
 	float *cs = sm, *sn = sm + a.rot_half, *red = sn + a.rot_half;
 	const int t = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
@@ -1898,12 +2010,12 @@ static inline int launch_qkv_post(const QkvPostArgs& a, int rows, cudaStream_t s
 		if (a.rot_half < 0 || 2 * a.rot_half > a.d || (size_t) a.rot_half * 8 > 40 * 1024) return set_error(XALM_ERR_INVALID, "qkv_post: %d pairs in a head of %d", a.rot_half, a.d);
 		const int units = (a.H + a.G) * ((a.d + 1) / 2) + a.G * a.dv;
 		const int parts = a.q_out && rows < 64 ? std::max(1, std::min(8, units / 512)) : 1; // short steps: several CTAs per token
-		qkv_rows_post_kernel<<<dim3(rows, parts), 256, ((size_t) 2 * a.rot_half + 33) * 4, s>>>(a);
+		launch_step(qkv_rows_post_kernel, dim3(rows, parts), 256, ((size_t) 2 * a.rot_half + 33) * 4, s, rows, a);
 		return launch_check("qkv_rows_post");
 	}
 	const int units = a.H + 2 * a.G, nw = units < 8 ? units : 8, wmax = a.d > a.dv ? a.d : a.dv;
 	if ((size_t) nw * wmax * 4 > 48 * 1024) return set_error(XALM_ERR_UNSUPPORTED, "qkv_post: heads of %d do not fit shared memory", wmax);
-	qkv_post_kernel<<<dim3(rows, (units + nw - 1) / nw), nw * 32, (size_t) nw * wmax * 4, s>>>(a);
+	launch_step(qkv_post_kernel, dim3(rows, (units + nw - 1) / nw), nw * 32, (size_t) nw * wmax * 4, s, rows, a);
 	return launch_check("qkv_post");
 }
 
@@ -1912,8 +2024,8 @@ static inline int launch_embed_pair(const EmbedPairArgs& a, bool w_bf16, int row
 	if (a.pair && a.buckets <= 0) return set_error(XALM_ERR_INVALID, "pair embedding: %d buckets", a.buckets);
 	const size_t smem = (size_t) (a.width + std::max(a.groups, 1)) * 4;
 	if (smem > 48 * 1024) return set_error(XALM_ERR_UNSUPPORTED, "embedding: a row of %d does not fit shared memory", a.width);
-	if (w_bf16) embed_pair_kernel<__nv_bfloat16><<<rows, norm_threads(a.width), smem, s>>>(a);
-	else embed_pair_kernel<float><<<rows, norm_threads(a.width), smem, s>>>(a);
+	if (w_bf16) launch_step(embed_pair_kernel<__nv_bfloat16>, rows, norm_threads(a.width), smem, s, rows, a);
+	else launch_step(embed_pair_kernel<float>, rows, norm_threads(a.width), smem, s, rows, a);
 	return launch_check("embed_pair");
 }
 
@@ -1928,10 +2040,10 @@ static inline int launch_hc_norm(const float* xs, int S, size_t stream_stride, c
 	const size_t smem = (size_t) (width + 33) * 4;
 	XALM_TRY(hc_norm_prepare(width));
 	const int nt = norm_threads(width);
-	if (S <= 1) hc_norm_kernel<1><<<rows, nt, smem, s>>>(xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
-	else if (S <= 2) hc_norm_kernel<2><<<rows, nt, smem, s>>>(xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
-	else if (S <= 4) hc_norm_kernel<4><<<rows, nt, smem, s>>>(xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
-	else hc_norm_kernel<MAX_STREAMS><<<rows, nt, smem, s>>>(xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
+	if (S <= 1) launch_step(hc_norm_kernel<1>, rows, nt, smem, s, rows, xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
+	else if (S <= 2) launch_step(hc_norm_kernel<2>, rows, nt, smem, s, rows, xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
+	else if (S <= 4) launch_step(hc_norm_kernel<4>, rows, nt, smem, s, rows, xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
+	else launch_step(hc_norm_kernel<MAX_STREAMS>, rows, nt, smem, s, rows, xs, S, stream_stride, a, w, one_plus, eps, width, h, sum_out);
 	return launch_check("hc_norm");
 }
 
@@ -1944,7 +2056,7 @@ static inline int layer_norm_prepare(int width) {
 	return XALM_OK;
 }
 static inline int launch_layer_norm(const float* x, int ldx, const float* w, const float* b, float eps, int width, float* h, int rows, cudaStream_t s) {
-	layer_norm_kernel<<<rows, norm_threads(width), (size_t) (width + 33) * 4, s>>>(x, ldx, w, b, eps, width, h);
+	launch_step(layer_norm_kernel, rows, norm_threads(width), (size_t) (width + 33) * 4, s, rows, x, ldx, w, b, eps, width, h);
 	return launch_check("layer_norm");
 }
 
@@ -1955,10 +2067,10 @@ static inline int launch_dual_norm_hc(const float* A, const float* B, const floa
 	const int nt = norm_threads(width);
 	if (next.h && !dual_norm_can_carry(width)) return set_error(XALM_ERR_UNSUPPORTED, "dual_norm_hc: a row of %d does not fit shared memory", width);
 	const size_t smem = (size_t) (33 + (next.h ? width : 0)) * 4;
-	if (e.S <= 1) dual_norm_hc_kernel<1><<<rows, nt, smem, s>>>(A, B, wa, wb, eps, width, e, next);
-	else if (e.S <= 2) dual_norm_hc_kernel<2><<<rows, nt, smem, s>>>(A, B, wa, wb, eps, width, e, next);
-	else if (e.S <= 4) dual_norm_hc_kernel<4><<<rows, nt, smem, s>>>(A, B, wa, wb, eps, width, e, next);
-	else dual_norm_hc_kernel<MAX_STREAMS><<<rows, nt, smem, s>>>(A, B, wa, wb, eps, width, e, next);
+	if (e.S <= 1) launch_step(dual_norm_hc_kernel<1>, rows, nt, smem, s, rows, A, B, wa, wb, eps, width, e, next);
+	else if (e.S <= 2) launch_step(dual_norm_hc_kernel<2>, rows, nt, smem, s, rows, A, B, wa, wb, eps, width, e, next);
+	else if (e.S <= 4) launch_step(dual_norm_hc_kernel<4>, rows, nt, smem, s, rows, A, B, wa, wb, eps, width, e, next);
+	else launch_step(dual_norm_hc_kernel<MAX_STREAMS>, rows, nt, smem, s, rows, A, B, wa, wb, eps, width, e, next);
 	return launch_check("dual_norm_hc");
 }
 
@@ -2026,7 +2138,7 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 		if (launches) *launches = a.n_splits > 1 ? 2 : 1;
 		XALM_TRY(launch_swa_one(a, rows, cache_f32, s));
 		if (a.n_splits > 1) {
-			swa_merge_kernel<<<dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s>>>(a);
+			launch_step(swa_merge_kernel, dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s, rows, a);
 			XALM_TRY(launch_check("swa_merge"));
 		}
 		return XALM_OK;
@@ -2068,7 +2180,7 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 	}
 	XALM_TRY(launch_check("swa_attn"));
 	if (a.n_splits > 1 && !a.tickets) {
-		swa_merge_kernel<<<dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s>>>(a);
+		launch_step(swa_merge_kernel, dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s, rows, a);
 		XALM_TRY(launch_check("swa_merge"));
 	}
 	return XALM_OK;
@@ -2085,11 +2197,13 @@ static inline int launch_hgrn2_cols(const Hgrn2Args& a, int warps, int nb, cudaS
 	cfg.blockDim = dim3(warps * 32);
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = s;
-	cudaLaunchAttribute at[1];
+	cudaLaunchAttribute at[2];
 	at[0].id = cudaLaunchAttributeClusterDimension;
 	at[0].val.clusterDim.x = nb; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at;
-	cfg.numAttrs = 1;
+	cfg.numAttrs = a.rows == 1 && pdl_next(s) ? 2 : 1;
 	const cudaError_t e = cudaLaunchKernelEx(&cfg, hgrn2_cols_kernel<DPL, KEYED>, a);
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "hgrn2 launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;

@@ -221,13 +221,14 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 		ha.proj = m->proj; ha.ld = (int) m->proj_ld; ha.q_off = L.off_rq; ha.f_off = L.off_rf; ha.v_off = L.off_rv;
 		ha.H = Hr; ha.d = dr; ha.dv = dvr;
 		ha.f_bias = L.fb; ha.lower = L.lower; ha.norm_w = L.rnorm; ha.eps = m->eps;
-		ha.state = L.state; ha.step = m->d_step; ha.out = m->ro; ha.max_rows = m->chunk; ha.activated = 1;
+		ha.state = L.state; ha.step = m->d_step; ha.out = m->ro; ha.max_rows = m->chunk; ha.rows = n; ha.activated = 1;
 		// the two mixers read the same projections and write different buffers: the recurrence runs on the side stream (a branch
 		// of the graph, when the step is captured) while the attention and its output projection run here
 		const bool overlap = tune("seq_overlap") != 0;
 		if (overlap) {
 			XALM_CUDA_CHECK(cudaEventRecord(m->ev_fork, s));
 			XALM_CUDA_CHECK(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
+			pdl_block(m->side);
 		}
 		XALM_TRY(launch_hgrn2(ha, overlap ? m->side : s));
 		(*nl)++;
@@ -238,7 +239,10 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 		RowsEpi est;
 		est.kind = EPI_STORE; est.out = m->ol; est.ldo = W;
 		XALM_TRY(rows_product(m, m->att, H * dv, L.w_lo, &L.t_lo, n, W, H * dv, est, nl));
-		if (overlap) XALM_CUDA_CHECK(cudaStreamWaitEvent(s, m->ev_join, 0));
+		if (overlap) {
+			XALM_CUDA_CHECK(cudaStreamWaitEvent(s, m->ev_join, 0));
+			pdl_block(s);
+		}
 		est.out = m->orr;
 		XALM_TRY(rows_product(m, m->ro, Hr * dvr, L.w_ro, &L.t_ro, n, W, Hr * dvr, est, nl));
 		NextRead nx; // the feed-forward's read of the streams rides along with the mixer's write when the row fits

@@ -255,7 +255,10 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 			XALM_TRY(launch_moe_combine(ca, n, s));
 			*nl += 2;
 		}
-		if (m->keep_layers) XALM_CUDA_CHECK(cudaMemcpyAsync(m->layer_sums + ri * hs, x, (size_t) n * W * 4, cudaMemcpyDeviceToDevice, s));
+		if (m->keep_layers) {
+			XALM_CUDA_CHECK(cudaMemcpyAsync(m->layer_sums + ri * hs, x, (size_t) n * W * 4, cudaMemcpyDeviceToDevice, s));
+			pdl_block(s);
+		}
 	}
 	if (want) {
 		const int rows = want == 2 ? n : 1, first = want == 2 ? 0 : n - 1;

@@ -281,6 +281,7 @@ struct Fork {
 		if (!on) return XALM_OK;
 		XALM_CUDA_CHECK(cudaEventRecord(m->ev_fork, m->stream));
 		XALM_CUDA_CHECK(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
+		pdl_block(m->side);
 		return XALM_OK;
 	}
 	int mark() const { // the side branch ends here
@@ -288,7 +289,10 @@ struct Fork {
 		return XALM_OK;
 	}
 	int join() const {
-		if (on) XALM_CUDA_CHECK(cudaStreamWaitEvent(m->stream, m->ev_join, 0));
+		if (on) {
+			XALM_CUDA_CHECK(cudaStreamWaitEvent(m->stream, m->ev_join, 0));
+			pdl_block(m->stream);
+		}
 		return XALM_OK;
 	}
 };
@@ -305,6 +309,7 @@ int ensure_graph(SeqModel* m, int mode) {
 	if (m->graph[mode]) return XALM_OK;
 	cudaGraph_t g = nullptr;
 	XALM_CUDA_CHECK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
+	pdl_block(m->stream);
 	int nl = 0;
 	const int rc = m->hooks->enqueue_pass(m, 1, mode ? 1 : 0, &nl);
 	cudaError_t e = cudaStreamEndCapture(m->stream, &g);
@@ -327,6 +332,7 @@ int run_pass(SeqModel* m, const int* tokens, int n, int want) {
 	const SeqStep st = {m->pos, n, m->prev_token};
 	XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_tokens, tokens, (size_t) n * 4, cudaMemcpyHostToDevice, m->stream));
 	XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_step, &st, sizeof st, cudaMemcpyHostToDevice, m->stream));
+	pdl_block(m->stream); // the pass's first kernel follows the copies
 	int nl = 0;
 	if (n == 1 && tune("seq_graph")) {
 		const int mode = want ? 1 : 0;

@@ -54,6 +54,7 @@ __host__ __device__ constexpr size_t swo_smem_floats(int lpk, int nch, int hb) {
 
 template <typename CT, int LPK, int NCH, int HB>
 __global__ void __launch_bounds__(swo_threads(NCH)) swa_one_kernel(SwaArgs a) {
+	pdl_enter();
 	namespace cg = cooperative_groups;
 	constexpr int DP = LPK * 8 * NCH, NTH = swo_threads(NCH), UNITS = NTH / LPK, KB = sizeof(CT) == 2 ? (NCH <= 2 ? 4 : 2) : (NCH == 1 ? 2 : 1), NV = KB * HB;
 	extern __shared__ __align__(16) float sm[];
@@ -277,11 +278,13 @@ static int launch_swa_one_inst(const SwaArgs& a, int rows, cudaStream_t s) {
 	cfg.blockDim = dim3(swo_threads(NCH));
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = s;
-	cudaLaunchAttribute at[1];
+	cudaLaunchAttribute at[2];
 	at[0].id = cudaLaunchAttributeClusterDimension;
 	at[0].val.clusterDim.x = SWO_CTAS; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at;
-	cfg.numAttrs = 1;
+	cfg.numAttrs = rows == 1 && pdl_next(s) ? 2 : 1;
 	const cudaError_t e = cudaLaunchKernelEx(&cfg, swa_one_kernel<CT, LPK, NCH, HB>, a);
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "swa_one launch failed: %s", cudaGetErrorString(e));
 	return launch_check("swa_one");
