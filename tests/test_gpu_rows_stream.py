@@ -1,4 +1,4 @@
-"""Products of one token with bf16 weights (four columns per warp, slices of K over warps): columns that do not fill a warp's four, lengths around a lane's
+"""Products of one token, and of five to thirty-one, with bf16 weights (four columns per warp, slices of K over warps): columns that do not fill a warp's four, lengths around a lane's
 pieces and around the slices, every epilogue that pairs columns, the chosen experts' products."""
 import numpy as np
 import pytest
@@ -19,11 +19,12 @@ def bound(K):
 
 @pytest.mark.parametrize("N", [1, 2, 3, 4, 7, 33, 2500])
 @pytest.mark.parametrize("K", [8, 248, 256, 264, 512, 1000, 2048, 4104])
-def test_plain_and_paired_columns(N, K):
+@pytest.mark.parametrize("T", [1, 5, 8, 9, 16, 17, 31])
+def test_plain_and_paired_columns(N, K, T):
     rng = np.random.default_rng(N * K)
-    x, w, u = rng.standard_normal((1, K)).astype(np.float32), bf16(rng.standard_normal((N, K)) / K ** 0.5), bf16(rng.standard_normal((N, K)) / K ** 0.5)
+    x, w, u = rng.standard_normal((T, K)).astype(np.float32), bf16(rng.standard_normal((N, K)) / K ** 0.5), bf16(rng.standard_normal((N, K)) / K ** 0.5)
     z, y = x.astype(np.float64) @ w.T, x.astype(np.float64) @ u.T
-    mul = rng.standard_normal((1, N)).astype(np.float32)
+    mul = rng.standard_normal((T, N)).astype(np.float32)
     got = capi.rows_act(x, w, act=0, cap=20.0, mul=mul, w_bf16=True)
     assert np.abs(got - 20 * np.tanh(z / 20) / (1 + np.exp(-mul))).max() < bound(K)
     got = capi.glu_rows(x, w, u, 7.0, w_bf16=True)
@@ -31,7 +32,7 @@ def test_plain_and_paired_columns(N, K):
     assert np.abs(got - g / (1 + np.exp(-1.702 * g)) * (np.clip(y, -7, 7) + 1)).max() < 4 * bound(K)
 
 
-@pytest.mark.parametrize("T,K,ff", [(1, 64, 24), (1, 1032, 40), (3, 256, 6), (2, 2048, 130)])
+@pytest.mark.parametrize("T,K,ff", [(1, 64, 24), (1, 1032, 40), (3, 256, 6), (2, 2048, 130), (17, 256, 6), (31, 1032, 130), (20, 64, 24)])
 def test_chosen_experts(T, K, ff):
     rng = np.random.default_rng(K + ff)
     E, top = 6, 2

@@ -600,6 +600,88 @@ __global__ void __launch_bounds__(256) rows_stream_kernel(const float* __restric
 	rows_stream_finish<KS>(e, 0, c0, N, warp, lane, ks, acc, red);
 }
 
+// ---- the same for a few tokens (5 to 31, too few for the tensor cores' tiles): TB of them share each read of the weights ---------------------------
+// Bound: memory up to about 10 tokens, FP32 FMAs above.  The 64 x 64 tiles of rows_gemm_kernel leave 9 tokens 1/7 of a tile and 32 CTAs for 2048
+// columns, and load one element at a time: 9 tokens of 2048 x 2048 took 161 us, here 9.
+// Every lane ends up with the sums of one (token of the first eight, column) and one (token of the second eight, column) pair.
+// v[k] of every lane -> lane k gets the sum over lanes of v[k]
+__device__ __forceinline__ float warp_sum_transposed32(float (&v)[32], int lane) {
+#pragma unroll
+	for (int s = 16; s >= 1; s >>= 1) {
+		const bool up = (lane & s) != 0;
+#pragma unroll
+		for (int k = 0; k < s; k++) {
+			const float send = up ? v[k] : v[k + s];
+			const float keep = up ? v[k + s] : v[k];
+			v[k] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+		}
+	}
+	return v[0];
+}
+// W (N, K) columns c0 .. c0 + 3 times nt <= TB rows; x(t): row t's K floats, e's row is out_row(t).  red: 8 x 32 * (TB / 8) floats.  Every thread of the CTA
+// calls it, with c0 >= N where it has no columns.
+template <int KS, int TB, typename X, typename R>
+__device__ __forceinline__ void rows_few_tile(const __nv_bfloat16* W, int c0, int N, int K, int nt, X x, R out_row, const RowsEpi& e, int warp, int lane, float* red) {
+	constexpr int STEP = 256 * KS, G = TB / 8;
+	const int ks = warp % KS, k0 = (ks * 32 + lane) * 8;
+	float acc[G][32] = {}; // [eight tokens][token * 4 + column]
+	if (c0 < N) {
+		const __nv_bfloat16* w[RS_COLS];
+#pragma unroll
+		for (int c = 0; c < RS_COLS; c++) w[c] = W + (size_t) min(c0 + c, N - 1) * K;
+		uint4 r[RS_COLS], nx[RS_COLS];
+		if (k0 < K)
+#pragma unroll
+			for (int c = 0; c < RS_COLS; c++) nx[c] = *reinterpret_cast<const uint4*>(w[c] + k0);
+		for (int k = k0; k < K; k += STEP) {
+#pragma unroll
+			for (int c = 0; c < RS_COLS; c++) r[c] = nx[c];
+			if (k + STEP < K)
+#pragma unroll
+				for (int c = 0; c < RS_COLS; c++) nx[c] = *reinterpret_cast<const uint4*>(w[c] + k + STEP);
+#pragma unroll
+			for (int t = 0; t < TB; t++)
+				if (t < nt) {
+					const float* xr = x(t) + k;
+					const float4 x0 = *reinterpret_cast<const float4*>(xr), x1 = *reinterpret_cast<const float4*>(xr + 4);
+#pragma unroll
+					for (int c = 0; c < RS_COLS; c++) acc[t / 8][t % 8 * 4 + c] = dot8_bf16(acc[t / 8][t % 8 * 4 + c], r[c], x0, x1);
+				}
+		}
+	}
+#pragma unroll
+	for (int g = 0; g < G; g++) {
+		float v = warp_sum_transposed32(acc[g], lane);
+		if (KS > 1) {
+			red[(warp * G + g) * 32 + lane] = v;
+			__syncthreads();
+			if (ks == 0)
+#pragma unroll
+				for (int j = 1; j < KS; j++) v += red[((warp + j) * G + g) * 32 + lane];
+		}
+		const float next = __shfl_xor_sync(0xffffffffu, v, 1);
+		const int t = g * 8 + lane / 4, col = c0 + lane % 4;
+		if (ks == 0 && t < nt && col < N) {
+			if (e.kind == EPI_GLU) {
+				if (!(lane & 1) && col + 1 < N) epi_apply(e, out_row(t), col, N, v, next);
+			} else epi_apply(e, out_row(t), col, N, v, 0.f);
+		}
+	}
+}
+template <int KS, int TB>
+__global__ void __launch_bounds__(256, 2) rows_few_kernel(const float* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int T, int N, int K, RowsEpi e) {
+	__shared__ float red[8 * 32 * (TB / 8)];
+	if (blockIdx.z) { // one product of a batch
+		A += (size_t) blockIdx.z * e.batch_a;
+		W += (size_t) blockIdx.z * e.batch_w;
+		e.out += (size_t) blockIdx.z * e.batch_o;
+		if (e.mul) e.mul += (size_t) blockIdx.z * e.batch_o;
+	}
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t0 = blockIdx.y * TB;
+	rows_few_tile<KS, TB>(W, (blockIdx.x * (8 / KS) + warp / KS) * RS_COLS, N, K, min(TB, T - t0), [&](int t) { return A + (size_t) (t0 + t) * lda; },
+	                      [&](int t) { return t0 + t; }, e, warp, lane, red);
+}
+
 // ---- sliding-window softmax attention with score mixing across heads -------------------------------------------------------------
 struct SwaArgs {
 	const float* q;    // (T, ldq): head h at columns q_off + h * d
@@ -1372,21 +1454,6 @@ inline size_t hgrn2_smem_bytes(int d, int dv) { return sizeof(float) * ((size_t)
 // barrier reads the others' through distributed shared memory and scales the rows it wrote.
 constexpr int HG_CW = 4, HG_TT = 8;
 
-// v[k] of every lane -> lane k gets the sum over lanes of v[k]
-__device__ __forceinline__ float warp_sum_transposed32(float (&v)[32], int lane) {
-#pragma unroll
-	for (int s = 16; s >= 1; s >>= 1) {
-		const bool up = (lane & s) != 0;
-#pragma unroll
-		for (int k = 0; k < s; k++) {
-			const float send = up ? v[k] : v[k + s];
-			const float keep = up ? v[k + s] : v[k];
-			v[k] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-		}
-	}
-	return v[0];
-}
-
 template <int DPL, int KEYED>
 __global__ void hgrn2_cols_kernel(Hgrn2Args a) {
 	pdl_enter();
@@ -1656,10 +1723,14 @@ static inline int launch_check(const char* what) {
 }
 static inline int norm_threads(int width) { return width >= 1024 ? 256 : width >= 256 ? 128 : 64; }
 
+// From this many tokens on, rows_gemm_kernel's tiles are at least half full (passes of 32 and more run on the tensor cores where their shapes allow)
+constexpr int ROWS_FEW = 32;
+
 // out(T,N) = A(T,K) . W(N,K)^T with epilogue e, IEEE fp32 arithmetic; W is bf16 or fp32
 // batch > 1: that many products in one launch, operands and output advancing by e.batch_a / batch_w / batch_o per product
 static inline int launch_rows(const float* A, int lda, const void* W, bool w_bf16, int T, int N, int K, const RowsEpi& e, cudaStream_t s, int batch = 1) {
-	if (T == 1 && w_bf16 && K % 8 == 0 && (e.batch_a % 4 == 0 && e.batch_w % 8 == 0) && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A)) & 15) == 0) {
+	const bool wide = w_bf16 && K % 8 == 0 && e.batch_a % 4 == 0 && e.batch_w % 8 == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A)) & 15) == 0;
+	if (T == 1 && wide) {
 		const int ks = rows_stream_ks(N, K, batch), sets = (N + RS_COLS - 1) / RS_COLS;
 		const dim3 grid((sets * ks + 7) / 8, 1, batch);
 		const __nv_bfloat16* w = (const __nv_bfloat16*) W;
@@ -1667,6 +1738,20 @@ static inline int launch_rows(const float* A, int lda, const void* W, bool w_bf1
 		else if (ks == 2) launch_step(rows_stream_kernel<2>, grid, 256, 0, s, T, A, w, N, K, e);
 		else if (ks == 4) launch_step(rows_stream_kernel<4>, grid, 256, 0, s, T, A, w, N, K, e);
 		else launch_step(rows_stream_kernel<8>, grid, 256, 0, s, T, A, w, N, K, e);
+	} else if (T > 4 && T < ROWS_FEW && wide && lda % 4 == 0) {
+		const int tb = T <= 8 ? 8 : 16, groups = (T + tb - 1) / tb, ks = rows_stream_ks(N, K, batch * groups), sets = (N + RS_COLS - 1) / RS_COLS;
+		const dim3 grid((sets * ks + 7) / 8, groups, batch);
+		const __nv_bfloat16* w = (const __nv_bfloat16*) W;
+#define XALM_ROWS_FEW(KS_)                                                                        \
+	do {                                                                                          \
+		if (tb == 8) rows_few_kernel<KS_, 8><<<grid, 256, 0, s>>>(A, lda, w, T, N, K, e);         \
+		else rows_few_kernel<KS_, 16><<<grid, 256, 0, s>>>(A, lda, w, T, N, K, e);                \
+	} while (0)
+		if (ks == 1) XALM_ROWS_FEW(1);
+		else if (ks == 2) XALM_ROWS_FEW(2);
+		else if (ks == 4) XALM_ROWS_FEW(4);
+		else XALM_ROWS_FEW(8);
+#undef XALM_ROWS_FEW
 	} else if (T <= 4) {
 		const int pairs = (N + 1) / 2;
 		int ks = 1; // warps per column pair: enough CTAs for two per SM, each slice of K at least 256 long

@@ -403,6 +403,29 @@ __global__ void __launch_bounds__(256) moe_stream_kernel(MoeGemmArgs a) {
 	rows_stream_finish<KS>(a.e, p, c0, a.N, warp, lane, ks, acc, red);
 }
 
+// ---- the same for steps between a matvec per pair and the tensor cores' passes: a tile's rows eight at a time against four columns per warp -----------
+// The 64-row tiles of moe_gemm_kernel, with two or three rows each, took 674 us for 9 tokens' 4 of 16 experts at width 2048 (268 MB of weights)
+template <int KS>
+__global__ void __launch_bounds__(256, 2) moe_few_kernel(MoeGemmArgs a) {
+	__shared__ float red[8 * 32];
+	__shared__ int pair[8];
+	__shared__ const float* row[8];
+	if ((int) blockIdx.y >= *a.n_tiles) return;
+	const int ex = a.tiles[3 * blockIdx.y], first = a.tiles[3 * blockIdx.y + 1], rows = a.tiles[3 * blockIdx.y + 2];
+	const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(a.W) + (size_t) ex * a.N * a.K;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	for (int r0 = 0; r0 < rows; r0 += 8) {
+		const int nt = min(8, rows - r0);
+		__syncthreads(); // the eight rows before are done
+		if (threadIdx.x < nt) {
+			pair[threadIdx.x] = a.sorted[first + r0 + threadIdx.x];
+			row[threadIdx.x] = a.A + (size_t) (pair[threadIdx.x] / a.a_div) * a.lda;
+		}
+		__syncthreads();
+		rows_few_tile<KS, 8>(W, (blockIdx.x * (8 / KS) + warp / KS) * RS_COLS, a.N, a.K, nt, [&](int t) { return row[t]; }, [&](int t) { return pair[t]; }, a.e, warp, lane, red);
+	}
+}
+
 // ---- launchers ------------------------------------------------------------------------------------------------------------------
 static inline size_t moe_router_smem(int K, int E, int n_groups) { return (size_t) (K + 2 * E + std::max(n_groups, 1)) * 4; }
 static inline int moe_prepare(int K, int E, int n_groups) { // outside a stream capture
@@ -458,6 +481,15 @@ static inline int launch_moe_gemm(const MoeGemmArgs& a, bool w_bf16, int pairs, 
 		else XALM_MOE_MATVEC(float);
 #undef XALM_MOE_MATVEC
 		return launch_check("moe_matvec");
+	}
+	if (rows < ROWS_FEW && w_bf16 && a.K % 8 == 0 && a.lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.W) | reinterpret_cast<uintptr_t>(a.A)) & 15) == 0) {
+		const int ks = rows_stream_ks(a.N, a.K, std::min(E, pairs));
+		const dim3 grid(((a.N + RS_COLS - 1) / RS_COLS * ks + 7) / 8, moe_max_tiles(pairs, E));
+		if (ks == 1) moe_few_kernel<1><<<grid, 256, 0, s>>>(a);
+		else if (ks == 2) moe_few_kernel<2><<<grid, 256, 0, s>>>(a);
+		else if (ks == 4) moe_few_kernel<4><<<grid, 256, 0, s>>>(a);
+		else moe_few_kernel<8><<<grid, 256, 0, s>>>(a);
+		return launch_check("moe_few");
 	}
 	const dim3 grid((a.N + 63) / 64, moe_max_tiles(pairs, E));
 	if (w_bf16) moe_gemm_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(a);
