@@ -46,3 +46,17 @@ def test_chosen_experts(T, K, ff):
             g = wg[e].astype(np.float64) @ x
             want = wd[e].astype(np.float64) @ (g / (1 + np.exp(-g)) * (wu[e].astype(np.float64) @ x))
             assert np.abs(out[t, r] - want).max() < 4 * bound(K) + 4 * bound(ff)
+
+
+@pytest.mark.parametrize("W,groups", [(64, 1), (96, 3), (1024, 8), (4096, 1), (4096, 8), (8192, 1)])
+@pytest.mark.parametrize("T", [1, 4])
+def test_group_norm_of_short_steps(W, groups, T):
+    rng = np.random.default_rng(W + groups)
+    parts, n_hist = 3, 5
+    y, pw, w, x = rng.standard_normal((T, parts, W)), rng.uniform(0.1, 1, (T, parts)), 1 + 0.2 * rng.standard_normal(W), rng.standard_normal((T, W))
+    hist, coef = rng.standard_normal((n_hist, T, W)), rng.standard_normal(n_hist + 1)
+    u = (y * pw[:, :, None]).sum(1).reshape(T, groups, -1)
+    want = x + (u / np.sqrt((u * u).mean(-1, keepdims=True) + 1e-5)).reshape(T, W) * w
+    got, avg = capi.group_norm_residual(y, w, groups, 1e-5, x_in=x, part_w=pw, hist=hist, dwa=coef)
+    assert np.abs(got - want).max() < 2e-5  # a dozen fp32 roundings of values below 8
+    assert np.abs(avg - ((coef[:-1, None, None] * hist).sum(0) + coef[-1] * want)).max() < 6e-5

@@ -246,8 +246,8 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 	const int W = m->width;
 	const size_t hs = (size_t) m->chunk * W;
 	const bool f32 = m->precision == XALM_PRECISION_F32;
-	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<n, norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, 1, hs, m->hist);
-	else embed_streams_kernel<float><<<n, norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, 1, hs, m->hist);
+	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, 1, hs, m->hist);
+	else embed_streams_kernel<float><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, 1, hs, m->hist);
 	XALM_SEQ_LAUNCH_CHECK("embed");
 	const float* x = m->hist; // what the layer reads: X_0, later the depth average (or the last result where a layer has none)
 	for (size_t li = 0; li < m->layers.size(); li++) {

@@ -248,8 +248,8 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 	cudaStream_t s = m->stream;
 	const int W = m->width;
 	const size_t hs = (size_t) m->chunk * W;
-	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<n, norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, 1, hs, m->x, m->embed_scale);
-	else embed_streams_kernel<float><<<n, norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, 1, hs, m->x, m->embed_scale);
+	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, 1, hs, m->x, m->embed_scale);
+	else embed_streams_kernel<float><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, 1, hs, m->x, m->embed_scale);
 	XALM_SEQ_LAUNCH_CHECK("embed");
 	for (size_t li = 0; li < m->layers.size(); li++) {
 		const Layer& L = m->layers[li];

@@ -37,7 +37,7 @@ struct LatentPostArgs {
 	const SeqStep* step;
 };
 
-// one CTA per token; shared memory: 33 floats
+// one CTA per token, or (steps of a few tokens, grid (rows, 2)) one for the query row and one for the cache row; shared memory: 33 floats
 static __global__ void latent_post_kernel(LatentPostArgs a) {
 	pdl_enter();
 	__shared__ float red[33];
@@ -45,13 +45,13 @@ static __global__ void latent_post_kernel(LatentPostArgs a) {
 	if (t >= a.step->n) return;
 	const float* row = a.proj + (size_t) t * a.ld;
 	const int pos = a.step->pos0 + t;
-	if (a.q_rank) {
+	if (a.q_rank && blockIdx.y == 0) {
 		float ss = 0.f;
 		for (int c = tid; c < a.q_rank; c += nth) ss = fmaf(row[a.q_off + c], row[a.q_off + c], ss);
 		const float r = 1.f / sqrtf(block_sum(ss, red) / (float) a.q_rank + a.eps);
 		for (int c = tid; c < a.q_rank; c += nth) a.cq[(size_t) t * a.ldc + c] = row[a.q_off + c] * r * a.q_norm[c];
 	}
-	if (!a.kv_rank) return;
+	if (!a.kv_rank || blockIdx.y != gridDim.y - 1) return;
 	float ss = 0.f;
 	for (int c = tid; c < a.kv_rank; c += nth) ss = fmaf(row[a.kv_off + c], row[a.kv_off + c], ss);
 	const float r = 1.f / sqrtf(block_sum(ss, red) / (float) a.kv_rank + a.eps);
@@ -79,7 +79,7 @@ static __global__ void latent_post_kernel(LatentPostArgs a) {
 static inline int launch_latent_post(const LatentPostArgs& a, int rows, cudaStream_t s) {
 	if (a.rot % 2 || (a.rot && !a.freq)) return set_error(XALM_ERR_INVALID, "latent_post: %d rotated columns", a.rot);
 	const int widest = std::max(a.q_rank, a.kv_rank);
-	launch_step(latent_post_kernel, rows, widest >= 512 ? 256 : widest >= 128 ? 128 : 64, 0, s, rows, a);
+	launch_step(latent_post_kernel, dim3(rows, rows <= 4 ? 2 : 1), rows <= 4 ? std::min(512, std::max(64, (widest + 63) / 64 * 32)) : widest >= 512 ? 256 : widest >= 128 ? 128 : 64, 0, s, rows, a);
 	return launch_check("latent_post");
 }
 

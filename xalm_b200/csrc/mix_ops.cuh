@@ -83,6 +83,11 @@ struct SeqStep {
 	int prev; // the token before the step's first one, -1 at a sequence's start (designs whose embedding looks at token pairs)
 };
 
+static inline int norm_threads(int width) { return width >= 1024 ? 256 : width >= 256 ? 128 : 64; }
+// A step of a few tokens leaves most SMs idle, and a row's kernel takes as long as its dependent trips to memory: a row's columns go over several CTAs
+// where they do not depend on one another.  (Four times the threads in one CTA did not help: 1024 threads take longer to start.)
+static inline int step_parts(int rows, int width) { return rows > 4 ? 1 : std::min(16, std::max(1, width / norm_threads(width))); }
+
 // ---- embedding -> streams -------------------------------------------------------------------------------------------------
 // positions: (max positions, width) learned rows, the one of the token's position in its sequence is added (unscaled); NULL: none
 template <typename WT>
@@ -92,7 +97,7 @@ __global__ void embed_streams_kernel(const WT* __restrict__ table, const int* __
 	const int t = blockIdx.x;
 	const WT* row = table + (size_t) tokens[t] * width;
 	const WT* prow = positions ? positions + (size_t) (step->pos0 + t) * width : nullptr;
-	for (int c = threadIdx.x; c < width; c += blockDim.x) {
+	for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
 		float v = ldf(row + c) * scale; // scale 1: the row as it is
 		if (prow) v += ldf(prow + c);
 		for (int s = 0; s < S; s++) xs[(size_t) s * stream_stride + (size_t) t * width + c] = v;
@@ -159,11 +164,14 @@ __global__ void embed_pair_kernel(EmbedPairArgs a) {
 template <int SS>
 __global__ void hc_norm_kernel(const float* __restrict__ xs, int S, size_t stream_stride, const float* __restrict__ a, const float* __restrict__ w,
                                int one_plus, float eps, int width, float* __restrict__ h, float* __restrict__ sum_out) {
-	pdl_enter();
 	extern __shared__ float sm[];
 	float* u = sm;            // width
 	float* red = sm + width;  // 33
 	const int t = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
+	float w0[4]; // the first columns' weights: on their way before the kernel before this one is done
+#pragma unroll
+	for (int k = 0; k < 4; k++) w0[k] = h && k * nth + tid < width ? w[k * nth + tid] : 0.f;
+	pdl_enter();
 	// Four columns per thread at a time, every load of the four issued before the first use: a one-token step runs one CTA of this
 	// kernel, and its time is the number of dependent trips to memory.
 	float av[SS];
@@ -198,7 +206,7 @@ __global__ void hc_norm_kernel(const float* __restrict__ xs, int S, size_t strea
 #pragma unroll
 		for (int k = 0; k < 4; k++) {
 			const int c = c0 + k * nth + tid;
-			wv[k] = (h && c < width) ? w[c] : 0.f;
+			wv[k] = !c0 ? w0[k] : (h && c < width) ? w[c] : 0.f;
 		}
 #pragma unroll
 		for (int k = 0; k < 4; k++) {
@@ -1721,7 +1729,6 @@ static inline int launch_check(const char* what) {
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "%s launch failed: %s", what, cudaGetErrorString(e));
 	return XALM_OK;
 }
-static inline int norm_threads(int width) { return width >= 1024 ? 256 : width >= 256 ? 128 : 64; }
 
 // From this many tokens on, rows_gemm_kernel's tiles are at least half full (passes of 32 and more run on the tensor cores where their shapes allow)
 constexpr int ROWS_FEW = 32;
@@ -1917,6 +1924,68 @@ static __global__ void group_norm_residual_kernel(GroupNormArgs a) {
 		}
 	}
 }
+// The same for steps of a few tokens, grid (rows, groups): a CTA per group, whose columns (four per thread) are read in one trip and stay in registers.
+// As one CTA per row the norms of 4096 columns in 8 groups took 7.4 us each, 15.6 us with two experts' rows joined; with this kernel and the embedding
+// row over 16 CTAs a Bolovik step at width 4096, which runs five of them, went from 347 to 316 us.
+static __global__ void group_norm_step_kernel(GroupNormArgs a) {
+	__shared__ float red[33];
+	const int t = blockIdx.x, tid = threadIdx.x, nth = blockDim.x, W = a.width, gs = W / a.groups, lo = blockIdx.y * gs;
+	float wv[4], v[4], xi[4], acc[4] = {}, ss = 0.f;
+	bool in[4];
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		in[k] = tid + k * nth < gs;
+		wv[k] = in[k] ? a.w[lo + tid + k * nth] : 0.f;
+	}
+	pdl_enter();
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		const int c = lo + tid + k * nth;
+		xi[k] = in[k] && a.x_in ? a.x_in[(size_t) t * W + c] : 0.f;
+		v[k] = in[k] && !a.part_w ? a.y[(size_t) t * a.ldy + c] : 0.f;
+	}
+	if (a.part_w)
+#pragma unroll 4
+		for (int p = 0; p < a.parts; p++) {
+			const size_t pk = (size_t) t * a.parts + p;
+			const float* y = a.y + (a.part_row ? (size_t) a.part_row[pk] : pk) * a.ldy + lo + tid;
+			const float pw = a.part_w[pk];
+#pragma unroll
+			for (int k = 0; k < 4; k++) v[k] = fmaf(pw, in[k] ? y[k * nth] : 0.f, v[k]);
+		}
+	if (a.dwa)
+#pragma unroll 4
+		for (int j = 0; j < a.n_hist; j++) {
+			const float* hv = a.hist + (size_t) j * a.hist_stride + (size_t) t * W + lo + tid;
+			const float cj = a.dwa[j];
+#pragma unroll
+			for (int k = 0; k < 4; k++) acc[k] = fmaf(cj, in[k] ? hv[k * nth] : 0.f, acc[k]);
+		}
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		if (a.gate && in[k]) {
+			const float z = a.gate[(size_t) t * a.ldg + lo + tid + k * nth];
+			v[k] *= z * sigmoidf_(z);
+		}
+		ss = fmaf(v[k], v[k], ss);
+	}
+	const float rinv = 1.f / sqrtf(block_sum(ss, red) / (float) gs + a.eps);
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		if (!in[k]) continue;
+		const int c = lo + tid + k * nth;
+		const size_t at = (size_t) t * W + c;
+		float o = v[k] * rinv * wv[k];
+		if (a.out_scale != 0.f) o *= a.out_scale;
+		if (a.x_in) o += xi[k];
+		a.x_out[a.ld_out ? (size_t) t * a.ld_out + c : at] = o;
+		if (a.dwa) {
+			o = fmaf(a.dwa[a.n_hist], o, acc[k]);
+			a.avg_out[at] = o;
+		}
+		if (a.keep_out) a.keep_out[at] = o;
+	}
+}
 static inline size_t group_norm_smem(int width, int groups) { return (size_t) (width + groups) * 4; }
 static inline int group_norm_prepare(int width, int groups) {
 	static bool raised = false;
@@ -1928,7 +1997,9 @@ static inline int group_norm_prepare(int width, int groups) {
 }
 static inline int launch_group_norm(const GroupNormArgs& a, int rows, cudaStream_t s) {
 	if (a.groups <= 0 || a.width % a.groups) return set_error(XALM_ERR_INVALID, "group norm: %d groups do not divide a row of %d", a.groups, a.width);
-	launch_step(group_norm_residual_kernel, rows, norm_threads(a.width), group_norm_smem(a.width, a.groups), s, rows, a);
+	const int gs = a.width / a.groups;
+	if (rows <= 4 && gs <= 4096 && a.groups <= 65535) launch_step(group_norm_step_kernel, dim3(rows, a.groups), std::max(32, (gs + 127) / 128 * 32), 0, s, rows, a);
+	else launch_step(group_norm_residual_kernel, rows, norm_threads(a.width), group_norm_smem(a.width, a.groups), s, rows, a);
 	return launch_check("group_norm_residual");
 }
 

@@ -216,9 +216,9 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 	const size_t hs = (size_t) m->chunk * W;
 	float *x = m->x, *x_next = m->x2; // a repetition's product reads the one and writes the other
 	if (m->w_bf16)
-		embed_streams_kernel<__nv_bfloat16><<<n, norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, 1, hs, x, 1.f,
+		embed_streams_kernel<__nv_bfloat16><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, 1, hs, x, 1.f,
 		                                                                  (const __nv_bfloat16*) m->positions, m->d_step);
-	else embed_streams_kernel<float><<<n, norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, 1, hs, x, 1.f, (const float*) m->positions, m->d_step);
+	else embed_streams_kernel<float><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, 1, hs, x, 1.f, (const float*) m->positions, m->d_step);
 	XALM_SEQ_LAUNCH_CHECK("embed");
 	if (m->loops) { // what the embedded row adds at the start of every repetition
 		RowsEpi e0;

@@ -188,8 +188,8 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 	const int W = m->width, S = m->S;
 	const size_t sstride = (size_t) m->chunk * W;
 	const int rt = norm_threads(W);
-	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<n, rt, 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, S, sstride, m->xs);
-	else embed_streams_kernel<float><<<n, rt, 0, s>>>((const float*) m->embed, m->d_tokens, W, S, sstride, m->xs);
+	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<dim3(n, step_parts(n, W)), rt, 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, S, sstride, m->xs);
+	else embed_streams_kernel<float><<<dim3(n, step_parts(n, W)), rt, 0, s>>>((const float*) m->embed, m->d_tokens, W, S, sstride, m->xs);
 	XALM_SEQ_LAUNCH_CHECK("embed");
 	for (size_t li = 0; li < m->layers.size(); li++) {
 		const Layer& L = m->layers[li];

@@ -219,8 +219,8 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 	const size_t hs = (size_t) m->chunk * W;
 	float* x = m->x;
 	const int copies = m->loops ? 2 : 1; // the residual stream, and x_0 for the passes to come
-	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<n, norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, copies, hs, x);
-	else embed_streams_kernel<float><<<n, norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, copies, hs, x);
+	if (m->w_bf16) embed_streams_kernel<__nv_bfloat16><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const __nv_bfloat16*) m->embed, m->d_tokens, W, copies, hs, x);
+	else embed_streams_kernel<float><<<dim3(n, step_parts(n, W)), norm_threads(W), 0, s>>>((const float*) m->embed, m->d_tokens, W, copies, hs, x);
 	XALM_SEQ_LAUNCH_CHECK("embed");
 	for (size_t ri = 0; ri < m->runs.size(); ri++) {
 		const Run& R = m->runs[ri];
