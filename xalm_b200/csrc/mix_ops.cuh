@@ -2250,6 +2250,14 @@ static inline bool swa_one_ok(const SwaArgs& a, int rows) {
 	       ((reinterpret_cast<uintptr_t>(a.kc) | reinterpret_cast<uintptr_t>(a.vc) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
 }
 
+// swa_mma.cu: passes of many tokens over a bf16 cache, on the tensor cores.  It takes heads of 32 to 128 channels in whole 16-byte pieces whose scores
+// do not mix, and fills a warp's 16 queries; smaller heads would be mostly padding.
+int launch_swa_mma(const SwaArgs& a, int rows, cudaStream_t s);
+static inline bool swa_mma_ok(const SwaArgs& a, int rows, bool cache_f32) {
+	return !cache_f32 && rows >= 16 && !a.talk && std::min(a.d, a.dv) >= 32 && std::max(a.d, a.dv) <= 128 && ((a.d | a.dv | a.ldk | a.ldv) & 7) == 0 &&
+	       ((a.ldq | a.q_off) & 3) == 0 && a.H <= 65535 && ((reinterpret_cast<uintptr_t>(a.kc) | reinterpret_cast<uintptr_t>(a.vc) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
+}
+
 // rows: tokens of the step; cache_f32: element type of the ring.  With n_splits > 1 the merge kernel follows.  Returns the number of
 // launches through *launches (1 or 2) when it is given.
 static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s, int* launches = nullptr) {
@@ -2282,6 +2290,10 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 			}
 			return XALM_OK;
 		}
+	}
+	if (swa_mma_ok(a, rows, cache_f32)) {
+		if (launches) *launches = 1;
+		return launch_swa_mma(a, rows, s);
 	}
 	const int tq = swa_pick_tq(a.H, a.G, a.d, a.dv, rows);
 	if (swa_one_ok(a, rows)) {

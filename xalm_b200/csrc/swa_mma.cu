@@ -1,0 +1,253 @@
+// swa_mma.cu — the attention of mix_ops.cuh (window, kept first positions, chunks, soft cap, distance biases, sink, gate; no mixing of heads) for passes
+// of many tokens over a bf16 cache, on the tensor cores in fp32 grade.
+//
+// Queries and probabilities are fp32 values: each enters as three bf16 planes (hi + mid + lo = its 24 bits), keys and values as the bf16 the cache
+// holds, so that every product is exact and only the fp32 sums round.  The tensor cores sum 16 products (of the small planes first) from zero; sums of more
+// are added in round-to-nearest, since the tensor cores' own additions truncate: chained over a head's channels and a key block, the result was
+// twice as far from float64 as the fp32 FMA kernel's.
+// A CTA takes 16 queries of one head per warp; 64 keys and their values at a time come through a two-deep cp.async ring; queries stay in shared memory
+// as planes, scores, probabilities and output in registers (m16n8k16 fragments).
+// Bound: the instructions around the products (splits, exponentials, adds: about half) and the mma.sync pipe, three products per one.  Against the fp32
+// FMA tiles of mix_ops.cuh: 1024 tokens of 16 heads of 128 over up to 2048 keys 1626 -> 200 us, of 8 heads in a window of 512 286 -> 94 us; 256 tokens
+// of 8 heads over up to 301 keys 105 -> 83 us (32 CTAs).  Distance from float64 at 128 channels and 1500 keys: 2.6e-7, the FMA kernel 4.4e-7.
+#define XALM_SECONDARY_TU
+#include "common.cuh"
+#include "family.h"
+#include "mix_ops.cuh"
+
+namespace xalm {
+namespace mix {
+
+constexpr int SMM_KEYS = 64, SMM_STAGES = 2;
+
+__device__ __forceinline__ void smm_ldsm4(uint32_t (&r)[4], uint32_t addr) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void smm_ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void smm_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+	asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+	             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+	             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// two fp32 values as three pairs of bf16 whose sums are the values
+__device__ __forceinline__ void smm_split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+	const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+	const float xr = x - __low2float(h), yr = y - __high2float(h);
+	const __nv_bfloat162 m = __floats2bfloat162_rn(xr, yr);
+	const __nv_bfloat162 l = __floats2bfloat162_rn(xr - __low2float(m), yr - __high2float(m));
+	hi = *reinterpret_cast<const uint32_t*>(&h);
+	mid = *reinterpret_cast<const uint32_t*>(&m);
+	lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// rows of D bf16 in 16-byte pieces, piece p of row r at place p ^ (r % 8): the eight rows of a fragment's 8x8 matrix fall on different banks
+template <int D>
+__device__ __forceinline__ uint32_t smm_at(int row, int piece) {
+	return (uint32_t) (row * (D * 2) + ((piece ^ (row & 7)) << 4));
+}
+__host__ __device__ constexpr size_t smm_smem(int dq, int dv, int warps) {
+	return (size_t) 3 * 16 * warps * dq * 2 + (size_t) SMM_STAGES * SMM_KEYS * (dq + dv) * 2 + (size_t) SMM_STAGES * SMM_KEYS * 4;
+}
+
+// DQ, DV: the channel counts rounded up to 64 or 128 (the rest is zero); WARPS * 16 queries
+template <int DQ, int DV, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
+	extern __shared__ __align__(128) uint8_t smem[];
+	constexpr int NTH = WARPS * 32, ROWS = WARPS * 16;
+	uint8_t* qs = smem;                                  // 3 planes x ROWS x DQ
+	uint8_t* ks = qs + (size_t) 3 * ROWS * DQ * 2;       // stages x SMM_KEYS x DQ
+	uint8_t* vs = ks + (size_t) SMM_STAGES * SMM_KEYS * DQ * 2;
+	int* kp = reinterpret_cast<int*>(vs + (size_t) SMM_STAGES * SMM_KEYS * DV * 2); // stages x SMM_KEYS positions (0x7fffffff: no key)
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = lane >> 2, ql = lane & 3;
+	const int n = a.step->n, pos0 = a.step->pos0, H = a.H, G = a.G, d = a.d, dv = a.dv;
+	const int t0 = ((int) gridDim.x - 1 - (int) blockIdx.x) * ROWS, h = blockIdx.y, g = h / (H / G); // the last queries see the most keys: they start first
+	const int nq = min(ROWS, n - t0);
+	if (nq <= 0) return;
+	const int i_lo = pos0 + t0, i_hi = i_lo + nq - 1;
+	const SwaKeys km = swa_keys(a, i_lo);
+	const int nk = km.ks + i_hi - km.j_first + 1;
+	const int ldk = a.ldk ? a.ldk : G * d, ldv = a.ldv ? a.ldv : G * dv;
+	const __nv_bfloat16* kc = reinterpret_cast<const __nv_bfloat16*>(a.kc) + (size_t) g * d;
+	const __nv_bfloat16* vc = reinterpret_cast<const __nv_bfloat16*>(a.vc) + (size_t) g * dv;
+
+	auto stage = [&](int j0, int buf) {
+		const uint32_t kb = smem_u32(ks) + (uint32_t) buf * SMM_KEYS * DQ * 2, vb = smem_u32(vs) + (uint32_t) buf * SMM_KEYS * DV * 2;
+		// PER threads share a key, whose slot is worked out once, and take alternate 16-byte pieces; size 0 writes zeros (beyond the last key or channel)
+		constexpr int PER = NTH / SMM_KEYS;
+		const int row = tid / PER, j = min(j0 + row, nk - 1), first = tid % PER;
+		const bool in = j0 + row < nk;
+		const size_t slot = km.slot(j);
+		if (first == 0) kp[buf * SMM_KEYS + row] = in ? km.pos(j) : 0x7fffffff;
+		const __nv_bfloat16 *kr = kc + slot * ldk, *vr = vc + slot * ldv;
+#pragma unroll
+		for (int p = 0; p < DQ / 8; p += PER) {
+			const int ok = in && (p + first) * 8 < d;
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kb + smm_at<DQ>(row, p + first)), "l"(kr + (ok ? (p + first) * 8 : 0)), "r"(ok ? 16 : 0) : "memory");
+		}
+#pragma unroll
+		for (int p = 0; p < DV / 8; p += PER) {
+			const int ok = in && (p + first) * 8 < dv;
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vb + smm_at<DV>(row, p + first)), "l"(vr + (ok ? (p + first) * 8 : 0)), "r"(ok ? 16 : 0) : "memory");
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	stage(0, 0);
+	// queries, as planes
+	for (int x = tid; x < ROWS * (DQ / 8); x += NTH) {
+		const int row = x / (DQ / 8), p = x % (DQ / 8);
+		float v[8] = {};
+		if (row < nq && p * 8 < d) ld8(a.q + (size_t) (t0 + row) * a.ldq + a.q_off + (size_t) h * d + p * 8, v);
+		uint32_t w[3][4];
+#pragma unroll
+		for (int e = 0; e < 4; e++) smm_split(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+#pragma unroll
+		for (int pl = 0; pl < 3; pl++)
+			*reinterpret_cast<uint4*>(qs + (size_t) pl * ROWS * DQ * 2 + smm_at<DQ>(row, p)) = make_uint4(w[pl][0], w[pl][1], w[pl][2], w[pl][3]);
+	}
+	float o[DV / 8][4] = {}, m[2] = {-INFINITY, -INFINITY}, l[2] = {};
+	const int r0 = warp * 16 + quad; // this thread's rows: r0 and r0 + 8 of the CTA's
+	const float slope = a.slope ? a.slope[h] : 0.f, b1 = a.r1 ? a.r1[h] : 0.f, b2 = a.r1 ? a.r2[h] : 0.f;
+	const int blocks = (nk + SMM_KEYS - 1) / SMM_KEYS;
+	const bool plain = !(a.softcap > 0.f) && !a.r1 && !a.slope, one_run = a.mask_chunk <= 0 || i_lo / a.mask_chunk == i_hi / a.mask_chunk;
+	for (int blk = 0; blk < blocks; blk++) {
+		const int buf = blk % SMM_STAGES, j0 = blk * SMM_KEYS;
+		if (blk + 1 < blocks) {
+			stage(j0 + SMM_KEYS, (blk + 1) % SMM_STAGES);
+			asm volatile("cp.async.wait_group 1;" ::: "memory");
+		} else asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads();
+		const uint32_t kb = smem_u32(ks) + (uint32_t) buf * SMM_KEYS * DQ * 2, vb = smem_u32(vs) + (uint32_t) buf * SMM_KEYS * DV * 2;
+		// ---- scores ----
+		float s[SMM_KEYS / 8][4] = {};
+#pragma unroll
+		for (int k = 0; k < DQ / 16; k++) {
+			uint32_t qa[3][4];
+#pragma unroll
+			for (int pl = 0; pl < 3; pl++) smm_ldsm4(qa[pl], smem_u32(qs) + (uint32_t) pl * ROWS * DQ * 2 + smm_at<DQ>(warp * 16 + (lane & 15), 2 * k + (lane >> 4)));
+#pragma unroll
+			for (int c = 0; c < SMM_KEYS / 16; c++) { // 16 keys
+				uint32_t b[4];
+				float part[2][4] = {};
+				smm_ldsm4(b, kb + smm_at<DQ>(c * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1)));
+#pragma unroll
+				for (int pl = 2; pl >= 0; pl--) {
+					smm_mma(part[0], qa[pl], b[0], b[1]);
+					smm_mma(part[1], qa[pl], b[2], b[3]);
+				}
+#pragma unroll
+				for (int x = 0; x < 2; x++)
+#pragma unroll
+					for (int e = 0; e < 4; e++) s[2 * c + x][e] += part[x][e];
+			}
+		}
+		// ---- scale, soft cap, biases, mask ----
+		const int* pos = kp + buf * SMM_KEYS;
+		float top[2] = {m[0], m[1]};
+		const int p_lo = km.pos(j0), p_hi = km.pos(min(j0 + SMM_KEYS, nk) - 1);
+		if (plain && j0 + SMM_KEYS <= nk && p_hi <= i_lo && (a.window >= 0x7fffffff || i_hi - p_lo < a.window || p_hi < a.keep_first) && one_run) {
+			// every query sees every key of the block, and the score is only scaled
+#pragma unroll
+			for (int c = 0; c < SMM_KEYS / 8; c++)
+#pragma unroll
+				for (int e = 0; e < 4; e++) {
+					s[c][e] *= a.scale;
+					top[e >> 1] = fmaxf(top[e >> 1], s[c][e]);
+				}
+		} else
+#pragma unroll
+		for (int c = 0; c < SMM_KEYS / 8; c++)
+#pragma unroll
+			for (int e = 0; e < 4; e++) {
+				const int i = i_lo + r0 + (e >> 1) * 8, j = pos[c * 8 + ql * 2 + (e & 1)];
+				float x = s[c][e] * a.scale;
+				if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+				const float dist = (float) max(i - j, 0);
+				if (a.r1) x -= b1 * log1pf(b2 * dist);
+				if (a.slope) x -= slope * dist;
+				const bool seen = j <= i && (a.window >= 0x7fffffff || i - j < a.window || j < a.keep_first) && (a.mask_chunk <= 0 || j >= i - i % a.mask_chunk);
+				s[c][e] = seen ? x : -INFINITY;
+				top[e >> 1] = fmaxf(top[e >> 1], s[c][e]);
+			}
+		// ---- softmax weights ----
+#pragma unroll
+		for (int r = 0; r < 2; r++) {
+			top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
+			top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
+			const float at = top[r] == -INFINITY ? 0.f : top[r], keep = m[r] == -INFINITY ? 0.f : expf(m[r] - at);
+			float sum = 0.f;
+#pragma unroll
+			for (int c = 0; c < SMM_KEYS / 8; c++)
+#pragma unroll
+				for (int e = 0; e < 2; e++) {
+					s[c][2 * r + e] = expf(s[c][2 * r + e] - at);
+					sum += s[c][2 * r + e];
+				}
+			l[r] = fmaf(l[r], keep, sum); // this lane's keys; joined at the end
+			m[r] = top[r];
+#pragma unroll
+			for (int c = 0; c < DV / 8; c++)
+#pragma unroll
+				for (int e = 0; e < 2; e++) o[c][2 * r + e] *= keep;
+		}
+		uint32_t p[3][SMM_KEYS / 16][4];
+#pragma unroll
+		for (int c = 0; c < SMM_KEYS / 16; c++)
+#pragma unroll
+			for (int e = 0; e < 4; e++) smm_split(s[2 * c + (e >> 1)][(e & 1) * 2], s[2 * c + (e >> 1)][(e & 1) * 2 + 1], p[0][c][e], p[1][c][e], p[2][c][e]);
+		// ---- values ----
+#pragma unroll
+		for (int c = 0; c < DV / 16; c++) { // 16 value channels
+#pragma unroll
+			for (int k = 0; k < SMM_KEYS / 16; k++) {
+				uint32_t b[4];
+				float part[2][4] = {};
+				smm_ldsm4_t(b, vb + smm_at<DV>(k * 16 + (lane & 15), 2 * c + (lane >> 4)));
+#pragma unroll
+				for (int pl = 2; pl >= 0; pl--) {
+					smm_mma(part[0], p[pl][k], b[0], b[1]);
+					smm_mma(part[1], p[pl][k], b[2], b[3]);
+				}
+#pragma unroll
+				for (int x = 0; x < 2; x++)
+#pragma unroll
+					for (int e = 0; e < 4; e++) o[2 * c + x][e] += part[x][e];
+			}
+		}
+		__syncthreads(); // the block's buffer is read
+	}
+#pragma unroll
+	for (int r = 0; r < 2; r++) {
+		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+		const int t = t0 + r0 + r * 8;
+		if (r0 + r * 8 >= nq) continue;
+		float* dst = a.out + (size_t) t * (a.ldo ? a.ldo : H * dv) + (size_t) h * dv;
+#pragma unroll
+		for (int c = 0; c < DV / 8; c++)
+#pragma unroll
+			for (int e = 0; e < 2; e++) {
+				const int col = c * 8 + ql * 2 + e;
+				if (col >= dv) continue;
+				float v = swa_finish(a, h, o[c][2 * r + e], l[r], m[r]);
+				if (a.gate) v *= swa_gate(a, t, h, col);
+				dst[col] = v;
+			}
+	}
+}
+
+template <int DQ, int DV>
+static int launch_swa_mma_inst(const SwaArgs& a, int rows, cudaStream_t s) {
+	constexpr int WARPS = 4; // two per CTA, for twice the CTAs, copied every key block for half the queries and were slower
+	XALM_CUDA_CHECK(cudaFuncSetAttribute(swa_mma_kernel<DQ, DV, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smm_smem(DQ, DV, WARPS)));
+	swa_mma_kernel<DQ, DV, WARPS><<<dim3((rows + WARPS * 16 - 1) / (WARPS * 16), a.H), WARPS * 32, smm_smem(DQ, DV, WARPS), s>>>(a);
+	return launch_check("swa_mma");
+}
+
+int launch_swa_mma(const SwaArgs& a, int rows, cudaStream_t s) {
+	if (a.d <= 64) return a.dv <= 64 ? launch_swa_mma_inst<64, 64>(a, rows, s) : launch_swa_mma_inst<64, 128>(a, rows, s);
+	return a.dv <= 64 ? launch_swa_mma_inst<128, 64>(a, rows, s) : launch_swa_mma_inst<128, 128>(a, rows, s);
+}
+
+} // namespace mix
+} // namespace xalm
