@@ -53,6 +53,12 @@ struct HostTensor {
 	std::vector<float> v;
 };
 
+struct StepIn { // a one-token step's inputs, as they lie at SeqModel::d_step
+	SeqStep step;
+	int token;
+};
+static_assert(sizeof(StepIn) == sizeof(SeqStep) + sizeof(int), "the first token follows the step");
+
 struct SeqModel;
 struct SeqHooks {
 	int (*parse_config)(SeqModel*, const char* json);        // sizes, constants, expected tensors; touches no device
@@ -88,15 +94,17 @@ struct SeqModel { // what a handle of these families points to (ModelHead first)
 	float *logits = nullptr, *layer_sums = nullptr;
 	int keep_layers = 0;                      // keep the residual stream after every layer of the last pass (read_state(100 + layer))
 	int graph_launches[2] = {0, 0};           // kernels in the captured one-token step (without / with logits)
+	SeqStep* d_step = nullptr; // with d_tokens right behind it
 	int* d_tokens = nullptr;
-	SeqStep* d_step = nullptr;
+	StepIn* h_step = nullptr;  // pinned: what a one-token step's graph copies there
 	float* h_logits = nullptr; // pinned, chunk x vocab
 	int* d_targets = nullptr;  // max_tokens, as d_probs and h_probs (pinned): the target probabilities of one prefill call
 	float *d_probs = nullptr, *h_probs = nullptr;
 	cudaStream_t stream = nullptr, own_stream = nullptr;
 	cudaStream_t side = nullptr; // for mixers of a layer that do not depend on one another
 	cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-	cudaGraphExec_t graph[2] = {nullptr, nullptr};
+	cudaGraphExec_t graph[2] = {nullptr, nullptr};    // a one-token step's kernels (without / with logits)
+	cudaGraphExec_t graph_io[2] = {nullptr, nullptr}; // and with the copies of its inputs and of its logits around them, for calls that wait for the step
 	int pos = 0; // tokens the running sequence holds
 	int prev_token = -1; // the last of them (-1: none yet), handed to the kernels as SeqStep.prev
 	int last_launches = 0;
@@ -305,38 +313,57 @@ int check_ready(SeqModel* m) {
 	return XALM_OK;
 }
 
-int ensure_graph(SeqModel* m, int mode) {
-	if (m->graph[mode]) return XALM_OK;
+int ensure_graph(SeqModel* m, int mode, bool io) {
+	cudaGraphExec_t* exec = io ? &m->graph_io[mode] : &m->graph[mode];
+	if (*exec) return XALM_OK;
 	cudaGraph_t g = nullptr;
 	XALM_CUDA_CHECK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
 	pdl_block(m->stream);
 	int nl = 0;
+	cudaError_t ec = io ? cudaMemcpyAsync(m->d_step, m->h_step, sizeof(StepIn), cudaMemcpyHostToDevice, m->stream) : cudaSuccess;
 	const int rc = m->hooks->enqueue_pass(m, 1, mode ? 1 : 0, &nl);
+	if (io && mode && ec == cudaSuccess) ec = cudaMemcpyAsync(m->h_logits, m->logits, (size_t) m->vocab * 4, cudaMemcpyDeviceToHost, m->stream);
 	cudaError_t e = cudaStreamEndCapture(m->stream, &g);
+	if (e == cudaSuccess) e = ec;
 	if (rc != XALM_OK) {
 		if (g) cudaGraphDestroy(g);
 		return rc;
 	}
-	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
+	if (e != cudaSuccess) {
+		if (g) cudaGraphDestroy(g);
+		return set_error(XALM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
+	}
 	m->graph_launches[mode] = nl;
-	e = cudaGraphInstantiate(&m->graph[mode], g, 0);
+	e = cudaGraphInstantiate(exec, g, 0);
 	cudaGraphDestroy(g);
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "cudaGraphInstantiate failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
 }
 
 // one pass of n <= chunk tokens at the sequence's position; the logits (want) stay on the device
-int run_pass(SeqModel* m, const int* tokens, int n, int want) {
+// waits: the caller waits for the pass before it returns, so that a one-token step may take its inputs from pinned memory and leave its logits in
+// h_logits, one graph launch in all.  (Two copies from pageable memory before the graph and one behind it cost a step 10 us.)
+int run_pass(SeqModel* m, const int* tokens, int n, int want, bool waits = false) {
 	for (int i = 0; i < n; i++)
 		if (tokens[i] < 0 || tokens[i] >= m->vocab) return set_error(XALM_ERR_INVALID, "token %d out of range", tokens[i]);
 	const SeqStep st = {m->pos, n, m->prev_token};
+	if (n == 1 && waits && tune("seq_graph")) {
+		const int mode = want ? 1 : 0;
+		XALM_TRY(ensure_graph(m, mode, true));
+		*m->h_step = {st, tokens[0]};
+		XALM_CUDA_CHECK(cudaGraphLaunch(m->graph_io[mode], m->stream));
+		m->last_launches = m->graph_launches[mode]; // as counted at capture
+		m->pos++;
+		m->prev_token = tokens[0];
+		return XALM_OK;
+	}
 	XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_tokens, tokens, (size_t) n * 4, cudaMemcpyHostToDevice, m->stream));
 	XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_step, &st, sizeof st, cudaMemcpyHostToDevice, m->stream));
 	pdl_block(m->stream); // the pass's first kernel follows the copies
 	int nl = 0;
 	if (n == 1 && tune("seq_graph")) {
 		const int mode = want ? 1 : 0;
-		XALM_TRY(ensure_graph(m, mode));
+		XALM_TRY(ensure_graph(m, mode, false));
 		XALM_CUDA_CHECK(cudaGraphLaunch(m->graph[mode], m->stream));
 		nl = m->graph_launches[mode]; // as counted at capture
 	} else {
@@ -370,7 +397,8 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 		const int nc = std::min(m->chunk, n - at);
 		const bool last = at + nc == n;
 		const int w = want == 2 ? 2 : (want == 1 && last ? 1 : 0);
-		XALM_TRY(run_pass(m, tokens + at, nc, w));
+		const bool io = last && nc == 1 && !probs && tune("seq_graph"); // (every call ends with a wait, but only its last pass is the last to read h_step)
+		XALM_TRY(run_pass(m, tokens + at, nc, w, io));
 		if (!w) continue;
 		const int rows = w == 2 ? nc : 1;
 		const int good = probs ? std::max(0, std::min(nc, n_probs - at)) : 0;
@@ -380,7 +408,7 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 			m->last_launches++;
 		}
 		if (logits_host || !probs) {
-			XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_logits, m->logits, (size_t) rows * V * 4, cudaMemcpyDeviceToHost, m->stream));
+			if (!io) XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_logits, m->logits, (size_t) rows * V * 4, cudaMemcpyDeviceToHost, m->stream));
 			XALM_CUDA_CHECK(cudaStreamSynchronize(m->stream));
 			if (logits_host) memcpy(logits_host + (w == 2 ? (size_t) at * V : 0), m->h_logits, (size_t) rows * V * 4);
 		}
@@ -400,12 +428,15 @@ void seq_destroy(SeqModel* m) {
 	if (!m) return;
 	cudaSetDevice(m->device);
 	if (m->stream) cudaStreamSynchronize(m->stream);
-	for (int i = 0; i < 2; i++)
+	for (int i = 0; i < 2; i++) {
 		if (m->graph[i]) cudaGraphExecDestroy(m->graph[i]);
+		if (m->graph_io[i]) cudaGraphExecDestroy(m->graph_io[i]);
+	}
 	for (void* p : m->allocs) cudaFree(p);
 	tc_weight_free(&m->t_head);
 	if (m->h_logits) cudaFreeHost(m->h_logits);
 	if (m->h_probs) cudaFreeHost(m->h_probs);
+	if (m->h_step) cudaFreeHost(m->h_step);
 	if (m->own_stream) cudaStreamDestroy(m->own_stream);
 	if (m->side) cudaStreamDestroy(m->side);
 	if (m->ev_fork) cudaEventDestroy(m->ev_fork);
@@ -505,8 +536,11 @@ int seq_finalize(SeqModel* m) {
 	const size_t C = (size_t) m->chunk;
 	XALM_TRY(dev_alloc(m, &m->logits, C * m->vocab));
 	if (m->keep_layers) XALM_TRY(dev_alloc(m, &m->layer_sums, (size_t) m->n_layers * C * W, true));
-	XALM_TRY(dev_alloc(m, &m->d_tokens, C));
-	XALM_TRY(dev_alloc(m, &m->d_step, 1));
+	uint8_t* in = nullptr;
+	XALM_TRY(dev_alloc(m, &in, sizeof(SeqStep) + C * sizeof(int)));
+	m->d_step = reinterpret_cast<SeqStep*>(in);
+	m->d_tokens = reinterpret_cast<int*>(in + sizeof(SeqStep));
+	XALM_CUDA_CHECK(cudaMallocHost(&m->h_step, sizeof(StepIn)));
 	XALM_CUDA_CHECK(cudaMallocHost(&m->h_logits, C * m->vocab * 4));
 	XALM_TRY(dev_alloc(m, &m->d_targets, (size_t) m->max_tokens));
 	XALM_TRY(dev_alloc(m, &m->d_probs, (size_t) m->max_tokens));
