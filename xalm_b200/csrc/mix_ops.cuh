@@ -610,7 +610,8 @@ __global__ void __launch_bounds__(256) rows_stream_kernel(const float* __restric
 
 // ---- the same for a few tokens (5 to 31, too few for the tensor cores' tiles): TB of them share each read of the weights ---------------------------
 // Bound: memory up to about 10 tokens, FP32 FMAs above.  The 64 x 64 tiles of rows_gemm_kernel leave 9 tokens 1/7 of a tile and 32 CTAs for 2048
-// columns, and load one element at a time: 9 tokens of 2048 x 2048 took 161 us, here 9.
+// columns, and load one element at a time: the products of a 9-token pass at width 2048
+// took 161 us on average, here 13.
 // Every lane ends up with the sums of one (token of the first eight, column) and one (token of the second eight, column) pair.
 // v[k] of every lane -> lane k gets the sum over lanes of v[k]
 __device__ __forceinline__ float warp_sum_transposed32(float (&v)[32], int lane) {

@@ -386,7 +386,7 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 	if ((long long) pos0 + n > m->max_tokens) return set_error(XALM_ERR_INVALID, "step: positions [%d, %d) exceed max_tokens %d", pos0, pos0 + n, m->max_tokens);
 	const int V = m->vocab;
 	// Target probabilities are taken on the device, so that of n x vocab logits only n floats cross PCIe (2048 positions of 32000 logits: 4.6 ms of
-	// copies and 240 ms of one host thread's exponentials before, 0.09 ms now).  The logits themselves are copied when they are asked for.
+	// copies and 240 ms of one host thread's exponentials before, 0.06 ms now).  The logits themselves are copied when they are asked for.
 	const bool probs = targets && probs_host;
 	int n_probs = 0; // the rows before the first target that is out of range
 	if (probs) {
