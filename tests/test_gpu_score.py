@@ -1,4 +1,6 @@
 """Target probabilities of config.json families (prefill with targets): the device kernel against softmax in float64 over the same pass's logits."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -43,4 +45,23 @@ def test_a_target_out_of_range_is_refused_after_the_rows_before_it():
     with pytest.raises(capi.XalmError, match="target 100 out of range"):
         m.prefill(toks, 0, want_logits=2, targets=targets, fetch_logits=False)
     assert m.info("position") == n
+    m.close()
+
+
+@pytest.mark.parametrize("n,bad", [(75, 70), (75, 40), (40, 32), (110, 109)])
+@pytest.mark.parametrize("what", ["token", "target"])
+def test_a_failing_pass_leaves_the_probabilities_of_the_rows_before_it(n, bad, what):
+    """Passes of 32.  A token that is out of range fails before its pass, a target after the rows before it."""
+    rng = np.random.default_rng(n + bad)
+    m = small_model(100, 32, 128)
+    toks, targets = rng.integers(0, 100, n).astype(np.int32), rng.integers(0, 100, n).astype(np.int32)
+    want = m.prefill(toks, 0, want_logits=2, targets=targets, fetch_logits=False)[1]
+    m.release()
+    (toks if what == "token" else targets)[bad] = 100
+    got = np.full(n, -1, np.float32)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    assert capi.lib().xalm_cuda_prefill(m._h, p(toks), n, 0, 2, None, p(targets), p(got)) != 0
+    rows = bad // 32 * 32 if what == "token" else bad
+    assert np.array_equal(got[:rows], want[:rows]) and (got[rows:] == -1).all()
+    assert m.info("position") == (rows if what == "token" else min(n, bad // 32 * 32 + 32))
     m.close()

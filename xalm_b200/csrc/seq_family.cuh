@@ -100,6 +100,7 @@ struct SeqModel { // what a handle of these families points to (ModelHead first)
 	float* h_logits = nullptr; // pinned, chunk x vocab
 	int* d_targets = nullptr;  // max_tokens, as d_probs and h_probs (pinned): the target probabilities of one prefill call
 	float *d_probs = nullptr, *h_probs = nullptr;
+	cudaEvent_t ev_probs[2] = {nullptr, nullptr}; // h_probs holds a pass's probabilities; passes take turns
 	cudaStream_t stream = nullptr, own_stream = nullptr;
 	cudaStream_t side = nullptr; // for mixers of a layer that do not depend on one another
 	cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -393,12 +394,29 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 		while (n_probs < n && targets[n_probs] >= 0 && targets[n_probs] < V) n_probs++;
 		XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_targets, targets, (size_t) n * 4, cudaMemcpyHostToDevice, m->stream));
 	}
-	for (int at = 0; at < n; at += m->chunk) {
+	// A pass's probabilities reach the caller once the pass behind it is enqueued, so that the device does not wait for the host in between; when a later
+	// pass fails, the caller has those of the passes before it.
+	struct {
+		int at, n;
+	} sent[2] = {}; // the last two passes' probabilities, on their way to h_probs
+	auto hand_out = [&](int k) -> int {
+		if (!sent[k].n) return XALM_OK;
+		XALM_CUDA_CHECK(cudaEventSynchronize(m->ev_probs[k]));
+		memcpy(probs_host + sent[k].at, m->h_probs + sent[k].at, (size_t) sent[k].n * 4);
+		sent[k].n = 0;
+		return XALM_OK;
+	};
+	int k = 0; // this pass's entry of sent
+	for (int at = 0; at < n; at += m->chunk, k ^= 1) {
 		const int nc = std::min(m->chunk, n - at);
 		const bool last = at + nc == n;
 		const int w = want == 2 ? 2 : (want == 1 && last ? 1 : 0);
 		const bool io = last && nc == 1 && !probs && tune("seq_graph"); // (every call ends with a wait, but only its last pass is the last to read h_step)
-		XALM_TRY(run_pass(m, tokens + at, nc, w, io));
+		const int rc = run_pass(m, tokens + at, nc, w, io);
+		if (rc != XALM_OK) {
+			hand_out(k ^ 1);
+			return rc;
+		}
 		if (!w) continue;
 		const int rows = w == 2 ? nc : 1;
 		const int good = probs ? std::max(0, std::min(nc, n_probs - at)) : 0;
@@ -406,19 +424,24 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 			target_prob_kernel<<<good, TARGET_PROB_THREADS, 0, m->stream>>>(m->logits, V, -INFINITY, m->d_targets + at, m->d_probs + at);
 			XALM_TRY(launch_check("target_prob"));
 			m->last_launches++;
+			XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_probs + at, m->d_probs + at, (size_t) good * 4, cudaMemcpyDeviceToHost, m->stream));
+			XALM_CUDA_CHECK(cudaEventRecord(m->ev_probs[k], m->stream));
+			sent[k].at = at;
+			sent[k].n = good;
 		}
 		if (logits_host || !probs) {
 			if (!io) XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_logits, m->logits, (size_t) rows * V * 4, cudaMemcpyDeviceToHost, m->stream));
 			XALM_CUDA_CHECK(cudaStreamSynchronize(m->stream));
 			if (logits_host) memcpy(logits_host + (w == 2 ? (size_t) at * V : 0), m->h_logits, (size_t) rows * V * 4);
 		}
-		if (probs && (last || good < nc)) {
-			XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_probs, m->d_probs, (size_t) n_probs * 4, cudaMemcpyDeviceToHost, m->stream));
+		XALM_TRY(hand_out(k ^ 1));
+		if (probs && good < nc) {
+			XALM_TRY(hand_out(k));
 			XALM_CUDA_CHECK(cudaStreamSynchronize(m->stream));
-			memcpy(probs_host, m->h_probs, (size_t) n_probs * 4);
-			if (good < nc) return set_error(XALM_ERR_INVALID, "step: target %d out of range", targets[n_probs]);
+			return set_error(XALM_ERR_INVALID, "step: target %d out of range", targets[n_probs]);
 		}
 	}
+	XALM_TRY(hand_out(k ^ 1));
 	XALM_CUDA_CHECK(cudaStreamSynchronize(m->stream));
 	return XALM_OK;
 }
@@ -441,6 +464,8 @@ void seq_destroy(SeqModel* m) {
 	if (m->side) cudaStreamDestroy(m->side);
 	if (m->ev_fork) cudaEventDestroy(m->ev_fork);
 	if (m->ev_join) cudaEventDestroy(m->ev_join);
+	for (cudaEvent_t e : m->ev_probs)
+		if (e) cudaEventDestroy(e);
 	m->hooks->destroy(m);
 }
 
@@ -466,6 +491,8 @@ int seq_create(const ModelFamily* family, const SeqHooks* hooks, const char* jso
 	if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking);
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming);
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming);
+	for (cudaEvent_t& ev : m->ev_probs)
+		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
 	if (e != cudaSuccess) { delete mm; return set_error(XALM_ERR_CUDA, "cudaStreamCreate failed: %s", cudaGetErrorString(e)); }
 	m->stream = m->own_stream;
 	*out = reinterpret_cast<xalm_cuda_model*>(m);
