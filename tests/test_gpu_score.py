@@ -65,3 +65,19 @@ def test_a_failing_pass_leaves_the_probabilities_of_the_rows_before_it(n, bad, w
     assert np.array_equal(got[:rows], want[:rows]) and (got[rows:] == -1).all()
     assert m.info("position") == (rows if what == "token" else min(n, bad // 32 * 32 + 32))
     m.close()
+
+
+def test_the_limit_of_positions_costs_no_memory_where_the_caches_are_windowed():
+    """A pass's probabilities need room for a pass.  Entries for every position up to the limit would be 1 GB on the device and 0.5 GB of pinned memory here."""
+    import torch
+
+    cfg = O.make_config(vocab=100, width=64, layers=[O.attention_layer(4, 2, 16, 16, window=32, mlp=O.dense(64))], groups=2)
+    free = []
+    for limit in (96, 96, 1 << 27):  # the first one loads the library's kernels
+        m = Model.from_json(cfg, O.random_weights(cfg, 1)).cuda(max_tokens=limit)
+        free.append(torch.cuda.mem_get_info()[0])
+        toks = np.arange(80) % 100
+        got = m.prefill(toks, 0, want_logits=2, targets=toks, fetch_logits=False)[1]
+        assert ((got > 0) & (got < 1)).all()
+        m.close()
+    assert free[1] - free[2] < 64 << 20

@@ -98,9 +98,9 @@ struct SeqModel { // what a handle of these families points to (ModelHead first)
 	int* d_tokens = nullptr;
 	StepIn* h_step = nullptr;  // pinned: what a one-token step's graph copies there
 	float* h_logits = nullptr; // pinned, chunk x vocab
-	int* d_targets = nullptr;  // max_tokens, as d_probs and h_probs (pinned): the target probabilities of one prefill call
-	float *d_probs = nullptr, *h_probs = nullptr;
-	cudaEvent_t ev_probs[2] = {nullptr, nullptr}; // h_probs holds a pass's probabilities; passes take turns
+	int* d_targets = nullptr;  // chunk, as d_probs: a pass's target probabilities
+	float *d_probs = nullptr, *h_probs = nullptr; // h_probs: pinned, two passes'
+	cudaEvent_t ev_probs[2] = {nullptr, nullptr}; // a half of h_probs holds its pass's probabilities
 	cudaStream_t stream = nullptr, own_stream = nullptr;
 	cudaStream_t side = nullptr; // for mixers of a layer that do not depend on one another
 	cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -390,19 +390,17 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 	// copies and 240 ms of one host thread's exponentials before, 0.06 ms now).  The logits themselves are copied when they are asked for.
 	const bool probs = targets && probs_host;
 	int n_probs = 0; // the rows before the first target that is out of range
-	if (probs) {
+	if (probs)
 		while (n_probs < n && targets[n_probs] >= 0 && targets[n_probs] < V) n_probs++;
-		XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_targets, targets, (size_t) n * 4, cudaMemcpyHostToDevice, m->stream));
-	}
 	// A pass's probabilities reach the caller once the pass behind it is enqueued, so that the device does not wait for the host in between; when a later
 	// pass fails, the caller has those of the passes before it.
 	struct {
 		int at, n;
-	} sent[2] = {}; // the last two passes' probabilities, on their way to h_probs
+	} sent[2] = {}; // the last two passes' probabilities, each on its way to its half of h_probs
 	auto hand_out = [&](int k) -> int {
 		if (!sent[k].n) return XALM_OK;
 		XALM_CUDA_CHECK(cudaEventSynchronize(m->ev_probs[k]));
-		memcpy(probs_host + sent[k].at, m->h_probs + sent[k].at, (size_t) sent[k].n * 4);
+		memcpy(probs_host + sent[k].at, m->h_probs + (size_t) k * m->chunk, (size_t) sent[k].n * 4);
 		sent[k].n = 0;
 		return XALM_OK;
 	};
@@ -421,10 +419,11 @@ int seq_step(SeqModel* m, const int* tokens, int n, int pos0, int want, float* l
 		const int rows = w == 2 ? nc : 1;
 		const int good = probs ? std::max(0, std::min(nc, n_probs - at)) : 0;
 		if (good) {
-			target_prob_kernel<<<good, TARGET_PROB_THREADS, 0, m->stream>>>(m->logits, V, -INFINITY, m->d_targets + at, m->d_probs + at);
+			XALM_CUDA_CHECK(cudaMemcpyAsync(m->d_targets, targets + at, (size_t) good * 4, cudaMemcpyHostToDevice, m->stream));
+			target_prob_kernel<<<good, TARGET_PROB_THREADS, 0, m->stream>>>(m->logits, V, -INFINITY, m->d_targets, m->d_probs);
 			XALM_TRY(launch_check("target_prob"));
 			m->last_launches++;
-			XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_probs + at, m->d_probs + at, (size_t) good * 4, cudaMemcpyDeviceToHost, m->stream));
+			XALM_CUDA_CHECK(cudaMemcpyAsync(m->h_probs + (size_t) k * m->chunk, m->d_probs, (size_t) good * 4, cudaMemcpyDeviceToHost, m->stream));
 			XALM_CUDA_CHECK(cudaEventRecord(m->ev_probs[k], m->stream));
 			sent[k].at = at;
 			sent[k].n = good;
@@ -569,9 +568,9 @@ int seq_finalize(SeqModel* m) {
 	m->d_tokens = reinterpret_cast<int*>(in + sizeof(SeqStep));
 	XALM_CUDA_CHECK(cudaMallocHost(&m->h_step, sizeof(StepIn)));
 	XALM_CUDA_CHECK(cudaMallocHost(&m->h_logits, C * m->vocab * 4));
-	XALM_TRY(dev_alloc(m, &m->d_targets, (size_t) m->max_tokens));
-	XALM_TRY(dev_alloc(m, &m->d_probs, (size_t) m->max_tokens));
-	XALM_CUDA_CHECK(cudaMallocHost(&m->h_probs, (size_t) m->max_tokens * 4));
+	XALM_TRY(dev_alloc(m, &m->d_targets, C));
+	XALM_TRY(dev_alloc(m, &m->d_probs, C));
+	XALM_CUDA_CHECK(cudaMallocHost(&m->h_probs, 2 * C * 4));
 	for (auto& [name, t] : m->tensors) std::vector<float>().swap(t.v); // the device owns the weights from here on
 	m->finalized = true;
 	return XALM_OK;
