@@ -67,6 +67,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 // The head of a kernel of a one-token step: its inputs are complete from here on, and the next kernel may take its place on the SMs.  In this order only
 // one kernel is ahead of the running one: with the other, a whole chain of waiting products took the SMs from the step's other branch.
+// Such a kernel is alive while the one before it still writes its inputs: what a step computes is therefore no __restrict__ parameter of it (the compiler
+// may then read it through the non-coherent path, or ahead of the wait); weights are.
 __device__ __forceinline__ void pdl_enter() {
 	pdl_wait();
 	pdl_launch_dependents();

@@ -91,8 +91,8 @@ static inline int step_parts(int rows, int width) { return rows > 4 ? 1 : std::m
 // ---- embedding -> streams -------------------------------------------------------------------------------------------------
 // positions: (max positions, width) learned rows, the one of the token's position in its sequence is added (unscaled); NULL: none
 template <typename WT>
-__global__ void embed_streams_kernel(const WT* __restrict__ table, const int* __restrict__ tokens, int width, int S, size_t stream_stride,
-                                     float* __restrict__ xs, float scale = 1.f, const WT* __restrict__ positions = nullptr, const SeqStep* step = nullptr) {
+__global__ void embed_streams_kernel(const WT* __restrict__ table, const int* tokens, int width, int S, size_t stream_stride, float* xs,
+                                     float scale = 1.f, const WT* __restrict__ positions = nullptr, const SeqStep* step = nullptr) {
 	pdl_enter();
 	const int t = blockIdx.x;
 	const WT* row = table + (size_t) tokens[t] * width;
@@ -162,8 +162,8 @@ __global__ void embed_pair_kernel(EmbedPairArgs a) {
 // `sum_out` (optional) receives the un-normed combination (the residual stream as a reader outside the model sees it).
 // SS: the most streams this instance takes (its loops are unrolled to SS: the code of a one-CTA launch should be short to fetch)
 template <int SS>
-__global__ void hc_norm_kernel(const float* __restrict__ xs, int S, size_t stream_stride, const float* __restrict__ a, const float* __restrict__ w,
-                               int one_plus, float eps, int width, float* __restrict__ h, float* __restrict__ sum_out) {
+__global__ void hc_norm_kernel(const float* xs, int S, size_t stream_stride, const float* __restrict__ a, const float* __restrict__ w, int one_plus,
+                               float eps, int width, float* h, float* sum_out) {
 	extern __shared__ float sm[];
 	float* u = sm;            // width
 	float* red = sm + width;  // 33
@@ -223,8 +223,7 @@ __global__ void hc_norm_kernel(const float* __restrict__ xs, int S, size_t strea
 // ---- layer norm ------------------------------------------------------------------------------------------------------------------
 // h[t] = (x[t] - mean) / sqrt(mean of the squared deviations + eps) * w + b (b NULL: no bias).  One CTA per row; the row stays in shared memory
 // between the two sums, so the deviations are taken from the finished mean.  Loads four columns per thread ahead, as hc_norm_kernel.
-static __global__ void layer_norm_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, const float* __restrict__ b, float eps, int width,
-                                         float* __restrict__ h) {
+static __global__ void layer_norm_kernel(const float* x, int ldx, const float* __restrict__ w, const float* __restrict__ b, float eps, int width, float* h) {
 	pdl_enter();
 	extern __shared__ float sm[];
 	float* u = sm;            // width
@@ -593,7 +592,7 @@ static inline int rows_stream_ks(int N, int K, int batch) {
 	return ks;
 }
 template <int KS>
-__global__ void __launch_bounds__(256) rows_stream_kernel(const float* __restrict__ A, const __nv_bfloat16* __restrict__ W, int N, int K, RowsEpi e) {
+__global__ void __launch_bounds__(256) rows_stream_kernel(const float* A, const __nv_bfloat16* __restrict__ W, int N, int K, RowsEpi e) {
 	__shared__ float red[8][RS_COLS];
 	if (blockIdx.z) { // one product of a batch
 		A += (size_t) blockIdx.z * e.batch_a;
@@ -1633,7 +1632,7 @@ struct NextRead {
 	float* h = nullptr;       // (T, width), NULL: nothing rides along
 };
 template <int SS>
-__global__ void dual_norm_hc_kernel(const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ wa, const float* __restrict__ wb,
+__global__ void dual_norm_hc_kernel(const float* A, const float* B, const float* __restrict__ wa, const float* __restrict__ wb,
                                     float eps, int width, RowsEpi e, NextRead next) {
 	pdl_enter();
 	extern __shared__ float sm[];

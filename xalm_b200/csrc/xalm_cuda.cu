@@ -460,8 +460,7 @@ static int launch_matvec(MatvecArgs a, cudaStream_t s, bool pdl) {
 // small kernels
 // ---------------------------------------------------------------------------------------------------------
 // _copy_embedding (infer.cpp:553-602) from the ON-DISK layout of the table (block formats: extension)
-__global__ void embed_kernel(int type, const uint8_t* __restrict__ table, size_t row_bytes, int dim, const StepParams* step,
-                             float* __restrict__ x) {
+__global__ void embed_kernel(int type, const uint8_t* __restrict__ table, size_t row_bytes, int dim, const StepParams* step, float* x) {
 	pdl_launch_dependents();
 	pdl_wait();
 	const uint8_t* row = table + (size_t) step->token * row_bytes;
@@ -507,7 +506,7 @@ __global__ void argmax_kernel(const float* __restrict__ logits, int n, int* __re
 	}
 }
 
-__global__ void residual_add_kernel(float* __restrict__ x, const float* __restrict__ y, int n) {
+__global__ void residual_add_kernel(float* x, const float* y, int n) {
 	pdl_launch_dependents();
 	pdl_wait();
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] += y[i];
@@ -526,7 +525,7 @@ struct PeerArgs {
 	int rank, size, stride;
 	uint2* recv[8];          // per rank: its receive area [2 slots][8 source ranks][dim] of {value, tag} words (fused exchange, matvec_tma.cuh)
 };
-__global__ void peer_allreduce_residual_kernel(const PeerArgs pa, float* __restrict__ x, int n, int idx, const StepParams* step) {
+__global__ void peer_allreduce_residual_kernel(const PeerArgs pa, float* x, int n, int idx, const StepParams* step) {
 	pdl_launch_dependents();
 	pdl_wait();
 	const int slot = idx & 1;
@@ -562,7 +561,7 @@ __global__ void peer_allreduce_residual_kernel(const PeerArgs pa, float* __restr
 // must still be CONSUMED before this rank moves on — the two-slot scheme is only safe while every rank executes
 // push(i), recv(i), push(i+1), ... (tests/test_tp_exchange_protocol.py shows the overwrite / deadlock without this).  One CTA polls
 // the tags of all P partials of that exchange and discards the values.
-__global__ void tp_drain_kernel(const uint2* __restrict__ recv, int n_ranks, int dim, int idx, const StepParams* step, unsigned int* err_flag) {
+__global__ void tp_drain_kernel(const uint2* recv, int n_ranks, int dim, int idx, const StepParams* step, unsigned int* err_flag) {
 	pdl_launch_dependents();
 	pdl_wait();
 	const unsigned int seq = step->ar_base + (unsigned int) idx + 1u;
