@@ -60,3 +60,14 @@ def test_group_norm_of_short_steps(W, groups, T):
     got, avg = capi.group_norm_residual(y, w, groups, 1e-5, x_in=x, part_w=pw, hist=hist, dwa=coef)
     assert np.abs(got - want).max() < 2e-5  # a dozen fp32 roundings of values below 8
     assert np.abs(avg - ((coef[:-1, None, None] * hist).sum(0) + coef[-1] * want)).max() < 6e-5
+
+
+@pytest.mark.parametrize("N", [1000, 4720, 4721, 9001])
+@pytest.mark.parametrize("K", [1, 9, 511, 1030])
+def test_one_token_of_rows_that_are_not_whole_pieces(N, K):
+    """K in slices below 4721 columns (from 512 on); the one-token instance for the others."""
+    rng = np.random.default_rng(N + K)
+    x, w = rng.standard_normal((1, K)).astype(np.float32), bf16(rng.standard_normal((N, K)) / K ** 0.5)
+    got = capi.rows_act(x, w, act=0, w_bf16=True)
+    z = x.astype(np.float64) @ w.T
+    assert np.abs(got - z).max() < 2 * bound(K)
