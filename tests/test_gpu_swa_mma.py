@@ -3,8 +3,10 @@ keys around the tiles, every mask and term of the score, and its error beside th
 import numpy as np
 import pytest
 
+import bolovik_oracle as O
 from test_gpu_swa_one import bf16, inputs, reference
 from xalm_b200 import capi
+from xalm_b200.model import Model
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +49,56 @@ def test_no_further_from_float64_than_fp32_sums():
     want = reference(q, k, v, pos0, H, G, 10 ** 6, scale=d ** -0.5)
     err = [np.linalg.norm(capi.swa_attention(q, k, v, pos0, H, G, d, d, 10 ** 6, d ** -0.5, cache_bf16=c) - want) / np.linalg.norm(want) for c in (True, False)]
     assert err[0] <= err[1]
+
+
+@pytest.mark.parametrize("T,pos0", [(16, 0), (16, 1040), (32, 330), (45, 63), (64, 512), (100, 29), (130, 700)])
+@pytest.mark.parametrize("n_splits", [2, 5, 16])
+def test_keys_split_over_several_ctas(T, pos0, n_splits):
+    """Splits of whole key blocks: fewer blocks than splits, one block each, several each; every term that is applied where the splits are joined."""
+    H, G, d, dv, rng = 4, 2, 40, 64, np.random.default_rng(T + pos0)
+    q, k, v = inputs(T, pos0 + T, H, G, d, dv, T + pos0)
+    sink, slope = rng.uniform(0.1, 1, H).astype(np.float32), rng.uniform(0.01, 0.1, H).astype(np.float32)
+    wide, heads = rng.standard_normal((T, H * dv)).astype(np.float32), rng.standard_normal((T, H)).astype(np.float32)
+    kw = dict(n_splits=n_splits, cache_bf16=True)
+    for window in (10 ** 6, 90):
+        want = reference(q, k, v, pos0, H, G, window, scale=0.2, softcap=5.0, gate=wide)
+        assert np.abs(capi.swa_attention(q, k, v, pos0, H, G, d, dv, window, 0.2, softcap=5.0, gate=wide, **kw) - want).max() < TOL
+    want = reference(q, k, v, pos0, H, G, 10 ** 6, scale=0.2, slope=slope, sink=sink, gate=heads)
+    assert np.abs(capi.biased_attention(q, k, v, pos0, H, G, d, dv, 0.2, slope=slope, sink=sink, gate=heads, **kw) - want).max() < TOL
+    want = reference(q, k, v, pos0, H, G, 50, keep=9, scale=0.2)
+    assert np.abs(capi.swa_attention_kept(q, k, v, pos0, H, G, d, dv, 50, 9, 0.2, **kw) - want).max() < TOL
+    want = reference(q, k, v, pos0, H, G, 10 ** 6, chunk=64, scale=0.2)
+    assert np.abs(capi.chunked_attention(q, k, v, pos0, H, G, d, dv, 64, 0.2, **kw) - want).max() < TOL
+
+
+@pytest.mark.parametrize("T", [16, 33, 64])
+@pytest.mark.parametrize("n_splits", [1, 4])
+def test_a_ring_that_has_wrapped(T, n_splits):
+    """The window's keys lie around the ring's end, behind slots of first positions that stay."""
+    H, G, d, pos0, window = 2, 1, 64, 1000, 150
+    q, k, v = inputs(T, pos0 + T, H, G, d, d, T)
+    for ring in (window - 1 + T, 257):
+        got = capi.swa_attention(q, k, v, pos0, H, G, d, d, window, 0.2, ring=ring, n_splits=n_splits, cache_bf16=True)
+        assert np.abs(got - reference(q, k, v, pos0, H, G, window, scale=0.2)).max() < TOL
+        got = capi.swa_attention_kept(q, k, v, pos0, H, G, d, d, window, 7, 0.2, ring=ring, n_splits=n_splits, cache_bf16=True)
+        assert np.abs(got - reference(q, k, v, pos0, H, G, window, keep=7, scale=0.2)).max() < TOL
+
+
+def test_splits_are_split():
+    """The sums of three splits, joined, are not those of one walk over the keys."""
+    q, k, v = inputs(40, 640, 4, 2, 64, 64, 5)
+    got = [capi.swa_attention(q, k, v, 600, 4, 2, 64, 64, 10 ** 6, 0.125, n_splits=s, cache_bf16=True) for s in (1, 3)]
+    assert not np.array_equal(*got) and np.abs(got[0] - got[1]).max() < TOL
+
+
+@pytest.mark.parametrize("limit,joins", [(64, 0), (100, 0), (128, 1), (4096, 1)])
+def test_a_short_pass_over_a_long_cache_splits_the_keys(limit, joins):
+    """8 CTAs of queries and heads, and a cache of `limit` slots: from two key blocks on the pass has a join's kernel."""
+    cfg = O.make_config(vocab=50, width=64, layers=[O.attention_layer(8, 2, 32, 32, mlp=O.dense(64))], groups=2)
+    count = []
+    for n in (64, limit):
+        m = Model.from_json(cfg, O.random_weights(cfg, 1), "BF16").cuda(max_tokens=n)
+        m.prefill(np.arange(20), 0, want_logits=0)
+        count.append(m.last_launch_count())
+        m.close()
+    assert count[1] == count[0] + joins

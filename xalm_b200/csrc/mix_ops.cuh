@@ -2255,11 +2255,30 @@ static inline bool swa_one_ok(const SwaArgs& a, int rows) {
 }
 
 // swa_mma.cu: passes of many tokens over a bf16 cache, on the tensor cores.  It takes heads of 32 to 128 channels in whole 16-byte pieces whose scores
-// do not mix, and fills a warp's 16 queries; smaller heads would be mostly padding.
+// do not mix, and fills a warp's 16 queries; smaller heads would be mostly padding.  Takes a.n_splits > 0
 int launch_swa_mma(const SwaArgs& a, int rows, cudaStream_t s);
+constexpr int SWA_MMA_ROWS = 64, SWA_MMA_KEYS = 64; // queries of one head per CTA; keys per step
 static inline bool swa_mma_ok(const SwaArgs& a, int rows, bool cache_f32) {
 	return !cache_f32 && rows >= 16 && !a.talk && std::min(a.d, a.dv) >= 32 && std::max(a.d, a.dv) <= 128 && ((a.d | a.dv | a.ldk | a.ldv) & 7) == 0 &&
 	       ((a.ldq | a.q_off) & 3) == 0 && a.H <= 65535 && ((reinterpret_cast<uintptr_t>(a.kc) | reinterpret_cast<uintptr_t>(a.vc) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
+}
+
+// Splits of the keys for the kernel above.  A CTA walks its keys at 2.4 (64 channels) to 4.2 us (128) per 64, so that a short pass over a long cache needs
+// more CTAs than its queries and heads give: up to two per SM, each with keys for a step.  Times with the best of 1 to 32 splits (the join's kernel
+// included), one split, and the tiled kernel as it would be launched: 16 tokens of 8 heads of 128 over 4096 keys 32, 342, 271 us; 64 tokens 42, 345, 252;
+// 64 tokens of 32 heads over 1024 keys 38, 132, 277; over 32768 416, -, 5689.  128 tokens of 32 heads (64 CTAs): four splits against one 54 : 129 us over
+// 1024 keys, 128 : 332 over 4096; 256 tokens (128 CTAs): two against one 88 : 122, 234 : 327.
+static inline int swa_mma_splits(const SwaArgs& a, int rows) {
+	if (!a.part_o || !a.part_ml) return 1;
+	const long long ctas = (long long) (rows + SWA_MMA_ROWS - 1) / SWA_MMA_ROWS * a.H;
+	long long reach = a.window < 0x7fffffff ? a.window : a.ring;
+	if (a.mask_chunk > 0) reach = std::min<long long>(reach, a.mask_chunk);
+	const long long keys = std::min<long long>(a.ring, reach + std::min(rows, SWA_MMA_ROWS)) + a.keep_first; // what a CTA's queries see at most
+	return (int) std::max<long long>(1, std::min({296 / ctas, keys / SWA_MMA_KEYS, (long long) a.part_cap / rows}));
+}
+static inline int launch_swa_merge(const SwaArgs& a, int rows, cudaStream_t s) {
+	launch_step(swa_merge_kernel, dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s, rows, a);
+	return launch_check("swa_merge");
 }
 
 // rows: tokens of the step; cache_f32: element type of the ring.  With n_splits > 1 the merge kernel follows.  Returns the number of
@@ -2296,8 +2315,10 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 		}
 	}
 	if (swa_mma_ok(a, rows, cache_f32)) {
-		if (launches) *launches = 1;
-		return launch_swa_mma(a, rows, s);
+		if (a.n_splits <= 0) a.n_splits = swa_mma_splits(a, rows);
+		if (launches) *launches = a.n_splits > 1 ? 2 : 1;
+		XALM_TRY(launch_swa_mma(a, rows, s));
+		return a.n_splits > 1 ? launch_swa_merge(a, rows, s) : XALM_OK;
 	}
 	const int tq = swa_pick_tq(a.H, a.G, a.d, a.dv, rows);
 	if (swa_one_ok(a, rows)) {
@@ -2309,11 +2330,7 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 		}
 		if (launches) *launches = a.n_splits > 1 ? 2 : 1;
 		XALM_TRY(launch_swa_one(a, rows, cache_f32, s));
-		if (a.n_splits > 1) {
-			launch_step(swa_merge_kernel, dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s, rows, a);
-			XALM_TRY(launch_check("swa_merge"));
-		}
-		return XALM_OK;
+		return a.n_splits > 1 ? launch_swa_merge(a, rows, s) : XALM_OK;
 	}
 	if (a.n_splits <= 0) { // enough CTAs for two waves, at least two key blocks each
 		const int qblocks = tq ? (rows + tq - 1) / tq : rows;
@@ -2351,11 +2368,7 @@ static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s
 		else swa_attn_kernel<__nv_bfloat16><<<dim3(rows, a.n_splits), 256, smem, s>>>(a);
 	}
 	XALM_TRY(launch_check("swa_attn"));
-	if (a.n_splits > 1 && !a.tickets) {
-		launch_step(swa_merge_kernel, dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s, rows, a);
-		XALM_TRY(launch_check("swa_merge"));
-	}
-	return XALM_OK;
+	return a.n_splits > 1 && !a.tickets ? launch_swa_merge(a, rows, s) : XALM_OK;
 }
 
 // max_rows: an upper bound of the step's tokens known on the host.  The cluster kernel takes d <= 256 and dv <= 1024; anything else

@@ -5,8 +5,9 @@
 // holds, so that every product is exact and only the fp32 sums round.  The tensor cores sum 16 products (of the small planes first) from zero; sums of more
 // are added in round-to-nearest, since the tensor cores' own additions truncate: chained over a head's channels and a key block, the result was
 // twice as far from float64 as the fp32 FMA kernel's.
-// A CTA takes 16 queries of one head per warp; 64 keys and their values at a time come through a two-deep cp.async ring; queries stay in shared memory
-// as planes, scores, probabilities and output in registers (m16n8k16 fragments).
+// A CTA takes 16 queries of one head per warp and, where few CTAs would run (swa_mma_splits), a share of the keys, whose parts swa_merge_kernel joins;
+// 64 keys and their values at a time come through a two-deep cp.async ring; queries stay in shared memory as planes, scores, probabilities and output in
+// registers (m16n8k16 fragments).
 // Bound: the instructions around the products (splits, exponentials, adds: about half) and the mma.sync pipe, three products per one.  Against the fp32
 // FMA tiles of mix_ops.cuh: 1024 tokens of 16 heads of 128 over up to 2048 keys 1626 -> 200 us, of 8 heads in a window of 512 286 -> 94 us; 256 tokens
 // of 8 heads over up to 301 keys 105 -> 83 us (32 CTAs).  Distance from float64 at 128 channels and 1500 keys: 2.6e-7, the FMA kernel 4.4e-7.
@@ -18,7 +19,7 @@
 namespace xalm {
 namespace mix {
 
-constexpr int SMM_KEYS = 64, SMM_STAGES = 2;
+constexpr int SMM_KEYS = SWA_MMA_KEYS, SMM_STAGES = 2;
 
 __device__ __forceinline__ void smm_ldsm4(uint32_t (&r)[4], uint32_t addr) {
 	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -67,6 +68,8 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 	const int i_lo = pos0 + t0, i_hi = i_lo + nq - 1;
 	const SwaKeys km = swa_keys(a, i_lo);
 	const int nk = km.ks + i_hi - km.j_first + 1;
+	const int per = ((nk + a.n_splits - 1) / a.n_splits + SMM_KEYS - 1) / SMM_KEYS * SMM_KEYS, sp = blockIdx.z; // whole key blocks for every split but the last
+	const int jb = min(nk, sp * per), je = min(nk, jb + per);
 	const int ldk = a.ldk ? a.ldk : G * d, ldv = a.ldv ? a.ldv : G * dv;
 	const __nv_bfloat16* kc = reinterpret_cast<const __nv_bfloat16*>(a.kc) + (size_t) g * d;
 	const __nv_bfloat16* vc = reinterpret_cast<const __nv_bfloat16*>(a.vc) + (size_t) g * dv;
@@ -75,8 +78,8 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 		const uint32_t kb = smem_u32(ks) + (uint32_t) buf * SMM_KEYS * DQ * 2, vb = smem_u32(vs) + (uint32_t) buf * SMM_KEYS * DV * 2;
 		// PER threads share a key, whose slot is worked out once, and take alternate 16-byte pieces; size 0 writes zeros (beyond the last key or channel)
 		constexpr int PER = NTH / SMM_KEYS;
-		const int row = tid / PER, j = min(j0 + row, nk - 1), first = tid % PER;
-		const bool in = j0 + row < nk;
+		const int row = tid / PER, j = min(j0 + row, je - 1), first = tid % PER;
+		const bool in = j0 + row < je;
 		const size_t slot = km.slot(j);
 		if (first == 0) kp[buf * SMM_KEYS + row] = in ? km.pos(j) : 0x7fffffff;
 		const __nv_bfloat16 *kr = kc + slot * ldk, *vr = vc + slot * ldv;
@@ -92,7 +95,7 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 		}
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
-	stage(0, 0);
+	if (jb < je) stage(jb, 0);
 	// queries, as planes
 	for (int x = tid; x < ROWS * (DQ / 8); x += NTH) {
 		const int row = x / (DQ / 8), p = x % (DQ / 8);
@@ -108,10 +111,10 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 	float o[DV / 8][4] = {}, m[2] = {-INFINITY, -INFINITY}, l[2] = {};
 	const int r0 = warp * 16 + quad; // this thread's rows: r0 and r0 + 8 of the CTA's
 	const float slope = a.slope ? a.slope[h] : 0.f, b1 = a.r1 ? a.r1[h] : 0.f, b2 = a.r1 ? a.r2[h] : 0.f;
-	const int blocks = (nk + SMM_KEYS - 1) / SMM_KEYS;
+	const int blocks = (je - jb + SMM_KEYS - 1) / SMM_KEYS;
 	const bool plain = !(a.softcap > 0.f) && !a.r1 && !a.slope, one_run = a.mask_chunk <= 0 || i_lo / a.mask_chunk == i_hi / a.mask_chunk;
 	for (int blk = 0; blk < blocks; blk++) {
-		const int buf = blk % SMM_STAGES, j0 = blk * SMM_KEYS;
+		const int buf = blk % SMM_STAGES, j0 = jb + blk * SMM_KEYS;
 		if (blk + 1 < blocks) {
 			stage(j0 + SMM_KEYS, (blk + 1) % SMM_STAGES);
 			asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -144,8 +147,8 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 		// ---- scale, soft cap, biases, mask ----
 		const int* pos = kp + buf * SMM_KEYS;
 		float top[2] = {m[0], m[1]};
-		const int p_lo = km.pos(j0), p_hi = km.pos(min(j0 + SMM_KEYS, nk) - 1);
-		if (plain && j0 + SMM_KEYS <= nk && p_hi <= i_lo && (a.window >= 0x7fffffff || i_hi - p_lo < a.window || p_hi < a.keep_first) && one_run) {
+		const int p_lo = km.pos(j0), p_hi = km.pos(min(j0 + SMM_KEYS, je) - 1);
+		if (plain && j0 + SMM_KEYS <= je && p_hi <= i_lo && (a.window >= 0x7fffffff || i_hi - p_lo < a.window || p_hi < a.keep_first) && one_run) {
 			// every query sees every key of the block, and the score is only scaled
 #pragma unroll
 			for (int c = 0; c < SMM_KEYS / 8; c++)
@@ -222,15 +225,24 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
 		const int t = t0 + r0 + r * 8;
 		if (r0 + r * 8 >= nq) continue;
-		float* dst = a.out + (size_t) t * (a.ldo ? a.ldo : H * dv) + (size_t) h * dv;
+		const bool parts = a.n_splits > 1; // swa_merge_kernel joins them
+		float* dst = parts ? a.part_o + ((size_t) t * a.n_splits + sp) * (H * dv) + (size_t) h * dv : a.out + (size_t) t * (a.ldo ? a.ldo : H * dv) + (size_t) h * dv;
+		if (parts && ql == 0) {
+			float* pml = a.part_ml + ((size_t) t * a.n_splits + sp) * (H * 2) + 2 * h;
+			pml[0] = m[r];
+			pml[1] = l[r];
+		}
 #pragma unroll
 		for (int c = 0; c < DV / 8; c++)
 #pragma unroll
 			for (int e = 0; e < 2; e++) {
 				const int col = c * 8 + ql * 2 + e;
 				if (col >= dv) continue;
-				float v = swa_finish(a, h, o[c][2 * r + e], l[r], m[r]);
-				if (a.gate) v *= swa_gate(a, t, h, col);
+				float v = o[c][2 * r + e];
+				if (!parts) {
+					v = swa_finish(a, h, v, l[r], m[r]);
+					if (a.gate) v *= swa_gate(a, t, h, col);
+				}
 				dst[col] = v;
 			}
 	}
@@ -238,9 +250,10 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 
 template <int DQ, int DV>
 static int launch_swa_mma_inst(const SwaArgs& a, int rows, cudaStream_t s) {
-	constexpr int WARPS = 4; // two per CTA, for twice the CTAs, copied every key block for half the queries and were slower
+	// Fewer warps per CTA for passes of 16 and 32 tokens, and two for twice the CTAs, copied every key block for fewer queries and were slower
+	constexpr int WARPS = SWA_MMA_ROWS / 16;
 	XALM_CUDA_CHECK(cudaFuncSetAttribute(swa_mma_kernel<DQ, DV, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smm_smem(DQ, DV, WARPS)));
-	swa_mma_kernel<DQ, DV, WARPS><<<dim3((rows + WARPS * 16 - 1) / (WARPS * 16), a.H), WARPS * 32, smm_smem(DQ, DV, WARPS), s>>>(a);
+	swa_mma_kernel<DQ, DV, WARPS><<<dim3((rows + WARPS * 16 - 1) / (WARPS * 16), a.H, a.n_splits), WARPS * 32, smm_smem(DQ, DV, WARPS), s>>>(a);
 	return launch_check("swa_mma");
 }
 
