@@ -102,3 +102,26 @@ def test_a_short_pass_over_a_long_cache_splits_the_keys(limit, joins):
         count.append(m.last_launch_count())
         m.close()
     assert count[1] == count[0] + joins
+
+
+@pytest.mark.parametrize("T,pos0,n_splits", [(64, 0, 1), (64, 0, 2), (100, 30, 1), (20, 200, 3)])
+@pytest.mark.parametrize("what", ["v inf", "v nan", "k inf", "q inf"])
+def test_infinities_and_nan_stay_with_the_queries_that_see_them(T, pos0, n_splits, what):
+    """A masked key's weight is zero, and zero times its value must not count; an infinite key whose score is minus infinity has no weight either."""
+    H, G, d = 2, 1, 64
+    q, k, v = inputs(T, pos0 + T, H, G, d, d, T)
+    j = pos0 + T // 2  # a position inside the pass
+    if what == "q inf":
+        q[T // 2, 3] = np.inf
+    else:
+        (v if what[0] == "v" else k)[[j, j - pos0 // 2], 3] = np.nan if what == "v nan" else np.inf
+    with np.errstate(invalid="ignore"):
+        for kw in (dict(), dict(window=20), dict(chunk=16)):
+            window, chunk = kw.get("window", 10 ** 6), kw.get("chunk", 0)
+            want = reference(q, k, v, pos0, H, G, window, chunk=chunk, scale=0.125)
+            if chunk:
+                got = capi.chunked_attention(q, k, v, pos0, H, G, d, d, chunk, 0.125, n_splits=n_splits, cache_bf16=True)
+            else:
+                got = capi.swa_attention(q, k, v, pos0, H, G, d, d, window, 0.125, n_splits=n_splits, cache_bf16=True)
+            assert np.isfinite(want).any() and not np.isfinite(want).all()
+            assert np.allclose(got, want, rtol=0, atol=TOL, equal_nan=True)

@@ -2264,10 +2264,10 @@ static inline bool swa_mma_ok(const SwaArgs& a, int rows, bool cache_f32) {
 }
 
 // Splits of the keys for the kernel above.  A CTA walks its keys at 2.4 (64 channels) to 4.2 us (128) per 64, so that a short pass over a long cache needs
-// more CTAs than its queries and heads give: up to two per SM, each with keys for a step.  Times with the best of 1 to 32 splits (the join's kernel
-// included), one split, and the tiled kernel as it would be launched: 16 tokens of 8 heads of 128 over 4096 keys 32, 342, 271 us; 64 tokens 42, 345, 252;
-// 64 tokens of 32 heads over 1024 keys 38, 132, 277; over 32768 416, -, 5689.  128 tokens of 32 heads (64 CTAs): four splits against one 54 : 129 us over
-// 1024 keys, 128 : 332 over 4096; 256 tokens (128 CTAs): two against one 88 : 122, 234 : 327.
+// more CTAs than its queries and heads give: up to two per SM, each with keys for a step.  With these splits (the join's kernel included), with one, and the
+// tiled kernel as it would be launched, heads of 128, caches flushed: 16 tokens of 8 heads over 4096 keys 39, 312, 271 us; 64 tokens 44, 314, 252; 64 tokens
+// of 32 heads over 1024 keys 44, 96, 277, over 4096 82, 314, 822; 128 tokens of 32 heads (64 CTAs) over 4096 133, 315, 1606; 45 tokens of 8 heads over 301
+// keys 28, 43, 119; 1024 tokens of 8 heads in a window of 512 (128 CTAs, two splits) 69, 70, 268.
 static inline int swa_mma_splits(const SwaArgs& a, int rows) {
 	if (!a.part_o || !a.part_ml) return 1;
 	const long long ctas = (long long) (rows + SWA_MMA_ROWS - 1) / SWA_MMA_ROWS * a.H;

@@ -9,8 +9,8 @@
 // 64 keys and their values at a time come through a two-deep cp.async ring; queries stay in shared memory as planes, scores, probabilities and output in
 // registers (m16n8k16 fragments).
 // Bound: the instructions around the products (splits, exponentials, adds: about half) and the mma.sync pipe, three products per one.  Against the fp32
-// FMA tiles of mix_ops.cuh: 1024 tokens of 16 heads of 128 over up to 2048 keys 1626 -> 200 us, of 8 heads in a window of 512 286 -> 94 us; 256 tokens
-// of 8 heads over up to 301 keys 105 -> 83 us (32 CTAs).  Distance from float64 at 128 channels and 1500 keys: 2.6e-7, the FMA kernel 4.4e-7.
+// FMA tiles of mix_ops.cuh, caches flushed: 1024 tokens of 16 heads of 128 over up to 2048 keys 1978 -> 215 us, of 8 heads in a window of 512 268 -> 69 us;
+// 256 tokens of 8 heads over up to 256 keys 93 -> 31 us (four splits).  Distance from float64 at 128 channels and 1500 keys: 2.6e-7, the FMA kernel 4.4e-7.
 #define XALM_SECONDARY_TU
 #include "common.cuh"
 #include "family.h"
@@ -49,6 +49,71 @@ __device__ __forceinline__ uint32_t smm_at(int row, int piece) {
 }
 __host__ __device__ constexpr size_t smm_smem(int dq, int dv, int warps) {
 	return (size_t) 3 * 16 * warps * dq * 2 + (size_t) SMM_STAGES * SMM_KEYS * (dq + dv) * 2 + (size_t) SMM_STAGES * SMM_KEYS * 4;
+}
+
+__device__ __forceinline__ bool smm_seen(const SwaArgs& a, int i, int j) {
+	return j <= i && (a.window >= 0x7fffffff || i - j < a.window || j < a.keep_first) && (a.mask_chunk <= 0 || j >= i - i % a.mask_chunk);
+}
+// scale, soft cap and distance biases of the raw score of positions i and j; slope, b1, b2: the head's
+__device__ __forceinline__ float smm_score(const SwaArgs& a, float x, int i, int j, float slope, float b1, float b2) {
+	x *= a.scale;
+	if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+	const float dist = (float) max(i - j, 0);
+	if (a.r1) x -= b1 * log1pf(b2 * dist);
+	if (a.slope) x -= slope * dist;
+	return x;
+}
+// row t's value of column col of head h, or split sp's part of it
+__device__ __forceinline__ void smm_store(const SwaArgs& a, int t, int h, int sp, int col, float o, float l, float m) {
+	if (a.n_splits > 1) { // swa_merge_kernel joins them
+		a.part_o[((size_t) t * a.n_splits + sp) * (a.H * a.dv) + (size_t) h * a.dv + col] = o;
+		if (col == 0) {
+			float* pml = a.part_ml + ((size_t) t * a.n_splits + sp) * (a.H * 2) + 2 * h;
+			pml[0] = m;
+			pml[1] = l;
+		}
+		return;
+	}
+	float v = swa_finish(a, h, o, l, m);
+	if (a.gate) v *= swa_gate(a, t, h, col);
+	a.out[(size_t) t * (a.ldo ? a.ldo : a.H * a.dv) + (size_t) h * a.dv + col] = v;
+}
+// The CTA's nq queries by fp32 FMAs, a warp per query, keys that a query does not see left out: for infinities and NaN, whose planes are not finite and
+// whose product with a masked key's weight of zero is NaN.
+template <int DV, int WARPS>
+__device__ __noinline__ void smm_nonfinite(const SwaArgs a, const SwaKeys km, const __nv_bfloat16* kc, const __nv_bfloat16* vc, int ldk, int ldv, int t0, int nq,
+                                              int i_lo, int h, int sp, int jb, int je, float slope, float b1, float b2) {
+	const int lane = threadIdx.x & 31;
+	for (int row = threadIdx.x >> 5; row < nq; row += WARPS) {
+		const int i = i_lo + row;
+		const float* q = a.q + (size_t) (t0 + row) * a.ldq + a.q_off + (size_t) h * a.d;
+		float m = -INFINITY, l = 0.f, o[DV / 32] = {};
+		for (int j0 = jb; j0 < je; j0 += 32) {
+			const int x = min(j0 + lane, je - 1), j = km.pos(x);
+			const bool seen = j0 + lane < je && smm_seen(a, i, j);
+			const __nv_bfloat16* k = kc + (size_t) km.slot(x) * ldk;
+			float s = 0.f;
+			for (int c = 0; c < a.d; c++) s = fmaf(q[c], __bfloat162float(k[c]), s);
+			s = seen ? smm_score(a, s, i, j, slope, b1, b2) : -INFINITY;
+			const float top = fmaxf(m, warp_max(s)), at = top == -INFINITY ? 0.f : top, keep = m == -INFINITY ? 0.f : expf(m - at), p = expf(s - at);
+			l = fmaf(l, keep, warp_sum(p));
+			m = top;
+#pragma unroll
+			for (int c = 0; c < DV / 32; c++) o[c] *= keep;
+			const unsigned sees = __ballot_sync(0xffffffffu, seen);
+			for (int y = 0; y < 32; y++) {
+				const float w = __shfl_sync(0xffffffffu, p, y);
+				if (!(sees >> y & 1)) continue;
+				const __nv_bfloat16* v = vc + (size_t) km.slot(j0 + y) * ldv;
+#pragma unroll
+				for (int c = 0; c < DV / 32; c++)
+					if (c * 32 + lane < a.dv) o[c] = fmaf(w, __bfloat162float(v[c * 32 + lane]), o[c]);
+			}
+		}
+#pragma unroll
+		for (int c = 0; c < DV / 32; c++)
+			if (c * 32 + lane < a.dv) smm_store(a, t0 + row, h, sp, c * 32 + lane, o[c], l, m);
+	}
 }
 
 // DQ, DV: the channel counts rounded up to 64 or 128 (the rest is zero); WARPS * 16 queries
@@ -163,13 +228,7 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 #pragma unroll
 			for (int e = 0; e < 4; e++) {
 				const int i = i_lo + r0 + (e >> 1) * 8, j = pos[c * 8 + ql * 2 + (e & 1)];
-				float x = s[c][e] * a.scale;
-				if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
-				const float dist = (float) max(i - j, 0);
-				if (a.r1) x -= b1 * log1pf(b2 * dist);
-				if (a.slope) x -= slope * dist;
-				const bool seen = j <= i && (a.window >= 0x7fffffff || i - j < a.window || j < a.keep_first) && (a.mask_chunk <= 0 || j >= i - i % a.mask_chunk);
-				s[c][e] = seen ? x : -INFINITY;
+				s[c][e] = smm_seen(a, i, j) ? smm_score(a, s[c][e], i, j, slope, b1, b2) : -INFINITY;
 				top[e >> 1] = fmaxf(top[e >> 1], s[c][e]);
 			}
 		// ---- softmax weights ----
@@ -219,34 +278,36 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 		}
 		__syncthreads(); // the block's buffer is read
 	}
+	bool finite = true;
 #pragma unroll
 	for (int r = 0; r < 2; r++) {
 		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
 		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
-		const int t = t0 + r0 + r * 8;
 		if (r0 + r * 8 >= nq) continue;
-		const bool parts = a.n_splits > 1; // swa_merge_kernel joins them
-		float* dst = parts ? a.part_o + ((size_t) t * a.n_splits + sp) * (H * dv) + (size_t) h * dv : a.out + (size_t) t * (a.ldo ? a.ldo : H * dv) + (size_t) h * dv;
-		if (parts && ql == 0) {
-			float* pml = a.part_ml + ((size_t) t * a.n_splits + sp) * (H * 2) + 2 * h;
-			pml[0] = m[r];
-			pml[1] = l[r];
-		}
+		finite &= isfinite(l[r]);
 #pragma unroll
-		for (int c = 0; c < DV / 8; c++)
-#pragma unroll
-			for (int e = 0; e < 2; e++) {
-				const int col = c * 8 + ql * 2 + e;
-				if (col >= dv) continue;
-				float v = o[c][2 * r + e];
-				if (!parts) {
-					v = swa_finish(a, h, v, l[r], m[r]);
-					if (a.gate) v *= swa_gate(a, t, h, col);
-				}
-				dst[col] = v;
-			}
+		for (int c = 0; c < DV / 8; c++) finite &= isfinite(o[c][2 * r]) && isfinite(o[c][2 * r + 1]);
 	}
+	if (__syncthreads_or(!finite)) {
+		smm_nonfinite<DV, WARPS>(a, km, kc, vc, ldk, ldv, t0, nq, i_lo, h, sp, jb, je, slope, b1, b2);
+		return;
+	}
+	// Through shared memory, a warp its own rows: with the store's code once per value of a thread, fetching it took 45 us of a CTA's time (16 tokens of 8
+	// heads over 1024 keys, one split: 139 -> 94 us)
+	constexpr int LDO = DV + 8; // floats: the eight rows of a fragment on different banks
+	float *os = reinterpret_cast<float*>(smem) + warp * 16 * LDO, *ls = reinterpret_cast<float*>(smem) + ROWS * LDO + warp * 32;
+#pragma unroll
+	for (int r = 0; r < 2; r++) {
+#pragma unroll
+		for (int c = 0; c < DV / 8; c++) *reinterpret_cast<float2*>(os + (quad + r * 8) * LDO + c * 8 + ql * 2) = make_float2(o[c][2 * r], o[c][2 * r + 1]);
+		if (ql == 0) *reinterpret_cast<float2*>(ls + (quad + r * 8) * 2) = make_float2(l[r], m[r]);
+	}
+	__syncwarp();
+	for (int row = 0; row < min(16, nq - warp * 16); row++)
+#pragma unroll 1
+		for (int col = lane; col < dv; col += 32) smm_store(a, t0 + warp * 16 + row, h, sp, col, os[row * LDO + col], ls[row * 2], ls[row * 2 + 1]);
 }
+static_assert(4 * (64 * (64 + 8) + 4 * 32) <= smm_smem(64, 64, 4) && 4 * (64 * (128 + 8) + 4 * 32) <= smm_smem(64, 128, 4), "the output's rows fit where queries and keys lay");
 
 template <int DQ, int DV>
 static int launch_swa_mma_inst(const SwaArgs& a, int rows, cudaStream_t s) {
