@@ -87,6 +87,23 @@ def test_latent_attention_over_rows(H, d, r, dv, R, T, pos0):
     close(capi.latent_attend(q, rows, pos0, H, d, r, dv, R, uk, uv, scale, freqs, gate=gate, n_splits=3), want * O.sigmoid(gate), F32_TOL)
 
 
+@pytest.mark.parametrize("T,pos0", [(1, 0), (1, 70), (4, 97)])
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("R,extra", [(760, 0), (768, 0), (1016, 8)])
+def test_short_steps_over_rows_at_and_beyond_the_cluster_kernels_channels(T, pos0, bf16, R, extra):
+    """Rows of 768 channels run as clusters; beyond them one CTA per query copies whole 16-byte pieces of rows whose values are a part of the keys."""
+    H, d, r, dv = 2, 16, 8, 8
+    rng = np.random.default_rng(R + T)
+    n = pos0 + T
+    rnd = O.bf16_round if bf16 else (lambda a: a)
+    c, k_rot, rows, uk, uv = latent_case(rng, n, H, d, r, dv, R, extra)
+    q = rng.standard_normal((T, H * (d + r)))
+    freqs = O.rotary_frequencies(r, 50.0)
+    want = O.attend_latents(q, rnd(c), rnd(k_rot), rnd(uk), rnd(uv), H=H, d=d, r=r, dv=dv, scale=0.1, freqs=freqs, first_pos=pos0)
+    got = capi.latent_attend(q, rnd(rows), pos0, H, d, r, dv, R, rnd(uk), rnd(uv), 0.1, freqs, cache_bf16=bf16, w_bf16=bf16)
+    close(got, want, F32_TOL)
+
+
 @pytest.mark.parametrize("T,pos0,far", [(1, 700, 3), (1, 700, 699), (2, 350, 31), (2, 350, 32), (48, 400, 0), (48, 400, 430)])
 @pytest.mark.parametrize("n_splits", [0, 1, 5])
 def test_latent_attention_finds_one_far_key(T, pos0, far, n_splits):
