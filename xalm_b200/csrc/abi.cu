@@ -39,7 +39,7 @@ static std::map<std::string, int>& tuning() {
 	    {"attn_splits", 0},  // 0 = auto (~1 CTA per SM, at most 32 splits per kv head)
 	    {"attn_min_split", 128},
 	    {"mv_cfg_rows", 0},  // 0 = auto, 1 = force config A (R4 KS1 NW4), 2 = force config B (R2 KS4 NW8)
-	    {"mega", 0},         // EXPERIMENTAL, measured slower than the kernel-per-op path (profiles/r2_token_kernel.md): one persistent kernel per
+	    {"mega", 0},         // EXPERIMENTAL, measured slower than the kernel-per-op path: one persistent kernel per
 	                         // token (decode_mega.cu) when the model allows — single GPU, integer weight formats
 	    {"mega_smem_kb", 170}, // shared memory per CTA the token kernel may take: the ring gets what the staged activations leave (3 stages on a
 	                           // 7B model: deeper rings measured no faster), the rest of the 228 KB stays L1

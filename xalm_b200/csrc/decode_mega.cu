@@ -1,7 +1,7 @@
 // decode_mega.cu — one persistent kernel per decode token (Model::forward, infer.cpp:604-638, batch 1).
 //
-// Why.  With one kernel per fused op (5 per layer, 162 per Mistral-7B token) the round-1 timeline
-// (profiles/r1_timeline_multikernel.md) shows ~36 us of HBM streaming per layer at roofline against 68 us measured: every
+// Why.  With one kernel per fused op (5 per layer, 162 per Mistral-7B token) a timeline taken inside the kernels
+// shows ~36 us of HBM streaming per layer at roofline against 68 us measured: every
 // kernel boundary drains the weight stream (ramp-up, tail, dependency flush, activation staging), and the 8-bit consumer
 // loop itself was issue/latency-bound.  Here a token is a list of PHASES run by the same resident CTAs, one per SM:
 //
@@ -19,7 +19,7 @@
 //     read with ld.global.cg (L2), never through L1.  (Tried and measured slower: hand-off by polling {value, tag} words —
 //     36 k threads polling the same 32 KB turn its L2 lines into a hot spot, 4-10 us per hand-off; and the same with a
 //     fence-free counter as a hint — without the fence the producers' stores take microseconds to reach L2 behind the weight
-//     stream, so the pollers spin just as long.  profiles/r2_token_kernel.md.)
+//     stream, so the pollers spin just as long.)
 //   * everything else a consumer needs after its input arrives is already on the SM: phase descriptors are fetched one
 //     phase ahead into shared memory, the token's scalars and the RoPE table are loaded once, norm weights are requested
 //     before the input is polled (all of these are read once per token, i.e. from DRAM behind the weight stream).

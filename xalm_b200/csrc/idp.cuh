@@ -3,7 +3,7 @@
 //
 // The reference multiplies dequantised weights d*q (+m) by fp32 activations (infer.cpp:104-135).  On the CUDA cores
 // that costs ~2.2 issue slots per 8-bit weight and ~4.3 per 4-bit weight (byte -> fp32 via PRMT, FADD2, FFMA2):
-// profiles/r1_matvec_tma_q8_0_w13.md shows the q8_0 kernel latency/issue-bound at 75 % of HBM peak and the 4/5-bit
+// the counters showed the q8_0 kernel latency/issue-bound at 75 % of HBM peak and the 4/5-bit
 // formats ALU-bound at 26-29 %.  Here the sum over a 32-element block is taken in INTEGERS with dp4a:
 //
 //     sum_j (d*q_j) * x_j  =  d * dx * sum_j q_j * X_j          x_j ~= dx * X_j,  X_j a 24-bit integer,
@@ -74,7 +74,7 @@ __device__ __forceinline__ void xq_store_block(const XqView& v, int blk, const f
 // The staging used by the kernels: EIGHT consecutive elements per lane, the four lanes 4k..4k+3 of a warp share a block (call with
 // all lanes of the warp).  Loads are coalesced (32 bytes per lane, 1 KB per warp instruction) and every thread of the CTA works;
 // the thread-per-block version above left half the CTA idle behind 32 line-strided loads per lane and took 7 us of a 25 us
-// kernel (profiles/r2_decode_timeline.md).  Same image in shared memory, bit for bit.
+// kernel.  Same image in shared memory, bit for bit.
 __device__ __forceinline__ void xq_store_group8(const XqView& v, int grp, const float (&x)[8]) {
 	uint32_t mb = 0;
 #pragma unroll

@@ -57,7 +57,7 @@ struct MatvecArgs {
 	int pf_kv;                   // 1: also prefetch rows [0, kv_len) of k_cache / v_cache (the attention kernel that follows QKV)
 	// rmsnorm weights of the NEXT norm-fused kernel (read once per token, i.e. from DRAM): CTA 0 pulls them into L2 at entry.  That
 	// kernel requests them before its dependency wait; coming from DRAM behind its own weight stream they took ~2.5 us, and the
-	// activation loads issued after them return in order behind them (profiles/r2_decode_timeline.md)
+	// activation loads issued after them return in order behind them
 	const uint8_t* pf_norm_ptr;
 	unsigned int pf_norm_bytes;
 	// tensor-parallel exchange fused into the matvec kernels (matvec_tma.cuh), LL style: the row-split matvecs (Wo, W2) PUSH every

@@ -4,7 +4,7 @@
 // cp.async.bulk, 8 consumer warps, rmsnorm prologue, QKV / GLU / residual / store epilogues, PDL, the fused tensor-parallel
 // exchange — but the consumers work in integers: the activations are staged ONCE per CTA as block floating point (three int8
 // limbs per element + one power-of-two scale per 32), and a 32-weight block costs 24 dp4a plus ~8 finishing instructions
-// instead of 64-136 PRMT / FADD2 / FFMA2.  Measured on the float core (profiles/r1_matvec_tma_q8_0_w13.md): q8_0 issue /
+// instead of 64-136 PRMT / FADD2 / FFMA2.  Measured on the float core: q8_0 issue /
 // latency-bound at 75 % of HBM peak (3.9 issue slots per weight with its per-tile reductions), q4_0..q5_1 ALU-bound at 26-29 %.
 //
 // Mapping: a tile is 8 rows, a ring stage 8 rows x 16 units (4096 elements).  Warp (kw, rw) = K-slice kw of 4 (32 blocks of 32
@@ -19,7 +19,7 @@ namespace xalm {
 
 constexpr int IDP_KW = 4, IDP_RW = 2, IDP_R = 4, IDP_RC = IDP_RW * IDP_R, IDP_U = 16;
 // Partial sums of the K-slice warps are handed to the tile's reducer warp through PB buffers, each with an mbarrier the 8 consumer
-// warps arrive on: nobody but the reducer ever waits (a CTA-wide bar.sync per tile was 26 % of all stall cycles, profiles/r2_idp_ncu.md).
+// warps arrive on: nobody but the reducer ever waits (a CTA-wide bar.sync per tile was 26 % of all stall cycles).
 // A buffer is reused PB tiles later; a warp cannot run more than NS stages (<= NS tiles) ahead of the slowest warp of its group (ring).
 __host__ __device__ inline int idp_pb(int NS) { return NS + 2 < 8 ? 8 : NS + 2; }
 constexpr int IDP_MP = 4; // staging passes of a norm-fused kernel: 8 elements x 256 lanes x 4 = n <= 8192
@@ -100,7 +100,7 @@ __global__ void __maxnreg__(96) matvec_idp_kernel(const IdpArgs ta) {
 					if (un == nu && nu == U && a.w.s0 == (size_t) ROW_STAGE) {
 						// the stage spans whole rows and a tile's rows are neighbours in memory: ONE copy per run of rows instead of
 						// one per row (the copy engine is bound by the NUMBER of bulk copies when they are a few KB each: q4_0 rows of
-						// 2304 bytes streamed no faster than q8_0 rows of 4352, profiles/r2_decode_timeline.md)
+						// 2304 bytes streamed no faster than q8_0 rows of 4352)
 						if (a.epi == EPI_GLU) { // rows [0, RC/2) are W1[o0..], rows [RC/2, RC) are W3[o0..]
 							const int o0 = row0 / 2;
 							bulk_g2s(dst, a.w.p0 + (size_t) o0 * a.w.s0, bytes * (RC / 2), &full[slot]);

@@ -2,7 +2,7 @@
 // (mma.sync.m16n8k32.s32.u8.u8), weights in fragment tiles (frag_layout.cuh).
 //
 // Why.  The dp4a core (matvec_idp.cuh) spends 24 IDP.4A plus ~30 unpack / convert / scale instructions per 32-weight block and
-// lane: 0.112 (q8_0) - 0.124 (q4_0) warp instructions per weight.  ncu (profiles/r2_ncu_q4_0_w13_details.txt): q4_0 W1|W3 runs at
+// lane: 0.112 (q8_0) - 0.124 (q4_0) warp instructions per weight.  ncu: q4_0 W1|W3 runs at
 // 30 % of DRAM peak with the issue slots 52 % busy and 0.9 eligible warps per scheduler — the consumers, not HBM, set the pace,
 // and q4_0 decodes no faster than q8_0 although it streams half the bytes.  Here ONE mma handles a 16-row x 32-element block
 // column (512 weights) against the three activation limbs at once, and the per-block float work is 2 IMAD + 2 I2F + 2 FFMA:
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const
 
 	if (warp == NCW + 1) {
 		// ===================== epilogue warp: K-slice sums -> rows -> epilogue.  The 16 multiplying warps never wait for each other's
-		// partial sums (with a rotating reducer among them, a third of all warp samples sat in that wait: profiles/r2_mma.md) ==========
+		// partial sums (with a rotating reducer among them, a third of all warp samples sat in that wait) ==========
 		pdl_wait();
 		float nscale = 1.f;
 		int pb = 0, pph = 0;

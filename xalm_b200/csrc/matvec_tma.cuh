@@ -3,7 +3,7 @@
 // conflict-free 128-bit shared loads.  Same math, prologue and epilogues as matvec.cuh (which stays as the path for
 // row lengths that are not a multiple of 256 and for the table-decoded formats).
 //
-// Why (profiles/r1_matvec_ldg_q8_0_w13.md): the LDG version is L1TEX-bound, not HBM-bound — every warp re-reads its
+// Why: the LDG version is L1TEX-bound, not HBM-bound — every warp re-reads its
 // activation chunk (and the norm weights) through L1 for every 4 rows, 3x the weight traffic, and tops out at ~40 % of
 // HBM peak.  Here:
 //   * one CTA per SM, grid-strided over row tiles; a dedicated producer warp keeps a ring of NS stages in flight

@@ -204,7 +204,7 @@ static int launch_matvec_tma(const MatvecArgs& a, cudaStream_t s, bool pdl) {
 	if (tune("tma_rc") == 4 && ppu >= 16) { RC = 4; KW = 8; }
 	if (tune("tma_rc") == 8 && ppu >= 16) { RC = 8; KW = 8; }
 	// norm-fused kernels (QKV, W1|W3, classifier; n = dim): 4 K-slices x 2 row groups use fewer registers (<= 72), so three
-	// CTAs fit per SM with 17 KB stages — measured faster than 2 x (8 K-slices) for these, slower for Wo/W2 (profiles/)
+	// CTAs fit per SM with 17 KB stages — measured faster than 2 x (8 K-slices) for these, slower for Wo/W2
 	bool norm_cfg = false;
 	if (a.norm_w != nullptr && ppu >= 16 && tune("tma_norm_kw4") && nu * ppu / 4 >= 32) { RC = 8; KW = 4; norm_cfg = true; }
 	if (a.norm_w == nullptr && vrows % 16 == 0 && tune("tma_short_rows")) {
@@ -642,7 +642,7 @@ static int attn_auto_splits(int n_kv_heads) {
 	int sms = 148;
 	int dev = 0;
 	if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	// about one CTA per SM, and never so many splits that the last-CTA merge dominates (measured: profiles/r1_attention_splits.md)
+	// about one CTA per SM, and never so many splits that the last-CTA merge dominates (measured)
 	int s = sms / n_kv_heads;
 	if (s > 32) s = 32;
 	return s < 1 ? 1 : s;
