@@ -309,7 +309,9 @@ int xalm_cuda_sync(xalm_cuda_model* m);
  * every position), 1 = logits of the last position -> logits_host[vocab], 2 = every position -> logits_host[n*vocab].
  * targets/probs_host (n entries each, or NULL; needs want_logits 2): probs_host[i] = Sampler::sample_prob(targets[i])
  * on the logits of position pos0+i (sampler.cpp:18-33) — what perplexity mode takes the log of (main.cpp:251).
- * logits_host may be NULL.  Synchronous.  Tensor-core operands are fp16 with fp32 accumulation; the "prefill_split"
+ * A call that fails after some of its positions have run (config.json families take a prompt in passes) leaves probs_host the probabilities
+ * before the failing pass, or before the target that is out of range.  logits_host may be NULL; together with targets the buffer of
+ * xalm_cuda_logits_host then keeps what it held.  Synchronous.  Tensor-core operands are fp16 with fp32 accumulation; the "prefill_split"
  * knob (xalm_cuda_tune) picks how fp32 values enter them: 3 (default) = hi+lo fp16 pairs for activations, weights and the
  * attention operands (3 MMAs per product; 32-layer 4k-token logits within ~1e-3 of the token-at-a-time path), 2 = pairs
  * for activations only, 1 = plain fp16 (fastest; ~4e-2 at that depth).  1e-2. */

@@ -88,7 +88,9 @@ int tune(const char* k) {
 // ---------------------------------------------------------------------------------------------------------
 // programmatic dependent launches (common.cuh)
 // ---------------------------------------------------------------------------------------------------------
-static std::vector<cudaStream_t>& blocked_streams() { // a few at most: a model's two streams, each asked about soon after
+// Streams this thread has blocked and not asked about since: a model's two at most, since a handle stands here once.  A pass of several tokens may never
+// ask; a handle that outlives its stream costs the next stream of that handle one launch that does not overlap.
+static std::vector<cudaStream_t>& blocked_streams() {
 	static thread_local std::vector<cudaStream_t> b;
 	return b;
 }

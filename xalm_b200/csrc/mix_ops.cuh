@@ -863,7 +863,8 @@ __global__ void __launch_bounds__(256) swa_attn_kernel(SwaArgs a) {
 	const int jb = sp * per, je = min(nk, jb + per); // virtual key indices
 	// staged rows: Ks[jj][G d], Vs[jj][G dv] in the cache's element type
 	const bool staged = a.stage_off > 0;
-	// one key/value head whose values are the first dv entries of the key rows (a latent cache): the staged key rows serve as values too
+	// one key/value head whose values are the first dv entries of the key rows (a latent cache of rows beyond 768 channels; swa_one.cu takes the shorter
+	// ones): the staged key rows serve as values too
 	const bool v_in_k = a.vc == a.kc && ldv == ldk && G == 1 && dv <= d;
 	const int vs_ld = v_in_k ? G * d : G * dv;
 	CT* Ks = reinterpret_cast<CT*>(sm + a.stage_off);
