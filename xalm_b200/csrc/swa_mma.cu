@@ -8,7 +8,8 @@
 // A CTA takes 16 queries of one head per warp and, where few CTAs would run (swa_mma_splits), a share of the keys, whose parts swa_merge_kernel joins;
 // 64 keys and their values at a time come through a two-deep cp.async ring; queries stay in shared memory as planes, scores, probabilities and output in
 // registers (m16n8k16 fragments).
-// Bound: the instructions around the products (splits, exponentials, adds: about half) and the mma.sync pipe, three products per one.  Against the fp32
+// Bound: latency, one or two warps per scheduler (115 KB a CTA) going through chains of three products, adds, exponentials and splits: at 1024 tokens of 16
+// heads over 1024 keys the mma.sync pipe is active 20 % and 26 % of the issue slots are used.  Against the fp32
 // FMA tiles of mix_ops.cuh, caches flushed: 1024 tokens of 16 heads of 128 over up to 2048 keys 1978 -> 215 us, of 8 heads in a window of 512 268 -> 69 us;
 // 256 tokens of 8 heads over up to 256 keys 93 -> 31 us (four splits).  Distance from float64 at 128 channels and 1500 keys: 2.6e-7, the FMA kernel 4.4e-7.
 #define XALM_SECONDARY_TU
