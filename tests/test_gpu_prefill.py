@@ -62,6 +62,25 @@ def test_gemm_shapes(shape):
     assert np.max(np.abs(out - ref)) <= 2e-5 * float(np.abs(ref).max()) + 1e-6
 
 
+@pytest.mark.parametrize("shape", [(5, 4096, 288), (33, 14336, 1024), (130, 2112, 544), (333, 4096, 4096), (257, 1088, 2496)])
+@pytest.mark.parametrize("split", [1, 2, 3])
+def test_gemm_few_tiles(shape, split):
+    """Shapes whose K steps a cluster's CTAs share: uneven shares, ragged rows and columns, one to five row tiles.  The tolerances are those of the tests
+    above: a share's sum is fp32 as the whole sum is, and there are at most 8 of them."""
+    Tn, K, N = shape
+    t = T.parse("f32")
+    a, w = synth.normal(6, 79, Tn * K, 1.0).reshape(Tn, K), synth.normal(6, 80, N * K, 0.05).reshape(N, K)
+    raw = np.ascontiguousarray(w).view(np.uint8).reshape(-1)
+    out = capi.gemm(a, raw, t.id, K, N, split)
+    if split == 3:
+        ref = a.astype(np.float64) @ w.astype(np.float64).T
+    else:
+        hi = _fp16(a)
+        ref = (hi.astype(np.float64) + (_fp16(a - hi) if split == 2 else 0.0)) @ _fp16(w).astype(np.float64).T
+    assert np.max(np.abs(out - ref)) <= 2e-5 * float(np.abs(ref).max()) + 1e-6
+    assert np.array_equal(out, capi.gemm(a, raw, t.id, K, N, split))
+
+
 def _oracle_all_logits(om, tokens):
     return np.stack([om.forward(int(tok), pos, 1).copy() for pos, tok in enumerate(tokens)])
 

@@ -36,6 +36,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -432,8 +433,177 @@ struct GemmCfg {
 	static constexpr size_t SMEM = (size_t) NS * STAGE + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 
-// GROUPED: M tiles come from a list, each with a matrix of its own
-template <int NA, int NB, bool GROUPED = false>
+// The accumulator of a tile as the epilogue sees it: N consecutive columns of this thread's row
+struct AccTmem { // as it lies in tensor memory
+	uint32_t taddr;
+	__device__ __forceinline__ void get(int c, float (&v)[8]) const { tmem_ld8(taddr + c, v); }
+	__device__ __forceinline__ void get(int c, float (&v)[16]) const { tmem_ld16(taddr + c, v); }
+	__device__ __forceinline__ void get(int c, float (&v)[32]) const { tmem_ld32(taddr + c, v); }
+};
+struct AccCluster { // summed over the cluster's CTAs, in the order of their ranks; each left its own in its shared memory, four columns x 128 rows at a time
+	uint32_t base; // of this thread's row, an address of this CTA
+	int ks;
+	template <int N>
+	__device__ __forceinline__ void get(int c, float (&v)[N]) const {
+#pragma unroll
+		for (int i = 0; i < N; i++) v[i] = 0.f;
+#pragma unroll 4
+		for (int r = 0; r < ks; r++) {
+			uint32_t a;
+			asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(base), "r"(r));
+#pragma unroll
+			for (int i = 0; i < N; i += 4) {
+				float4 x;
+				asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+				             : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+				             : "r"(a + (uint32_t) ((c + i) / 4 * GB_M * 16)));
+				v[i] += x.x; v[i + 1] += x.y; v[i + 2] += x.z; v[i + 3] += x.w;
+			}
+		}
+	}
+};
+__device__ __forceinline__ void cluster_barrier() { // every thread of the cluster's CTAs
+	__syncwarp();
+	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The fused epilogue of tile (mt, nt) for this thread's row, chunks of columns part, part + parts, ... (one CTA: all of them)
+template <bool GROUPED, typename Acc>
+__device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc, int mt, int nt, int row_in_tile, int part, int parts) {
+	const int m = mt * GB_M + row_in_tile;
+	const bool mrow = GROUPED ? row_in_tile < g.gtiles[3 * mt + 2] : m < g.M;
+	if (GROUPED && g.epi == GEPI_ACT) {
+		for (int c = part * 16; c < GB_N; c += parts * 16) {
+			float v[16];
+			acc.get(c, v);
+			const int n0 = nt * GB_N + c;
+			if (!mrow || n0 >= g.N) continue;
+			float h[8];
+			if (g.gact.glu) { // gate and up columns alternate: 16 columns are 8 values
+#pragma unroll
+				for (int i = 0; i < 8; i++) h[i] = mix::glu_apply(g.gact.act, v[2 * i], v[2 * i + 1], g.gact.limit, g.gact.alpha);
+				store_a8(g.o, m, n0 / 2, h);
+			} else {
+#pragma unroll
+				for (int half = 0; half < 2; half++) {
+#pragma unroll
+					for (int i = 0; i < 8; i++) h[i] = mix::act_apply(g.gact.act, v[8 * half + i]);
+					store_a8(g.o, m, n0 + 8 * half, h);
+				}
+			}
+		}
+	} else if (g.epi == GEPI_GLU) {
+		for (int c = part * 8; c < GB_N / 2; c += parts * 8) {
+			float gt[8], up[8];
+			acc.get(c, gt);
+			acc.get(GB_N / 2 + c, up);
+			const int o0 = nt * (GB_N / 2) + c;
+			if (mrow && o0 < g.N) {
+				float h[8];
+#pragma unroll
+				for (int i = 0; i < 8; i++) h[i] = (g.act == XALM_SILU ? act_silu(gt[i]) : act_gelu(gt[i])) * up[i]; // infer.cpp:470-488
+				store_a8(g.o, m, o0, h);
+			}
+		}
+	} else if (g.epi == GEPI_QKV) {
+		// 16 columns = 8 rotation pairs at a time; q_dim, kv_dim and head_dim are multiples of 16, so a chunk never straddles
+		// the q | k | v regions or a head, and leaves as two 16-byte stores
+		const int pos = g.pos0 + m;
+		const float2* cs_row = g.rope_cs + (size_t) (mrow ? m : 0) * (g.head_dim / 2);
+		for (int c = part * 16; c < GB_N; c += parts * 16) {
+			float v[16];
+			acc.get(c, v);
+			const int n0 = nt * GB_N + c;
+			if (!mrow || n0 >= g.N) continue;
+			const int region = n0 < g.q_dim ? 0 : (n0 < g.q_dim + g.kv_dim ? 1 : 2);
+			const int j0 = n0 - (region == 0 ? 0 : region == 1 ? g.q_dim : g.q_dim + g.kv_dim); // column inside the region
+#pragma unroll
+			for (int i = 0; i < 16; i++) v[i] = clipf(v[i], g.qkv_clip); // infer.cpp:389-399
+			if (region < 2) { // rope (infer.cpp:305-322) on q and k: the same sincosf(pos * freq) values as the decode kernels
+				const float4* cs4 = reinterpret_cast<const float4*>(cs_row + ((j0 % g.head_dim) >> 1));
+#pragma unroll
+				for (int i = 0; i < 4; i++) {
+					const float4 t = cs4[i]; // {cos, sin} of two consecutive pairs
+					const float a0 = v[4 * i], b0 = v[4 * i + 1], a1 = v[4 * i + 2], b1 = v[4 * i + 3];
+					v[4 * i] = a0 * t.x - b0 * t.y; v[4 * i + 1] = a0 * t.y + b0 * t.x;
+					v[4 * i + 2] = a1 * t.z - b1 * t.w; v[4 * i + 3] = a1 * t.w + b1 * t.z;
+				}
+			}
+			__half2 h[8];
+#pragma unroll
+			for (int i = 0; i < 8; i++) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+			if (region == 0 && g.qt_hi) { // head_dim 128: tile ((head * n_qb + m / 128) * 2 + hd half), row m % 128
+				const int head = j0 >> 7, hc = j0 & 127;
+				const size_t toff = ((size_t) (head * g.n_qb + (m >> 7)) * 2 + (hc >> 6)) * A_TILE_BYTES;
+				const size_t o0 = toff + tile_inner_off(m & 127, hc & 63), o1 = toff + tile_inner_off(m & 127, (hc & 63) + 8);
+				*reinterpret_cast<uint4*>(g.qt_hi + o0) = reinterpret_cast<const uint4*>(h)[0];
+				*reinterpret_cast<uint4*>(g.qt_hi + o1) = reinterpret_cast<const uint4*>(h)[1];
+				if (g.qt_lo) {
+					__half2 l[8];
+#pragma unroll
+					for (int i = 0; i < 8; i++) {
+						const float2 f = __half22float2(h[i]);
+						l[i] = __floats2half2_rn(v[2 * i] - f.x, v[2 * i + 1] - f.y);
+					}
+					*reinterpret_cast<uint4*>(g.qt_lo + o0) = reinterpret_cast<const uint4*>(l)[0];
+					*reinterpret_cast<uint4*>(g.qt_lo + o1) = reinterpret_cast<const uint4*>(l)[1];
+				}
+				continue;
+			}
+			__half* dst = region == 0 ? g.q_out + (size_t) m * g.q_dim + j0
+			            : region == 1 ? g.k_cache + (size_t) pos * g.kv_dim + j0 : g.v_cache + (size_t) pos * g.kv_dim + j0;
+			reinterpret_cast<uint4*>(dst)[0] = reinterpret_cast<const uint4*>(h)[0];
+			reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<const uint4*>(h)[1];
+			if (region > 0 && g.kt) { // the same values as operand tiles (key = pos: this path is only taken with pos0 == 0)
+				const int kvh = j0 >> 7, hc = j0 & 127;
+				const size_t blk = (size_t) (kvh * g.n_kb_total + (pos >> 7)) * 2;
+				if (region == 1) { // K tile (kv head, 128-key block, hd half): row = key, 64 hd columns
+					uint8_t* t = g.kt + (blk + (hc >> 6)) * A_TILE_BYTES;
+					*reinterpret_cast<uint4*>(t + tile_inner_off(pos & 127, hc & 63)) = reinterpret_cast<const uint4*>(h)[0];
+					*reinterpret_cast<uint4*>(t + tile_inner_off(pos & 127, (hc & 63) + 8)) = reinterpret_cast<const uint4*>(h)[1];
+				} else {           // V^T tile (kv head, 128-key block, key half): row = hd, 64 key columns; a warp covers 32 consecutive keys
+					uint8_t* t = g.vt + (blk + ((pos & 127) >> 6)) * A_TILE_BYTES;
+					const __half* hv = reinterpret_cast<const __half*>(h);
+#pragma unroll
+					for (int i = 0; i < 16; i++) *reinterpret_cast<__half*>(t + tile_inner_off(hc + i, pos & 63)) = hv[i];
+				}
+			}
+			if (region == 0 && g.q_lo) {
+				__half2 l[8];
+#pragma unroll
+				for (int i = 0; i < 8; i++) {
+					const float2 f = __half22float2(h[i]);
+					l[i] = __floats2half2_rn(v[2 * i] - f.x, v[2 * i + 1] - f.y);
+				}
+				uint4* dl = reinterpret_cast<uint4*>(g.q_lo + (size_t) m * g.q_dim + j0);
+				dl[0] = reinterpret_cast<const uint4*>(l)[0];
+				dl[1] = reinterpret_cast<const uint4*>(l)[1];
+			}
+		}
+	} else {
+		for (int c = part * 32; c < GB_N; c += parts * 32) { // 32 columns = one full 128-byte line per thread
+			float v[32];
+			acc.get(c, v);
+			const int n0 = nt * GB_N + c;
+			if (!mrow || n0 >= g.N) continue;
+			float* o = g.out + (size_t) (GROUPED ? g.gtiles[3 * mt + 1] + row_in_tile : m - g.out_row0) * g.ldo + n0;
+#pragma unroll
+			for (int i = 0; i < 32; i += 4) {
+				if (n0 + i >= g.N) break;
+				float4 r = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+				if (g.epi == GEPI_RESID) {
+					const float4 x = *reinterpret_cast<const float4*>(o + i);
+					r.x += x.x; r.y += x.y; r.z += x.z; r.w += x.w; // infer.cpp:450-452, :492-494
+				}
+				*reinterpret_cast<float4*>(o + i) = r;
+			}
+		}
+	}
+}
+
+// GROUPED: M tiles come from a list, each with a matrix of its own.  SPLIT: the CTAs of a cluster share a tile's K steps (gemm_split)
+template <int NA, int NB, bool GROUPED = false, bool SPLIT = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs g) {
 	using Cfg = GemmCfg<NA, NB>;
 	constexpr int NS = Cfg::NS;
@@ -468,17 +638,24 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 	const int MT = GROUPED ? *g.gn_tiles : g.MT;
 	const int n_tiles = MT * g.NT;
 	const int KT = g.KT;
+	int rank = 0, ks = 1;
+	if constexpr (SPLIT) {
+		asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+		asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(ks));
+	}
+	const int first_tile = (int) blockIdx.x / ks, tile_step = (int) gridDim.x / ks;
+	const int k_lo = rank * KT / ks, k_hi = (rank + 1) * KT / ks; // this CTA's K steps of every tile
 
 	if (warp == 0) {
-		if (lane == 0) {
-			int slot = 0, phase = 0;
-			for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+		int slot = 0, phase = 0;
+		for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
+			if (lane == 0) {
 				const int mt = g.mt0 + tile % MT, nt = tile / MT;
 				const uint8_t* ah = g.a_hi + (size_t) mt * KT * A_TILE_BYTES;
 				const uint8_t* al = NA == 2 ? g.a_lo + (size_t) mt * KT * A_TILE_BYTES : nullptr;
 				const uint8_t* bt = (GROUPED ? g.gb[g.gtiles[3 * mt]] : g.b) + (size_t) nt * KT * B_TILE_BYTES;
 				const uint8_t* bl = NB == 2 ? g.b_lo + (size_t) nt * KT * B_TILE_BYTES : nullptr;
-				for (int kt = 0; kt < KT; kt++) {
+				for (int kt = k_lo; kt < k_hi; kt++) {
 					mb_wait(&empty[slot], phase ^ 1);
 					uint8_t* st = smem + (size_t) slot * Cfg::STAGE;
 					mb_expect_tx(&full[slot], Cfg::STAGE);
@@ -489,17 +666,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 					if (++slot == NS) { slot = 0; phase ^= 1; }
 				}
 			}
+			if constexpr (SPLIT) { cluster_barrier(); cluster_barrier(); }
 		}
 		__syncwarp();
 	} else if (warp == 1) {
-		if (lane == 0) {
-			constexpr uint32_t idesc = instr_desc_f16(GB_M, GB_N);
-			int slot = 0, phase = 0, acc = 0, acc_phase = 0;
-			for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+		constexpr uint32_t idesc = instr_desc_f16(GB_M, GB_N);
+		int slot = 0, phase = 0, acc = 0, acc_phase = 0;
+		for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
+			if (lane == 0) {
 				mb_wait(&tempty[acc], acc_phase ^ 1);
 				tc_fence_after();
 				const uint32_t d_tmem = tmem_base + (uint32_t) acc * GB_N;
-				for (int kt = 0; kt < KT; kt++) {
+				for (int kt = k_lo; kt < k_hi; kt++) {
 					mb_wait(&full[slot], phase);
 					tc_fence_after();
 					const uint32_t sa = s_u32(smem + (size_t) slot * Cfg::STAGE);
@@ -510,7 +688,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 #pragma unroll
 						for (int k = 0; k < GB_K / UMMA_K; k++) {
 							// advancing K by 16 fp16 = 32 bytes inside the 128-byte swizzle row: +2 in the (>>4) address field
-							umma_f16(d_tmem, adesc + (uint64_t) (2 * k), bdesc + (uint64_t) (2 * k), idesc, (uint32_t) ((kt | k | p) != 0));
+							umma_f16(d_tmem, adesc + (uint64_t) (2 * k), bdesc + (uint64_t) (2 * k), idesc, (uint32_t) (((kt - k_lo) | k | p) != 0));
 						}
 					}
 					umma_commit(&empty[slot]); // frees the stage once these MMAs have read it
@@ -520,148 +698,41 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 				acc ^= 1;
 				if (acc == 0) acc_phase ^= 1;
 			}
+			if constexpr (SPLIT) { cluster_barrier(); cluster_barrier(); }
 		}
 		__syncwarp();
 	} else {
 		const int quad = warp & 3; // TMEM lanes [32*quad, 32*quad+32) are the ones this warp may read
 		int acc = 0, acc_phase = 0;
-		for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+		for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
 			const int mt = g.mt0 + tile % MT, nt = tile / MT;
 			mb_wait(&tfull[acc], acc_phase);
 			tc_fence_after();
-			const int m = mt * GB_M + quad * 32 + lane;
-			const bool mrow = GROUPED ? quad * 32 + lane < g.gtiles[3 * mt + 2] : m < g.M;
 			const uint32_t taddr = tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N;
-			if (GROUPED && g.epi == GEPI_ACT) {
-				for (int c = 0; c < GB_N; c += 16) {
-					float v[16];
-					tmem_ld16(taddr + c, v);
-					const int n0 = nt * GB_N + c;
-					if (!mrow || n0 >= g.N) continue;
-					float h[8];
-					if (g.gact.glu) { // gate and up columns alternate: 16 columns are 8 values
+			if constexpr (SPLIT) {
+				const int rows = GROUPED ? g.gtiles[3 * mt + 2] : g.M - mt * GB_M;
+				uint8_t* own = smem + (size_t) (quad * 32 + lane) * 16; // where the ring was: every stage of this tile has been read
+				if (quad * 32 < rows) { // rows that nobody stores stay where they are
+					for (int c = 0; c < GB_N; c += 32) {
+						float v[32];
+						tmem_ld32(taddr + c, v);
 #pragma unroll
-						for (int i = 0; i < 8; i++) h[i] = mix::glu_apply(g.gact.act, v[2 * i], v[2 * i + 1], g.gact.limit, g.gact.alpha);
-						store_a8(g.o, m, n0 / 2, h);
-					} else {
-#pragma unroll
-						for (int half = 0; half < 2; half++) {
-#pragma unroll
-							for (int i = 0; i < 8; i++) h[i] = mix::act_apply(g.gact.act, v[8 * half + i]);
-							store_a8(g.o, m, n0 + 8 * half, h);
-						}
+						for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(own + (size_t) ((c + i) / 4) * (GB_M * 16)) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
 					}
 				}
-			} else if (g.epi == GEPI_GLU) {
-				for (int c = 0; c < GB_N / 2; c += 8) {
-					float gt[8], up[8];
-					tmem_ld8(taddr + c, gt);
-					tmem_ld8(taddr + GB_N / 2 + c, up);
-					const int o0 = nt * (GB_N / 2) + c;
-					if (mrow && o0 < g.N) {
-						float h[8];
-#pragma unroll
-						for (int i = 0; i < 8; i++) h[i] = (g.act == XALM_SILU ? act_silu(gt[i]) : act_gelu(gt[i])) * up[i]; // infer.cpp:470-488
-						store_a8(g.o, m, o0, h);
-					}
-				}
-			} else if (g.epi == GEPI_QKV) {
-				// 16 columns = 8 rotation pairs at a time; q_dim, kv_dim and head_dim are multiples of 16, so a chunk never straddles
-				// the q | k | v regions or a head, and leaves as two 16-byte stores
-				const int pos = g.pos0 + m;
-				const float2* cs_row = g.rope_cs + (size_t) (mrow ? m : 0) * (g.head_dim / 2);
-				for (int c = 0; c < GB_N; c += 16) {
-					float v[16];
-					tmem_ld16(taddr + c, v);
-					const int n0 = nt * GB_N + c;
-					if (!mrow || n0 >= g.N) continue;
-					const int region = n0 < g.q_dim ? 0 : (n0 < g.q_dim + g.kv_dim ? 1 : 2);
-					const int j0 = n0 - (region == 0 ? 0 : region == 1 ? g.q_dim : g.q_dim + g.kv_dim); // column inside the region
-#pragma unroll
-					for (int i = 0; i < 16; i++) v[i] = clipf(v[i], g.qkv_clip); // infer.cpp:389-399
-					if (region < 2) { // rope (infer.cpp:305-322) on q and k: the same sincosf(pos * freq) values as the decode kernels
-						const float4* cs4 = reinterpret_cast<const float4*>(cs_row + ((j0 % g.head_dim) >> 1));
-#pragma unroll
-						for (int i = 0; i < 4; i++) {
-							const float4 t = cs4[i]; // {cos, sin} of two consecutive pairs
-							const float a0 = v[4 * i], b0 = v[4 * i + 1], a1 = v[4 * i + 2], b1 = v[4 * i + 3];
-							v[4 * i] = a0 * t.x - b0 * t.y; v[4 * i + 1] = a0 * t.y + b0 * t.x;
-							v[4 * i + 2] = a1 * t.z - b1 * t.w; v[4 * i + 3] = a1 * t.w + b1 * t.z;
-						}
-					}
-					__half2 h[8];
-#pragma unroll
-					for (int i = 0; i < 8; i++) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-					if (region == 0 && g.qt_hi) { // head_dim 128: tile ((head * n_qb + m / 128) * 2 + hd half), row m % 128
-						const int head = j0 >> 7, hc = j0 & 127;
-						const size_t toff = ((size_t) (head * g.n_qb + (m >> 7)) * 2 + (hc >> 6)) * A_TILE_BYTES;
-						const size_t o0 = toff + tile_inner_off(m & 127, hc & 63), o1 = toff + tile_inner_off(m & 127, (hc & 63) + 8);
-						*reinterpret_cast<uint4*>(g.qt_hi + o0) = reinterpret_cast<const uint4*>(h)[0];
-						*reinterpret_cast<uint4*>(g.qt_hi + o1) = reinterpret_cast<const uint4*>(h)[1];
-						if (g.qt_lo) {
-							__half2 l[8];
-#pragma unroll
-							for (int i = 0; i < 8; i++) {
-								const float2 f = __half22float2(h[i]);
-								l[i] = __floats2half2_rn(v[2 * i] - f.x, v[2 * i + 1] - f.y);
-							}
-							*reinterpret_cast<uint4*>(g.qt_lo + o0) = reinterpret_cast<const uint4*>(l)[0];
-							*reinterpret_cast<uint4*>(g.qt_lo + o1) = reinterpret_cast<const uint4*>(l)[1];
-						}
-						continue;
-					}
-					__half* dst = region == 0 ? g.q_out + (size_t) m * g.q_dim + j0
-					            : region == 1 ? g.k_cache + (size_t) pos * g.kv_dim + j0 : g.v_cache + (size_t) pos * g.kv_dim + j0;
-					reinterpret_cast<uint4*>(dst)[0] = reinterpret_cast<const uint4*>(h)[0];
-					reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<const uint4*>(h)[1];
-					if (region > 0 && g.kt) { // the same values as operand tiles (key = pos: this path is only taken with pos0 == 0)
-						const int kvh = j0 >> 7, hc = j0 & 127;
-						const size_t blk = (size_t) (kvh * g.n_kb_total + (pos >> 7)) * 2;
-						if (region == 1) { // K tile (kv head, 128-key block, hd half): row = key, 64 hd columns
-							uint8_t* t = g.kt + (blk + (hc >> 6)) * A_TILE_BYTES;
-							*reinterpret_cast<uint4*>(t + tile_inner_off(pos & 127, hc & 63)) = reinterpret_cast<const uint4*>(h)[0];
-							*reinterpret_cast<uint4*>(t + tile_inner_off(pos & 127, (hc & 63) + 8)) = reinterpret_cast<const uint4*>(h)[1];
-						} else {           // V^T tile (kv head, 128-key block, key half): row = hd, 64 key columns; a warp covers 32 consecutive keys
-							uint8_t* t = g.vt + (blk + ((pos & 127) >> 6)) * A_TILE_BYTES;
-							const __half* hv = reinterpret_cast<const __half*>(h);
-#pragma unroll
-							for (int i = 0; i < 16; i++) *reinterpret_cast<__half*>(t + tile_inner_off(hc + i, pos & 63)) = hv[i];
-						}
-					}
-					if (region == 0 && g.q_lo) {
-						__half2 l[8];
-#pragma unroll
-						for (int i = 0; i < 8; i++) {
-							const float2 f = __half22float2(h[i]);
-							l[i] = __floats2half2_rn(v[2 * i] - f.x, v[2 * i + 1] - f.y);
-						}
-						uint4* dl = reinterpret_cast<uint4*>(g.q_lo + (size_t) m * g.q_dim + j0);
-						dl[0] = reinterpret_cast<const uint4*>(l)[0];
-						dl[1] = reinterpret_cast<const uint4*>(l)[1];
-					}
-				}
+				tc_fence_before();
+				__syncwarp();
+				if (lane == 0) mb_arrive(&tempty[acc]);
+				cluster_barrier();
+				if (quad * 32 < rows) gemm_epilogue<GROUPED>(g, AccCluster{s_u32(own), ks}, mt, nt, quad * 32 + lane, rank, ks);
+				asm volatile("fence.proxy.async;" ::: "memory"); // the next tile's copies land where the sums lay
+				cluster_barrier();
 			} else {
-				for (int c = 0; c < GB_N; c += 32) { // 32 columns = one full 128-byte line per thread
-					float v[32];
-					tmem_ld32(taddr + c, v);
-					const int n0 = nt * GB_N + c;
-					if (!mrow || n0 >= g.N) continue;
-					float* o = g.out + (size_t) (GROUPED ? g.gtiles[3 * mt + 1] + quad * 32 + lane : m - g.out_row0) * g.ldo + n0;
-#pragma unroll
-					for (int i = 0; i < 32; i += 4) {
-						if (n0 + i >= g.N) break;
-						float4 r = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-						if (g.epi == GEPI_RESID) {
-							const float4 x = *reinterpret_cast<const float4*>(o + i);
-							r.x += x.x; r.y += x.y; r.z += x.z; r.w += x.w; // infer.cpp:450-452, :492-494
-						}
-						*reinterpret_cast<float4*>(o + i) = r;
-					}
-				}
+				gemm_epilogue<GROUPED>(g, AccTmem{taddr}, mt, nt, quad * 32 + lane, 0, 1);
+				tc_fence_before();
+				__syncwarp();
+				if (lane == 0) mb_arrive(&tempty[acc]);
 			}
-			tc_fence_before();
-			__syncwarp();
-			if (lane == 0) mb_arrive(&tempty[acc]);
 			acc ^= 1;
 			if (acc == 0) acc_phase ^= 1;
 		}
@@ -1389,16 +1460,80 @@ static int launch_gemm_inst(const GemmArgs& g, int grid, cudaStream_t s) {
 	gemm_tc_kernel<NA, NB, GROUPED><<<grid, GEMM_THREADS, GemmCfg<NA, NB>::SMEM, s>>>(g);
 	return XALM_OK;
 }
+constexpr int GEMM_MAX_SPLIT = 8; // the portable cluster size
+template <int NA, int NB>
+static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int grid, int ks, cudaStream_t s) {
+	static_assert(GB_M * GB_N * 4 <= GemmCfg<NA, NB>::NS * GemmCfg<NA, NB>::STAGE, "a tile's sums fit where the ring lay");
+	cfg->gridDim = dim3((unsigned) grid);
+	cfg->blockDim = dim3(GEMM_THREADS);
+	cfg->dynamicSmemBytes = GemmCfg<NA, NB>::SMEM;
+	cfg->stream = s;
+	at->id = cudaLaunchAttributeClusterDimension;
+	at->val.clusterDim.x = (unsigned) ks; at->val.clusterDim.y = 1; at->val.clusterDim.z = 1;
+	cfg->attrs = at;
+	cfg->numAttrs = 1;
+}
+// How many CTAs, one cluster, share a tile's K steps.  Few tiles (short prompts, narrow matrices) leave SMs idle while a CTA's time is its K steps, each
+// of which waits for the 48 to 96 KB that one SM draws in.  (Splitting the columns instead would read the activations once per part.)  Each CTA sums its
+// share of the steps, the sums are joined through distributed shared memory and every CTA finishes its share of the columns: there is no workspace,
+// and the order of the sum does not depend on who is first.
+// The rule estimates waves x (K steps + join), with as many clusters at a time as the device says fit; STEP and the join's 4 us + 0.5 us per CTA are
+// fitted to back-to-back launches, us without -> with the split chosen (planes of activations / weights; tokens x columns x K):
+//   1/1: 45 x 1024 x 4096 24.7 -> 12.4 (8 CTAs), 256 x 2048 x 2048 18.5 -> 14.4 (4), 1024 x 1024 x 4096 26.7 -> 18.5 (4), 1024 x 2048 x 8192 45.2 -> 30.8 (2)
+//   2/1: 33 x 4096 x 4096 42.0 -> 18.5 (5), 333 x 4096 x 4096 45.2 -> 30.0 (2), 333 x 4096 x 14336 139 -> 78 (5, two waves)
+//   2/2: 33 x 4096 x 14336 242 -> 57 (6), 333 x 6144 x 4096 82 -> 49 (2), 500 x 2048 x 6144 94 -> 37 (4)
+// From about 80 tiles on, and for 16 K steps with 8 tiles and more, one CTA per tile is as fast or faster and the rule says so.
+template <int NA, int NB>
+static int gemm_split(int tiles, int KT) {
+	static std::atomic<int> fits[GEMM_MAX_SPLIT + 1]; // clusters of this size that run at a time, 0: not asked yet
+	constexpr float STEP = NA == 1 ? 0.36f : NB == 1 ? 0.58f : 1.08f; // us
+	const float whole = (float) cdiv(tiles, sm_count()) * (float) KT * STEP;
+	int best = 1;
+	float best_us = whole;
+	for (int ks = 2; ks <= GEMM_MAX_SPLIT && ks <= KT && tiles * ks <= 2 * sm_count(); ks++) {
+		int n = fits[ks].load(std::memory_order_relaxed);
+		if (!n) {
+			cudaLaunchConfig_t cfg = {};
+			cudaLaunchAttribute at[1];
+			gemm_cluster_config<NA, NB>(&cfg, at, sm_count() / ks * ks, ks, nullptr);
+			if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<NA, NB, false, true>, &cfg) != cudaSuccess || n <= 0) {
+				cudaGetLastError();
+				n = -1;
+			}
+			fits[ks].store(n, std::memory_order_relaxed);
+		}
+		if (n <= 0) continue;
+		const float us = (float) cdiv(tiles, n) * ((float) cdiv(KT, ks) * STEP + 4.f + 0.5f * (float) ks);
+		if (us < best_us) { best_us = us; best = ks; }
+	}
+	return best;
+}
+template <int NA, int NB>
+static int launch_gemm_planes(const GemmArgs& g, int tiles, cudaStream_t s) {
+	static std::atomic<bool> attr{false};
+	if (!attr.load()) {
+		XALM_CUDA_CHECK(cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM));
+		attr.store(true);
+	}
+	const int ks = gemm_split<NA, NB>(tiles, g.KT);
+	cudaError_t e;
+	if (ks > 1) {
+		cudaLaunchConfig_t cfg = {};
+		cudaLaunchAttribute at[1];
+		gemm_cluster_config<NA, NB>(&cfg, at, std::min(tiles, sm_count() / ks) * ks, ks, s);
+		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, false, true>, g);
+	} else {
+		XALM_TRY((launch_gemm_inst<NA, NB>(g, std::min(tiles, sm_count()), s)));
+		e = cudaGetLastError();
+	}
+	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "gemm_tc launch failed: %s", cudaGetErrorString(e));
+	return XALM_OK;
+}
 static int launch_gemm(const GemmArgs& g, int na, int nb, cudaStream_t s) {
 	const int tiles = g.MT * g.NT;
 	if (tiles <= 0) return XALM_OK;
-	const int grid = std::min(tiles, sm_count());
-	if (na == 2 && nb == 2) XALM_TRY((launch_gemm_inst<2, 2>(g, grid, s)));
-	else if (na == 2) XALM_TRY((launch_gemm_inst<2, 1>(g, grid, s)));
-	else XALM_TRY((launch_gemm_inst<1, 1>(g, grid, s)));
-	cudaError_t e = cudaGetLastError();
-	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "gemm_tc launch failed: %s", cudaGetErrorString(e));
-	return XALM_OK;
+	if (na == 2 && nb == 2) return launch_gemm_planes<2, 2>(g, tiles, s);
+	return na == 2 ? launch_gemm_planes<2, 1>(g, tiles, s) : launch_gemm_planes<1, 1>(g, tiles, s);
 }
 
 // weights of `w` (rows [0, n_valid) or the GLU pairing) -> B tiles in `dst` (+ rounding residuals in dst_lo when not NULL)
