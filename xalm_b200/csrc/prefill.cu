@@ -18,9 +18,9 @@
 // Operand layout ("A tiles"/"B tiles"): 128 (A) or 256 (B) rows x 64 K-elements of fp16, stored as the exact
 // shared-memory image tcgen05.mma wants for a K-major SWIZZLE_128B operand (8-row x 128-byte atoms, 16-byte chunks
 // XOR-swizzled by row%8), tile after tile.  One cp.async.bulk (TMA engine) brings a whole 16/32 KB tile into shared
-// memory — no tensor map, no per-thread staging.  Weights are dequantised from their decode layout into B tiles once
-// per GEMM (dequant_tiles_kernel: every format the decode path takes), which costs 2 bytes written + read per weight
-// against 2*T flops per weight: ~10 % of the GEMM at T = 4096.
+// memory, without per-thread staging.  fp16 weights are cut out of their rows by a tensor map (weight_map); other formats are dequantised from
+// their decode layout into B tiles once per GEMM (dequant_tiles_kernel: every format the decode path takes), which costs 2 bytes written + read per
+// weight and plane against 2*T flops per weight: ~10 % of the GEMM at T = 4096.
 //
 // Numerics: tensor-core operands are fp16 with fp32 accumulation.  split=1 rounds every operand to fp16 (fastest; ten rounding
 // stages per layer add up to ~4e-2 on the logits of a 32-layer model).  split=2 keeps the activations to ~fp32 by feeding
@@ -28,6 +28,7 @@
 // (hi.hi + lo.hi + hi.lo) and for q and the softmax probabilities in attention: logits within ~1e-3 of the token-at-a-time
 // fp32 path at 32 layers x 4096 tokens.  Tolerance in tests: 1e-2 (north star: "within max-abs 1e-2 (fp16)").
 #define XALM_SECONDARY_TU
+#include <cuda.h> // CUtensorMap: types only, the encoder is asked of the runtime
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <float.h>
@@ -263,6 +264,12 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 	             "r"(bytes), "r"(s_u32(bar))
 	             : "memory");
 }
+// box of a row-major matrix (elements k0.., rows r0..) -> shared memory as the swizzled K-major operand image; k0 is a multiple of 64 elements
+__device__ __forceinline__ void tensor_load(void* dst, const CUtensorMap* map, int k0, int r0, uint64_t* bar) {
+	asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(s_u32(dst)), "l"(map), "r"(k0),
+	             "r"(r0), "r"(s_u32(bar))
+	             : "memory");
+}
 // one lane of a converged warp (elect.sync): lets the compiler keep the tcgen05 issue in a warp-uniform branch
 __device__ __forceinline__ bool elect_one() {
 	uint32_t pred;
@@ -389,7 +396,9 @@ enum { GEPI_STORE = 0, GEPI_RESID = 1, GEPI_GLU = 2, GEPI_QKV = 3, GEPI_ACT = 4 
 struct GemmArgs {
 	const uint8_t* a_hi;
 	const uint8_t* a_lo;
-	const uint8_t* b;
+	const uint8_t* b;    // NULL: one weight plane, its tiles cut out of the row-major fp16 matrix by the kernel's tensor map
+	int b_box;          // rows of the map's box: GB_N, or GB_N / 2 where a tile takes two (rows nt * b_box of the matrix and of glu_off)
+	int glu_off;
 	const uint8_t* b_lo; // residual plane of the weights (NB = 2)
 	int MT, NT, KT;     // tile counts; M tiles are [mt0, mt0 + MT)
 	int mt0;
@@ -604,7 +613,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 
 // GROUPED: M tiles come from a list, each with a matrix of its own.  SPLIT: the CTAs of a cluster share a tile's K steps (gemm_split)
 template <int NA, int NB, bool GROUPED = false, bool SPLIT = false>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs g) {
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap b_map) {
 	using Cfg = GemmCfg<NA, NB>;
 	constexpr int NS = Cfg::NS;
 	extern __shared__ uint8_t smem_raw[];
@@ -661,7 +670,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 					mb_expect_tx(&full[slot], Cfg::STAGE);
 					bulk_load(st, ah + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
 					if (NA == 2) bulk_load(st + A_TILE_BYTES, al + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
-					bulk_load(st + NA * A_TILE_BYTES, bt + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
+					if (NB == 1 && !GROUPED && !g.b) {
+						tensor_load(st + NA * A_TILE_BYTES, &b_map, kt * GB_K, nt * g.b_box, &full[slot]);
+						if (g.b_box < GB_N) tensor_load(st + NA * A_TILE_BYTES + B_TILE_BYTES / 2, &b_map, kt * GB_K, g.glu_off + nt * g.b_box, &full[slot]);
+					} else bulk_load(st + NA * A_TILE_BYTES, bt + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
 					if (NB == 2) bulk_load(st + NA * A_TILE_BYTES + B_TILE_BYTES, bl + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
 					if (++slot == NS) { slot = 0; phase ^= 1; }
 				}
@@ -1451,13 +1463,13 @@ const float* prefill_logits_dev(const PrefillScratch* s, int* rows) {
 }
 
 template <int NA, int NB, bool GROUPED = false>
-static int launch_gemm_inst(const GemmArgs& g, int grid, cudaStream_t s) {
+static int launch_gemm_inst(const GemmArgs& g, const CUtensorMap& b_map, int grid, cudaStream_t s) {
 	static bool attr = false;
 	if (!attr) {
 		XALM_CUDA_CHECK(cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM));
 		attr = true;
 	}
-	gemm_tc_kernel<NA, NB, GROUPED><<<grid, GEMM_THREADS, GemmCfg<NA, NB>::SMEM, s>>>(g);
+	gemm_tc_kernel<NA, NB, GROUPED><<<grid, GEMM_THREADS, GemmCfg<NA, NB>::SMEM, s>>>(g, b_map);
 	return XALM_OK;
 }
 constexpr int GEMM_MAX_SPLIT = 8; // the portable cluster size
@@ -1482,6 +1494,7 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 //   1/1: 45 x 1024 x 4096 24.7 -> 12.4 (8 CTAs), 256 x 2048 x 2048 18.5 -> 14.4 (4), 1024 x 1024 x 4096 26.7 -> 18.5 (4), 1024 x 2048 x 8192 45.2 -> 30.8 (2)
 //   2/1: 33 x 4096 x 4096 42.0 -> 18.5 (5), 333 x 4096 x 4096 45.2 -> 30.0 (2), 333 x 4096 x 14336 139 -> 78 (5, two waves)
 //   2/2: 33 x 4096 x 14336 242 -> 57 (6), 333 x 6144 x 4096 82 -> 49 (2), 500 x 2048 x 6144 94 -> 37 (4)
+// Against float64 the result is nearer, 2 to 5 times at 4 to 8 shares: the tensor cores' own additions truncate, and a share has fewer of them.
 // From about 80 tiles on, and for 16 K steps with 8 tiles and more, one CTA per tile is as fast or faster and the rule says so.
 template <int NA, int NB>
 static int gemm_split(int tiles, int KT) {
@@ -1509,7 +1522,7 @@ static int gemm_split(int tiles, int KT) {
 	return best;
 }
 template <int NA, int NB>
-static int launch_gemm_planes(const GemmArgs& g, int tiles, cudaStream_t s) {
+static int launch_gemm_planes(const GemmArgs& g, const CUtensorMap& b_map, int tiles, cudaStream_t s) {
 	static std::atomic<bool> attr{false};
 	if (!attr.load()) {
 		XALM_CUDA_CHECK(cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM));
@@ -1521,19 +1534,41 @@ static int launch_gemm_planes(const GemmArgs& g, int tiles, cudaStream_t s) {
 		cudaLaunchConfig_t cfg = {};
 		cudaLaunchAttribute at[1];
 		gemm_cluster_config<NA, NB>(&cfg, at, std::min(tiles, sm_count() / ks) * ks, ks, s);
-		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, false, true>, g);
+		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, false, true>, g, b_map);
 	} else {
-		XALM_TRY((launch_gemm_inst<NA, NB>(g, std::min(tiles, sm_count()), s)));
+		XALM_TRY((launch_gemm_inst<NA, NB>(g, b_map, std::min(tiles, sm_count()), s)));
 		e = cudaGetLastError();
 	}
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "gemm_tc launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
 }
-static int launch_gemm(const GemmArgs& g, int na, int nb, cudaStream_t s) {
+static int launch_gemm(const GemmArgs& g, int na, int nb, cudaStream_t s, const CUtensorMap& b_map = CUtensorMap()) {
 	const int tiles = g.MT * g.NT;
 	if (tiles <= 0) return XALM_OK;
-	if (na == 2 && nb == 2) return launch_gemm_planes<2, 2>(g, tiles, s);
-	return na == 2 ? launch_gemm_planes<2, 1>(g, tiles, s) : launch_gemm_planes<1, 1>(g, tiles, s);
+	if (na == 2 && nb == 2) return launch_gemm_planes<2, 2>(g, b_map, tiles, s);
+	return na == 2 ? launch_gemm_planes<2, 1>(g, b_map, tiles, s) : launch_gemm_planes<1, 1>(g, b_map, tiles, s);
+}
+
+// fp16 rows are their own operand tiles: the copy engine cuts 64-element pieces of box_rows rows out of them and swizzles them on the way, where writing
+// tiles first and reading them back is twice the matrix more traffic (333 tokens of three 7B layers: 1770 -> 1262 us).  false: not this matrix (another type, rows that do not start on 16 bytes, a
+// driver without the encoder); its tiles are written by dequant_tiles_kernel.
+static bool weight_map(const WMat& w, int K, int box_rows, CUtensorMap* map) {
+	typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+	                           CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+	static const Encode encode = [] {
+		void* f = nullptr;
+		cudaDriverEntryPointQueryResult q;
+		if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+			cudaGetLastError();
+			return (Encode) nullptr;
+		}
+		return (Encode) f;
+	}();
+	if (!encode || w.type != XALM_F16 || w.layout_frag || w.layout_units || K % 8 || w.s0 % 16 || (uintptr_t) w.p0 % 16) return false;
+	const cuuint64_t dims[2] = {(cuuint64_t) K, (cuuint64_t) w.rows}, strides[1] = {(cuuint64_t) w.s0};
+	const cuuint32_t box[2] = {GB_K, (cuuint32_t) box_rows}, steps[2] = {1, 1};
+	return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint8_t*>(w.p0), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+	              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // weights of `w` (rows [0, n_valid) or the GLU pairing) -> B tiles in `dst` (+ rounding residuals in dst_lo when not NULL)
@@ -1666,8 +1701,16 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		if (precise) XALM_TRY(sc.q_lo.ensure((size_t) Tp * pm.q_dim * 2, true, s));
 	}
 	XALM_TRY(sc.rope.ensure((size_t) T * (c.head_dim / 2) * sizeof(float2), false, s));
-	size_t wt_tiles = std::max({(size_t) NT_qkv * KT_dim, (size_t) NT_dim * KT_q, (size_t) NT_glu * KT_dim, (size_t) NT_dim * KT_h});
-	if (want_logits) wt_tiles = std::max(wt_tiles, (size_t) NT_cls * KT_dim);
+	CUtensorMap b_map;
+	size_t wt_tiles = 0; // of the matrices whose tiles are written
+	auto need_tiles = [&](const WMat& w, int K, int NT, int KT) {
+		if (!weight_map(w, K, GB_N, &b_map)) wt_tiles = std::max(wt_tiles, (size_t) NT * KT);
+	};
+	for (const PrefillLayer& P : pm.layers) {
+		need_tiles(P.wqkv, c.dim, NT_qkv, KT_dim); need_tiles(P.wo, pm.q_dim, NT_dim, KT_q);
+		need_tiles(P.w13, c.dim, NT_glu, KT_dim); need_tiles(P.w2, c.hidden_dim, NT_dim, KT_h);
+	}
+	if (want_logits) need_tiles(pm.wcls, c.dim, NT_cls, KT_dim);
 	for (int i = 0; i < 2; i++) {
 		XALM_TRY(sc.wt[i].ensure(wt_tiles * B_TILE_BYTES, false, s));
 		if (precise) XALM_TRY(sc.wt_lo[i].ensure(wt_tiles * B_TILE_BYTES, false, s));
@@ -1694,6 +1737,7 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 	int prepared = 0; // weight sets dequantised (issued) so far
 	auto nb_of = [&](const WMat& w) { return precise && w.type != XALM_F16 ? 2 : 1; }; // f16 weights are exact in one plane
 	auto prep = [&](const WMat& w, bool glu, int glu_off, int n_valid, int K, int NT, int KT) -> int {
+		if (weight_map(w, K, glu ? GB_N / 2 : GB_N, &b_map)) return XALM_OK;
 		const int b = prepared & 1;
 		if (prepared >= 2) XALM_CUDA_CHECK(cudaStreamWaitEvent(ds, sc.ev_gemm[b], 0)); // the GEMM that last read this buffer
 		t_begin("dequant");
@@ -1704,8 +1748,17 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		launches++;
 		return XALM_OK;
 	};
-	auto run = [&](GemmArgs& g, const WMat& w) -> int {
+	auto run = [&](GemmArgs& g, const WMat& w, int K, int glu_off) -> int {
 		const int b = job & 1;
+		g.b_box = glu_off ? GB_N / 2 : GB_N;
+		g.glu_off = glu_off;
+		if (weight_map(w, K, g.b_box, &b_map)) {
+			t_begin("gemm_f16");
+			XALM_TRY(launch_gemm(g, na, 1, s, b_map));
+			t_end();
+			launches++;
+			return XALM_OK;
+		}
 		g.b = sc.wt[b].p;
 		g.b_lo = sc.wt_lo[b].p;
 		XALM_CUDA_CHECK(cudaStreamWaitEvent(s, sc.ev_deq[b], 0));
@@ -1744,7 +1797,7 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		if (attn_tc) { g.qt_hi = sc.qt_hi.p; g.qt_lo = precise ? sc.qt_lo.p : nullptr; g.n_qb = n_qb; }
 		const bool tiles_from_epilogue = attn_tc && pos0 == 0 && getenv("XALM_ATTN_RETILE") == nullptr; // later chunks re-tile the whole cache prefix
 		if (tiles_from_epilogue) { g.kt = sc.kt.p; g.vt = sc.vt.p; g.n_kb_total = n_kb_total; }
-		XALM_TRY(run(g, P.wqkv));
+		XALM_TRY(run(g, P.wqkv, c.dim, 0));
 		t_begin("attention");
 		if (attn_tc) {
 			if (!tiles_from_epilogue)
@@ -1762,7 +1815,7 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		g = {};
 		g.a_hi = xb2.hi; g.a_lo = xb2.lo;
 		g.MT = MT; g.NT = NT_dim; g.KT = KT_q; g.M = T; g.N = c.dim; g.epi = GEPI_RESID; g.out = x; g.ldo = c.dim;
-		XALM_TRY(run(g, P.wo));
+		XALM_TRY(run(g, P.wo, pm.q_dim, 0));
 		// ---- feed-forward half ----
 		t_begin("rmsnorm");
 		rmsnorm_rows_kernel<<<norm_grid, 128, 0, s>>>(x, T, c.dim, P.rms_ffn, P.rms_ffn_type, c.norm_eps, xb);
@@ -1771,13 +1824,13 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		g = {};
 		g.a_hi = xb.hi; g.a_lo = xb.lo;
 		g.MT = MT; g.NT = NT_glu; g.KT = KT_dim; g.M = T; g.N = c.hidden_dim; g.epi = GEPI_GLU; g.o = hb; g.act = c.act;
-		XALM_TRY(run(g, P.w13));
+		XALM_TRY(run(g, P.w13, c.dim, P.glu_off));
 		if (l + 1 < L) XALM_TRY(prep_qkv(l + 1));
 		else if (want_logits) XALM_TRY(prep(pm.wcls, false, 0, c.vocab_size, c.dim, NT_cls, KT_dim));
 		g = {};
 		g.a_hi = hb.hi; g.a_lo = hb.lo;
 		g.MT = MT; g.NT = NT_dim; g.KT = KT_h; g.M = T; g.N = c.dim; g.epi = GEPI_RESID; g.out = x; g.ldo = c.dim;
-		XALM_TRY(run(g, P.w2));
+		XALM_TRY(run(g, P.w2, c.hidden_dim, 0));
 		launches += 3;
 	}
 	if (want_logits) {
@@ -1790,7 +1843,7 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		g.mt0 = want_logits == 1 ? MT - 1 : 0;
 		g.MT = want_logits == 1 ? 1 : MT;
 		g.out_row0 = logit_row0;
-		XALM_TRY(run(g, pm.wcls));
+		XALM_TRY(run(g, pm.wcls, c.dim, 0));
 		launches++;
 		if (targets && probs_host) {
 			XALM_TRY(sc.targets.ensure((size_t) T * 4, false, s));
@@ -1837,21 +1890,25 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 int prefill_gemm_dev(const WMat& w, const float* a_dev, int T, float* out_dev, int split, cudaStream_t s) {
 	const int K = w.n, N = w.rows;
 	if (K % 8) return set_error(XALM_ERR_INVALID, "gemm: K %% 8 != 0");
-	const int na = split >= 2 ? 2 : 1, nb = split >= 3 ? 2 : 1;
+	const int na = split >= 2 ? 2 : 1;
 	const int MT = cdiv(T, GB_M), KT = cdiv(K, GB_K), NT = cdiv(N, GB_N);
 	DevBuf ah, al, bt, bl;
+	CUtensorMap b_map;
+	const bool mapped = weight_map(w, K, GB_N, &b_map);
+	const int nb = split >= 3 && !mapped ? 2 : 1;
 	XALM_TRY(ah.ensure((size_t) MT * KT * A_TILE_BYTES, true, s));
 	if (na == 2) XALM_TRY(al.ensure((size_t) MT * KT * A_TILE_BYTES, true, s));
-	XALM_TRY(bt.ensure((size_t) NT * KT * B_TILE_BYTES, false, s));
+	if (!mapped) XALM_TRY(bt.ensure((size_t) NT * KT * B_TILE_BYTES, false, s));
 	if (nb == 2) XALM_TRY(bl.ensure((size_t) NT * KT * B_TILE_BYTES, false, s));
 	ATiles at{ah.p, na == 2 ? al.p : nullptr, KT};
 	pack_a_kernel<<<std::min(cdiv(T * (K / 8), 256), sm_count() * 8), 256, 0, s>>>(a_dev, T, K, at);
-	int rc = launch_dequant_tiles(w, false, 0, N, K, NT, KT, bt.p, nb == 2 ? bl.p : nullptr, s);
+	int rc = mapped ? XALM_OK : launch_dequant_tiles(w, false, 0, N, K, NT, KT, bt.p, nb == 2 ? bl.p : nullptr, s);
 	if (rc == XALM_OK) {
 		GemmArgs g = {};
 		g.a_hi = at.hi; g.a_lo = at.lo; g.b = bt.p; g.b_lo = bl.p;
 		g.MT = MT; g.NT = NT; g.KT = KT; g.M = T; g.N = N; g.epi = GEPI_STORE; g.out = out_dev; g.ldo = N;
-		rc = launch_gemm(g, na, nb, s);
+		g.b_box = GB_N;
+		rc = launch_gemm(g, na, nb, s, b_map);
 	}
 	cudaError_t e = cudaStreamSynchronize(s);
 	ah.release(); al.release(); bt.release(); bl.release();
@@ -1954,8 +2011,8 @@ static int launch_group(const TcGroup& t, const uint8_t* a_hi, const uint8_t* a_
 	g.NT = cdiv(t.N, GB_N); g.KT = t.K / GB_K; g.N = t.N;
 	g.gtiles = t.tiles; g.gn_tiles = t.n_tiles; g.gb = t.b;
 	const int grid = std::min(t.max_tiles * g.NT, sm_count());
-	if (a_lo) XALM_TRY((launch_gemm_inst<2, 1, true>(g, grid, s)));
-	else XALM_TRY((launch_gemm_inst<1, 1, true>(g, grid, s)));
+	if (a_lo) XALM_TRY((launch_gemm_inst<2, 1, true>(g, CUtensorMap(), grid, s)));
+	else XALM_TRY((launch_gemm_inst<1, 1, true>(g, CUtensorMap(), grid, s)));
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "grouped gemm_tc launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
