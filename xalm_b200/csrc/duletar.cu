@@ -225,8 +225,10 @@ int enqueue_retention(Du* m, const Layer& L, int n, int* nl) {
 	ha.norm_plain = 1; ha.eps = m->eps;
 	ha.gate = m->proj; ha.ldg = m->proj_ld; ha.g_off = L.off_g;
 	ha.state = L.state; ha.step = m->d_step; ha.out = m->att; ha.max_rows = m->chunk; ha.rows = n;
-	XALM_TRY(launch_hgrn2(ha, s));
-	(*nl)++;
+	ha.ws = m->rec_ws; ha.ws_floats = m->rec_ws_floats;
+	int launches = 1;
+	XALM_TRY(launch_hgrn2(ha, s, &launches));
+	*nl += launches;
 	return XALM_OK;
 }
 
@@ -312,6 +314,7 @@ int finalize(SeqModel* sm) {
 			if (!hgrn2_cols_ok(d, dv, m->chunk) && hgrn2_smem_bytes(d, dv) > 200 * 1024)
 				return set_error(XALM_ERR_UNSUPPORTED, "layer %zu: a retention state of %d x %d per head", li, d, dv);
 			XALM_TRY(hgrn2_prepare(d, dv));
+			m->rec_ws_floats = std::max(m->rec_ws_floats, hgrn2_chunk_floats(H, d, dv, m->chunk));
 		} else {
 			XALM_TRY(latent_upload(m, p + "mix.", li, &L.lat, &m->lat, &m->parts));
 			if (L.kv_from < 0) XALM_TRY(latent_cache_alloc(m, L.lat, &L.cache));
@@ -345,6 +348,7 @@ int finalize(SeqModel* sm) {
 	XALM_TRY(dev_alloc(m, &m->x, C * W));
 	XALM_TRY(dev_alloc(m, &m->hn, C * W));
 	XALM_TRY(dev_alloc(m, &m->proj, C * m->proj_ld));
+	if (m->rec_ws_floats) XALM_TRY(dev_alloc(m, &m->rec_ws, m->rec_ws_floats));
 	XALM_TRY(latent_alloc(m, &m->lat));
 	XALM_TRY(dev_alloc(m, &m->att, C * max_att));
 	XALM_TRY(dev_alloc(m, &m->ffh, C * max_ff));

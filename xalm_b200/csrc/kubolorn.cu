@@ -289,8 +289,10 @@ int enqueue_gla(Kb* m, const Layer& L, const Run& R, int n, const Fork& fk, int*
 	ha.gate = m->proj; ha.ldg = m->proj_ld; ha.g_off = L.off_g;
 	ha.state = R.state; ha.step = m->d_step; ha.out = m->att; ha.max_rows = m->chunk; ha.rows = n;
 	XALM_TRY(fk.open());
-	XALM_TRY(launch_hgrn2(ha, fk.side()));
-	(*nl)++;
+	ha.ws = m->rec_ws; ha.ws_floats = m->rec_ws_floats;
+	int launches = 1;
+	XALM_TRY(launch_hgrn2(ha, fk.side(), &launches));
+	*nl += launches;
 	return fk.mark();
 }
 
@@ -320,8 +322,9 @@ int enqueue_parallel(Kb* m, const Layer& L, const Run& R, int n, const Fork& fk,
 	ha.keyed = 2; ha.qk_rep = L.sH / L.sG; ha.dt_off = L.off_dt; ha.dt_bias = L.dt_bias; ha.A_log = L.A_log; ha.skip = L.D;
 	ha.eps = m->eps;
 	ha.state = R.state; ha.step = m->d_step; ha.out = m->yssd; ha.max_rows = m->chunk; ha.rows = n;
-	XALM_TRY(launch_hgrn2(ha, side));
-	(*nl)++;
+	ha.ws = m->rec_ws; ha.ws_floats = m->rec_ws_floats;
+	XALM_TRY(launch_hgrn2(ha, side, &launches));
+	*nl += launches;
 	GroupNormArgs g;
 	g.y = m->yssd; g.ldy = L.inner();
 	g.gate = m->proj + L.off_z; g.ldg = m->proj_ld;
@@ -463,6 +466,7 @@ int finalize(SeqModel* sm) {
 			if (!hgrn2_cols_ok(d, dv, m->chunk, true) && hgrn2_smem_bytes(d, dv) > 200 * 1024)
 				return set_error(XALM_ERR_UNSUPPORTED, "layer %zu: a recurrent state of %d x %d per head", li, d, dv);
 			XALM_TRY(hgrn2_prepare(d, dv));
+			m->rec_ws_floats = std::max(m->rec_ws_floats, hgrn2_chunk_floats(H, d, dv, m->chunk));
 			max_proj = std::max(max_proj, (size_t) L.off_alpha + H * d);
 		} else {
 			const int H = L.aH, G = L.aG, d = L.ad, inner = L.inner(), Cc = L.conv_channels();
@@ -495,6 +499,7 @@ int finalize(SeqModel* sm) {
 			if (!hgrn2_cols_ok(L.sN, L.sP, m->chunk, true) && hgrn2_smem_bytes(L.sN, L.sP) > 200 * 1024)
 				return set_error(XALM_ERR_UNSUPPORTED, "layer %zu: a recurrent state of %d x %d per head", li, L.sN, L.sP);
 			XALM_TRY(hgrn2_prepare(L.sN, L.sP));
+			m->rec_ws_floats = std::max(m->rec_ws_floats, hgrn2_chunk_floats(L.sH, L.sN, L.sP, m->chunk));
 			max_proj = std::max(max_proj, (size_t) L.off_conv + Cc);
 			max_yssd = std::max(max_yssd, (size_t) inner);
 			max_hd = std::max(max_hd, (size_t) H * d);
@@ -545,6 +550,7 @@ int finalize(SeqModel* sm) {
 	XALM_TRY(dev_alloc(m, &m->h2, C * W));
 	XALM_TRY(dev_alloc(m, &m->hn, C * W));
 	XALM_TRY(dev_alloc(m, &m->proj, C * m->proj_ld));
+	if (m->rec_ws_floats) XALM_TRY(dev_alloc(m, &m->rec_ws, m->rec_ws_floats));
 	XALM_TRY(dev_alloc(m, &m->att, C * max_att));
 	XALM_TRY(dev_alloc(m, &m->yssd, C * max_yssd));
 	XALM_TRY(dev_alloc(m, &m->ffh, C * max_ff));

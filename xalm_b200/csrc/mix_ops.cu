@@ -156,6 +156,9 @@ int xalm_cuda_hgrn2(float* out, float* state, const float* qz, const float* fz, 
 	a.out = d_out;
 	a.max_rows = T;
 	if (!a.proj || !a.state || !a.step || !d_out) return set_error(XALM_ERR_CUDA, "hgrn2: device allocation failed");
+	a.rows = T;
+	a.ws_floats = hgrn2_chunk_floats(H, d, dv, T);
+	if (a.ws_floats) a.ws = pool.raw<float>(a.ws_floats);
 	XALM_TRY(launch_hgrn2(a, nullptr));
 	XALM_TRY(finish("hgrn2"));
 	XALM_CUDA_CHECK(cudaMemcpy(out, d_out, (size_t) T * H * dv * 4, cudaMemcpyDeviceToHost));
@@ -488,6 +491,9 @@ int xalm_cuda_retention(float* out, float* state, const float* q, const float* k
 		XALM_TRY(launch_rope_heads(ra, T, nullptr));
 	}
 	XALM_TRY(hgrn2_prepare(d, dv));
+	a.rows = T;
+	a.ws_floats = hgrn2_chunk_floats(H, d, dv, T);
+	if (a.ws_floats) a.ws = pool.raw<float>(a.ws_floats);
 	XALM_TRY(launch_hgrn2(a, nullptr));
 	XALM_TRY(finish("retention"));
 	XALM_CUDA_CHECK(cudaMemcpy(out, a.out, (size_t) T * H * dv * 4, cudaMemcpyDeviceToHost));
@@ -814,6 +820,9 @@ int xalm_cuda_keyed_recurrence(float* out, float* state, const float* q, const f
 	a.max_rows = T;
 	if (!a.proj || !a.state || !a.step || !a.out) return set_error(XALM_ERR_CUDA, "keyed_recurrence: device allocation failed");
 	XALM_TRY(hgrn2_prepare(d, dv));
+	a.rows = T;
+	a.ws_floats = hgrn2_chunk_floats(H, d, dv, T);
+	if (a.ws_floats) a.ws = pool.raw<float>(a.ws_floats);
 	XALM_TRY(launch_hgrn2(a, nullptr));
 	XALM_TRY(finish("keyed_recurrence"));
 	XALM_CUDA_CHECK(cudaMemcpy(out, a.out, (size_t) T * H * dv * 4, cudaMemcpyDeviceToHost));

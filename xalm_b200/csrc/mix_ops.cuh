@@ -1363,7 +1363,14 @@ struct Hgrn2Args {
 	int dt_off;
 	const float *dt_bias, *A_log; // (H)
 	const float* skip;   // (H) or NULL
+	float* ws;           // workspace of long passes (hgrn2_chunk_floats), or NULL: they run token by token
+	size_t ws_floats;
 };
+// From this many tokens on a pass goes over its chunks at once (rec_chunk.cu): 43 us for three launches at 48 tokens of 8 heads of 64 x 128 and 46 at 256,
+// where the scan takes 0.6 us per token
+constexpr int HG_CHUNK_ROWS = 80;
+size_t hgrn2_chunk_floats(int H, int d, int dv, int rows); // 0: not this shape
+int launch_hgrn2_chunks(const Hgrn2Args& a, cudaStream_t s);
 constexpr int HG_TC = 8; // tokens staged at a time
 __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 // decay, key factor and query of channel i of head h for one token's row, in a keyed mode
@@ -2425,11 +2432,24 @@ static inline bool hgrn2_cols_ok(int d, int dv, int max_rows, bool keyed = false
 	return nb <= 8 && dpl <= 8 && warps * 32 * regs <= 65536 && max_rows > 0 && hgrn2_cols_smem_bytes(dpl <= 1 ? 1 : dpl <= 2 ? 2 : dpl <= 4 ? 4 : 8, warps, max_rows) <= 160 * 1024;
 }
 
-static inline int launch_hgrn2(const Hgrn2Args& a, cudaStream_t s) {
+// 16-byte loads of every row that the chunked kernels read or write
+static inline bool hgrn2_chunks_ok(const Hgrn2Args& a) {
+	const size_t need = a.ws ? hgrn2_chunk_floats(a.H, a.d, a.dv, a.rows) : 0;
+	const int cols = a.ld | a.d | a.dv | a.q_off | a.v_off | (a.keyed || a.decay ? a.k_off : 0) | (a.decay || a.keyed == 2 ? 0 : a.f_off);
+	const uintptr_t at = (uintptr_t) a.proj | (uintptr_t) a.out | (uintptr_t) a.state | (uintptr_t) a.ws;
+	return need && need <= a.ws_floats && cols % 4 == 0 && at % 16 == 0;
+}
+// *launches: the kernels launched
+static inline int launch_hgrn2(const Hgrn2Args& a, cudaStream_t s, int* launches = nullptr) {
+	if (launches) *launches = 1;
 	const int warps = hgrn2_cols_warps(a.dv);
 	const int nb = (a.dv + warps * HG_CW - 1) / (warps * HG_CW);
 	const int dpl = (a.d + 31) / 32;
 	if (a.keyed && a.H % std::max(a.qk_rep, 1)) return set_error(XALM_ERR_INVALID, "recurrence: %d heads in groups of %d", a.H, a.qk_rep);
+	if (hgrn2_chunks_ok(a)) {
+		if (launches) *launches = 3;
+		return launch_hgrn2_chunks(a, s);
+	}
 	if (hgrn2_cols_ok(a.d, a.dv, a.max_rows, a.keyed != 0)) {
 		if (a.keyed) {
 			if (dpl <= 1) return launch_hgrn2_cols<1, 1>(a, warps, nb, s);

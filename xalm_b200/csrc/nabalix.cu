@@ -230,8 +230,10 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 			XALM_CUDA_CHECK(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
 			pdl_block(m->side);
 		}
-		XALM_TRY(launch_hgrn2(ha, overlap ? m->side : s));
-		(*nl)++;
+		ha.ws = m->rec_ws; ha.ws_floats = m->rec_ws_floats;
+		int rec_launches = 1;
+		XALM_TRY(launch_hgrn2(ha, overlap ? m->side : s, &rec_launches));
+		*nl += rec_launches;
 		if (overlap) XALM_CUDA_CHECK(cudaEventRecord(m->ev_join, m->side));
 		int swa_launches = 1;
 		XALM_TRY(launch_swa(sa, n, m->precision == XALM_PRECISION_F32, s, &swa_launches));
@@ -346,6 +348,7 @@ int finalize(SeqModel* sm) {
 			return set_error(XALM_ERR_UNSUPPORTED, "layer %zu: recurrence state needs %zu bytes of shared memory", li, hsm);
 		XALM_TRY(swa_prepare(H, d, dv));
 		XALM_TRY(hgrn2_prepare(dr, dvr));
+		m->rec_ws_floats = std::max(m->rec_ws_floats, hgrn2_chunk_floats(Hr, dr, dvr, m->chunk));
 	}
 	XALM_TRY(hc_norm_prepare(W));
 	for (Layer& L : m->layers) {
@@ -363,6 +366,7 @@ int finalize(SeqModel* sm) {
 	XALM_TRY(dev_alloc(m, &m->xs, (size_t) S * C * W));
 	XALM_TRY(dev_alloc(m, &m->h, C * W));
 	XALM_TRY(dev_alloc(m, &m->proj, C * m->proj_ld));
+	if (m->rec_ws_floats) XALM_TRY(dev_alloc(m, &m->rec_ws, m->rec_ws_floats));
 	XALM_TRY(dev_alloc(m, &m->att, C * max_att));
 	XALM_TRY(dev_alloc(m, &m->ro, C * max_ro));
 	XALM_TRY(dev_alloc(m, &m->ol, C * W));

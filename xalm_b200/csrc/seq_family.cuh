@@ -88,6 +88,8 @@ struct SeqModel { // what a handle of these families points to (ModelHead first)
 	uint8_t *a_hi = nullptr, *a_lo = nullptr; // activation operand planes of the tensor-core path
 	float* tc_out = nullptr;                  // its plain fp32 product, when an epilogue follows
 	size_t tc_a_bytes = 0, tc_cols = 4;       // what the registered weights need of them
+	float* rec_ws = nullptr;                  // workspace of a pass's recurrences; a layer's has been joined before the next layer's starts
+	size_t rec_ws_floats = 0;
 	int tc_min_rows = 32;
 	float* final_norm = nullptr;
 	int chunk = 256;                          // most positions of one pass
