@@ -287,8 +287,10 @@ int enqueue_pass(SeqModel* sm, int n, int want, int* nl) {
 			da.eps = m->eps; da.unit_eps = 1e-6f; da.q_scale = 1.f / sqrtf((float) d);
 			da.conv_state = L.conv_state; da.state = L.state;
 			da.prep = m->prep; da.ldp = m->prep_ld; da.out = m->att; da.step = m->d_step;
-			XALM_TRY(launch_delta(da, n, s));
-			*nl += 2;
+			da.ws = m->rec_ws; da.ws_floats = m->rec_ws_floats;
+			int launches = 2;
+			XALM_TRY(launch_delta(da, n, s, &launches));
+			*nl += launches;
 		}
 		est.out = m->y; est.ldo = W;
 		XALM_TRY(rows_product(m, m->att, H * dv, L.w_o, &L.t_o, n, W, H * dv, est, nl));
@@ -372,6 +374,7 @@ int finalize(SeqModel* sm) {
 			XALM_TRY(dev_alloc(m, &L.state, (size_t) H * d * dv, true));
 			XALM_TRY(dev_alloc(m, &L.conv_state, (size_t) std::max(1, L.taps - 1) * (2 * G * d + H * dv), true));
 			XALM_TRY(delta_prepare(d, dv));
+			m->rec_ws_floats = std::max(m->rec_ws_floats, delta_chunk_floats(H, d, dv, m->chunk));
 			max_prep = std::max(max_prep, (size_t) 2 * G * d + H * dv + 2 * H);
 		}
 		XALM_TRY(upload_rows(m, {T(p + "mix.o")}, H * dv, false, &L.w_o, &L.m_o));
@@ -403,6 +406,7 @@ int finalize(SeqModel* sm) {
 	XALM_TRY(dev_alloc(m, &m->xavg, C * W));
 	XALM_TRY(dev_alloc(m, &m->proj, C * m->proj_ld));
 	XALM_TRY(dev_alloc(m, &m->prep, C * m->prep_ld));
+	if (m->rec_ws_floats) XALM_TRY(dev_alloc(m, &m->rec_ws, m->rec_ws_floats));
 	XALM_TRY(dev_alloc(m, &m->att, C * max_att));
 	XALM_TRY(dev_alloc(m, &m->y, C * W));
 	XALM_TRY(dev_alloc(m, &m->ffh, C * max_ff));

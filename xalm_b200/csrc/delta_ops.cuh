@@ -11,7 +11,7 @@
 // A column of S evolves on its own (u_c needs only S[:, c]): one to four neighbouring lanes own a column, its d values in their registers
 // (d <= 256; beyond that in shared memory), k and q of the token are broadcast from shared memory, and the only sums across lanes are
 // the two dot products inside a column's lanes and the per-head norm.
-// The scan is sequential in the tokens by construction: the state keeps the exact fp32 recurrence.  Everything is fp32 (expf, log1pf).
+// The scan is sequential in the tokens by construction: the state keeps the exact fp32 recurrence.  Long passes: delta_chunk.cu.  Everything is fp32 (expf, log1pf).
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -38,7 +38,13 @@ struct DeltaArgs {
 	int ldp;
 	float* out;        // (T, H * dv)
 	const SeqStep* step;
+	float* ws;         // workspace of long passes (delta_chunk_floats), or NULL: they run token by token
+	size_t ws_floats;
 };
+// From this many tokens on a pass goes chunk by chunk (delta_chunk.cu): 30 us for its three kernels at 64 tokens of 8 heads of 64 x 128, the scan 39 us at 63
+constexpr int DELTA_CHUNK_ROWS = 64;
+size_t delta_chunk_floats(int H, int d, int dv, int rows); // 0: not this shape
+int launch_delta_chunks(const DeltaArgs& a, int rows, cudaStream_t s);
 
 
 // grid (tokens, 2 G + H): a CTA convolves one head — a q head, a k head (both scaled to unit length afterwards) or a v head; the CTA of
@@ -286,11 +292,21 @@ static inline int delta_prepare(int d, int dv) { // outside a stream capture
 	}
 	return XALM_OK;
 }
-// rows: tokens of the step (host-side bound); two launches
-static inline int launch_delta(const DeltaArgs& a, int rows, cudaStream_t s) {
+// The chunked kernels copy 16 bytes at a time out of prep; the convolutions' state comes from the pass alone
+static inline bool delta_chunks_ok(const DeltaArgs& a, int rows) {
+	const size_t need = a.ws ? delta_chunk_floats(a.H, a.d, a.dv, rows) : 0;
+	return need && need <= a.ws_floats && (a.ldp | a.d | a.dv) % 4 == 0 && ((uintptr_t) a.prep | (uintptr_t) a.ws) % 16 == 0 && a.taps <= DELTA_CHUNK_ROWS;
+}
+// rows: tokens of the step (host-side bound).  *launches: the kernels launched
+static inline int launch_delta(const DeltaArgs& a, int rows, cudaStream_t s, int* launches = nullptr) {
+	if (launches) *launches = 2;
 	if (a.H % a.G || a.taps < 1 || !delta_ok(a.d, a.dv)) return set_error(XALM_ERR_UNSUPPORTED, "delta rule: heads %d / %d, state %d x %d", a.H, a.G, a.d, a.dv);
 	launch_step(delta_prep_kernel, dim3(rows, 2 * a.G + a.H), 128, 0, s, rows, a);
 	XALM_TRY(launch_check("delta_prep"));
+	if (delta_chunks_ok(a, rows)) {
+		if (launches) *launches = 4;
+		return launch_delta_chunks(a, rows, s);
+	}
 	const DeltaShape z = delta_shape(a.d, a.dv);
 	const size_t smem = delta_rule_smem(a.d, a.dv);
 #define XALM_DELTA_LAUNCH(DS_, NS_) launch_step(delta_rule_kernel<DS_, NS_>, a.H, z.threads, smem, s, rows, a)

@@ -330,7 +330,9 @@ int xalm_cuda_delta_rule(float* out, float* state, float* conv_state, const floa
 	const size_t ncs = (size_t) std::max(1, taps - 1) * Cc;
 	a.conv_state = pool.put(conv_state, ncs);
 	a.state = pool.put(state, (size_t) H * d * dv);
-	a.ldp = Cc + 2 * H;
+	a.ldp = (Cc + 2 * H + 3) / 4 * 4;
+	a.ws_floats = delta_chunk_floats(H, d, dv, T);
+	if (a.ws_floats) a.ws = pool.raw<float>(a.ws_floats);
 	a.prep = pool.raw<float>((size_t) T * a.ldp);
 	a.out = pool.raw<float>((size_t) T * nv);
 	a.step = pool.put(&st, 1);
