@@ -2263,11 +2263,12 @@ static inline bool swa_one_ok(const SwaArgs& a, int rows) {
 }
 
 // swa_mma.cu: passes of many tokens over a bf16 cache, on the tensor cores.  It takes heads of 32 to 128 channels in whole 16-byte pieces whose scores
-// do not mix, and fills a warp's 16 queries; smaller heads would be mostly padding.  Takes a.n_splits > 0
+// do not mix; smaller heads would be mostly padding.  From 5 tokens on, since a tile that is mostly padding still beats the tiled kernel: 9 tokens of 16 heads of
+// 128 over 777 keys 165 -> 25 us.  Takes a.n_splits > 0
 int launch_swa_mma(const SwaArgs& a, int rows, cudaStream_t s);
 constexpr int SWA_MMA_ROWS = 64, SWA_MMA_KEYS = 64; // queries of one head per CTA; keys per step
 static inline bool swa_mma_ok(const SwaArgs& a, int rows, bool cache_f32) {
-	return !cache_f32 && rows >= 16 && !a.talk && std::min(a.d, a.dv) >= 32 && std::max(a.d, a.dv) <= 128 && ((a.d | a.dv | a.ldk | a.ldv) & 7) == 0 &&
+	return !cache_f32 && rows > 4 && !a.talk && std::min(a.d, a.dv) >= 32 && std::max(a.d, a.dv) <= 128 && ((a.d | a.dv | a.ldk | a.ldv) & 7) == 0 &&
 	       ((a.ldq | a.q_off) & 3) == 0 && a.H <= 65535 && ((reinterpret_cast<uintptr_t>(a.kc) | reinterpret_cast<uintptr_t>(a.vc) | reinterpret_cast<uintptr_t>(a.q)) & 15) == 0;
 }
 
@@ -2284,6 +2285,24 @@ static inline int swa_mma_splits(const SwaArgs& a, int rows) {
 	const long long keys = std::min<long long>(a.ring, reach + std::min(rows, SWA_MMA_ROWS)) + a.keep_first; // what a CTA's queries see at most
 	return (int) std::max<long long>(1, std::min({296 / ctas, keys / SWA_MMA_KEYS, (long long) a.part_cap / rows}));
 }
+// A latent for passes of more than the few tokens that swa_one.cu takes: keys that are the values too, of one head of more than the 128 channels above.
+// Takes a.n_splits > 0
+int launch_swa_latent(const SwaArgs& a, int rows, cudaStream_t s);
+constexpr int SWA_LATENT_ROWS = 32; // (query, head) pairs per CTA
+static inline bool swa_latent_ok(const SwaArgs& a, int rows, bool cache_f32) {
+	return !cache_f32 && rows > 4 && !a.talk && a.G == 1 && a.vc == a.kc && (a.ldv ? a.ldv : a.dv) == (a.ldk ? a.ldk : a.d) && a.dv <= a.d && a.dv >= 32 && a.dv <= 512 &&
+	       a.d > 128 && a.d <= 576 && ((a.d | a.dv | a.ldk) & 7) == 0 && ((a.ldq | a.q_off) & 1) == 0 && (reinterpret_cast<uintptr_t>(a.kc) & 15) == 0 &&
+	       (reinterpret_cast<uintptr_t>(a.q) & 7) == 0;
+}
+// CTAs for every SM (two per SM up to 256 channels), each with a block of keys at least
+static inline int swa_latent_splits(const SwaArgs& a, int rows) {
+	if (!a.part_o || !a.part_ml) return 1;
+	const long long ctas = ((long long) rows * a.H + SWA_LATENT_ROWS - 1) / SWA_LATENT_ROWS;
+	long long reach = a.window < 0x7fffffff ? a.window : a.ring;
+	if (a.mask_chunk > 0) reach = std::min<long long>(reach, a.mask_chunk);
+	const long long keys = std::min<long long>(a.ring, reach + std::min(rows, SWA_LATENT_ROWS)) + a.keep_first;
+	return (int) std::max<long long>(1, std::min({(a.d <= 256 ? 296 : 148) / ctas, keys / SWA_MMA_KEYS, (long long) a.part_cap / rows, 65535ll}));
+}
 static inline int launch_swa_merge(const SwaArgs& a, int rows, cudaStream_t s) {
 	launch_step(swa_merge_kernel, dim3(rows, (a.H * a.dv + 127) / 128), 128, 0, s, rows, a);
 	return launch_check("swa_merge");
@@ -2293,6 +2312,12 @@ static inline int launch_swa_merge(const SwaArgs& a, int rows, cudaStream_t s) {
 // launches through *launches (1 or 2) when it is given.
 static inline int launch_swa(SwaArgs a, int rows, bool cache_f32, cudaStream_t s, int* launches = nullptr) {
 	if (a.mask_chunk > 0 && a.keep_first > 0) return set_error(XALM_ERR_UNSUPPORTED, "attention: kept first positions together with chunks");
+	if (swa_latent_ok(a, rows, cache_f32)) {
+		if (a.n_splits <= 0) a.n_splits = swa_latent_splits(a, rows);
+		if (launches) *launches = a.n_splits > 1 ? 2 : 1;
+		XALM_TRY(launch_swa_latent(a, rows, s));
+		return a.n_splits > 1 ? launch_swa_merge(a, rows, s) : XALM_OK;
+	}
 	// One key/value group, no score mixing, more than a few rows, and all heads together do not fit a CTA's shared memory in the tiled kernel
 	// (many heads over a wide latent): the heads run in 2, 4 or 8 launches, each a smaller attention of its own on its share of the query
 	// and output columns, with its own slice of the partial buffers and ticket counters.

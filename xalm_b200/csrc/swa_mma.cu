@@ -29,9 +29,17 @@ __device__ __forceinline__ void smm_ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
 	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 __device__ __forceinline__ void smm_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-	asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+	asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
 	             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
 	             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the three planes of A times two pairs of fragments of B (four tiles of 8 columns), small planes first; four sums at a time, so that a product does not wait
+// for the one before it
+__device__ __forceinline__ void smm_planes(float (&part)[4][4], const uint32_t (&a)[3][4], const uint32_t (&b)[2][4]) {
+#pragma unroll
+	for (int pl = 2; pl >= 0; pl--)
+#pragma unroll
+		for (int x = 0; x < 4; x++) smm_mma(part[x], a[pl], b[x >> 1][2 * (x & 1)], b[x >> 1][2 * (x & 1) + 1]);
 }
 // two fp32 values as three pairs of bf16 whose sums are the values
 __device__ __forceinline__ void smm_split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -79,42 +87,98 @@ __device__ __forceinline__ void smm_store(const SwaArgs& a, int t, int h, int sp
 	if (a.gate) v *= swa_gate(a, t, h, col);
 	a.out[(size_t) t * (a.ldo ? a.ldo : a.H * a.dv) + (size_t) h * a.dv + col] = v;
 }
-// The CTA's nq queries by fp32 FMAs, a warp per query, keys that a query does not see left out: for infinities and NaN, whose planes are not finite and
-// whose product with a masked key's weight of zero is NaN.
+// Rows first, first + step, ... of a tile from shared memory (row r at os + r * LDS_, its l and m at lm[2 r]) to their places, a warp a row, four neighbouring
+// columns a lane; place(r, t, h) says whose row it is.  What a row's columns share (the softmax's denominator with the sink, a head's gate) is worked out
+// once.  (swa_mma_kernel's rows of 128 channels at most are no faster this way.)
+template <int LDS_, typename Place>
+__device__ __forceinline__ void smm_store_rows(const SwaArgs& a, const float* os, const float* lm, int first, int step, int nrows, int sp, Place place) {
+	const int lane = threadIdx.x & 31, dv = a.dv, ldo = a.ldo ? a.ldo : a.H * dv;
+	float* out = a.n_splits > 1 ? a.part_o : a.out;
+	const bool wide = ((ldo | dv) & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+#pragma unroll 1
+	for (int r = first; r < nrows; r += step) {
+		int t, h;
+		place(r, t, h);
+		const float l = lm[2 * r], m = lm[2 * r + 1];
+		float c = 1.f, den = 1.f, g = 1.f;
+		size_t at;
+		if (a.n_splits > 1) { // swa_merge_kernel joins them
+			at = ((size_t) t * a.n_splits + sp) * (a.H * dv) + (size_t) h * dv;
+			if (lane == 0) {
+				float* pml = a.part_ml + ((size_t) t * a.n_splits + sp) * (a.H * 2) + 2 * h;
+				pml[0] = m;
+				pml[1] = l;
+			}
+		} else { // as swa_finish
+			at = (size_t) t * ldo + (size_t) h * dv;
+			den = l;
+			if (a.sink) {
+				const float sk = a.sink[h];
+				if (sk > m) {
+					c = expf(m - sk);
+					den = fmaf(den, c, 1.f);
+				} else den += expf(sk - m);
+			}
+			if (a.gate && a.gate_per_head) g = swa_gate(a, t, h, 0);
+		}
+#pragma unroll 1
+		for (int col = lane * 4; col < dv; col += 128) {
+			const float4 x = *reinterpret_cast<const float4*>(os + r * LDS_ + col);
+			float o[4] = {x.x, x.y, x.z, x.w};
+			if (a.n_splits <= 1) {
+#pragma unroll
+				for (int e = 0; e < 4; e++) {
+					o[e] = o[e] * c / den;
+					if (a.out_scale != 0.f) o[e] *= a.out_scale;
+					if (a.gate) o[e] *= a.gate_per_head ? g : swa_gate(a, t, h, col + e);
+				}
+			}
+			if (wide) *reinterpret_cast<float4*>(out + at + col) = make_float4(o[0], o[1], o[2], o[3]);
+			else
+#pragma unroll
+				for (int e = 0; e < 4; e++) out[at + col + e] = o[e];
+		}
+	}
+}
+// A query by fp32 FMAs on one warp, keys that it does not see left out: for infinities and NaN, whose planes are not finite and whose product with a masked
+// key's weight of zero is NaN.  t: its row, i: its position; DV: the value channels rounded up
+template <int DV>
+__device__ __forceinline__ void smm_nonfinite_row(const SwaArgs& a, const SwaKeys& km, const __nv_bfloat16* kc, const __nv_bfloat16* vc, int ldk, int ldv, int t, int i,
+                                                  int h, int sp, int jb, int je, float slope, float b1, float b2) {
+	const int lane = threadIdx.x & 31;
+	const float* q = a.q + (size_t) t * a.ldq + a.q_off + (size_t) h * a.d;
+	float m = -INFINITY, l = 0.f, o[DV / 32] = {};
+	for (int j0 = jb; j0 < je; j0 += 32) {
+		const int x = min(j0 + lane, je - 1), j = km.pos(x);
+		const bool seen = j0 + lane < je && smm_seen(a, i, j);
+		const __nv_bfloat16* k = kc + (size_t) km.slot(x) * ldk;
+		float s = 0.f;
+		for (int c = 0; c < a.d; c++) s = fmaf(q[c], __bfloat162float(k[c]), s);
+		s = seen ? smm_score(a, s, i, j, slope, b1, b2) : -INFINITY;
+		const float top = fmaxf(m, warp_max(s)), at = top == -INFINITY ? 0.f : top, keep = m == -INFINITY ? 0.f : expf(m - at), p = expf(s - at);
+		l = fmaf(l, keep, warp_sum(p));
+		m = top;
+#pragma unroll
+		for (int c = 0; c < DV / 32; c++) o[c] *= keep;
+		const unsigned sees = __ballot_sync(0xffffffffu, seen);
+		for (int y = 0; y < 32; y++) {
+			const float w = __shfl_sync(0xffffffffu, p, y);
+			if (!(sees >> y & 1)) continue;
+			const __nv_bfloat16* v = vc + (size_t) km.slot(j0 + y) * ldv;
+#pragma unroll
+			for (int c = 0; c < DV / 32; c++)
+				if (c * 32 + lane < a.dv) o[c] = fmaf(w, __bfloat162float(v[c * 32 + lane]), o[c]);
+		}
+	}
+#pragma unroll
+	for (int c = 0; c < DV / 32; c++)
+		if (c * 32 + lane < a.dv) smm_store(a, t, h, sp, c * 32 + lane, o[c], l, m);
+}
+// the CTA's nq queries, a warp per query
 template <int DV, int WARPS>
 __device__ __noinline__ void smm_nonfinite(const SwaArgs a, const SwaKeys km, const __nv_bfloat16* kc, const __nv_bfloat16* vc, int ldk, int ldv, int t0, int nq,
                                               int i_lo, int h, int sp, int jb, int je, float slope, float b1, float b2) {
-	const int lane = threadIdx.x & 31;
-	for (int row = threadIdx.x >> 5; row < nq; row += WARPS) {
-		const int i = i_lo + row;
-		const float* q = a.q + (size_t) (t0 + row) * a.ldq + a.q_off + (size_t) h * a.d;
-		float m = -INFINITY, l = 0.f, o[DV / 32] = {};
-		for (int j0 = jb; j0 < je; j0 += 32) {
-			const int x = min(j0 + lane, je - 1), j = km.pos(x);
-			const bool seen = j0 + lane < je && smm_seen(a, i, j);
-			const __nv_bfloat16* k = kc + (size_t) km.slot(x) * ldk;
-			float s = 0.f;
-			for (int c = 0; c < a.d; c++) s = fmaf(q[c], __bfloat162float(k[c]), s);
-			s = seen ? smm_score(a, s, i, j, slope, b1, b2) : -INFINITY;
-			const float top = fmaxf(m, warp_max(s)), at = top == -INFINITY ? 0.f : top, keep = m == -INFINITY ? 0.f : expf(m - at), p = expf(s - at);
-			l = fmaf(l, keep, warp_sum(p));
-			m = top;
-#pragma unroll
-			for (int c = 0; c < DV / 32; c++) o[c] *= keep;
-			const unsigned sees = __ballot_sync(0xffffffffu, seen);
-			for (int y = 0; y < 32; y++) {
-				const float w = __shfl_sync(0xffffffffu, p, y);
-				if (!(sees >> y & 1)) continue;
-				const __nv_bfloat16* v = vc + (size_t) km.slot(j0 + y) * ldv;
-#pragma unroll
-				for (int c = 0; c < DV / 32; c++)
-					if (c * 32 + lane < a.dv) o[c] = fmaf(w, __bfloat162float(v[c * 32 + lane]), o[c]);
-			}
-		}
-#pragma unroll
-		for (int c = 0; c < DV / 32; c++)
-			if (c * 32 + lane < a.dv) smm_store(a, t0 + row, h, sp, c * 32 + lane, o[c], l, m);
-	}
+	for (int row = threadIdx.x >> 5; row < nq; row += WARPS) smm_nonfinite_row<DV>(a, km, kc, vc, ldk, ldv, t0 + row, i_lo + row, h, sp, jb, je, slope, b1, b2);
 }
 
 // DQ, DV: the channel counts rounded up to 64 or 128 (the rest is zero); WARPS * 16 queries
@@ -195,17 +259,14 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 #pragma unroll
 			for (int pl = 0; pl < 3; pl++) smm_ldsm4(qa[pl], smem_u32(qs) + (uint32_t) pl * ROWS * DQ * 2 + smm_at<DQ>(warp * 16 + (lane & 15), 2 * k + (lane >> 4)));
 #pragma unroll
-			for (int c = 0; c < SMM_KEYS / 16; c++) { // 16 keys
-				uint32_t b[4];
-				float part[2][4] = {};
-				smm_ldsm4(b, kb + smm_at<DQ>(c * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1)));
+			for (int c = 0; c < SMM_KEYS / 16; c += 2) { // 32 keys
+				uint32_t b[2][4];
+				float part[4][4] = {};
 #pragma unroll
-				for (int pl = 2; pl >= 0; pl--) {
-					smm_mma(part[0], qa[pl], b[0], b[1]);
-					smm_mma(part[1], qa[pl], b[2], b[3]);
-				}
+				for (int x = 0; x < 2; x++) smm_ldsm4(b[x], kb + smm_at<DQ>((c + x) * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1)));
+				smm_planes(part, qa, b);
 #pragma unroll
-				for (int x = 0; x < 2; x++)
+				for (int x = 0; x < 4; x++)
 #pragma unroll
 					for (int e = 0; e < 4; e++) s[2 * c + x][e] += part[x][e];
 			}
@@ -253,26 +314,23 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 #pragma unroll
 				for (int e = 0; e < 2; e++) o[c][2 * r + e] *= keep;
 		}
-		uint32_t p[3][SMM_KEYS / 16][4];
+		uint32_t p[SMM_KEYS / 16][3][4];
 #pragma unroll
 		for (int c = 0; c < SMM_KEYS / 16; c++)
 #pragma unroll
-			for (int e = 0; e < 4; e++) smm_split(s[2 * c + (e >> 1)][(e & 1) * 2], s[2 * c + (e >> 1)][(e & 1) * 2 + 1], p[0][c][e], p[1][c][e], p[2][c][e]);
+			for (int e = 0; e < 4; e++) smm_split(s[2 * c + (e >> 1)][(e & 1) * 2], s[2 * c + (e >> 1)][(e & 1) * 2 + 1], p[c][0][e], p[c][1][e], p[c][2][e]);
 		// ---- values ----
 #pragma unroll
-		for (int c = 0; c < DV / 16; c++) { // 16 value channels
+		for (int c = 0; c < DV / 16; c += 2) { // 32 value channels
 #pragma unroll
 			for (int k = 0; k < SMM_KEYS / 16; k++) {
-				uint32_t b[4];
-				float part[2][4] = {};
-				smm_ldsm4_t(b, vb + smm_at<DV>(k * 16 + (lane & 15), 2 * c + (lane >> 4)));
+				uint32_t b[2][4];
+				float part[4][4] = {};
 #pragma unroll
-				for (int pl = 2; pl >= 0; pl--) {
-					smm_mma(part[0], p[pl][k], b[0], b[1]);
-					smm_mma(part[1], p[pl][k], b[2], b[3]);
-				}
+				for (int x = 0; x < 2; x++) smm_ldsm4_t(b[x], vb + smm_at<DV>(k * 16 + (lane & 15), 2 * (c + x) + (lane >> 4)));
+				smm_planes(part, p[k], b);
 #pragma unroll
-				for (int x = 0; x < 2; x++)
+				for (int x = 0; x < 4; x++)
 #pragma unroll
 					for (int e = 0; e < 4; e++) o[2 * c + x][e] += part[x][e];
 			}
@@ -309,6 +367,209 @@ __global__ void __launch_bounds__(WARPS * 32) swa_mma_kernel(SwaArgs a) {
 		for (int col = lane; col < dv; col += 32) smm_store(a, t0 + warp * 16 + row, h, sp, col, os[row * LDO + col], ls[row * 2], ls[row * 2 + 1]);
 }
 static_assert(4 * (64 * (64 + 8) + 4 * 32) <= smm_smem(64, 64, 4) && 4 * (64 * (128 + 8) + 4 * 32) <= smm_smem(64, 128, 4), "the output's rows fit where queries and keys lay");
+
+// ---- a latent: one head of up to 576 channels of keys, whose first channels are the values, for all query heads -------------------------------
+// Rows of a tile are (query, head) pairs, 32 a CTA.  Two groups of W warps, 16 rows each: for the scores a warp takes a W-th of the channels (its queries'
+// planes stay in registers) and all 64 keys of a block, for the output a W-th of the value channels.  The parts of the scores meet in shared memory, where a
+// warp makes its share of the rows' weights of them.  Products and sums as above.
+// Bound: latency of a scheduler's four warps; the mma.sync pipe at 512 channels is next (3072 products of 16 x 8 x 16 per 64 keys).  W = 8 where W = 4 would
+// leave two warps per scheduler (256 tokens of 16 heads of 512 over 256 to 777 keys 93 -> 72 us).  The fp32 FMA tiles of mix_ops.cuh, which took these passes
+// before, and this kernel, caches flushed: 256 tokens of 16 heads of 512 496 -> 72 us, 9 tokens of them over 777 keys 244 -> 19 us, 1024 tokens of 8 heads of 256
+// in a window of 512 357 -> 110 us.  Distance from float64 at 512 channels and 764 keys: within 5 % of the FMA kernel's.
+constexpr int SML_ROWS = SWA_LATENT_ROWS, SML_LDS = SMM_KEYS + 4; // floats of a row of scores
+template <int W, int NK, int NV>
+struct SmlCfg { // NK, NV: 16 channels of keys and of values per warp
+	static constexpr int TH = 2 * W * 32, DQ = W * NK * 16, DV = W * NV * 16, RPW = SML_ROWS / (2 * W); // RPW: rows whose weights a warp makes
+	static constexpr size_t SMEM = (size_t) SMM_STAGES * SMM_KEYS * DQ * 2 + (size_t) W * SML_ROWS * SML_LDS * 4 + (size_t) 3 * SML_ROWS * SMM_KEYS * 2 +
+	                               (size_t) SMM_STAGES * SMM_KEYS * 4 + 4 * SML_ROWS * 4;
+	static constexpr int PER_SM = 2 * (SMEM + 1024) <= 228 * 1024 && TH <= 256 ? 2 : 1;
+};
+template <int DV, int TH>
+__device__ __noinline__ void sml_nonfinite(const SwaArgs a, const SwaKeys km, const __nv_bfloat16* kc, int ldk, int row0, int nrows, int pos0, int sp, int jb, int je) {
+	for (int row = threadIdx.x >> 5; row < nrows; row += TH / 32) {
+		const int t = (row0 + row) / a.H, h = (row0 + row) % a.H;
+		smm_nonfinite_row<DV>(a, km, kc, kc, ldk, ldk, t, pos0 + t, h, sp, jb, je, a.slope ? a.slope[h] : 0.f, a.r1 ? a.r1[h] : 0.f, a.r1 ? a.r2[h] : 0.f);
+	}
+}
+
+template <int W, int NK, int NV>
+__global__ void __launch_bounds__(SmlCfg<W, NK, NV>::TH, SmlCfg<W, NK, NV>::PER_SM) swa_latent_kernel(SwaArgs a) {
+	using Cfg = SmlCfg<W, NK, NV>;
+	extern __shared__ __align__(128) uint8_t smem[];
+	constexpr int TH = Cfg::TH, DQ = Cfg::DQ, DV = Cfg::DV, RPW = Cfg::RPW, LDO = DV + 8;
+	static_assert((size_t) SML_ROWS * LDO * 4 <= (size_t) SMM_STAGES * SMM_KEYS * DQ * 2, "the output's rows fit where the keys lay");
+	uint8_t* ks = smem;                                                                       // stages x SMM_KEYS x DQ
+	float* sc = reinterpret_cast<float*>(ks + (size_t) SMM_STAGES * SMM_KEYS * DQ * 2);       // W parts x SML_ROWS x SML_LDS
+	uint8_t* ps = reinterpret_cast<uint8_t*>(sc + W * SML_ROWS * SML_LDS);                    // 3 planes x SML_ROWS x SMM_KEYS
+	int* kp = reinterpret_cast<int*>(ps + (size_t) 3 * SML_ROWS * SMM_KEYS * 2);              // stages x SMM_KEYS positions (0x7fffffff: no key)
+	float *keeps = reinterpret_cast<float*>(kp + SMM_STAGES * SMM_KEYS), *lm = keeps + SML_ROWS;
+	int* at_row = reinterpret_cast<int*>(lm + 2 * SML_ROWS); // rows' positions
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = lane >> 2, ql = lane & 3, rg = warp / W, qt = warp % W;
+	const int n = a.step->n, pos0 = a.step->pos0, H = a.H, d = a.d, dv = a.dv;
+	const int row0 = ((int) gridDim.x - 1 - (int) blockIdx.x) * SML_ROWS, nrows = min(SML_ROWS, n * H - row0);
+	if (nrows <= 0) return;
+	const int i_lo = pos0 + row0 / H, i_hi = pos0 + (row0 + nrows - 1) / H;
+	const SwaKeys km = swa_keys(a, i_lo);
+	const int nk = km.ks + i_hi - km.j_first + 1;
+	const int per = ((nk + a.n_splits - 1) / a.n_splits + SMM_KEYS - 1) / SMM_KEYS * SMM_KEYS, sp = blockIdx.y;
+	const int jb = min(nk, sp * per), je = min(nk, jb + per);
+	const int ldk = a.ldk ? a.ldk : d;
+	const __nv_bfloat16* kc = reinterpret_cast<const __nv_bfloat16*>(a.kc);
+	auto stage = [&](int j0, int buf) {
+		const uint32_t kb = smem_u32(ks) + (uint32_t) buf * SMM_KEYS * DQ * 2;
+		constexpr int PER = TH / SMM_KEYS;
+		const int row = tid / PER, first = tid % PER;
+		const bool in = j0 + row < je;
+		const int j = min(j0 + row, je - 1);
+		if (first == 0) kp[buf * SMM_KEYS + row] = in ? km.pos(j) : 0x7fffffff;
+		const __nv_bfloat16* kr = kc + (size_t) km.slot(j) * ldk;
+#pragma unroll
+		for (int p = 0; p < DQ / 8; p += PER) {
+			const int ok = in && (p + first) * 8 < d;
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kb + smm_at<DQ>(row, p + first)), "l"(kr + (ok ? (p + first) * 8 : 0)), "r"(ok ? 16 : 0) : "memory");
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	if (jb < je) stage(jb, 0);
+	uint32_t qf[NK][3][4]; // this warp's rows and channels as operand fragments, three planes
+#pragma unroll
+	for (int k = 0; k < NK; k++)
+#pragma unroll
+		for (int e = 0; e < 4; e++) {
+			const int row = rg * 16 + quad + (e & 1) * 8, col = (qt * NK + k) * 16 + ql * 2 + (e >> 1) * 8;
+			float2 v = make_float2(0.f, 0.f);
+			if (row < nrows && col < d) v = *reinterpret_cast<const float2*>(a.q + (size_t) ((row0 + row) / H) * a.ldq + a.q_off + (size_t) ((row0 + row) % H) * d + col);
+			smm_split(v.x, v.y, qf[k][0][e], qf[k][1][e], qf[k][2][e]);
+		}
+	float o[2 * NV][4] = {}; // rows quad, quad + 8 of the group; value channels (qt * NV + ..) * 16 ..
+	float m[RPW], l[RPW]; // of rows RPW warp .. (l: this lane's keys)
+#pragma unroll
+	for (int r = 0; r < RPW; r++) { m[r] = -INFINITY; l[r] = 0.f; }
+	const bool biased = a.r1 || a.slope;
+	if (tid < SML_ROWS) at_row[tid] = pos0 + (row0 + min(tid, nrows - 1)) / H;
+	const int blocks = (je - jb + SMM_KEYS - 1) / SMM_KEYS;
+	for (int blk = 0; blk < blocks; blk++) {
+		const int buf = blk % SMM_STAGES, j0 = jb + blk * SMM_KEYS;
+		asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads(); // the block's keys are there, and nobody reads the block before it any more
+		if (blk + 1 < blocks) stage(j0 + SMM_KEYS, (blk + 1) % SMM_STAGES);
+		const uint32_t kb = smem_u32(ks) + (uint32_t) buf * SMM_KEYS * DQ * 2;
+		{ // ---- scores over this warp's channels ----
+#pragma unroll 1
+			for (int half = 0; half < SMM_KEYS; half += 32) {
+				float s[4][4] = {};
+#pragma unroll
+				for (int k = 0; k < NK; k++) {
+					uint32_t b[2][4];
+					float part[4][4] = {};
+#pragma unroll
+					for (int x = 0; x < 2; x++) smm_ldsm4(b[x], kb + smm_at<DQ>(half + x * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * (qt * NK + k) + ((lane >> 3) & 1)));
+					smm_planes(part, qf[k], b);
+#pragma unroll
+					for (int x = 0; x < 4; x++)
+#pragma unroll
+						for (int e = 0; e < 4; e++) s[x][e] += part[x][e];
+				}
+				float* dst = sc + ((size_t) qt * SML_ROWS + rg * 16 + quad) * SML_LDS + half + ql * 2;
+#pragma unroll
+				for (int c = 0; c < 4; c++)
+#pragma unroll
+					for (int r = 0; r < 2; r++) *reinterpret_cast<float2*>(dst + r * 8 * SML_LDS + c * 8) = make_float2(s[c][2 * r], s[c][2 * r + 1]);
+			}
+		}
+		__syncthreads();
+		// ---- weights: a lane takes two neighbouring keys ----
+#pragma unroll
+		for (int r = 0; r < RPW; r++) {
+			const int row = warp * RPW + r;
+			float z[2] = {};
+#pragma unroll
+			for (int q = 0; q < W; q++) {
+				const float2 v = *reinterpret_cast<const float2*>(sc + ((size_t) q * SML_ROWS + row) * SML_LDS + lane * 2);
+				z[0] += v.x; z[1] += v.y;
+			}
+			const int2 j = *reinterpret_cast<const int2*>(kp + buf * SMM_KEYS + lane * 2);
+			const int i = at_row[row];
+			float slope = 0.f, b1 = 0.f, b2 = 0.f;
+			if (biased) {
+				const int h = (row0 + min(row, nrows - 1)) % H;
+				if (a.slope) slope = a.slope[h];
+				if (a.r1) { b1 = a.r1[h]; b2 = a.r2[h]; }
+			}
+			z[0] = smm_seen(a, i, j.x) ? smm_score(a, z[0], i, j.x, slope, b1, b2) : -INFINITY;
+			z[1] = smm_seen(a, i, j.y) ? smm_score(a, z[1], i, j.y, slope, b1, b2) : -INFINITY;
+			const float top = fmaxf(m[r], warp_max(fmaxf(z[0], z[1]))), at = top == -INFINITY ? 0.f : top, keep = m[r] == -INFINITY ? 0.f : expf(m[r] - at);
+			const float p0 = expf(z[0] - at), p1 = expf(z[1] - at);
+			l[r] = fmaf(l[r], keep, p0 + p1);
+			m[r] = top;
+			if (lane == 0) keeps[row] = keep;
+			uint32_t pl[3];
+			smm_split(p0, p1, pl[0], pl[1], pl[2]);
+#pragma unroll
+			for (int x = 0; x < 3; x++) *reinterpret_cast<uint32_t*>(ps + (size_t) x * SML_ROWS * SMM_KEYS * 2 + smm_at<SMM_KEYS>(row, lane >> 2) + (lane & 3) * 4) = pl[x];
+		}
+		__syncthreads();
+		// ---- values ----
+		const float k0 = keeps[rg * 16 + quad], k1 = keeps[rg * 16 + quad + 8];
+#pragma unroll
+		for (int c = 0; c < 2 * NV; c++) { o[c][0] *= k0; o[c][1] *= k0; o[c][2] *= k1; o[c][3] *= k1; }
+#pragma unroll 1
+		for (int k = 0; k < SMM_KEYS / 16; k++) {
+			uint32_t pa[3][4];
+#pragma unroll
+			for (int pl = 0; pl < 3; pl++) smm_ldsm4(pa[pl], smem_u32(ps) + (uint32_t) pl * SML_ROWS * SMM_KEYS * 2 + smm_at<SMM_KEYS>(rg * 16 + (lane & 15), 2 * k + (lane >> 4)));
+#pragma unroll
+			for (int c = 0; c < NV; c += 2) { // 32 value channels
+				uint32_t b[2][4];
+				float part[4][4] = {};
+#pragma unroll
+				for (int x = 0; x < 2; x++) smm_ldsm4_t(b[x], kb + smm_at<DQ>(k * 16 + (lane & 15), 2 * (qt * NV + c + x) + (lane >> 4)));
+				smm_planes(part, pa, b);
+#pragma unroll
+				for (int x = 0; x < 4; x++)
+#pragma unroll
+					for (int e = 0; e < 4; e++) o[2 * c + x][e] += part[x][e];
+			}
+		}
+	}
+	bool finite = true;
+#pragma unroll
+	for (int r = 0; r < RPW; r++) {
+		l[r] = warp_sum(l[r]);
+		if (warp * RPW + r < nrows) finite &= isfinite(l[r]);
+		if (lane == 0) *reinterpret_cast<float2*>(lm + 2 * (warp * RPW + r)) = make_float2(l[r], m[r]);
+	}
+#pragma unroll
+	for (int r = 0; r < 2; r++)
+		if (rg * 16 + quad + r * 8 < nrows)
+#pragma unroll
+			for (int c = 0; c < 2 * NV; c++) finite &= isfinite(o[c][2 * r]) && isfinite(o[c][2 * r + 1]);
+	if (__syncthreads_or(!finite)) {
+		sml_nonfinite<DV, TH>(a, km, kc, ldk, row0, nrows, pos0, sp, jb, je);
+		return;
+	}
+	float* os = reinterpret_cast<float*>(smem);
+#pragma unroll
+	for (int r = 0; r < 2; r++)
+#pragma unroll
+		for (int c = 0; c < 2 * NV; c++)
+			*reinterpret_cast<float2*>(os + (rg * 16 + quad + r * 8) * LDO + (qt * NV * 2 + c) * 8 + ql * 2) = make_float2(o[c][2 * r], o[c][2 * r + 1]);
+	__syncthreads();
+	smm_store_rows<LDO>(a, os, lm, warp, TH / 32, nrows, sp, [&](int r, int& t, int& h) { t = (row0 + r) / H; h = (row0 + r) % H; });
+}
+
+template <int W, int NK, int NV>
+static int launch_swa_latent_inst(const SwaArgs& a, int rows, cudaStream_t s) {
+	using Cfg = SmlCfg<W, NK, NV>;
+	XALM_CUDA_CHECK(cudaFuncSetAttribute(swa_latent_kernel<W, NK, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) Cfg::SMEM));
+	swa_latent_kernel<W, NK, NV><<<dim3((unsigned) (((long long) rows * a.H + SML_ROWS - 1) / SML_ROWS), a.n_splits), Cfg::TH, Cfg::SMEM, s>>>(a);
+	return launch_check("swa_latent");
+}
+int launch_swa_latent(const SwaArgs& a, int rows, cudaStream_t s) {
+	if (a.d <= 256) return launch_swa_latent_inst<4, 4, 4>(a, rows, s);
+	if (a.d <= 320 && a.dv <= 256) return launch_swa_latent_inst<4, 5, 4>(a, rows, s);
+	return a.d <= 512 ? launch_swa_latent_inst<8, 4, 4>(a, rows, s) : launch_swa_latent_inst<4, 9, 8>(a, rows, s);
+}
 
 template <int DQ, int DV>
 static int launch_swa_mma_inst(const SwaArgs& a, int rows, cudaStream_t s) {
