@@ -2264,7 +2264,7 @@ static inline bool swa_one_ok(const SwaArgs& a, int rows) {
 
 // swa_mma.cu: passes of many tokens over a bf16 cache, on the tensor cores.  It takes heads of 32 to 128 channels in whole 16-byte pieces whose scores
 // do not mix; smaller heads would be mostly padding.  From 5 tokens on, since a tile that is mostly padding still beats the tiled kernel: 9 tokens of 16 heads of
-// 128 over 777 keys 165 -> 25 us.  Takes a.n_splits > 0
+// 128 over 777 keys 165 -> 22 + 4 us.  Takes a.n_splits > 0
 int launch_swa_mma(const SwaArgs& a, int rows, cudaStream_t s);
 constexpr int SWA_MMA_ROWS = 64, SWA_MMA_KEYS = 64; // queries of one head per CTA; keys per step
 static inline bool swa_mma_ok(const SwaArgs& a, int rows, bool cache_f32) {

@@ -391,7 +391,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 //   warps 2-5 epilogue: tcgen05.ld the 128 x 256 fp32 accumulator (one TMEM lane quadrant per warp) and apply the
 //             fused epilogue, while the MMA warp already fills the OTHER accumulator buffer (2 x 256 of the 512 columns)
 // ------------------------------------------------------------------------------------------------------------------
-enum { GEPI_STORE = 0, GEPI_RESID = 1, GEPI_GLU = 2, GEPI_QKV = 3, GEPI_ACT = 4 /* grouped launches */ };
+enum { GEPI_STORE = 0, GEPI_RESID = 1, GEPI_GLU = 2, GEPI_QKV = 3, GEPI_ACT = 4 /* grouped launches */, GEPI_FUSED = 5 /* TcEpi's CAP, ACT, GLU */ };
 
 struct GemmArgs {
 	const uint8_t* a_hi;
@@ -430,6 +430,7 @@ struct GemmArgs {
 	const int* gn_tiles;
 	const uint8_t* const* gb;
 	TcAct gact;
+	TcEpi fused;
 };
 
 constexpr int GEMM_THREADS = 192;
@@ -500,6 +501,29 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 					for (int i = 0; i < 8; i++) h[i] = mix::act_apply(g.gact.act, v[8 * half + i]);
 					store_a8(g.o, m, n0 + 8 * half, h);
 				}
+			}
+		}
+	} else if (!GROUPED && g.epi == GEPI_FUSED) {
+		for (int c = part * 8; c < GB_N; c += parts * 8) {
+			float v[8];
+			acc.get(c, v);
+			const int n0 = nt * GB_N + c;
+			if (!mrow || n0 >= g.N) continue;
+			float* o = g.out + (size_t) (m - g.out_row0) * g.ldo;
+			if (g.fused.kind == TcEpi::GLU) { // N % 8 == 0: eight columns are four values
+#pragma unroll
+				for (int i = 0; i < 4; i++) v[i] = mix::glu_apply(g.fused.act, v[2 * i], v[2 * i + 1], g.fused.limit, g.fused.alpha);
+				*reinterpret_cast<float4*>(o + n0 / 2) = make_float4(v[0], v[1], v[2], v[3]);
+			} else {
+				if (g.fused.kind == TcEpi::CAP) {
+#pragma unroll
+					for (int i = 0; i < 8; i++) v[i] = g.fused.limit * tanhf(v[i] / g.fused.limit);
+				} else {
+#pragma unroll
+					for (int i = 0; i < 8; i++) v[i] = mix::act_apply(g.fused.act, v[i]);
+				}
+				*reinterpret_cast<float4*>(o + n0) = make_float4(v[0], v[1], v[2], v[3]);
+				if (n0 + 4 < g.N) *reinterpret_cast<float4*>(o + n0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
 			}
 		}
 	} else if (g.epi == GEPI_GLU) {
@@ -1970,14 +1994,16 @@ void tc_weight_free(TcWeight* w) {
 }
 size_t tc_a_plane_bytes(int T, int K) { return (size_t) cdiv(T, GB_M) * cdiv(K, GB_K) * A_TILE_BYTES; }
 
-int tc_gemm(const TcWeight& w, const float* a_dev, int T, float* out_dev, int ldo, uint8_t* a_hi, uint8_t* a_lo, cudaStream_t s) {
-	if (!tc_shape_ok(w.N, w.K, ldo) || T <= 0) return set_error(XALM_ERR_INVALID, "tc_gemm: shape (%d x %d) . (%d x %d)^T, ldo %d", T, w.K, w.N, w.K, ldo);
+int tc_gemm(const TcWeight& w, const float* a_dev, int T, float* out_dev, int ldo, uint8_t* a_hi, uint8_t* a_lo, cudaStream_t s, const TcEpi& epi) {
+	if (!tc_shape_ok(w.N, w.K, ldo) || !tc_epi_ok(epi, w.N, ldo, out_dev) || T <= 0) return set_error(XALM_ERR_INVALID, "tc_gemm: shape (%d x %d) . (%d x %d)^T, ldo %d", T, w.K, w.N, w.K, ldo);
 	const int MT = cdiv(T, GB_M);
 	ATiles at{a_hi, a_lo, w.KT};
 	pack_a_kernel<<<std::min(cdiv(T * (w.K / 8), 256), sm_count() * 8), 256, 0, s>>>(a_dev, T, w.K, at);
 	GemmArgs g = {};
 	g.a_hi = a_hi; g.a_lo = a_lo; g.b = w.hi; g.b_lo = w.lo;
-	g.MT = MT; g.NT = w.NT; g.KT = w.KT; g.M = T; g.N = w.N; g.epi = GEPI_STORE; g.out = out_dev; g.ldo = ldo;
+	g.MT = MT; g.NT = w.NT; g.KT = w.KT; g.M = T; g.N = w.N; g.out = out_dev; g.ldo = ldo;
+	g.epi = epi.kind == TcEpi::STORE ? GEPI_STORE : epi.kind == TcEpi::ADD ? GEPI_RESID : GEPI_FUSED;
+	g.fused = epi;
 	return launch_gemm(g, a_lo ? 2 : 1, w.lo ? 2 : 1, s);
 }
 

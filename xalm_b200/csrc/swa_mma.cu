@@ -374,7 +374,7 @@ static_assert(4 * (64 * (64 + 8) + 4 * 32) <= smm_smem(64, 64, 4) && 4 * (64 * (
 // warp makes its share of the rows' weights of them.  Products and sums as above.
 // Bound: latency of a scheduler's four warps; the mma.sync pipe at 512 channels is next (3072 products of 16 x 8 x 16 per 64 keys).  W = 8 where W = 4 would
 // leave two warps per scheduler (256 tokens of 16 heads of 512 over 256 to 777 keys 93 -> 72 us).  The fp32 FMA tiles of mix_ops.cuh, which took these passes
-// before, and this kernel, caches flushed: 256 tokens of 16 heads of 512 496 -> 72 us, 9 tokens of them over 777 keys 244 -> 19 us, 1024 tokens of 8 heads of 256
+// before, and this kernel, caches flushed: 256 tokens of 16 heads of 512 496 -> 72 us, 9 tokens of them over 777 keys 244 -> 24 + 6 us (twelve splits and their join), 1024 tokens of 8 heads of 256
 // in a window of 512 357 -> 110 us.  Distance from float64 at 512 channels and 764 keys: within 5 % of the FMA kernel's.
 constexpr int SML_ROWS = SWA_LATENT_ROWS, SML_LDS = SMM_KEYS + 4; // floats of a row of scores
 template <int W, int NK, int NV>
