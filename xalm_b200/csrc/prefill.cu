@@ -635,7 +635,64 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 	}
 }
 
-// GROUPED: M tiles come from a list, each with a matrix of its own.  SPLIT: the CTAs of a cluster share a tile's K steps (gemm_split)
+// K steps [k_lo, k_hi) of tile (mt, nt) into the ring
+template <int NA, int NB, bool GROUPED>
+__device__ __forceinline__ void gemm_load_steps(const GemmArgs& g, const CUtensorMap& b_map, int mt, int nt, int k_lo, int k_hi, uint8_t* smem, uint64_t* full,
+                                                uint64_t* empty, int& slot, int& phase) {
+	using Cfg = GemmCfg<NA, NB>;
+	const int KT = g.KT;
+	const uint8_t* ah = g.a_hi + (size_t) mt * KT * A_TILE_BYTES;
+	const uint8_t* al = NA == 2 ? g.a_lo + (size_t) mt * KT * A_TILE_BYTES : nullptr;
+	const uint8_t* bt = (GROUPED ? g.gb[g.gtiles[3 * mt]] : g.b) + (size_t) nt * KT * B_TILE_BYTES;
+	const uint8_t* bl = NB == 2 ? g.b_lo + (size_t) nt * KT * B_TILE_BYTES : nullptr;
+	for (int kt = k_lo; kt < k_hi; kt++) {
+		mb_wait(&empty[slot], phase ^ 1);
+		uint8_t* st = smem + (size_t) slot * Cfg::STAGE;
+		mb_expect_tx(&full[slot], Cfg::STAGE);
+		bulk_load(st, ah + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
+		if (NA == 2) bulk_load(st + A_TILE_BYTES, al + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
+		if (NB == 1 && !GROUPED && !g.b) {
+			tensor_load(st + NA * A_TILE_BYTES, &b_map, kt * GB_K, nt * g.b_box, &full[slot]);
+			if (g.b_box < GB_N) tensor_load(st + NA * A_TILE_BYTES + B_TILE_BYTES / 2, &b_map, kt * GB_K, g.glu_off + nt * g.b_box, &full[slot]);
+		} else bulk_load(st + NA * A_TILE_BYTES, bt + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
+		if (NB == 2) bulk_load(st + NA * A_TILE_BYTES + B_TILE_BYTES, bl + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
+		if (++slot == Cfg::NS) { slot = 0; phase ^= 1; }
+	}
+}
+// the next accumulator from the next n K steps of the ring
+template <int NA, int NB>
+__device__ __forceinline__ void gemm_mma_steps(int n, uint32_t tmem_base, uint8_t* smem, uint64_t* full, uint64_t* empty, uint64_t* tfull, uint64_t* tempty, int& slot,
+                                               int& phase, int& acc, int& acc_phase) {
+	using Cfg = GemmCfg<NA, NB>;
+	constexpr uint32_t idesc = instr_desc_f16(GB_M, GB_N);
+	mb_wait(&tempty[acc], acc_phase ^ 1);
+	tc_fence_after();
+	const uint32_t d_tmem = tmem_base + (uint32_t) acc * GB_N;
+	for (int kt = 0; kt < n; kt++) {
+		mb_wait(&full[slot], phase);
+		tc_fence_after();
+		const uint32_t sa = s_u32(smem + (size_t) slot * Cfg::STAGE);
+#pragma unroll
+		for (int p = 0; p < NA + NB - 1; p++) { // (a_hi, b_hi), (a_lo, b_hi), (a_hi, b_lo)
+			const uint64_t adesc = smem_desc(sa + (p == 1 ? A_TILE_BYTES : 0));
+			const uint64_t bdesc = smem_desc(sa + NA * A_TILE_BYTES + (p == 2 ? B_TILE_BYTES : 0));
+#pragma unroll
+			for (int k = 0; k < GB_K / UMMA_K; k++) {
+				// advancing K by 16 fp16 = 32 bytes inside the 128-byte swizzle row: +2 in the (>>4) address field
+				umma_f16(d_tmem, adesc + (uint64_t) (2 * k), bdesc + (uint64_t) (2 * k), idesc, (uint32_t) ((kt | k | p) != 0));
+			}
+		}
+		umma_commit(&empty[slot]); // frees the stage once these MMAs have read it
+		if (++slot == Cfg::NS) { slot = 0; phase ^= 1; }
+	}
+	umma_commit(&tfull[acc]);
+	acc ^= 1;
+	if (acc == 0) acc_phase ^= 1;
+}
+
+// GROUPED: M tiles come from a list, each with a matrix of its own.  SPLIT: the CTAs of a cluster share a tile's K steps (gemm_split).
+// The two forms have loops of their own: with one loop whose bounds and strides depend on the cluster, one CTA per tile was 1 to 2 % slower although the
+// cluster's size is a constant there (4096 x 4096 x 14336: one plane each 326 us, 320; two planes each 939 us, 928)
 template <int NA, int NB, bool GROUPED = false, bool SPLIT = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap b_map) {
 	using Cfg = GemmCfg<NA, NB>;
@@ -671,81 +728,48 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 	const int MT = GROUPED ? *g.gn_tiles : g.MT;
 	const int n_tiles = MT * g.NT;
 	const int KT = g.KT;
-	int rank = 0, ks = 1;
+	struct { int rank, ks, tile0, tiles, k_lo, k_hi; } cl; // of SPLIT: this CTA's place in its cluster, the cluster's tiles, this CTA's K steps of each
 	if constexpr (SPLIT) {
-		asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-		asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(ks));
+		asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cl.rank));
+		asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cl.ks));
+		cl.tile0 = (int) blockIdx.x / cl.ks; cl.tiles = (int) gridDim.x / cl.ks;
+		cl.k_lo = cl.rank * KT / cl.ks; cl.k_hi = (cl.rank + 1) * KT / cl.ks;
 	}
-	const int first_tile = (int) blockIdx.x / ks, tile_step = (int) gridDim.x / ks;
-	const int k_lo = rank * KT / ks, k_hi = (rank + 1) * KT / ks; // this CTA's K steps of every tile
 
 	if (warp == 0) {
 		int slot = 0, phase = 0;
-		for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
-			if (lane == 0) {
-				const int mt = g.mt0 + tile % MT, nt = tile / MT;
-				const uint8_t* ah = g.a_hi + (size_t) mt * KT * A_TILE_BYTES;
-				const uint8_t* al = NA == 2 ? g.a_lo + (size_t) mt * KT * A_TILE_BYTES : nullptr;
-				const uint8_t* bt = (GROUPED ? g.gb[g.gtiles[3 * mt]] : g.b) + (size_t) nt * KT * B_TILE_BYTES;
-				const uint8_t* bl = NB == 2 ? g.b_lo + (size_t) nt * KT * B_TILE_BYTES : nullptr;
-				for (int kt = k_lo; kt < k_hi; kt++) {
-					mb_wait(&empty[slot], phase ^ 1);
-					uint8_t* st = smem + (size_t) slot * Cfg::STAGE;
-					mb_expect_tx(&full[slot], Cfg::STAGE);
-					bulk_load(st, ah + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
-					if (NA == 2) bulk_load(st + A_TILE_BYTES, al + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
-					if (NB == 1 && !GROUPED && !g.b) {
-						tensor_load(st + NA * A_TILE_BYTES, &b_map, kt * GB_K, nt * g.b_box, &full[slot]);
-						if (g.b_box < GB_N) tensor_load(st + NA * A_TILE_BYTES + B_TILE_BYTES / 2, &b_map, kt * GB_K, g.glu_off + nt * g.b_box, &full[slot]);
-					} else bulk_load(st + NA * A_TILE_BYTES, bt + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
-					if (NB == 2) bulk_load(st + NA * A_TILE_BYTES + B_TILE_BYTES, bl + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
-					if (++slot == NS) { slot = 0; phase ^= 1; }
-				}
+		if constexpr (SPLIT) {
+			for (int tile = cl.tile0; tile < n_tiles; tile += cl.tiles) {
+				if (lane == 0) gemm_load_steps<NA, NB, GROUPED>(g, b_map, g.mt0 + tile % MT, tile / MT, cl.k_lo, cl.k_hi, smem, full, empty, slot, phase);
+				cluster_barrier();
+				cluster_barrier();
 			}
-			if constexpr (SPLIT) { cluster_barrier(); cluster_barrier(); }
+		} else if (lane == 0) {
+			for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
+				gemm_load_steps<NA, NB, GROUPED>(g, b_map, g.mt0 + tile % MT, tile / MT, 0, KT, smem, full, empty, slot, phase);
 		}
 		__syncwarp();
 	} else if (warp == 1) {
-		constexpr uint32_t idesc = instr_desc_f16(GB_M, GB_N);
 		int slot = 0, phase = 0, acc = 0, acc_phase = 0;
-		for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
-			if (lane == 0) {
-				mb_wait(&tempty[acc], acc_phase ^ 1);
-				tc_fence_after();
-				const uint32_t d_tmem = tmem_base + (uint32_t) acc * GB_N;
-				for (int kt = k_lo; kt < k_hi; kt++) {
-					mb_wait(&full[slot], phase);
-					tc_fence_after();
-					const uint32_t sa = s_u32(smem + (size_t) slot * Cfg::STAGE);
-#pragma unroll
-					for (int p = 0; p < NA + NB - 1; p++) { // (a_hi, b_hi), (a_lo, b_hi), (a_hi, b_lo)
-						const uint64_t adesc = smem_desc(sa + (p == 1 ? A_TILE_BYTES : 0));
-						const uint64_t bdesc = smem_desc(sa + NA * A_TILE_BYTES + (p == 2 ? B_TILE_BYTES : 0));
-#pragma unroll
-						for (int k = 0; k < GB_K / UMMA_K; k++) {
-							// advancing K by 16 fp16 = 32 bytes inside the 128-byte swizzle row: +2 in the (>>4) address field
-							umma_f16(d_tmem, adesc + (uint64_t) (2 * k), bdesc + (uint64_t) (2 * k), idesc, (uint32_t) (((kt - k_lo) | k | p) != 0));
-						}
-					}
-					umma_commit(&empty[slot]); // frees the stage once these MMAs have read it
-					if (++slot == NS) { slot = 0; phase ^= 1; }
-				}
-				umma_commit(&tfull[acc]);
-				acc ^= 1;
-				if (acc == 0) acc_phase ^= 1;
+		if constexpr (SPLIT) {
+			for (int tile = cl.tile0; tile < n_tiles; tile += cl.tiles) {
+				if (lane == 0) gemm_mma_steps<NA, NB>(cl.k_hi - cl.k_lo, tmem_base, smem, full, empty, tfull, tempty, slot, phase, acc, acc_phase);
+				cluster_barrier();
+				cluster_barrier();
 			}
-			if constexpr (SPLIT) { cluster_barrier(); cluster_barrier(); }
+		} else if (lane == 0) {
+			for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) gemm_mma_steps<NA, NB>(KT, tmem_base, smem, full, empty, tfull, tempty, slot, phase, acc, acc_phase);
 		}
 		__syncwarp();
 	} else {
 		const int quad = warp & 3; // TMEM lanes [32*quad, 32*quad+32) are the ones this warp may read
 		int acc = 0, acc_phase = 0;
-		for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
-			const int mt = g.mt0 + tile % MT, nt = tile / MT;
-			mb_wait(&tfull[acc], acc_phase);
-			tc_fence_after();
-			const uint32_t taddr = tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N;
-			if constexpr (SPLIT) {
+		if constexpr (SPLIT) {
+			for (int tile = cl.tile0; tile < n_tiles; tile += cl.tiles) {
+				const int mt = g.mt0 + tile % MT, nt = tile / MT;
+				mb_wait(&tfull[acc], acc_phase);
+				tc_fence_after();
+				const uint32_t taddr = tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N;
 				const int rows = GROUPED ? g.gtiles[3 * mt + 2] : g.M - mt * GB_M;
 				uint8_t* own = smem + (size_t) (quad * 32 + lane) * 16; // where the ring was: every stage of this tile has been read
 				if (quad * 32 < rows) { // rows that nobody stores stay where they are
@@ -760,17 +784,24 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 				__syncwarp();
 				if (lane == 0) mb_arrive(&tempty[acc]);
 				cluster_barrier();
-				if (quad * 32 < rows) gemm_epilogue<GROUPED>(g, AccCluster{s_u32(own), ks}, mt, nt, quad * 32 + lane, rank, ks);
+				if (quad * 32 < rows) gemm_epilogue<GROUPED>(g, AccCluster{s_u32(own), cl.ks}, mt, nt, quad * 32 + lane, cl.rank, cl.ks);
 				asm volatile("fence.proxy.async;" ::: "memory"); // the next tile's copies land where the sums lay
 				cluster_barrier();
-			} else {
-				gemm_epilogue<GROUPED>(g, AccTmem{taddr}, mt, nt, quad * 32 + lane, 0, 1);
+				acc ^= 1;
+				if (acc == 0) acc_phase ^= 1;
+			}
+		} else {
+			for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+				const int mt = g.mt0 + tile % MT, nt = tile / MT;
+				mb_wait(&tfull[acc], acc_phase);
+				tc_fence_after();
+				gemm_epilogue<GROUPED>(g, AccTmem{tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N}, mt, nt, quad * 32 + lane, 0, 1);
 				tc_fence_before();
 				__syncwarp();
 				if (lane == 0) mb_arrive(&tempty[acc]);
+				acc ^= 1;
+				if (acc == 0) acc_phase ^= 1;
 			}
-			acc ^= 1;
-			if (acc == 0) acc_phase ^= 1;
 		}
 	}
 	tc_fence_before();
