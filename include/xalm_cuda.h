@@ -220,6 +220,9 @@ int xalm_cuda_rows_act(float* out, const float* x, const float* w, int T, int N,
  * qk_post: proj (T, (H + G) d) = [q | k]; q_out = turned q; k_out (ring, G d) the turned keys and v_out (ring, G d) the keys as they came, row
  *   p % ring for position p.  Turn: the first 2 rot_half entries of a head, entry i with i + rot_half, by p * freq[i], cos and sin times rot_mag.
  * rows_act_bias: out = act(x W^T + bias); act as rows_act, 4 tanh-gelu, 5 sigmoid(.)^act_pow.
+ * rows_tc: x (T, K) . w (N, K)^T on the tcgen05 GEMM of passes of many tokens (K % 64 == 0, N % 4 == 0; w rounded to bf16, x as a_planes = 1 or 2 fp16
+ *   planes).  kind 0: stored; 1: added to out; 2: limit * tanh(. / limit); 3: max(., 0)^2; 4: tanh-gelu; 5: pairs of neighbouring columns (gate, up) become
+ *   one by glu_act as glu of moe_ffn_routed (out (T, N / 2), N % 8 == 0).  fused: by the GEMM's epilogue; else by a kernel that reads the plain product.
  * gated_group_norm: out[:, :W] of rows ld_out wide = grouped RMS norm of y * silu(gate) (gate NULL: of y), times w, times out_scale (0: 1). */
 int xalm_cuda_norm_conv(float* out, float* hist, const float* x, int T, int W, int groups, int taps, int readers, const float* w, const float* cw, float eps);
 int xalm_cuda_short_conv(float* out, float* hist, const float* x, int T, int C, int taps, const float* w, const float* bias, int act);
@@ -233,6 +236,7 @@ int xalm_cuda_sink_attention(float* out, const float* q, const float* k, const f
 int xalm_cuda_qk_post(float* q_out, float* k_out, float* v_out, const float* proj, int T, int pos0, int H, int G, int d, const float* freq, int rot_half,
                       float rot_mag, int ring);
 int xalm_cuda_rows_act_bias(float* out, const float* x, const float* w, int T, int N, int K, int act, const float* bias, float act_pow, int w_bf16);
+int xalm_cuda_rows_tc(float* out, const float* x, const float* w, int T, int N, int K, int kind, int glu_act, float limit, float alpha, int a_planes, int fused);
 int xalm_cuda_gated_group_norm(float* out, const float* y, const float* gate, const float* w, int T, int W, int groups, float eps, float out_scale, int ld_out);
 
 /* Mechanisms of unrotated attention and of mixtures with identity experts (fp32 host arrays in and out):

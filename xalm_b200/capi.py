@@ -108,6 +108,7 @@ SYMBOLS = {
     "xalm_cuda_sink_attention": (_i, [_vp] * 4 + [_i] * 6 + [C.c_float, _vp, C.c_float, _i, _i]),
     "xalm_cuda_qk_post": (_i, [_vp] * 4 + [_i] * 5 + [_vp, _i, C.c_float, _i]),
     "xalm_cuda_rows_act_bias": (_i, [_vp] * 3 + [_i] * 4 + [_vp, C.c_float, _i]),
+    "xalm_cuda_rows_tc": (_i, [_vp] * 3 + [_i] * 5 + [C.c_float, C.c_float, _i, _i]),
     "xalm_cuda_gated_group_norm": (_i, [_vp] * 4 + [_i] * 3 + [C.c_float, C.c_float, _i]),
     "xalm_cuda_layer_norm": (_i, [_vp] * 4 + [_i, _i, C.c_float]),
     "xalm_cuda_embed_positions": (_i, [_vp, _vp, _i, _i, _vp, _i, _vp, _i, _i]),
@@ -511,6 +512,17 @@ def rows_act_bias(x, w, act, bias=None, act_pow=1.0, w_bf16=False):
     T, K = x.shape
     out = np.empty((T, w.shape[0]), dtype=np.float32)
     check(lib().xalm_cuda_rows_act_bias(_p(out), _p(x), _p(w), T, w.shape[0], K, act, _pn(bias), act_pow, int(w_bf16)))
+    return out
+
+
+ROWS_TC = {"store": 0, "add": 1, "cap": 2, "relu2": 3, "gelu": 4, "glu": 5}
+
+
+def rows_tc(x, w, kind="store", glu_act=1, limit=0.0, alpha=1.702, add=None, planes=1, fused=True):
+    x, w = _f(x), _f(w)
+    T, N = x.shape[0], w.shape[0]
+    out = np.array(add, dtype=np.float32, order="C") if kind == "add" else np.empty((T, N // 2 if kind == "glu" else N), dtype=np.float32)
+    check(lib().xalm_cuda_rows_tc(_p(out), _p(x), _p(w), T, N, x.shape[1], ROWS_TC[kind], glu_act, limit, alpha, planes, int(fused)))
     return out
 
 

@@ -13,6 +13,7 @@
 #include "mix_ops.cuh"
 #include "delta_ops.cuh"
 #include "conv_ops.cuh"
+#include "prefill.h"
 #include "latent_ops.cuh"
 #include "moe_ops.cuh"
 
@@ -849,6 +850,45 @@ int xalm_cuda_rows_act_bias(float* out, const float* x, const float* w, int T, i
 	XALM_TRY(launch_rows(d_x, K, d_w, w_bf16 != 0, T, N, K, e, nullptr));
 	XALM_TRY(finish("rows_act_bias"));
 	XALM_CUDA_CHECK(cudaMemcpy(out, d_out, (size_t) T * N * 4, cudaMemcpyDeviceToHost));
+	return XALM_OK;
+}
+
+int xalm_cuda_rows_tc(float* out, const float* x, const float* w, int T, int N, int K, int kind, int glu_act, float limit, float alpha, int a_planes, int fused) {
+	if (!out || !x || !w || T <= 0 || N <= 0 || K <= 0 || a_planes < 1 || a_planes > 2 || kind < TcEpi::STORE || kind > TcEpi::GLU || glu_act < GLU_CLAMPED || glu_act > GLU_GELU_TANH)
+		return set_error(XALM_ERR_INVALID, "rows_tc: bad argument");
+	TcEpi te;
+	te.kind = (TcEpi::Kind) kind; te.act = glu_act; te.limit = limit; te.alpha = alpha;
+	const int cols = te.kind == TcEpi::GLU ? N / 2 : N;
+	if (!tc_shape_ok(N, K, cols) || !tc_epi_ok(te, N, cols, nullptr)) return set_error(XALM_ERR_UNSUPPORTED, "rows_tc: (%d x %d) . (%d x %d)^T", T, K, N, K);
+	Pool pool;
+	std::vector<uint16_t> wb((size_t) N * K);
+	for (size_t i = 0; i < wb.size(); i++) wb[i] = bf16_bits(w[i]);
+	const uint16_t* d_w = pool.put(wb.data(), wb.size());
+	const float* d_x = pool.put(x, (size_t) T * K);
+	float *d_out = pool.put(out, (size_t) T * cols), *d_plain = pool.raw<float>((size_t) T * N);
+	uint8_t *hi = pool.raw<uint8_t>(tc_a_plane_bytes(T, K)), *lo = pool.raw<uint8_t>(tc_a_plane_bytes(T, K));
+	if (!d_w || !d_x || !d_out || !d_plain || !hi || !lo) return set_error(XALM_ERR_CUDA, "rows_tc: device allocation failed");
+	XALM_CUDA_CHECK(cudaMemset(hi, 0, tc_a_plane_bytes(T, K)));
+	XALM_CUDA_CHECK(cudaMemset(lo, 0, tc_a_plane_bytes(T, K)));
+	WMat wm = WMat();
+	wm.type = XALM_BF16; wm.rows = N; wm.n = K; wm.p0 = reinterpret_cast<const uint8_t*>(d_w); wm.s0 = (size_t) K * 2;
+	TcWeight tw;
+	int rc = tc_weight_build(wm, 1, &tw, nullptr);
+	if (rc == XALM_OK && fused) rc = tc_gemm(tw, d_x, T, d_out, cols, hi, a_planes == 2 ? lo : nullptr, nullptr, te);
+	else if (rc == XALM_OK) {
+		RowsEpi e;
+		e.out = d_out; e.ldo = cols;
+		if (te.kind == TcEpi::ADD) { e.kind = EPI_HC; e.xs = d_out; e.stream_stride = (size_t) T * N; }
+		else if (te.kind == TcEpi::CAP) e.cap = limit;
+		else if (te.kind == TcEpi::RELU2 || te.kind == TcEpi::GELU) { e.kind = EPI_ACT; e.act = te.kind == TcEpi::GELU ? ACT_GELU_TANH : ACT_RELU_SQUARED; }
+		else if (te.kind == TcEpi::GLU) { e.kind = EPI_GLU; e.glu_act = glu_act; e.limit = limit; e.alpha = alpha; }
+		rc = tc_gemm(tw, d_x, T, d_plain, N, hi, a_planes == 2 ? lo : nullptr, nullptr);
+		if (rc == XALM_OK) rc = launch_rows_epilogue(d_plain, N, T, N, e, nullptr);
+	}
+	if (rc == XALM_OK) rc = finish("rows_tc");
+	tc_weight_free(&tw);
+	XALM_TRY(rc);
+	XALM_CUDA_CHECK(cudaMemcpy(out, d_out, (size_t) T * cols * 4, cudaMemcpyDeviceToHost));
 	return XALM_OK;
 }
 

@@ -391,7 +391,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 //   warps 2-5 epilogue: tcgen05.ld the 128 x 256 fp32 accumulator (one TMEM lane quadrant per warp) and apply the
 //             fused epilogue, while the MMA warp already fills the OTHER accumulator buffer (2 x 256 of the 512 columns)
 // ------------------------------------------------------------------------------------------------------------------
-enum { GEPI_STORE = 0, GEPI_RESID = 1, GEPI_GLU = 2, GEPI_QKV = 3, GEPI_ACT = 4 /* grouped launches */, GEPI_FUSED = 5 /* TcEpi's CAP, ACT, GLU */ };
+enum { GEPI_STORE = 0, GEPI_RESID = 1, GEPI_GLU = 2, GEPI_QKV = 3, GEPI_ACT = 4 /* grouped launches */, GEPI_FUSED = 5 /* TcEpi's CAP, RELU2, GELU, GLU */ };
 
 struct GemmArgs {
 	const uint8_t* a_hi;
@@ -518,9 +518,12 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 				if (g.fused.kind == TcEpi::CAP) {
 #pragma unroll
 					for (int i = 0; i < 8; i++) v[i] = g.fused.limit * tanhf(v[i] / g.fused.limit);
-				} else {
+				} else if (g.fused.kind == TcEpi::GELU) {
 #pragma unroll
-					for (int i = 0; i < 8; i++) v[i] = mix::act_apply(g.fused.act, v[i]);
+					for (int i = 0; i < 8; i++) v[i] = mix::gelu_tanhf_(v[i]);
+				} else { // chosen per value instead: 33 x 4096 x 1024 with squared ReLU 35 us, 19 so; with GELU 47, 21
+#pragma unroll
+					for (int i = 0; i < 8; i++) v[i] = mix::act_apply(mix::ACT_RELU_SQUARED, v[i]);
 				}
 				*reinterpret_cast<float4*>(o + n0) = make_float4(v[0], v[1], v[2], v[3]);
 				if (n0 + 4 < g.N) *reinterpret_cast<float4*>(o + n0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
@@ -1554,6 +1557,14 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 template <int NA, int NB>
 static int gemm_split(int tiles, int KT) {
 	static std::atomic<int> fits[GEMM_MAX_SPLIT + 1]; // clusters of this size that run at a time, 0: not asked yet
+	static std::atomic<bool> attr{false};
+	if (!attr.load()) {
+		if (cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM) != cudaSuccess) {
+			cudaGetLastError();
+			return 1;
+		}
+		attr.store(true);
+	}
 	constexpr float STEP = NA == 1 ? 0.36f : NB == 1 ? 0.58f : 1.08f; // us
 	const float whole = (float) cdiv(tiles, sm_count()) * (float) KT * STEP;
 	int best = 1;
@@ -1578,11 +1589,6 @@ static int gemm_split(int tiles, int KT) {
 }
 template <int NA, int NB>
 static int launch_gemm_planes(const GemmArgs& g, const CUtensorMap& b_map, int tiles, cudaStream_t s) {
-	static std::atomic<bool> attr{false};
-	if (!attr.load()) {
-		XALM_CUDA_CHECK(cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM));
-		attr.store(true);
-	}
 	const int ks = gemm_split<NA, NB>(tiles, g.KT);
 	cudaError_t e;
 	if (ks > 1) {
@@ -2025,6 +2031,20 @@ void tc_weight_free(TcWeight* w) {
 }
 size_t tc_a_plane_bytes(int T, int K) { return (size_t) cdiv(T, GB_M) * cdiv(K, GB_K) * A_TILE_BYTES; }
 
+// An epilogue of the GEMM runs on four warps of a CTA and, in a CTA's last tile, beside nothing; the kernel that does it on the stored product has the whole
+// GPU but reads and writes the product again.  Where a cluster shares a tile, its CTAs share the columns too and the GEMM is faster throughout (1.03 to 1.5
+// times from 33 tokens on).  Else it depends on the product's size and on what a value takes; us of plain GEMM and kernel -> GEMM with the epilogue, caches warm,
+// tokens x columns x K:
+//   residual (a read per value), soft cap and gates with a sigmoid (quotients): from 2^21 values on.  1024 x 1024 x 1024 29 -> 33, 400 x 4096 x 1024 31 -> 33,
+//     512 x 4096 x 1024 35 -> 33; soft cap 33 x 32000 x 1024 33 -> 41, 64 x 32000 x 1024 42 -> 39, 1024 x 32000 x 1024 246 -> 151; SiLU gate 33 x 8192 x 1024
+//     19 -> 27, 256 x 8192 x 1024 27 -> 27, 2048 x 8192 x 1024 90 -> 70
+//   squared ReLU, GELU and its gate: from 2^19 on.  GELU 64 x 4096 x 1024 19.8 -> 20.7, 128 x 4096 x 1024 24.8 -> 20.7, 1024 x 8192 x 1024 70 -> 33
+bool tc_epi_pays(const TcEpi& e, const TcWeight& w, int T, int a_planes) {
+	if (e.kind == TcEpi::STORE) return true;
+	const int tiles = cdiv(T, GB_M) * w.NT, ks = a_planes == 1 ? gemm_split<1, 1>(tiles, w.KT) : w.lo ? gemm_split<2, 2>(tiles, w.KT) : gemm_split<2, 1>(tiles, w.KT);
+	const bool light = e.kind == TcEpi::RELU2 || e.kind == TcEpi::GELU || (e.kind == TcEpi::GLU && e.act == mix::GLU_GELU_TANH);
+	return ks > 1 || (size_t) T * w.N >= (light ? (size_t) 1 << 19 : (size_t) 1 << 21);
+}
 int tc_gemm(const TcWeight& w, const float* a_dev, int T, float* out_dev, int ldo, uint8_t* a_hi, uint8_t* a_lo, cudaStream_t s, const TcEpi& epi) {
 	if (!tc_shape_ok(w.N, w.K, ldo) || !tc_epi_ok(epi, w.N, ldo, out_dev) || T <= 0) return set_error(XALM_ERR_INVALID, "tc_gemm: shape (%d x %d) . (%d x %d)^T, ldo %d", T, w.K, w.N, w.K, ldo);
 	const int MT = cdiv(T, GB_M);

@@ -65,18 +65,20 @@ inline bool tc_shape_ok(int N, int K, int ldo) { return K % 64 == 0 && N % 4 == 
 int tc_weight_build(const WMat& w, int planes, TcWeight* out, cudaStream_t s); // allocates out->hi (/lo); W in its decode layout
 void tc_weight_free(TcWeight* w);
 size_t tc_a_plane_bytes(int T, int K); // one operand plane of T x K activations
-// a_hi / a_lo: caller-owned planes of tc_a_plane_bytes(T, K) bytes (a_lo NULL: one fp16 plane; else hi + lo = fp32-grade activations).
-// Two launches (pack, GEMM) on stream s; nothing is synchronised.
 struct TcEpi { // what happens to a product on its way out
-	enum Kind { STORE, ADD /* out += */, CAP /* limit * tanh(. / limit) */, ACT, GLU /* pairs of neighbouring columns (gate, up) become one */ };
+	enum Kind { STORE, ADD /* out += */, CAP /* limit * tanh(. / limit) */, RELU2 /* max(., 0)^2 */, GELU /* the tanh form */, GLU /* pairs of neighbouring columns (gate, up) become one */ };
 	Kind kind = STORE;
-	int act = 0; // ACT: ACT_* (no parameters); GLU: GLU_* (act_ops.cuh)
+	int act = 0; // GLU: GLU_* (act_ops.cuh)
 	float limit = 0.f, alpha = 0.f;
 };
 // whether the GEMM can do it for N columns into rows of ldo floats at out: it writes 16 bytes at a time
 inline bool tc_epi_ok(const TcEpi& e, int N, int ldo, const void* out) {
 	return N % (e.kind == TcEpi::GLU ? 8 : 4) == 0 && ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
 }
+// whether the GEMM is faster at it for T rows (a_planes: 1 or 2) than a kernel that reads the plain product
+bool tc_epi_pays(const TcEpi& e, const TcWeight& w, int T, int a_planes);
+// a_hi / a_lo: caller-owned planes of tc_a_plane_bytes(T, K) bytes (a_lo NULL: one fp16 plane; else hi + lo = fp32-grade activations).
+// Two launches (pack, GEMM) on stream s; nothing is synchronised.
 int tc_gemm(const TcWeight& w, const float* a_dev, int T, float* out_dev, int ldo, uint8_t* a_hi, uint8_t* a_lo, cudaStream_t s, const TcEpi& epi = TcEpi());
 
 

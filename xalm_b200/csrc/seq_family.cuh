@@ -258,11 +258,10 @@ int tc_register(SeqModel* m, const WMat& wm, TcWeight* t) {
 // ---- row products ---------------------------------------------------------------------------------------------------------------
 // Passes of few tokens and the fp32 mode: the fp32 FMA kernels of mix_ops.cuh with the epilogue fused.  Passes of tc_min_rows tokens
 // or more in the 16-bit mode: the tcgen05 GEMM of prefill.cu on the weight's resident fp16 tiles (activations packed to fp16, one
-// plane, or hi + lo with "seq_tc" = 2), fp32 accumulation, then the same epilogue as an elementwise kernel.
+// plane, or hi + lo with "seq_tc" = 2), fp32 accumulation.  What needs nothing but the product (and the residual stream's row) the GEMM does itself where
+// that is faster (tc_epi_pays), with the same functions; else the same epilogue as an elementwise kernel.
 int rows_product(SeqModel* m, const float* A, int lda, const void* W, const TcWeight* tw, int T, int N, int K, const RowsEpi& e, int* nl) {
 	if (m->use_tc && tw && tw->hi && T >= m->tc_min_rows && lda == K) {
-		// What needs nothing but the product (and the residual stream's row) the GEMM does itself, with the same functions: as a kernel of its own the epilogue
-		// reads and writes the product again (scoring 1900 tokens with soft-capped logits 2093 -> 1946 us, 2048 with a gated feed-forward 1413 -> 1381)
 		TcEpi te;
 		float* out = e.out;
 		int ldo = e.ldo;
@@ -270,9 +269,9 @@ int rows_product(SeqModel* m, const float* A, int lda, const void* W, const TcWe
 		if (e.kind == EPI_STORE && !e.mul && !e.add) {
 			fused = true;
 			if (e.cap > 0.f) { te.kind = TcEpi::CAP; te.limit = e.cap; }
-		} else if (e.kind == EPI_ACT && !e.bias && e.act != ACT_SIGMOID_POW) {
+		} else if (e.kind == EPI_ACT && !e.bias && (e.act == ACT_RELU_SQUARED || e.act == ACT_GELU_TANH)) {
 			fused = true;
-			te.kind = TcEpi::ACT; te.act = e.act;
+			te.kind = e.act == ACT_GELU_TANH ? TcEpi::GELU : TcEpi::RELU2;
 		} else if (e.kind == EPI_GLU) {
 			fused = true;
 			te.kind = TcEpi::GLU; te.act = e.glu_act; te.limit = e.limit; te.alpha = e.alpha;
@@ -281,7 +280,7 @@ int rows_product(SeqModel* m, const float* A, int lda, const void* W, const TcWe
 			te.kind = TcEpi::ADD;
 			out = e.xs; ldo = N;
 		}
-		if (fused && tc_epi_ok(te, N, ldo, out)) {
+		if (fused && tc_epi_ok(te, N, ldo, out) && tc_epi_pays(te, *tw, T, m->a_lo ? 2 : 1)) {
 			*nl += 2;
 			return tc_gemm(*tw, A, T, out, ldo, m->a_hi, m->a_lo, m->stream, te);
 		}
