@@ -396,8 +396,8 @@ enum { GEPI_STORE = 0, GEPI_RESID = 1, GEPI_GLU = 2, GEPI_QKV = 3, GEPI_ACT = 4 
 struct GemmArgs {
 	const uint8_t* a_hi;
 	const uint8_t* a_lo;
-	const uint8_t* b;    // NULL: one weight plane, its tiles cut out of the row-major fp16 matrix by the kernel's tensor map
-	int b_box;          // rows of the map's box: GB_N, or GB_N / 2 where a tile takes two (rows nt * b_box of the matrix and of glu_off)
+	const uint8_t* b;
+	int b_box;          // GF_MAP: rows of the map's box: GB_N, or GB_N / 2 where a tile takes two (rows nt * b_box of the matrix and of glu_off)
 	int glu_off;
 	const uint8_t* b_lo; // residual plane of the weights (NB = 2)
 	int MT, NT, KT;     // tile counts; M tiles are [mt0, mt0 + MT)
@@ -432,6 +432,18 @@ struct GemmArgs {
 	TcAct gact;
 	TcEpi fused;
 };
+
+// What a launch is for; an instance of gemm_tc_kernel holds only the operands and epilogues that its launches use.  With all of them in one, a launch carried
+// the tensor map's 128 bytes and all epilogues' code: passes of 33 to 320 tokens of a 1024 wide Mizerax model, 12 short products a layer pair, took 1 to 2 %
+// longer (128 tokens 443 us, 441 so; 434 to 443 before the map and the fused epilogues came)
+enum GemmFor {
+	GF_TILES, // a prompt's products on weight tiles: GEPI_STORE, _RESID, _GLU, _QKV
+	GF_MAP,   // the same on fp16 rows through a tensor map
+	GF_ROWS,  // tc_gemm: GEPI_STORE, _RESID, _FUSED
+	GF_GROUP, // M tiles come from a list, each with a matrix of its own: GEPI_STORE, _ACT
+};
+template <int FOR> struct GemmMap {};
+template <> struct GemmMap<GF_MAP> { CUtensorMap m; };
 
 constexpr int GEMM_THREADS = 192;
 // NA activation planes x NB weight planes: (1,1) fp16 x fp16; (2,1) hi+lo activations; (2,2) hi+lo on both sides, three MMAs per
@@ -479,8 +491,9 @@ __device__ __forceinline__ void cluster_barrier() { // every thread of the clust
 }
 
 // The fused epilogue of tile (mt, nt) for this thread's row, chunks of columns part, part + parts, ... (one CTA: all of them)
-template <bool GROUPED, typename Acc>
+template <int FOR, typename Acc>
 __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc, int mt, int nt, int row_in_tile, int part, int parts) {
+	constexpr bool GROUPED = FOR == GF_GROUP, PROMPT = FOR == GF_TILES || FOR == GF_MAP;
 	const int m = mt * GB_M + row_in_tile;
 	const bool mrow = GROUPED ? row_in_tile < g.gtiles[3 * mt + 2] : m < g.M;
 	if (GROUPED && g.epi == GEPI_ACT) {
@@ -503,7 +516,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 				}
 			}
 		}
-	} else if (!GROUPED && g.epi == GEPI_FUSED) {
+	} else if (FOR == GF_ROWS && g.epi == GEPI_FUSED) {
 		for (int c = part * 8; c < GB_N; c += parts * 8) {
 			float v[8];
 			acc.get(c, v);
@@ -529,7 +542,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 				if (n0 + 4 < g.N) *reinterpret_cast<float4*>(o + n0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
 			}
 		}
-	} else if (g.epi == GEPI_GLU) {
+	} else if (PROMPT && g.epi == GEPI_GLU) {
 		for (int c = part * 8; c < GB_N / 2; c += parts * 8) {
 			float gt[8], up[8];
 			acc.get(c, gt);
@@ -542,7 +555,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 				store_a8(g.o, m, o0, h);
 			}
 		}
-	} else if (g.epi == GEPI_QKV) {
+	} else if (PROMPT && g.epi == GEPI_QKV) {
 		// 16 columns = 8 rotation pairs at a time; q_dim, kv_dim and head_dim are multiples of 16, so a chunk never straddles
 		// the q | k | v regions or a head, and leaves as two 16-byte stores
 		const int pos = g.pos0 + m;
@@ -639,14 +652,14 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, const Acc& acc,
 }
 
 // K steps [k_lo, k_hi) of tile (mt, nt) into the ring
-template <int NA, int NB, bool GROUPED>
-__device__ __forceinline__ void gemm_load_steps(const GemmArgs& g, const CUtensorMap& b_map, int mt, int nt, int k_lo, int k_hi, uint8_t* smem, uint64_t* full,
+template <int NA, int NB, int FOR>
+__device__ __forceinline__ void gemm_load_steps(const GemmArgs& g, const GemmMap<FOR>& map, int mt, int nt, int k_lo, int k_hi, uint8_t* smem, uint64_t* full,
                                                 uint64_t* empty, int& slot, int& phase) {
 	using Cfg = GemmCfg<NA, NB>;
 	const int KT = g.KT;
 	const uint8_t* ah = g.a_hi + (size_t) mt * KT * A_TILE_BYTES;
 	const uint8_t* al = NA == 2 ? g.a_lo + (size_t) mt * KT * A_TILE_BYTES : nullptr;
-	const uint8_t* bt = (GROUPED ? g.gb[g.gtiles[3 * mt]] : g.b) + (size_t) nt * KT * B_TILE_BYTES;
+	const uint8_t* bt = (FOR == GF_GROUP ? g.gb[g.gtiles[3 * mt]] : g.b) + (size_t) nt * KT * B_TILE_BYTES;
 	const uint8_t* bl = NB == 2 ? g.b_lo + (size_t) nt * KT * B_TILE_BYTES : nullptr;
 	for (int kt = k_lo; kt < k_hi; kt++) {
 		mb_wait(&empty[slot], phase ^ 1);
@@ -654,9 +667,9 @@ __device__ __forceinline__ void gemm_load_steps(const GemmArgs& g, const CUtenso
 		mb_expect_tx(&full[slot], Cfg::STAGE);
 		bulk_load(st, ah + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
 		if (NA == 2) bulk_load(st + A_TILE_BYTES, al + (size_t) kt * A_TILE_BYTES, A_TILE_BYTES, &full[slot]);
-		if (NB == 1 && !GROUPED && !g.b) {
-			tensor_load(st + NA * A_TILE_BYTES, &b_map, kt * GB_K, nt * g.b_box, &full[slot]);
-			if (g.b_box < GB_N) tensor_load(st + NA * A_TILE_BYTES + B_TILE_BYTES / 2, &b_map, kt * GB_K, g.glu_off + nt * g.b_box, &full[slot]);
+		if constexpr (FOR == GF_MAP) {
+			tensor_load(st + NA * A_TILE_BYTES, &map.m, kt * GB_K, nt * g.b_box, &full[slot]);
+			if (g.b_box < GB_N) tensor_load(st + NA * A_TILE_BYTES + B_TILE_BYTES / 2, &map.m, kt * GB_K, g.glu_off + nt * g.b_box, &full[slot]);
 		} else bulk_load(st + NA * A_TILE_BYTES, bt + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
 		if (NB == 2) bulk_load(st + NA * A_TILE_BYTES + B_TILE_BYTES, bl + (size_t) kt * B_TILE_BYTES, B_TILE_BYTES, &full[slot]);
 		if (++slot == Cfg::NS) { slot = 0; phase ^= 1; }
@@ -693,11 +706,11 @@ __device__ __forceinline__ void gemm_mma_steps(int n, uint32_t tmem_base, uint8_
 	if (acc == 0) acc_phase ^= 1;
 }
 
-// GROUPED: M tiles come from a list, each with a matrix of its own.  SPLIT: the CTAs of a cluster share a tile's K steps (gemm_split).
+// SPLIT: the CTAs of a cluster share a tile's K steps (gemm_split).
 // The two forms have loops of their own: with one loop whose bounds and strides depend on the cluster, one CTA per tile was 1 to 2 % slower although the
 // cluster's size is a constant there (4096 x 4096 x 14336: one plane each 326 us, 320; two planes each 939 us, 928)
-template <int NA, int NB, bool GROUPED = false, bool SPLIT = false>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap b_map) {
+template <int NA, int NB, int FOR, bool SPLIT = false>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs g, const __grid_constant__ GemmMap<FOR> map) {
 	using Cfg = GemmCfg<NA, NB>;
 	constexpr int NS = Cfg::NS;
 	extern __shared__ uint8_t smem_raw[];
@@ -728,7 +741,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 	tc_fence_after();
 	const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
-	const int MT = GROUPED ? *g.gn_tiles : g.MT;
+	const int MT = FOR == GF_GROUP ? *g.gn_tiles : g.MT;
 	const int n_tiles = MT * g.NT;
 	const int KT = g.KT;
 	struct { int rank, ks, tile0, tiles, k_lo, k_hi; } cl; // of SPLIT: this CTA's place in its cluster, the cluster's tiles, this CTA's K steps of each
@@ -743,13 +756,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 		int slot = 0, phase = 0;
 		if constexpr (SPLIT) {
 			for (int tile = cl.tile0; tile < n_tiles; tile += cl.tiles) {
-				if (lane == 0) gemm_load_steps<NA, NB, GROUPED>(g, b_map, g.mt0 + tile % MT, tile / MT, cl.k_lo, cl.k_hi, smem, full, empty, slot, phase);
+				if (lane == 0) gemm_load_steps<NA, NB, FOR>(g, map, g.mt0 + tile % MT, tile / MT, cl.k_lo, cl.k_hi, smem, full, empty, slot, phase);
 				cluster_barrier();
 				cluster_barrier();
 			}
 		} else if (lane == 0) {
 			for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
-				gemm_load_steps<NA, NB, GROUPED>(g, b_map, g.mt0 + tile % MT, tile / MT, 0, KT, smem, full, empty, slot, phase);
+				gemm_load_steps<NA, NB, FOR>(g, map, g.mt0 + tile % MT, tile / MT, 0, KT, smem, full, empty, slot, phase);
 		}
 		__syncwarp();
 	} else if (warp == 1) {
@@ -773,7 +786,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 				mb_wait(&tfull[acc], acc_phase);
 				tc_fence_after();
 				const uint32_t taddr = tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N;
-				const int rows = GROUPED ? g.gtiles[3 * mt + 2] : g.M - mt * GB_M;
+				const int rows = g.M - mt * GB_M;
 				uint8_t* own = smem + (size_t) (quad * 32 + lane) * 16; // where the ring was: every stage of this tile has been read
 				if (quad * 32 < rows) { // rows that nobody stores stay where they are
 					for (int c = 0; c < GB_N; c += 32) {
@@ -787,7 +800,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 				__syncwarp();
 				if (lane == 0) mb_arrive(&tempty[acc]);
 				cluster_barrier();
-				if (quad * 32 < rows) gemm_epilogue<GROUPED>(g, AccCluster{s_u32(own), cl.ks}, mt, nt, quad * 32 + lane, cl.rank, cl.ks);
+				if (quad * 32 < rows) gemm_epilogue<FOR>(g, AccCluster{s_u32(own), cl.ks}, mt, nt, quad * 32 + lane, cl.rank, cl.ks);
 				asm volatile("fence.proxy.async;" ::: "memory"); // the next tile's copies land where the sums lay
 				cluster_barrier();
 				acc ^= 1;
@@ -798,7 +811,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 				const int mt = g.mt0 + tile % MT, nt = tile / MT;
 				mb_wait(&tfull[acc], acc_phase);
 				tc_fence_after();
-				gemm_epilogue<GROUPED>(g, AccTmem{tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N}, mt, nt, quad * 32 + lane, 0, 1);
+				gemm_epilogue<FOR>(g, AccTmem{tmem_base + ((uint32_t) (quad * 32) << 16) + (uint32_t) acc * GB_N}, mt, nt, quad * 32 + lane, 0, 1);
 				tc_fence_before();
 				__syncwarp();
 				if (lane == 0) mb_arrive(&tempty[acc]);
@@ -1520,14 +1533,14 @@ const float* prefill_logits_dev(const PrefillScratch* s, int* rows) {
 	return s ? reinterpret_cast<const float*>(s->logits.p) : nullptr;
 }
 
-template <int NA, int NB, bool GROUPED = false>
-static int launch_gemm_inst(const GemmArgs& g, const CUtensorMap& b_map, int grid, cudaStream_t s) {
+template <int NA, int NB, int FOR>
+static int launch_gemm_inst(const GemmArgs& g, const GemmMap<FOR>& map, int grid, cudaStream_t s) {
 	static bool attr = false;
 	if (!attr) {
-		XALM_CUDA_CHECK(cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM));
+		XALM_CUDA_CHECK(cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, FOR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM));
 		attr = true;
 	}
-	gemm_tc_kernel<NA, NB, GROUPED><<<grid, GEMM_THREADS, GemmCfg<NA, NB>::SMEM, s>>>(g, b_map);
+	gemm_tc_kernel<NA, NB, FOR><<<grid, GEMM_THREADS, GemmCfg<NA, NB>::SMEM, s>>>(g, map);
 	return XALM_OK;
 }
 constexpr int GEMM_MAX_SPLIT = 8; // the portable cluster size
@@ -1554,12 +1567,12 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 //   2/2: 33 x 4096 x 14336 242 -> 57 (6), 333 x 6144 x 4096 82 -> 49 (2), 500 x 2048 x 6144 94 -> 37 (4)
 // Against float64 the result is nearer, 2 to 5 times at 4 to 8 shares: the tensor cores' own additions truncate, and a share has fewer of them.
 // From about 80 tiles on, and for 16 K steps with 8 tiles and more, one CTA per tile is as fast or faster and the rule says so.
-template <int NA, int NB>
+template <int NA, int NB, int FOR>
 static int gemm_split(int tiles, int KT) {
 	static std::atomic<int> fits[GEMM_MAX_SPLIT + 1]; // clusters of this size that run at a time, 0: not asked yet
 	static std::atomic<bool> attr{false};
 	if (!attr.load()) {
-		if (cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM) != cudaSuccess) {
+		if (cudaFuncSetAttribute(gemm_tc_kernel<NA, NB, FOR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) GemmCfg<NA, NB>::SMEM) != cudaSuccess) {
 			cudaGetLastError();
 			return 1;
 		}
@@ -1575,7 +1588,7 @@ static int gemm_split(int tiles, int KT) {
 			cudaLaunchConfig_t cfg = {};
 			cudaLaunchAttribute at[1];
 			gemm_cluster_config<NA, NB>(&cfg, at, sm_count() / ks * ks, ks, nullptr);
-			if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<NA, NB, false, true>, &cfg) != cudaSuccess || n <= 0) {
+			if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<NA, NB, FOR, true>, &cfg) != cudaSuccess || n <= 0) {
 				cudaGetLastError();
 				n = -1;
 			}
@@ -1587,27 +1600,35 @@ static int gemm_split(int tiles, int KT) {
 	}
 	return best;
 }
-template <int NA, int NB>
-static int launch_gemm_planes(const GemmArgs& g, const CUtensorMap& b_map, int tiles, cudaStream_t s) {
-	const int ks = gemm_split<NA, NB>(tiles, g.KT);
+template <int NA, int NB, int FOR>
+static int launch_gemm_planes(const GemmArgs& g, const GemmMap<FOR>& map, int tiles, cudaStream_t s) {
+	const int ks = gemm_split<NA, NB, FOR>(tiles, g.KT);
 	cudaError_t e;
 	if (ks > 1) {
 		cudaLaunchConfig_t cfg = {};
 		cudaLaunchAttribute at[1];
 		gemm_cluster_config<NA, NB>(&cfg, at, std::min(tiles, sm_count() / ks) * ks, ks, s);
-		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, false, true>, g, b_map);
+		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, FOR, true>, g, map);
 	} else {
-		XALM_TRY((launch_gemm_inst<NA, NB>(g, b_map, std::min(tiles, sm_count()), s)));
+		XALM_TRY((launch_gemm_inst<NA, NB, FOR>(g, map, std::min(tiles, sm_count()), s)));
 		e = cudaGetLastError();
 	}
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "gemm_tc launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
 }
-static int launch_gemm(const GemmArgs& g, int na, int nb, cudaStream_t s, const CUtensorMap& b_map = CUtensorMap()) {
+template <int FOR>
+static int launch_gemm(const GemmArgs& g, int na, int nb, cudaStream_t s) {
 	const int tiles = g.MT * g.NT;
 	if (tiles <= 0) return XALM_OK;
-	if (na == 2 && nb == 2) return launch_gemm_planes<2, 2>(g, b_map, tiles, s);
-	return na == 2 ? launch_gemm_planes<2, 1>(g, b_map, tiles, s) : launch_gemm_planes<1, 1>(g, b_map, tiles, s);
+	const GemmMap<FOR> none;
+	if (na == 2 && nb == 2) return launch_gemm_planes<2, 2, FOR>(g, none, tiles, s);
+	return na == 2 ? launch_gemm_planes<2, 1, FOR>(g, none, tiles, s) : launch_gemm_planes<1, 1, FOR>(g, none, tiles, s);
+}
+static int launch_gemm_map(const GemmArgs& g, const CUtensorMap& b_map, int na, cudaStream_t s) { // one weight plane
+	const int tiles = g.MT * g.NT;
+	if (tiles <= 0) return XALM_OK;
+	const GemmMap<GF_MAP> map = {b_map};
+	return na == 2 ? launch_gemm_planes<2, 1, GF_MAP>(g, map, tiles, s) : launch_gemm_planes<1, 1, GF_MAP>(g, map, tiles, s);
 }
 
 // fp16 rows are their own operand tiles: the copy engine cuts 64-element pieces of box_rows rows out of them and swizzles them on the way, where writing
@@ -1815,7 +1836,7 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		g.glu_off = glu_off;
 		if (weight_map(w, K, g.b_box, &b_map)) {
 			t_begin("gemm_f16");
-			XALM_TRY(launch_gemm(g, na, 1, s, b_map));
+			XALM_TRY(launch_gemm_map(g, b_map, na, s));
 			t_end();
 			launches++;
 			return XALM_OK;
@@ -1824,7 +1845,7 @@ int prefill_run(const PrefillModel& pm, PrefillScratch** scratch, const int* tok
 		g.b_lo = sc.wt_lo[b].p;
 		XALM_CUDA_CHECK(cudaStreamWaitEvent(s, sc.ev_deq[b], 0));
 		t_begin(g.epi == GEPI_QKV ? "gemm_qkv" : g.epi == GEPI_GLU ? "gemm_w13" : g.epi == GEPI_STORE ? "gemm_cls" : g.KT == KT_q ? "gemm_wo" : "gemm_w2");
-		XALM_TRY(launch_gemm(g, na, nb_of(w), s));
+		XALM_TRY(launch_gemm<GF_TILES>(g, na, nb_of(w), s));
 		t_end();
 		XALM_CUDA_CHECK(cudaEventRecord(sc.ev_gemm[b], s));
 		job++;
@@ -1969,7 +1990,7 @@ int prefill_gemm_dev(const WMat& w, const float* a_dev, int T, float* out_dev, i
 		g.a_hi = at.hi; g.a_lo = at.lo; g.b = bt.p; g.b_lo = bl.p;
 		g.MT = MT; g.NT = NT; g.KT = KT; g.M = T; g.N = N; g.epi = GEPI_STORE; g.out = out_dev; g.ldo = N;
 		g.b_box = GB_N;
-		rc = launch_gemm(g, na, nb, s, b_map);
+		rc = mapped ? launch_gemm_map(g, b_map, na, s) : launch_gemm<GF_TILES>(g, na, nb, s);
 	}
 	cudaError_t e = cudaStreamSynchronize(s);
 	ah.release(); al.release(); bt.release(); bl.release();
@@ -1998,9 +2019,9 @@ int prefill_bench_gemm(int T, int N, int K, int split, int iters, float* ms_per_
 	cudaEvent_t e0, e1;
 	XALM_CUDA_CHECK(cudaEventCreate(&e0));
 	XALM_CUDA_CHECK(cudaEventCreate(&e1));
-	for (int i = 0; i < 3; i++) XALM_TRY(launch_gemm(g, na, nb, s));
+	for (int i = 0; i < 3; i++) XALM_TRY(launch_gemm<GF_TILES>(g, na, nb, s));
 	XALM_CUDA_CHECK(cudaEventRecord(e0, s));
-	for (int i = 0; i < iters; i++) XALM_TRY(launch_gemm(g, na, nb, s));
+	for (int i = 0; i < iters; i++) XALM_TRY(launch_gemm<GF_TILES>(g, na, nb, s));
 	XALM_CUDA_CHECK(cudaEventRecord(e1, s));
 	XALM_CUDA_CHECK(cudaStreamSynchronize(s));
 	float ms = 0.f;
@@ -2041,7 +2062,7 @@ size_t tc_a_plane_bytes(int T, int K) { return (size_t) cdiv(T, GB_M) * cdiv(K, 
 //   squared ReLU, GELU and its gate: from 2^19 on.  GELU 64 x 4096 x 1024 19.8 -> 20.7, 128 x 4096 x 1024 24.8 -> 20.7, 1024 x 8192 x 1024 70 -> 33
 bool tc_epi_pays(const TcEpi& e, const TcWeight& w, int T, int a_planes) {
 	if (e.kind == TcEpi::STORE) return true;
-	const int tiles = cdiv(T, GB_M) * w.NT, ks = a_planes == 1 ? gemm_split<1, 1>(tiles, w.KT) : w.lo ? gemm_split<2, 2>(tiles, w.KT) : gemm_split<2, 1>(tiles, w.KT);
+	const int tiles = cdiv(T, GB_M) * w.NT, ks = a_planes == 1 ? gemm_split<1, 1, GF_ROWS>(tiles, w.KT) : w.lo ? gemm_split<2, 2, GF_ROWS>(tiles, w.KT) : gemm_split<2, 1, GF_ROWS>(tiles, w.KT);
 	const bool light = e.kind == TcEpi::RELU2 || e.kind == TcEpi::GELU || (e.kind == TcEpi::GLU && e.act == mix::GLU_GELU_TANH);
 	return ks > 1 || (size_t) T * w.N >= (light ? (size_t) 1 << 19 : (size_t) 1 << 21);
 }
@@ -2055,7 +2076,7 @@ int tc_gemm(const TcWeight& w, const float* a_dev, int T, float* out_dev, int ld
 	g.MT = MT; g.NT = w.NT; g.KT = w.KT; g.M = T; g.N = w.N; g.out = out_dev; g.ldo = ldo;
 	g.epi = epi.kind == TcEpi::STORE ? GEPI_STORE : epi.kind == TcEpi::ADD ? GEPI_RESID : GEPI_FUSED;
 	g.fused = epi;
-	return launch_gemm(g, a_lo ? 2 : 1, w.lo ? 2 : 1, s);
+	return launch_gemm<GF_ROWS>(g, a_lo ? 2 : 1, w.lo ? 2 : 1, s);
 }
 
 // ---- groups of matrices (prefill.h) -----------------------------------------------------------------------------------------------
@@ -2088,8 +2109,8 @@ static int launch_group(const TcGroup& t, const uint8_t* a_hi, const uint8_t* a_
 	g.NT = cdiv(t.N, GB_N); g.KT = t.K / GB_K; g.N = t.N;
 	g.gtiles = t.tiles; g.gn_tiles = t.n_tiles; g.gb = t.b;
 	const int grid = std::min(t.max_tiles * g.NT, sm_count());
-	if (a_lo) XALM_TRY((launch_gemm_inst<2, 1, true>(g, CUtensorMap(), grid, s)));
-	else XALM_TRY((launch_gemm_inst<1, 1, true>(g, CUtensorMap(), grid, s)));
+	if (a_lo) XALM_TRY((launch_gemm_inst<2, 1, GF_GROUP>(g, GemmMap<GF_GROUP>(), grid, s)));
+	else XALM_TRY((launch_gemm_inst<1, 1, GF_GROUP>(g, GemmMap<GF_GROUP>(), grid, s)));
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "grouped gemm_tc launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
