@@ -1566,7 +1566,9 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 //   2/1: 33 x 4096 x 4096 42.0 -> 18.5 (5), 333 x 4096 x 4096 45.2 -> 30.0 (2), 333 x 4096 x 14336 139 -> 78 (5, two waves)
 //   2/2: 33 x 4096 x 14336 242 -> 57 (6), 333 x 6144 x 4096 82 -> 49 (2), 500 x 2048 x 6144 94 -> 37 (4)
 // Against float64 the result is nearer, 2 to 5 times at 4 to 8 shares: the tensor cores' own additions truncate, and a share has fewer of them.
-// From about 80 tiles on, and for 16 K steps with 8 tiles and more, one CTA per tile is as fast or faster and the rule says so.
+// With one plane each the rule leaves one CTA per tile from about 80 tiles on where K is not long (640 x 4096 x 14336 86 -> 74, x 4096 28 both ways) and for 16
+// K steps with 8 tiles and more.  Two planes take longer per step and share more often: 16 steps up to 36 tiles (2/1 256 x 4096 x 1024 18.5 -> 15.3, 2/2
+// 22.6 -> 16.8), 64 steps at 80 tiles with 2/2 (640 x 4096 x 4096 76 -> 68).  A twentieth less is asked for, since 2/1 lost there (45.8 -> 47.2 in three shares).
 template <int NA, int NB, int FOR>
 static int gemm_split(int tiles, int KT) {
 	static std::atomic<int> fits[GEMM_MAX_SPLIT + 1]; // clusters of this size that run at a time, 0: not asked yet
@@ -1581,7 +1583,7 @@ static int gemm_split(int tiles, int KT) {
 	constexpr float STEP = NA == 1 ? 0.36f : NB == 1 ? 0.58f : 1.08f; // us
 	const float whole = (float) cdiv(tiles, sm_count()) * (float) KT * STEP;
 	int best = 1;
-	float best_us = whole;
+	float best_us = 0.95f * whole;
 	for (int ks = 2; ks <= GEMM_MAX_SPLIT && ks <= KT && tiles * ks <= 2 * sm_count(); ks++) {
 		int n = fits[ks].load(std::memory_order_relaxed);
 		if (!n) {
