@@ -213,3 +213,14 @@ def test_prefill_4096_tokens_vs_oracle():
     lg_o = om.forward(int(toks[n]), n, 1)
     assert np.max(np.abs(st.logits() - lg_o)) <= LOGIT_TOL
     gm.close(); om.close()
+
+
+@pytest.mark.parametrize("hidden", [416, 544, 640])
+def test_prefill_f16_hidden_sizes_that_end_inside_a_tile(hidden):
+    """Gate and up rows of a tile come as two boxes of 128 rows each; here the last boxes reach past the gate's rows, past the matrix, and past K."""
+    config, om, gm = synth_pair("tiny", "f16", seed=11, std=0.06, hidden_dim=hidden)
+    tokens = np.random.default_rng(5).integers(3, config["vocab_size"], size=70).astype(np.int32)
+    ref = _oracle_all_logits(om, tokens)
+    got = gm.prefill(tokens, 0, want_logits=2)
+    assert np.max(np.abs(got - ref)) <= 1e-3
+    gm.close(); om.close()

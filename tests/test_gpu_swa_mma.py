@@ -125,3 +125,22 @@ def test_infinities_and_nan_stay_with_the_queries_that_see_them(T, pos0, n_split
                 got = capi.swa_attention(q, k, v, pos0, H, G, d, d, window, 0.125, n_splits=n_splits, cache_bf16=True)
             assert np.isfinite(want).any() and not np.isfinite(want).all()
             assert np.allclose(got, want, rtol=0, atol=TOL, equal_nan=True)
+
+
+@pytest.mark.parametrize("T", [5, 9, 15])
+@pytest.mark.parametrize("H,G,d,dv", [(3, 1, 40, 40), (4, 2, 72, 40), (2, 2, 128, 128), (1, 1, 32, 32)])
+def test_passes_of_a_few_tokens(H, G, d, dv, T):
+    """Tiles of mostly padding, warps without a query; short caches in one piece and long ones whose keys are split."""
+    for pos0, splits in ((0, 1), (3, 2), (700, 5), (1500, 7)):
+        q, k, v = inputs(T, pos0 + T, H, G, d, dv, H * d + T)
+        want = reference(q * np.float32(1.001), k, v, pos0, H, G, 10 ** 6, scale=d ** -0.5)
+        got = capi.swa_attention(q * np.float32(1.001), k, v, pos0, H, G, d, dv, 10 ** 6, d ** -0.5, n_splits=splits, cache_bf16=True)
+        assert np.abs(got - want).max() < TOL
+        got = capi.swa_attention_kept(q, k, v, pos0, H, G, d, dv, 50, 9, 0.2, n_splits=splits, cache_bf16=True)
+        assert np.abs(got - reference(q, k, v, pos0, H, G, 50, keep=9, scale=0.2)).max() < TOL
+
+
+@pytest.mark.parametrize("T,pos0,n_splits", [(5, 0, 1), (9, 300, 4), (15, 70, 1)])
+@pytest.mark.parametrize("what", ["v inf", "v nan", "k inf", "q inf"])
+def test_infinities_and_nan_in_passes_of_a_few_tokens(T, pos0, n_splits, what):
+    test_infinities_and_nan_stay_with_the_queries_that_see_them(T, pos0, n_splits, what)
