@@ -400,7 +400,9 @@ static int launch_chunks(const DeltaArgs& a, int rows, cudaStream_t s) {
 	XALM_CUDA_CHECK(cudaFuncSetAttribute(delta_local_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dc_local_smem(D)));
 	delta_local_kernel<D><<<dim3(chunks, a.H), DC_TH, dc_local_smem(D), s>>>(a, chunks);
 	XALM_TRY(launch_check("delta_local"));
-	// eight value channels per CTA where sixteen would leave half of the SMs idle: every CTA of a head reads the head's W, q, k and P
+	// eight value channels per CTA where sixteen would leave a third of the SMs idle: every CTA of a head reads the head's W, q, k and P.  All kernels of a pass, us
+	// with 8 -> 16 channels: 1024 tokens of 8 heads of 64 x 128 (64 CTAs of 16) 120 -> 138, of 16 of 64 x 64 (64) 151 -> 169, of 12 of 64 x 128 (96) 183 -> 159,
+	// of 12 of 128 x 128 (96) 261 -> 196, of 24 of 64 x 64 (96) 224 -> 202; 64 and 256 tokens likewise
 	if (a.H * ((a.dv + 15) / 16) >= 96) XALM_TRY((launch_states<D, 16>(a, chunks, s)));
 	else XALM_TRY((launch_states<D, 8>(a, chunks, s)));
 	delta_finish_kernel<<<(rows * a.H + 7) / 8, 256, 0, s>>>(a);

@@ -1367,7 +1367,10 @@ struct Hgrn2Args {
 	size_t ws_floats;
 };
 // From this many tokens on a pass goes over its chunks at once (rec_chunk.cu): 43 us for three launches at 48 tokens of 8 heads of 64 x 128 and 46 at 256,
-// where the scan takes 0.6 us per token
+// where the scan takes 0.4 to 0.6 us per token.  In whole passes, beside the layer's other branch, scan -> chunks: Kubolorn at width 2048 (16 heads) 80 tokens
+// 427 -> 403 us, 128 475 -> 425; Nabalix at 2048 (8) 96 600 -> 583, at 1024 (4) 80 441 -> 440, 128 480 -> 466; Duletar at 1024 (4, no branch) 96 449 -> 440.
+// Kubolorn at 1024 (8) is the one that loses: 80 336 -> 346, 96 338 -> 348, 128 357 -> 358, 160 368 -> 353, since the grouped products beside the recurrence
+// wait for the SMs that rec_output_kernel holds
 constexpr int HG_CHUNK_ROWS = 80;
 size_t hgrn2_chunk_floats(int H, int d, int dv, int rows); // 0: not this shape
 int launch_hgrn2_chunks(const Hgrn2Args& a, cudaStream_t s);
@@ -2263,8 +2266,9 @@ static inline bool swa_one_ok(const SwaArgs& a, int rows) {
 }
 
 // swa_mma.cu: passes of many tokens over a bf16 cache, on the tensor cores.  It takes heads of 32 to 128 channels in whole 16-byte pieces whose scores
-// do not mix; smaller heads would be mostly padding.  From 5 tokens on, since a tile that is mostly padding still beats the tiled kernel: 9 tokens of 16 heads of
-// 128 over 777 keys 165 -> 22 + 4 us.  Takes a.n_splits > 0
+// do not mix; smaller heads would be mostly padding.  From 5 tokens on, since a tile that is mostly padding still beats the tiled kernel.  5 tokens, caches
+// flushed: 16 heads of 128 over 5 keys 205 -> 24 us, over 4005 305 -> 40; 4 heads of 64 over 517 keys 47 -> 22; one head of 32 over 69 keys 21 -> 22, over 4005
+// 29 -> 26.  9 and 15 tokens: 1.2 to 11 times as fast for 1 to 32 heads of 32, 64 and 128.  Takes a.n_splits > 0
 int launch_swa_mma(const SwaArgs& a, int rows, cudaStream_t s);
 constexpr int SWA_MMA_ROWS = 64, SWA_MMA_KEYS = 64; // queries of one head per CTA; keys per step
 static inline bool swa_mma_ok(const SwaArgs& a, int rows, bool cache_f32) {
@@ -2286,7 +2290,7 @@ static inline int swa_mma_splits(const SwaArgs& a, int rows) {
 	return (int) std::max<long long>(1, std::min({296 / ctas, keys / SWA_MMA_KEYS, (long long) a.part_cap / rows}));
 }
 // A latent for passes of more than the few tokens that swa_one.cu takes: keys that are the values too, of one head of more than the 128 channels above.
-// Takes a.n_splits > 0
+// Against the tiled kernel 1.3 to 15 times as fast for 5 to 64 tokens of 1 to 16 heads of 136 to 576 channels over 5 to 4000 keys.  Takes a.n_splits > 0
 int launch_swa_latent(const SwaArgs& a, int rows, cudaStream_t s);
 constexpr int SWA_LATENT_ROWS = 32; // (query, head) pairs per CTA
 static inline bool swa_latent_ok(const SwaArgs& a, int rows, bool cache_f32) {

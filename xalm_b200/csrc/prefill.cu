@@ -1,4 +1,4 @@
-// prefill.cu — batched prefill / perplexity (BASELINE config 3): the whole prompt goes through every layer at once,
+// prefill.cu — batched prefill / perplexity: the whole prompt goes through every layer at once,
 // the seven per-layer contractions become GEMMs on the 5th-generation tensor cores (tcgen05.mma, accumulators in
 // TMEM), everything else stays the reference's arithmetic (infer.cpp:365-496) applied to T rows instead of one.
 //
@@ -26,7 +26,7 @@
 // stages per layer add up to ~4e-2 on the logits of a 32-layer model).  split=2 keeps the activations to ~fp32 by feeding
 // hi = fp16(a) and lo = fp16(a - hi) as two MMAs against the same weight tile.  split=3 (default) does the same for the weights
 // (hi.hi + lo.hi + hi.lo) and for q and the softmax probabilities in attention: logits within ~1e-3 of the token-at-a-time
-// fp32 path at 32 layers x 4096 tokens.  Tolerance in tests: 1e-2 (north star: "within max-abs 1e-2 (fp16)").
+// fp32 path at 32 layers x 4096 tokens.  Tolerance in tests: 1e-2.
 #define XALM_SECONDARY_TU
 #include <cuda.h> // CUtensorMap: types only, the encoder is asked of the runtime
 #include <cuda_fp16.h>
@@ -1565,7 +1565,8 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 //   1/1: 45 x 1024 x 4096 24.7 -> 12.4 (8 CTAs), 256 x 2048 x 2048 18.5 -> 14.4 (4), 1024 x 1024 x 4096 26.7 -> 18.5 (4), 1024 x 2048 x 8192 45.2 -> 30.8 (2)
 //   2/1: 33 x 4096 x 4096 42.0 -> 18.5 (5), 333 x 4096 x 4096 45.2 -> 30.0 (2), 333 x 4096 x 14336 139 -> 78 (5, two waves)
 //   2/2: 33 x 4096 x 14336 242 -> 57 (6), 333 x 6144 x 4096 82 -> 49 (2), 500 x 2048 x 6144 94 -> 37 (4)
-// Against float64 the result is nearer, 2 to 5 times at 4 to 8 shares: the tensor cores' own additions truncate, and a share has fewer of them.
+// Against float64 the result is nearer, 2 times at two shares (333 x 4096 x 4096, 2/2: 1.46e-5 -> 7.4e-6 in the 2-norm) to 7 at eight (33 x 1024 x 4096, 2/1:
+// 9.7e-6 -> 1.3e-6): the tensor cores' own additions truncate, and a share has fewer of them.
 // With one plane each the rule leaves one CTA per tile from about 80 tiles on where K is not long (640 x 4096 x 14336 86 -> 74, x 4096 28 both ways) and for 16
 // K steps with 8 tiles and more.  Two planes take longer per step and share more often: 16 steps up to 36 tiles (2/1 256 x 4096 x 1024 18.5 -> 15.3, 2/2
 // 22.6 -> 16.8), 64 steps at 80 tiles with 2/2 (640 x 4096 x 4096 76 -> 68).  A twentieth less is asked for, since 2/1 lost there (45.8 -> 47.2 in three shares).

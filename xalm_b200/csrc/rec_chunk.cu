@@ -11,9 +11,10 @@
 // which would make A a plain product of two matrices, overflow where a decay is small.  A product with s > t is not formed, so that an infinity
 // or a NaN stays with the tokens that see it.
 //
-// Bound: latency and the issue slots of two CTAs per SM, 60 thousand warp instructions per chunk and head at 64 x 128 (a third the walk over t, half the
-// two products with v).  The scan of hgrn2_cols_kernel takes token after token on a warp per scheduler, 0.6 us each whatever the heads; here all chunks
-// and heads are there at once.  1024 tokens of 16 heads of 64 x 128: 505 us as a scan, 38 + 8 + 21 us as the three kernels (caches flushed).
+// Bound: latency and issue slots, 56 thousand warp instructions per chunk and head at 64 x 128 (a third the walk over t, half the two products with v), 29 % of
+// the slots used at 1024 tokens of 8 heads.  Two CTAs of rec_local_kernel fit an SM at up to 64 key channels (100 KB each), one at 128 (149 KB).  The scan of
+// hgrn2_cols_kernel takes token after token on a warp per scheduler, 0.4 to 0.6 us each (8 and 16 heads of 64 x 128); here all chunks and heads are there at
+// once.  1024 tokens of 16 heads of 64 x 128: 505 us as a scan, 38 + 8 + 21 us as the three kernels (caches flushed).
 #define XALM_SECONDARY_TU
 #include "common.cuh"
 #include "family.h"

@@ -372,8 +372,11 @@ static_assert(4 * (64 * (64 + 8) + 4 * 32) <= smm_smem(64, 64, 4) && 4 * (64 * (
 // Rows of a tile are (query, head) pairs, 32 a CTA.  Two groups of W warps, 16 rows each: for the scores a warp takes a W-th of the channels (its queries'
 // planes stay in registers) and all 64 keys of a block, for the output a W-th of the value channels.  The parts of the scores meet in shared memory, where a
 // warp makes its share of the rows' weights of them.  Products and sums as above.
-// Bound: latency of a scheduler's four warps; the mma.sync pipe at 512 channels is next (3072 products of 16 x 8 x 16 per 64 keys).  W = 8 where W = 4 would
-// leave two warps per scheduler (256 tokens of 16 heads of 512 over 256 to 777 keys 93 -> 72 us).  The fp32 FMA tiles of mix_ops.cuh, which took these passes
+// Bound: latency of a scheduler's four warps (1024 tokens of 8 heads of 256: issue slots 30 %, mma.sync pipe 17 %); at 512 channels the pipe is next (3072
+// products of 16 x 8 x 16 per 64 keys).  Registers are short: at the 128 of two CTAs per SM the queries' planes of 256 channels spill in part (7 % of the warp
+// instructions are spill stores and loads), a few of the instances for 512 and 576 channels too.  W = 8 where W = 4 would
+// leave two warps per scheduler (256 tokens of 16 heads of 512 over 256 to 777 keys 93 -> 72 us).  The instance for up to 320 channels with values of 256 against
+// the one for 512 (320 and 328 channels, 64 tokens of 8 heads over 4000 keys): 69 us, 79; 33 tokens over 33 keys 26, 26.  The fp32 FMA tiles of mix_ops.cuh, which took these passes
 // before, and this kernel, caches flushed: 256 tokens of 16 heads of 512 496 -> 72 us, 9 tokens of them over 777 keys 244 -> 24 + 6 us (twelve splits and their join), 1024 tokens of 8 heads of 256
 // in a window of 512 357 -> 110 us.  Distance from float64 at 512 channels and 764 keys: within 5 % of the FMA kernel's.
 constexpr int SML_ROWS = SWA_LATENT_ROWS, SML_LDS = SMM_KEYS + 4; // floats of a row of scores
