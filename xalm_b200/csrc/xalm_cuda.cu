@@ -1390,7 +1390,8 @@ static int enqueue_token(xalm_cuda_model* m, int mode, cudaStream_t s, int* n_la
 		if (const int pf_mb = tune("tail_prefetch_mb")) { // chain: every kernel warms L2 with the head of the next kernel's stream
 			auto head = [&](const WMat& w, const uint8_t** ptr, unsigned long long* bytes) {
 				*ptr = w.p0;
-				*bytes = std::min<unsigned long long>((unsigned long long) w.s0 * w.rows, (unsigned long long) pf_mb << 20);
+				// (s0: bytes of a row, or of a 16-row tile; 16 times too many of them run past the allocation, where a prefetch takes microseconds to fail)
+				*bytes = std::min<unsigned long long>((unsigned long long) w.s0 * (w.layout_frag ? w.rows / MMA_RC : w.rows), (unsigned long long) pf_mb << 20);
 			};
 			a_qkv.pf_kv = 1;
 			head(a_wo.w, &a_at.pf_ptr, &a_at.pf_bytes);
