@@ -955,9 +955,9 @@ def main():
     k_bytes = 2 * hidden_l * cfg["dim"] * wtype.bytes // wtype.block
     nbuf = max(2, int(np.ceil(600e6 / k_bytes)))
     # which matvec the MODEL runs for this format and sharding (xalm_cuda.cu: alloc_wmat): the tensor-core kernel (matvec_mma.cuh) for the
-    # 4/5-bit formats and, under tensor parallelism, for the 8-bit ones; the dp4a kernel (matvec_idp.cuh) for 8-bit on one GPU
+    # integer formats; with XALM_MMA=2 the dp4a kernel (matvec_idp.cuh) for the 8-bit ones on one GPU
     int_fmt = args.wtype in ("q8_0", "q8", "q4_0", "q4_1", "q5_0", "q5_1")
-    mma_mode = int(os.environ.get("XALM_MMA", "2"))
+    mma_mode = int(os.environ.get("XALM_MMA", "1"))
     mma_kernel = int_fmt and (2 * hidden_l) % 16 == 0 and (mma_mode == 1 or (mma_mode == 2 and (world > 1 or args.wtype not in ("q8_0", "q8"))))
     idp_kernel = int_fmt and not mma_kernel and cfg["dim"] % 256 == 0 and (2 * hidden_l) % 8 == 0
     if mma_kernel:
@@ -978,7 +978,7 @@ def main():
     line = {
         "metric": "decode_tokens_per_s", "value": tps, "unit": "tok/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": ("f32 activations and accumulation; integer weight formats multiply in int8 (" + ("mma.sync m16n8k32 u8" if mma_kernel else "dp4a") +
+        "dtype": ("f32 activations and accumulation; integer weight formats multiply in int8 (" + ("mma.sync m16n8k32 s8" if mma_kernel else "dp4a") +
                   ") against 3 x int8 block-floating activation limbs") if (idp_kernel or mma_kernel) else "f32",
         "data": "synthetic", "config": workload_config(args, cfg),
         "e2e": {"value": e2e_tps, "unit": "tok/s", "h2d_bytes_per_step": 32, "d2h_bytes_per_step": cfg["vocab_size"] * 4,

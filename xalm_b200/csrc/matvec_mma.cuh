@@ -5,19 +5,26 @@
 // lane: 0.112 (q8_0) - 0.124 (q4_0) warp instructions per weight.  ncu: q4_0 W1|W3 runs at
 // 30 % of DRAM peak with the issue slots 52 % busy and 0.9 eligible warps per scheduler — the consumers, not HBM, set the pace,
 // and q4_0 decodes no faster than q8_0 although it streams half the bytes.  Here ONE mma handles a 16-row x 32-element block
-// column (512 weights) against the three activation limbs at once, and the per-block float work is 2 IMAD + 2 I2F + 2 FFMA:
-// ~0.04 warp instructions per weight.
+// column (512 weights) against the three activation limbs at once, and the per-block float work is 2 IMAD + 2 I2F + 2 FFMA.
 //
 // Arithmetic (exact in integers, like idp.cuh).  Activations are staged once per CTA as block floating point, x_k ~= dx * X_k
 // with |X_k| < 2^23 and one power-of-two dx per 32 elements, but in OFFSET form X'_k = X_k + 2^23 (three unsigned byte limbs
 // l0' l1' l2'), because the mma has one signedness per operand.  The B operand (32 k x 8 columns) holds
-//     column 0: l2'   column 1: l1'   column 2: l0'   column 3: ones   columns 4-7: zero
-// and the stored weight bytes u_k = q_k + BIAS are the A operand.  With the accumulators initialised to
-//     c(l2') = -BIAS S2',  c(l1') = -BIAS S1',  c(l0') = -BIAS (S0' - 4096),  c(ones) = 0       (S' = limb sums of the block)
-// the lane that holds columns (0, 1) forms v = 256 c1 + c0, the lane that holds (2, 3) forms v = c0 - 128 c1 (this removes the
-// 2^23 offset: 2^23 = 128 * 65536), and  sum_k (u_k - BIAS) X_k = 65536 v(2,3) + v(0,1)  exactly.  Each lane accumulates
-// float(v) * (d * dx [* 65536]) in fp32; lanes are added at the end of a tile.  With a one-hot x everything is exact and the
+//     column 0: l2'   column 1: l1'   column 2: l0'   columns 3-7: ones (of which only column 3 is used)
+// and the A operand the quants q_k as signed bytes, times MUL where that takes fewer instructions: a 4-bit quant stays in a byte's
+// upper half, whose top bit turned makes it 16 (q - 8).  The formats with a minimum have unsigned quants.  Nothing is left to
+// correct for in the accumulators, which start at zero.  The lane that holds columns (0, 1) forms v = 256 c1 + c0, the lane that
+// holds (2, 3) forms v = c0 - 128 c1 (this removes the 2^23 offset: 2^23 = 128 * 65536), and
+// MUL sum_k q_k X_k = 65536 v(2,3) + v(0,1)  exactly.  Each lane accumulates float(v) * (d * dx) in fp32; at the end of a tile the
+// factors 65536 and 1 / MUL are applied and the lanes are added.  With a one-hot x everything is exact and the
 // kernel returns the dequantised weight bit for bit (d*q exact, d*q+m rounds once).
+//
+// Bound: the 8-bit formats HBM (28672 x 4096 21.2 us, 19.7 with the multiplication left out), the 4-bit ones the consumers' issue slots and what they read
+// from shared memory (16.2 us, 12.0).  A record used to take biased weights, accumulator inits of 16 bytes and a branch around the limbs of unused
+// columns, 30 instructions of which 22 are left; 128 records a stage instead of 64 take the per-stage work off the 4-bit formats.  Back to back, buffers
+// beyond L2, before -> after: q4_0 28672 x 4096 17.6 -> 16.2 us, 4096 x 14336 11.4 -> 9.3, 4096 x 4096 5.0 -> 4.4; q8_0 28672 x 4096
+// 21.5 -> 21.2, 4096 x 14336 13.6 -> 12.5 (dp4a 22.9, 13.2).  Tried and not faster: the same in fp16 mma (twice the tensor instructions and wider
+// activations: 21.0 us), a warp's activations held in registers for two or four tiles (17.9, 19.1), 8 or 24 multiplying warps (16.6, 18.4).
 //
 // Skeleton: as matvec_idp.cuh — persistent CTAs (one per SM), a producer warp streaming records into an mbarrier ring with ONE
 // cp.async.bulk per stage (a tile's records are contiguous), 16 consumer warps, rmsnorm prologue (1/rms applied to the row
@@ -30,24 +37,24 @@
 namespace xalm {
 
 constexpr int MMA_RC = 16;  // rows per tile
-constexpr int MMA_SB = 64;  // records (32-element block columns) per ring stage
 constexpr int MMA_NCW = 16; // consumer warps
 constexpr int MMA_NT = MMA_NCW * 32;
 constexpr int MMA_MP = 2;   // activation groups a lane keeps in flight (8 elements each): one pass for n <= 8192
 
-// ---- activation image in shared memory: 3 limb planes (stride n + 16 bytes: the three planes a quarter-warp reads fall into
-//      different banks) + one 64-byte table entry per block, 16 bytes per lane position: {c-init (l2'), c-init (l1'), dx, sum x} {c-init (l0'), 0, dx * 65536, 0} {0} {0}
+// ---- activation image in shared memory: four planes of bytes (l2', l1', l0', ones; the eight bytes a lane position feeds the mma for a block lie together:
+//      elements 4 tig .., then 16 + 4 tig ..; planes n + 32 bytes apart, so that the four a half-warp reads fall into different banks) and one entry per
+//      block: dx, or {dx, sum x} for the formats with a minimum ----
 struct XmView {
 	uint8_t* q;
-	int4* tbl;
+	float* tbl;
 	int ps; // plane stride
 };
-__host__ __device__ inline size_t xm_bytes(int n) { return ((size_t) 3 * (n + 16) + (size_t) (n / 32) * 64 + 127) / 128 * 128; }
-__device__ __forceinline__ XmView xm_view(uint8_t* base, int n) { return {base, reinterpret_cast<int4*>(base + (size_t) 3 * (n + 16)), n + 16}; }
+__host__ __device__ inline size_t xm_bytes(int n) { return ((size_t) 4 * (n + 32) + (size_t) (n / 32) * 8 + 127) / 128 * 128; }
+__device__ __forceinline__ XmView xm_view(uint8_t* base, int n) { return {base, reinterpret_cast<float*>(base + (size_t) 4 * (n + 32)), n + 32}; }
 
 // eight consecutive elements per lane, the four lanes 4k .. 4k+3 of a warp share a block (call with all lanes of the warp)
 // (lanes past the end of the vector pass valid = false and take part in the shuffles only)
-template <int BIAS>
+template <bool HAS_MIN>
 __device__ __forceinline__ void xm_store_group8(const XmView& v, int grp, const float (&x)[8], bool valid = true) {
 	uint32_t mb = 0;
 #pragma unroll
@@ -59,47 +66,50 @@ __device__ __forceinline__ void xm_store_group8(const XmView& v, int grp, const 
 	const float sc = live ? __uint_as_float((uint32_t) (276 - eb) << 23) : 0.f;
 	const float dx = live ? __uint_as_float((uint32_t) (eb - 22) << 23) : 0.f;
 	uint32_t w[3][2];
-	uint32_t s0 = 0, s1 = 0, s2 = 0;
+	int sum = 0;
 #pragma unroll
 	for (int q = 0; q < 2; q++) {
 		int X[4];
 #pragma unroll
-		for (int e = 0; e < 4; e++) X[e] = min(__float2int_rn(x[4 * q + e] * sc), 8388607) + 8388608; // offset form: 0 .. 2^24 - 1
+		for (int e = 0; e < 4; e++) {
+			X[e] = min(__float2int_rn(x[4 * q + e] * sc), 8388607);
+			if (HAS_MIN) sum += X[e];
+			X[e] += 8388608; // offset form: 0 .. 2^24 - 1
+		}
 #pragma unroll
 		for (int k = 0; k < 3; k++) {
 			const uint32_t sel = (uint32_t) k | ((uint32_t) (4 + k) << 4);
 			const uint32_t lo = prmt((uint32_t) X[0], (uint32_t) X[1], sel), hi = prmt((uint32_t) X[2], (uint32_t) X[3], sel);
-			w[2 - k][q] = prmt(lo, hi, 0x5410u);
+			w[k][q] = prmt(lo, hi, 0x5410u);
 		}
-		asm("dp4a.u32.u32 %0, %1, %2, %0;" : "+r"(s0) : "r"(w[0][q]), "r"(0x01010101u));
-		asm("dp4a.u32.u32 %0, %1, %2, %0;" : "+r"(s1) : "r"(w[1][q]), "r"(0x01010101u));
-		asm("dp4a.u32.u32 %0, %1, %2, %0;" : "+r"(s2) : "r"(w[2][q]), "r"(0x01010101u));
 	}
-	uint32_t u = s1 | (s2 << 16); // block totals <= 32 * 255 < 2^16
-	u += __shfl_xor_sync(0xffffffffu, u, 1);
-	u += __shfl_xor_sync(0xffffffffu, u, 2);
-	s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-	s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+	if (HAS_MIN) { // (32 x 2^23 at most)
+		sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+		sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+	}
 	if (!valid) return;
+	uint8_t* o = v.q + (size_t) (grp >> 2) * 32 + (grp & 1) * 16 + ((grp >> 1) & 1) * 4;
 #pragma unroll
-	for (int k = 0; k < 3; k++) *reinterpret_cast<uint2*>(v.q + (size_t) k * v.ps + (size_t) grp * 8) = make_uint2(w[k][0], w[k][1]);
+	for (int k = 0; k < 3; k++) {
+		*reinterpret_cast<uint32_t*>(o + (size_t) k * v.ps) = w[k][0];
+		*reinterpret_cast<uint32_t*>(o + (size_t) k * v.ps + 8) = w[k][1];
+	}
 	if ((grp & 3) == 0) {
-		const int S0 = (int) s0, S1 = (int) (u & 0xFFFFu), S2 = (int) (u >> 16);
-		const int tot = (S0 - 4096) * 65536 + S1 * 256 + S2; // sum of the block's X (the offsets removed)
-		const float sx = __int2float_rn(tot) * dx;
-		int4* e = v.tbl + 4 * (grp >> 2); // one entry per lane position tig (columns 2 tig, 2 tig + 1); positions 2, 3 hold the zero columns
-		e[0] = make_int4(-BIAS * S2, -BIAS * S1, (int) __float_as_uint(dx), (int) __float_as_uint(sx));
-		e[1] = make_int4(-BIAS * (S0 - 4096), 0, (int) __float_as_uint(dx * 65536.f), 0);
-		e[2] = make_int4(0, 0, 0, 0);
-		e[3] = make_int4(0, 0, 0, 0);
+		if (HAS_MIN) *reinterpret_cast<float2*>(v.tbl + 2 * (grp >> 2)) = make_float2(dx, __int2float_rn(sum) * dx);
+		else v.tbl[grp >> 2] = dx;
 	}
 }
 
-// d = a * b + c with separate accumulator-in registers: the c-init values are used as they come from the table, no copies
-__device__ __forceinline__ void mma_u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0, int c1) {
-	asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
-	             : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-	             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1));
+template <bool SIGNED>
+__device__ __forceinline__ void mma_i8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+	if (SIGNED)
+		asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+		    : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+		    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+	else
+		asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+		    : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+		    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
 
 // ---- weight side: the A fragment and the scales of one record -------------------------------------------------------------
@@ -107,22 +117,22 @@ template <int TYPE>
 struct MmaFmt;
 template <>
 struct MmaFmt<XALM_Q8_0> {
-	static constexpr int RB = 544, BIAS = 128;
+	static constexpr int RB = 544, MUL = 1;
 	static constexpr bool HAS_MIN = false;
 	static __device__ __forceinline__ void load(const uint8_t* rec, int lane, int g, uint32_t (&a)[4], float& d0, float& d1, float&, float&) {
 		const uint4 q = *reinterpret_cast<const uint4*>(rec + lane * 16);
-		a[0] = q.x; a[1] = q.y; a[2] = q.z; a[3] = q.w;
+		a[0] = q.x ^ 0x80808080u; a[1] = q.y ^ 0x80808080u; a[2] = q.z ^ 0x80808080u; a[3] = q.w ^ 0x80808080u;
 		const float2 d = __half22float2(*reinterpret_cast<const __half2*>(rec + 512 + g * 4));
 		d0 = d.x; d1 = d.y;
 	}
 };
 template <>
 struct MmaFmt<XALM_Q8> {
-	static constexpr int RB = 512, BIAS = 128;
+	static constexpr int RB = 512, MUL = 1;
 	static constexpr bool HAS_MIN = false;
 	static __device__ __forceinline__ void load(const uint8_t* rec, int lane, int, uint32_t (&a)[4], float& d0, float& d1, float&, float&) {
 		const uint4 q = *reinterpret_cast<const uint4*>(rec + lane * 16);
-		a[0] = q.x; a[1] = q.y; a[2] = q.z; a[3] = q.w;
+		a[0] = q.x ^ 0x80808080u; a[1] = q.y ^ 0x80808080u; a[2] = q.z ^ 0x80808080u; a[3] = q.w ^ 0x80808080u;
 		d0 = d1 = 1.f / 100.f; // types.h:423-424
 	}
 };
@@ -139,17 +149,19 @@ __device__ __forceinline__ void mma_fifth_bits(const uint8_t* rec, int lane, uin
 }
 template <>
 struct MmaFmt<XALM_Q4_0> { // d * (q - 8)
-	static constexpr int RB = 288, BIAS = 8;
+	static constexpr int RB = 288, MUL = 16;
 	static constexpr bool HAS_MIN = false;
 	static __device__ __forceinline__ void load(const uint8_t* rec, int lane, int g, uint32_t (&a)[4], float& d0, float& d1, float&, float&) {
-		mma_nibbles(rec, lane, a);
+		const uint2 q = *reinterpret_cast<const uint2*>(rec + lane * 8); // a nibble in a byte's upper half, its top bit turned: 16 (q - 8) as a signed byte
+		a[0] = ((q.x << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[1] = (q.x & 0xF0F0F0F0u) ^ 0x80808080u;
+		a[2] = ((q.y << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[3] = (q.y & 0xF0F0F0F0u) ^ 0x80808080u;
 		const float2 d = __half22float2(*reinterpret_cast<const __half2*>(rec + 256 + g * 4));
 		d0 = d.x; d1 = d.y;
 	}
 };
 template <>
 struct MmaFmt<XALM_Q4_1> { // d * q + m
-	static constexpr int RB = 320, BIAS = 0;
+	static constexpr int RB = 320, MUL = 1;
 	static constexpr bool HAS_MIN = true;
 	static __device__ __forceinline__ void load(const uint8_t* rec, int lane, int g, uint32_t (&a)[4], float& d0, float& d1, float& m0, float& m1) {
 		mma_nibbles(rec, lane, a);
@@ -160,18 +172,20 @@ struct MmaFmt<XALM_Q4_1> { // d * q + m
 };
 template <>
 struct MmaFmt<XALM_Q5_0> { // d * ((ql | qh << 4) - 16)
-	static constexpr int RB = 352, BIAS = 16;
+	static constexpr int RB = 352, MUL = 8;
 	static constexpr bool HAS_MIN = false;
 	static __device__ __forceinline__ void load(const uint8_t* rec, int lane, int g, uint32_t (&a)[4], float& d0, float& d1, float&, float&) {
 		mma_nibbles(rec, lane, a);
 		mma_fifth_bits(rec, lane, a);
+#pragma unroll
+		for (int k = 0; k < 4; k++) a[k] = (a[k] << 3) ^ 0x80808080u; // 8 (q - 16) as a signed byte
 		const float2 d = __half22float2(*reinterpret_cast<const __half2*>(rec + 320 + g * 4));
 		d0 = d.x; d1 = d.y;
 	}
 };
 template <>
 struct MmaFmt<XALM_Q5_1> { // d * (ql | qh << 4) + m
-	static constexpr int RB = 384, BIAS = 0;
+	static constexpr int RB = 384, MUL = 1;
 	static constexpr bool HAS_MIN = true;
 	static __device__ __forceinline__ void load(const uint8_t* rec, int lane, int g, uint32_t (&a)[4], float& d0, float& d1, float& m0, float& m1) {
 		mma_nibbles(rec, lane, a);
@@ -183,11 +197,13 @@ struct MmaFmt<XALM_Q5_1> { // d * (ql | qh << 4) + m
 };
 
 __host__ __device__ inline bool mma_supported(int t) { return frag_record_bytes(t) != 0; }
+// records (32-element block columns) per ring stage: about 36 KB
+__host__ __device__ constexpr int mma_sb(int record_bytes) { return record_bytes > 400 ? 64 : 128; }
 __host__ __device__ inline int mma_pb(int NS) { return NS + 2 < 8 ? 8 : NS + 2; } // partial-sum buffers (tiles in flight), as idp_pb
 
 __host__ __device__ inline size_t mma_smem_bytes(int type, int n, int NS) {
 	size_t s = xm_bytes(n);
-	s += (size_t) NS * MMA_SB * frag_record_bytes(type);
+	s += (size_t) NS * mma_sb(frag_record_bytes(type)) * frag_record_bytes(type);
 	s += (size_t) mma_pb(NS) * MMA_NCW * MMA_RC * sizeof(float);
 	s += (2 * (size_t) NS + 2 * mma_pb(NS)) * sizeof(uint64_t);
 	s += MMA_NCW * sizeof(float);
@@ -201,9 +217,9 @@ struct MmaArgs {
 };
 
 template <int TYPE, bool NORM>
-__global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const MmaArgs ta) {
+__global__ void __maxnreg__(80) matvec_mma_kernel(const MmaArgs ta) {
 	using F = MmaFmt<TYPE>;
-	constexpr int RC = MMA_RC, SB = MMA_SB, NCW = MMA_NCW, NT = MMA_NT, RB = F::RB, MP = MMA_MP;
+	constexpr int RC = MMA_RC, NCW = MMA_NCW, NT = MMA_NT, RB = F::RB, SB = mma_sb(RB), MP = MMA_MP, QB = 4 * NCW; // QB: records that are unrolled
 	constexpr int STAGE = SB * RB;
 	auto cbar = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
 	const MatvecArgs& a = ta.a;
@@ -339,6 +355,8 @@ __global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const
 			if (grp < ngrp) load_gw(grp, gw[p]);
 		}
 	}
+	const XmView xv = xm_view(smem, n);
+	for (int i = tid * 16; i < n; i += NT * 16) *reinterpret_cast<uint4*>(xv.q + (size_t) 3 * xv.ps + i) = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
 	pdl_wait(); // activations / KV ring of earlier kernels are visible from here on
 	tl_mark(tl, 2);
 	if (a.epi == EPI_QKV && blockIdx.x == 0 && a.step->kv_sink > 0) { // re-rotate the attention sinks (infer.cpp:393-399)
@@ -381,7 +399,6 @@ __global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const
 		}
 	}
 	// ---- stage activations: quantise(NORM ? x * g : x); the scalar 1/rms is applied to the row sums (y = scale * sum w (x g)) ----
-	const XmView xv = xm_view(smem, n);
 	float ss = 0.f;
 	{
 		auto load_group = [&](int grp, float (&v)[8]) {
@@ -440,7 +457,7 @@ __global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const
 							xr[p][e] = xr[p][e] * g; // infer.cpp:233-235 without the scalar
 						}
 					}
-					xm_store_group8<F::BIAS>(xv, grp, xr[p], valid);
+					xm_store_group8<F::HAS_MIN>(xv, grp, xr[p], valid);
 				}
 			}
 		}
@@ -454,64 +471,61 @@ __global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const
 
 	// this lane's place in the mma fragments
 	const int g = lane >> 2, tig = lane & 3;
-	const int vmul = tig == 0 ? 256 : tig == 1 ? -128 : 0; // v = c_odd * vmul + c_even
-	const uint8_t* bp = xv.q + (size_t) (g == 0 ? 2 : g == 1 ? 1 : 0) * xv.ps + tig * 4; // B column g: l2', l1', l0' (then ones, zeros)
-	const uint32_t bdef = g == 3 ? 0x01010101u : 0u;
-	const int4* tp = xv.tbl + tig;
+	const int vmul = tig == 0 ? 256 : -128; // v = c_odd * vmul + c_even: columns (l2', l1') of lane position 0, (l0', ones) of 1; 2 and 3 are not used
+	const float yend = (tig == 0 ? 1.f : 65536.f) / F::MUL;
+	constexpr int TW = F::HAS_MIN ? 2 : 1; // floats of a block's table entry
+	const uint8_t* bp = xv.q + (size_t) min(g, 3) * xv.ps + tig * 8 + warp * 32;
+	const float* tp = xv.tbl + warp * TW;
+	const uint8_t* rp = ring + (size_t) warp * RB;
+	float y0, y1; // rows g and g + 8 of the tile, this lane's columns
+	// one record (16 rows x 32 elements): rec = its bytes, bq = this lane's limb bytes of the block, tq = its table entry
+	auto record = [&](const uint8_t* rec, const uint8_t* bq, const float* tq) {
+		uint32_t A[4];
+		float d0, d1, m0 = 0.f, m1 = 0.f;
+		F::load(rec, lane, g, A, d0, d1, m0, m1);
+		const uint2 B = *reinterpret_cast<const uint2*>(bq);
+		int c[4];
+		mma_i8<!F::HAS_MIN>(c, A, B.x, B.y);
+		const float dx = tq[0];
+		y0 = fmaf(__int2float_rn(c[1] * vmul + c[0]), d0 * dx, y0);
+		y1 = fmaf(__int2float_rn(c[3] * vmul + c[2]), d1 * dx, y1);
+		if (F::HAS_MIN) { // lane position 0 only
+			const float sx = tig == 0 ? tq[1] : 0.f;
+			y0 = fmaf(m0, sx, y0);
+			y1 = fmaf(m1, sx, y1);
+		}
+	};
 
 	int slot = 0, phase = 0;
-	int pb_next = 0, pph_next = 0;
+	int pb = 0, pph = 0;
 	for (int tt = 0; tt < my_tiles; tt++) {
-		const int pb = pb_next, pph = pph_next;
-		if (++pb_next == PB) { pb_next = 0; pph_next ^= 1; }
-		float y0 = 0.f, y1 = 0.f; // rows g and g + 8 of the tile, this lane's columns
+		y0 = y1 = 0.f;
 		for (int kr = 0; kr < kranges; kr++) {
-			const int b0 = kr * SB;
-			const int nbs = min(SB, nb - b0);
-			const uint8_t* st = ring + (size_t) slot * STAGE;
+			const uint8_t *rec = rp + (size_t) slot * STAGE, *bq = bp + (size_t) kr * (SB * 32);
+			const float* tq = tp + kr * (SB * TW);
 			mbar_wait(&full[slot], phase);
-			// one record (16 rows x 32 elements): rec = its bytes, bq = this lane's limb bytes of the block, tq = its table entry
-			auto record = [&](const uint8_t* rec, const uint8_t* bq, const int4* tq) {
-				uint32_t A[4];
-				float d0, d1, m0 = 0.f, m1 = 0.f;
-				F::load(rec, lane, g, A, d0, d1, m0, m1);
-				uint32_t B0 = bdef, B1 = bdef;
-				if (lane < 12) {
-					B0 = *reinterpret_cast<const uint32_t*>(bq);
-					B1 = *reinterpret_cast<const uint32_t*>(bq + 16);
-				}
-				const int4 tb = *tq;
-				int c[4];
-				mma_u8(c, A, B0, B1, tb.x, tb.y);
-				const int v0 = c[1] * vmul + c[0], v1 = c[3] * vmul + c[2];
-				const float dxl = __int_as_float(tb.z);
-				y0 = fmaf(__int2float_rn(v0), d0 * dxl, y0);
-				y1 = fmaf(__int2float_rn(v1), d1 * dxl, y1);
-				if (F::HAS_MIN) {
-					const float sxl = __int_as_float(tb.w);
-					y0 = fmaf(m0, sxl, y0);
-					y1 = fmaf(m1, sxl, y1);
-				}
-			};
-			if (nbs == SB) { // a full stage: this warp's four records sit at fixed offsets (every address = base + immediate)
-				const uint8_t* rec = st + (size_t) warp * RB;
-				const uint8_t* bq = bp + (size_t) (b0 + warp) * 32;
-				const int4* tq = tp + 4 * (b0 + warp);
+			const int left = nb - kr * SB;
 #pragma unroll
-				for (int i = 0; i < SB / NCW; i++) record(rec + (size_t) i * NCW * RB, bq + (size_t) i * NCW * 32, tq + i * NCW * 4);
-			} else {
-				for (int j = warp; j < nbs; j += NCW) record(st + (size_t) j * RB, bp + (size_t) (b0 + j) * 32, tp + 4 * (b0 + j));
+			for (int q = 0; q < SB; q += QB) {
+				if (left >= q + QB) { // this warp's four records sit at fixed offsets (every address = base + immediate)
+#pragma unroll
+					for (int i = q / NCW; i < (q + QB) / NCW; i++) record(rec + (size_t) i * NCW * RB, bq + (size_t) i * NCW * 32, tq + i * NCW * TW);
+				} else {
+#pragma unroll 1
+					for (int j = q; warp + j < left; j += NCW) record(rec + (size_t) j * RB, bq + (size_t) j * 32, tq + j * TW);
+					break;
+				}
 			}
 			__syncwarp();
 			if (lane == 0) mbar_arrive(&empty[slot]);
 			if (++slot == NS) { slot = 0; phase ^= 1; }
 		}
 		if (tl >= 0 && tt < 4) tl_begin(510 + 10 * tt + a.epi); // timeline event: tile tt multiplied
-		// ---- the four lanes of a quad -> one sum per row, warps -> shared memory (fixed order: bit-reproducible run to run) ----
+		// ---- lane positions 0 and 1 of a quad -> one sum per row, warps -> shared memory (fixed order: bit-reproducible run to run) ----
+		y0 *= yend;
+		y1 *= yend;
 		y0 += __shfl_xor_sync(0xffffffffu, y0, 1);
 		y1 += __shfl_xor_sync(0xffffffffu, y1, 1);
-		y0 += __shfl_xor_sync(0xffffffffu, y0, 2);
-		y1 += __shfl_xor_sync(0xffffffffu, y1, 2);
 		if (tt >= PB) mbar_wait(&pfree[pb], pph ^ 1); // the epilogue warp has read what this buffer held PB tiles ago
 		if (tig == 0) {
 			float* pt = part + (pb * NCW + warp) * RC;
@@ -520,6 +534,7 @@ __global__ void __launch_bounds__((MMA_NCW + 2) * 32, 1) matvec_mma_kernel(const
 		}
 		__syncwarp();
 		if (lane == 0) mbar_arrive(&pbar[pb]); // (release: this warp's partial sums are visible to whoever completes the wait)
+		if (++pb == PB) { pb = 0; pph ^= 1; }
 	}
 	tl_mark(tl, 3);
 }

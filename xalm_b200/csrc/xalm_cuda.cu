@@ -679,8 +679,8 @@ static int alloc_wmat(DevAlloc& da, WMat& m, int type, int rows, int n, int glu_
 	m.type = type; m.rows = rows; m.n = n; m.flags = 0; m.layout_units = 0; m.layout_frag = 0; m.glu_half = 0;
 	TypeInfo tinfo;
 	type_info(type, &tinfo);
-	// 2 (default): the 4/5-bit formats always; the 8-bit ones under tensor parallelism, where the per-rank rows are short (the dp4a kernel
-	// maps one 32-element block to a lane: rows of 512 elements keep 16 of its 256 lanes busy) — TP2 611 -> 637 tok/s
+	// 1 (default): all of them.  2: the 4/5-bit formats; the 8-bit ones under tensor parallelism, where the per-rank rows are short (the dp4a kernel
+	// maps one 32-element block to a lane: rows of 512 elements keep 16 of its 256 lanes busy)
 	const bool mma_on = tune("mma") == 1 || (tune("mma") == 2 && (sharded || (type != XALM_Q8_0 && type != XALM_Q8)));
 	if (mma_supported(type) && n % 32 == 0 && rows % MMA_RC == 0 && glu_half % 8 == 0 && mma_on && tune("tma") && !tune("mega") &&
 	    mma_smem_bytes(type, n, 2) <= 226 * 1024) {
