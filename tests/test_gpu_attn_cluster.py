@@ -1,0 +1,55 @@
+"""One-token attention as a cluster of CTAs per kv head (xalm_b200/csrc/attn_cluster.cu) against float64 and, for what is not finite, against the split kernel."""
+import numpy as np
+import pytest
+
+from xalm_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+def both(q, k, v, hd, n, nh, nkv):
+    out = []
+    for on in (0, 1):
+        capi.tune("attn_cluster", on)
+        out.append(capi.mha(q, k.view(np.uint16), v.view(np.uint16), hd, n, len(k), nh, nkv))
+    capi.tune("attn_cluster", 1)
+    return out
+
+
+def inputs(hd, n, nh, nkv, seed, scale=1.0):
+    r = np.random.default_rng(seed)
+    return ((scale * r.standard_normal(nh * hd)).astype(np.float32), *(r.standard_normal((n + 3, nkv * hd)).astype(np.float16) for _ in range(2)))
+
+
+# one slot; the ends of a 16-slot unit; one unit for every warp of a cluster of 16 (1024 slots) and one more; long enough for the ring to be refilled
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 257, 1024, 1025, 3001])
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 32, 8), (128, 8, 1), (64, 8, 2), (32, 8, 1), (256, 16, 2), (128, 80, 20)])
+def test_against_float64(hd, nh, nkv, n):
+    q, k, v = inputs(hd, n, nh, nkv, n + hd, scale=2.0)
+    got = both(q, k, v, hd, n, nh, nkv)[1]
+    K, V = (a[:n].astype(np.float64).reshape(n, nkv, hd) for a in (k, v))
+    for h in range(nh):
+        s = K[:, h // (nh // nkv)] @ q[h * hd:(h + 1) * hd].astype(np.float64) / np.sqrt(hd)
+        p = np.exp(s - s.max())
+        want = p / p.sum() @ V[:, h // (nh // nkv)]
+        # fp32: a score of up to 10 is off by some of its last bits (2^-24 each), which moves its weight by as much; sums of weights times values of order 1
+        assert np.max(np.abs(got[h * hd:(h + 1) * hd] - want)) < 64 * 10 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("what", ["key inf", "key -inf", "key nan", "value inf", "value -inf", "value nan", "query inf", "query nan", "query large", "query tiny"])
+def test_what_is_not_finite_goes_where_the_split_kernel_sends_it(what):
+    hd, n, nh, nkv = 128, 300, 32, 8
+    q, k, v = inputs(hd, n, nh, nkv, 5)
+    kind, val = what.split()
+    if kind == "query":
+        if val in ("inf", "nan"):
+            q[5] = float(val)
+        else:
+            q *= 1e30 if val == "large" else 1e-30
+    else:
+        (k if kind == "key" else v)[77, 3 * hd + 9] = float(val)
+    a, b = both(q, k, v, hd, n, nh, nkv)
+    for f in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(f(a), f(b))
+    fin = np.isfinite(a)
+    assert np.max(np.abs(a[fin] - b[fin])) < 64 * 10 * 2.0 ** -24

@@ -44,9 +44,9 @@ def _sources(d, exts):
 # build_cuda(families=["Nabalix"]) compiles abi.cu and what FAMILY_TUS names for those families, nothing else; the list of
 # linked units is kept beside the objects, and a later call that asks for more relinks.
 _ENGINE_TUS = ["mix_ops.cu", "swa_one.cu", "swa_mma.cu", "rec_chunk.cu", "delta_chunk.cu", "prefill.cu"]  # what the config.json families share
-FAMILY_TUS = {"Llama": ["xalm_cuda.cu", "prefill.cu", "decode_mega.cu"],
+FAMILY_TUS = {"Llama": ["xalm_cuda.cu", "attn_cluster.cu", "prefill.cu", "decode_mega.cu"],
               **{f: [f.lower() + ".cu", *_ENGINE_TUS] for f in ("Nabalix", "Bolovik", "Duletar", "Kubolorn", "Mizerax", "Pavitar")}}
-CUDA_TUS = ["abi.cu", "xalm_cuda.cu", "prefill.cu", "decode_mega.cu", "nabalix.cu", "bolovik.cu", "duletar.cu", "kubolorn.cu", "mizerax.cu", "pavitar.cu", "mix_ops.cu", "swa_one.cu", "swa_mma.cu", "rec_chunk.cu", "delta_chunk.cu"]
+CUDA_TUS = ["abi.cu", "xalm_cuda.cu", "attn_cluster.cu", "prefill.cu", "decode_mega.cu", "nabalix.cu", "bolovik.cu", "duletar.cu", "kubolorn.cu", "mizerax.cu", "pavitar.cu", "mix_ops.cu", "swa_one.cu", "swa_mma.cu", "rec_chunk.cu", "delta_chunk.cu"]
 
 
 def _tus(families):

@@ -38,6 +38,7 @@ static std::map<std::string, int>& tuning() {
 	    {"graph", 1},        // replay a captured CUDA graph per token
 	    {"attn_splits", 0},  // 0 = auto (~1 CTA per SM, at most 32 splits per kv head)
 	    {"attn_min_split", 128},
+	    {"attn_cluster", 1}, // one-token attention of four or eight query heads per kv head on the tensor cores (attn_cluster.cu); 0 = the split kernel
 	    {"mv_cfg_rows", 0},  // 0 = auto, 1 = force config A (R4 KS1 NW4), 2 = force config B (R2 KS4 NW8)
 	    {"mega", 0},         // EXPERIMENTAL, measured slower than the kernel-per-op path: one persistent kernel per
 	                         // token (decode_mega.cu) when the model allows — single GPU, integer weight formats

@@ -308,6 +308,10 @@ __global__ void __launch_bounds__(NW * 32) attn_decode_kernel(const AttnArgs a) 
 	}
 }
 
+// attn_cluster.cu: the same on the tensor cores, a cluster of CTAs per kv head.  attn_cluster_size: CTAs per cluster, 0: attn_decode_kernel is for these heads
+int attn_cluster_size(int head_dim, int G, int n_kv_heads, int max_kv_len);
+int launch_attn_cluster(const AttnArgs& a, int head_dim, int G, int C, cudaStream_t s, bool pdl);
+
 #ifndef XALM_SECONDARY_TU // non-template kernel: defined once, in xalm_cuda.cu's translation unit
 // ---- attention probabilities for the `att` scratch argument of mha (model.h:289-307): test hook only, one CTA per
 //      head, the three passes of infer.cpp:340-349 as written. ----

@@ -1,4 +1,17 @@
-// attn_cluster.cu — attention of one query token over the fp16 KV ring (the semantics of attention.cuh) on the tensor cores, a cluster of CTAs per kv head.
+// attn_cluster.cu — attention of one query token over the fp16 KV ring (the semantics of attention.cuh) on the tensor cores: a cluster of CTAs per kv head.
+//
+// Bound: latency.  A step's keys and values are 1 to 17 MB a layer (0.2 to 2.6 us of memory time) that the projection before has pulled into L2.  The split
+// kernel of attention.cuh walks them with fp32 FMAs (24 instructions per key and head for 128 channels, 177 registers) and joins its splits by a store, a fence, a
+// ticket and the last CTA's loads.  Here a warp takes 16 slots at a time with ldmatrix and m16n8k16: one product covers all query heads of the kv head, about
+// 250 instructions for 16 keys of four heads; the slots go round the cluster's warps, so that short contexts use all of them; what this step does not write is fetched
+// before the kernel waits for the projection; and the parts are pushed to the CTA that owns their channels through distributed shared memory, one barrier in all.
+// Queries and probabilities are fp32 values: each enters as three fp16 planes, scaled by powers of two, whose products with the cache's fp16 are exact.  Sums
+// of 16 products start from zero and are added in round-to-nearest as a tree, since the tensor cores' own additions truncate.  Distance from float64 over
+// 20 to 3002 keys and queries of deviation 0.3, 1 and 3: 0.99 times the split kernel's (0.86 to 1.13).  A warp that meets a score or a sum that is not finite
+// does its keys again in fp32 FMAs, so that an infinity or a NaN goes where it goes there (its zero planes would spread it).
+// A step's attention in the graph, split kernel before: 7B at position 3001 12.3 -> 9.5 us; per token, with it and without: 7B q8_0 1938 -> 1870 us, 8 layers of
+// q4_0 at 700 458 -> 428, 6 layers of bf16 at width 2048 and position 1777 275 -> 256.  Tried and not faster: rings of the neighbouring products cut
+// so that this kernel's CTAs fit beside them (no difference).
 #define XALM_SECONDARY_TU
 #include "attention.cuh"
 #include "family.h"
@@ -8,7 +21,6 @@ namespace xalm {
 constexpr int AC_NW = 4, AC_KEYS = 16, AC_MAX_CTAS = 16; // warps per CTA; slots of a unit (one product's keys); most CTAs of a cluster
 constexpr float AC_PSCALE = 16384.f;                     // probabilities enter the tensor cores times 2^14: their third fp16 plane stays above the subnormals' step
 __host__ __device__ constexpr int ac_stages(int hd) { return hd >= 256 ? 1 : hd == 128 ? 2 : 4; } // units a warp holds: 64 KB a CTA at most
-__host__ __device__ constexpr int ac_heads(int G) { return G == 8 ? 8 : 4; }                       // query heads of a kv head, padded
 __host__ __device__ constexpr size_t ac_ring_bytes(int hd) { return (size_t) AC_NW * ac_stages(hd) * 2 * AC_KEYS * hd * 2; }
 __host__ __device__ constexpr size_t ac_smem_bytes(int hd, int gp) {
 	return ac_ring_bytes(hd) + (size_t) 4 * gp * hd * 2 + ((size_t) hd * gp + AC_MAX_CTAS * 8) * 4 + (size_t) AC_MAX_CTAS * gp * 8 + (size_t) AC_NW * gp * 8 + gp * 4;
@@ -53,8 +65,8 @@ __device__ __forceinline__ void ac_cp_wait() { asm volatile("cp.async.wait_group
 
 enum { AC_EARLY = 0, AC_LATE = 1, AC_ALL = 2 }; // rows that this step's QKV kernel does not write | those it does | all
 
-template <int HD, int GP>
-__global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnArgs a, int G) {
+template <int HD, int GP> // GP: query heads of a kv head
+__global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnArgs a) {
 	constexpr int NW = AC_NW, NST = ac_stages(HD), KEYS = AC_KEYS, NTH = NW * 32, PIECES = HD / 8, TILE = KEYS * HD; // TILE: halves of a unit's keys
 	extern __shared__ __align__(128) uint8_t smem[];
 	__half* ring = reinterpret_cast<__half*>(smem);                    // [NW][NST][K | V][KEYS][HD]
@@ -109,7 +121,7 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		uint32_t top = 0;
 #pragma unroll
 		for (int e = 0; e < E; e++) {
-			q[e] = h < G ? __ldcg(a.q + (size_t) (kvh * G + h) * HD + lane + 32 * e) : 0.f;
+			q[e] = __ldcg(a.q + (size_t) (kvh * GP + h) * HD + lane + 32 * e);
 			top = max(top, __float_as_uint(q[e]) & 0x7fffffffu);
 		}
 		top = __reduce_max_sync(0xffffffffu, top) >> 23;
@@ -258,13 +270,13 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		for (int h = 0; h < GP; h++) {
 			float o[E] = {}, mh = -CUDART_INF_F, lh = 0.f;
 #pragma unroll 1
-			for (int u = u0; h < G && u < nu; u += du)
+			for (int u = u0; u < nu; u += du)
 #pragma unroll 1
 				for (int slot = u * KEYS; slot < min(kv_len, (u + 1) * KEYS); slot++) {
 					float x = 0.f;
 #pragma unroll
 					for (int e = 0; e < E; e++)
-						x += __ldcg(a.q + (size_t) (kvh * G + h) * HD + lane + 32 * e) * __half2float(__ldcg(kbase + (size_t) slot * kv_stride + lane + 32 * e));
+						x += __ldcg(a.q + (size_t) (kvh * GP + h) * HD + lane + 32 * e) * __half2float(__ldcg(kbase + (size_t) slot * kv_stride + lane + 32 * e));
 					x = warp_sum(x) * inv_sqrt;
 					const float mn = fmaxf(mh, x);
 					if (mn == -CUDART_INF_F) continue;
@@ -345,7 +357,7 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		den += __shfl_xor_sync(0xffffffffu, den, 1);
 		num += __shfl_xor_sync(0xffffffffu, num, 2);
 		den += __shfl_xor_sync(0xffffffffu, den, 2);
-		if (in && part == 0 && h < G) a.out[(size_t) (kvh * G + h) * HD + rank * own + x / GP] = num * (1.f / AC_PSCALE) / den;
+		if (in && part == 0) a.out[(size_t) (kvh * GP + h) * HD + rank * own + x / GP] = num * (1.f / AC_PSCALE) / den;
 	}
 }
 
@@ -369,8 +381,10 @@ static cudaError_t ac_config(int n_kv, int C, cudaStream_t s, bool pdl, cudaLaun
 }
 template <int HD, int GP>
 static int ac_size(int n_kv) {
+	int sms = 148, dev = 0;
+	if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	for (int C = AC_MAX_CTAS; C >= 1; C /= 2) {
-		if (C > 1 && C * n_kv > 148) continue;
+		if (C > 1 && C * n_kv > sms) continue;
 		cudaLaunchConfig_t cfg;
 		cudaLaunchAttribute at[2];
 		int n = 0;
@@ -383,23 +397,21 @@ static int ac_size(int n_kv) {
 	return 0;
 }
 
-#define XALM_AC_CASES(CALL)                                    \
-	if (gp == 4) {                                             \
-		if (head_dim == 32) { CALL(32, 4); }                   \
-		if (head_dim == 64) { CALL(64, 4); }                   \
-		if (head_dim == 128) { CALL(128, 4); }                 \
-		if (head_dim == 256) { CALL(256, 4); }                 \
-	} else {                                                   \
-		if (head_dim == 32) { CALL(32, 8); }                   \
-		if (head_dim == 64) { CALL(64, 8); }                   \
-		if (head_dim == 128) { CALL(128, 8); }                 \
-		if (head_dim == 256) { CALL(256, 8); }                 \
-	}
+#define XALM_AC_CASES(CALL)                                                              \
+	if (G == 4 && head_dim == 32) { CALL(32, 4); }                                       \
+	if (G == 4 && head_dim == 64) { CALL(64, 4); }                                       \
+	if (G == 4 && head_dim == 128) { CALL(128, 4); }                                     \
+	if (G == 8 && head_dim == 32) { CALL(32, 8); }                                       \
+	if (G == 8 && head_dim == 64) { CALL(64, 8); }                                       \
+	if (G == 8 && head_dim == 128) { CALL(128, 8); }                                     \
+	if (G == 8 && head_dim == 256) { CALL(256, 8); }
 
-// CTAs per kv head so that all clusters run at once on the current device; 0: this kernel cannot take the model's heads
-int attn_cluster_size(int head_dim, int G, int n_kv_heads) {
-	if (G != 1 && G != 2 && G != 4 && G != 8) return 0;
-	const int gp = ac_heads(G);
+// CTAs per kv head so that all clusters run at once on the current device; 0: the split kernel is the faster one for these heads.  Alone, back to back, buffers
+// beyond L2 (split kernel / this one, us): four heads of 128 over 8 kv heads 10.3 / 8.2 at 500 keys, 14.4 / 12.4 at 4096, 28.7 / 28.7 at 16384, 47 / 51 at 32768;
+// eight heads 14.4 / 10.3, 20.5 / 16.1, 49 / 35, 84 / 59; two heads 8.3 / 8.3, 12.4 / 12.3, 22.6 / 28.7; one head 10.1 / 10.3, 22.6 / 22.6.  Of 256 channels: eight
+// heads 26.6 / 14.4, 41 / 29, four 14.4 / 11.4, 20.5 / 22.6.
+int attn_cluster_size(int head_dim, int G, int n_kv_heads, int max_kv_len) {
+	if (G == 4 && max_kv_len > 16384) return 0;
 #define XALM_AC_SIZE(HD_, GP_) return ac_size<HD_, GP_>(n_kv_heads)
 	XALM_AC_CASES(XALM_AC_SIZE)
 #undef XALM_AC_SIZE
@@ -408,13 +420,12 @@ int attn_cluster_size(int head_dim, int G, int n_kv_heads) {
 
 // C: attn_cluster_size's answer
 int launch_attn_cluster(const AttnArgs& a, int head_dim, int G, int C, cudaStream_t s, bool pdl) {
-	const int gp = ac_heads(G);
 	cudaError_t e = cudaErrorInvalidValue;
 	cudaLaunchConfig_t cfg;
 	cudaLaunchAttribute at[2];
-#define XALM_AC_LAUNCH(HD_, GP_)                                                                \
-	e = ac_config<HD_, GP_>(a.n_kv_heads, C, s, pdl, &cfg, at);                                 \
-	if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD_, GP_>, a, G);
+#define XALM_AC_LAUNCH(HD_, GP_)                                                        \
+	e = ac_config<HD_, GP_>(a.n_kv_heads, C, s, pdl, &cfg, at);                         \
+	if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD_, GP_>, a);
 	XALM_AC_CASES(XALM_AC_LAUNCH)
 #undef XALM_AC_LAUNCH
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "attention launch failed: %s", cudaGetErrorString(e));

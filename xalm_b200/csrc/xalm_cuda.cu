@@ -5,7 +5,7 @@
 // Per token (Model::_forward_cpu, infer.cpp:604-638 / Block::_block_cpu, infer.cpp:365-496):
 //   embed                                   x = dequant(embed[token])
 //   per layer  matvec[norm -> QKV -> rope]  q fp32, k/v fp16 -> KV ring   (+ sink re-rotation)
-//              attn_decode                  xb2 = softmax(q k^T / sqrt(hd)) v      (split-K, GQA)
+//              attn_cluster / attn_decode   xb2 = softmax(q k^T / sqrt(hd)) v      (keys split, GQA)
 //              matvec[Wo, residual]         x += Wo xb2                    (TP: partial -> allreduce -> add)
 //              matvec[norm -> W1|W3 -> GLU] hb = act(W1 xb) * (W3 xb)
 //              matvec[W2, residual]         x += W2 hb                     (TP: partial -> allreduce -> add)
@@ -840,6 +840,7 @@ struct xalm_cuda_model {
 	float *attn_acc = nullptr, *attn_ml = nullptr;
 	unsigned int* tickets = nullptr;
 	int attn_splits = 0;
+	int attn_cluster = 0; // CTAs per kv head of attn_cluster.cu; 0: the split kernel of attention.cuh
 	StepParams* d_step = nullptr;
 	StepParams* h_step = nullptr; // pinned ring
 	cudaEvent_t h_step_ev[64];
@@ -1413,7 +1414,7 @@ static int enqueue_token(xalm_cuda_model* m, int mode, cudaStream_t s, int* n_la
 			nl++;
 		}
 		{
-			XALM_TRY(launch_attn(a_at, c.head_dim, G, s, pdl));
+			XALM_TRY(m->attn_cluster ? launch_attn_cluster(a_at, c.head_dim, G, m->attn_cluster, s, pdl) : launch_attn(a_at, c.head_dim, G, s, pdl));
 			nl++;
 		}
 		{ // Wo + residual
@@ -1571,6 +1572,7 @@ int xalm_cuda_finalize(xalm_cuda_model* m) {
 	XALM_CUDA_CHECK(cudaMemcpy(m->rope_freq, freq.data(), freq.size() * sizeof(float), cudaMemcpyHostToDevice));
 	const int G = c.n_heads / c.n_kv_heads;
 	m->attn_splits = attn_auto_splits(m->n_kv_heads_l);
+	m->attn_cluster = tune("attn_cluster") ? attn_cluster_size(c.head_dim, G, m->n_kv_heads_l, c.max_seq_len) : 0;
 	// the last-CTA merge parks 3 floats per (split, head) in the 8 x G x head_dim floats of the per-warp partial area (attention.cuh)
 	if (m->attn_splits > 8 * c.head_dim / 3) m->attn_splits = 8 * c.head_dim / 3;
 	XALM_TRY(fzero(&m->attn_acc, (size_t) m->n_kv_heads_l * m->attn_splits * G * c.head_dim));
@@ -1860,7 +1862,8 @@ int xalm_cuda_mha(float* xout, float* att, const uint16_t* kb, const uint16_t* v
 	a.q = (const float*) dq; a.k_cache = (const __half*) dk; a.v_cache = (const __half*) dv; a.out = (float*) dout;
 	a.kv_len_fixed = kv_len; a.n_kv_heads = n_kv_heads; a.n_splits = splits; a.min_split = tune("attn_min_split");
 	a.part_acc = (float*) dacc; a.part_ml = (float*) dml; a.tickets = (unsigned int*) dtick;
-	XALM_TRY(launch_attn(a, head_dim, G, 0, false));
+	const int C = tune("attn_cluster") ? attn_cluster_size(head_dim, G, n_kv_heads, kv_len) : 0;
+	XALM_TRY(C ? launch_attn_cluster(a, head_dim, G, C, 0, false) : launch_attn(a, head_dim, G, 0, false));
 	if (att) {
 		XALM_TRY(t.alloc(&datt, (size_t) n_heads * max_seq_len * sizeof(float)));
 		XALM_CUDA_CHECK(cudaMemset(datt, 0, (size_t) n_heads * max_seq_len * sizeof(float)));
