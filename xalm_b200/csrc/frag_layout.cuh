@@ -34,49 +34,43 @@ __host__ __device__ inline int frag_record_bytes(int t) {
 }
 __host__ __device__ inline int frag_quant_bytes(int t) { return (t == XALM_Q8_0 || t == XALM_Q8) ? 512 : 256; }
 
-// physical row of the uploaded (stacked) matrix -> virtual row of the tile order
-__host__ __device__ inline int frag_virtual_row(int glu_half, int r) {
-	if (!glu_half) return r;
-	const int o = r < glu_half ? r : r - glu_half;
-	return (o / 8) * 16 + (r < glu_half ? 0 : 8) + o % 8;
-}
-
-// ---- element access (the batched prefill's dequantiser, tests): 8 consecutive elements k0 .. k0+7 (k0 % 8 == 0) of physical row r
-__device__ __forceinline__ void frag_decode8(const WMat& w, int t, int r, int k0, float (&v)[8]) {
-	const int vr = frag_virtual_row(w.glu_half, r);
-	const int T = vr >> 4, g = vr & 7, hi = (vr >> 3) & 1;
-	const int nb = w.n / 32, blk = k0 / 32, kk0 = k0 % 32;
-	const int rb = frag_record_bytes(t), qb = frag_quant_bytes(t);
-	const uint8_t* rec = w.p0 + ((size_t) T * nb + blk) * rb;
-	const int half = kk0 / 16;
-	const int j = half * 2 + hi;
-	float d = 0.01f, mn = 0.f; // Q8: fixed scale 1/100
-	if (t == XALM_Q8_0 || t == XALM_Q4_0) d = f16_bits_to_f32(*reinterpret_cast<const uint16_t*>(rec + qb + g * 4 + hi * 2));
-	if (t == XALM_Q5_0) d = f16_bits_to_f32(*reinterpret_cast<const uint16_t*>(rec + qb + 64 + g * 4 + hi * 2));
-	if (t == XALM_Q4_1 || t == XALM_Q5_1) {
-		const uint8_t* sp = rec + qb + (t == XALM_Q5_1 ? 64 : 0) + g * 8 + hi * 2;
-		d = f16_bits_to_f32(*reinterpret_cast<const uint16_t*>(sp));
-		mn = f16_bits_to_f32(*reinterpret_cast<const uint16_t*>(sp + 4));
-	}
+// ---- element access (the batched prefill's dequantiser): elements 8 c .. 8 c + 7 of block `blk` of the tile's rows g and g + 8, which share a record's words
+template <int t>
+__device__ __forceinline__ void frag_decode8(const WMat& w, int tile, int g, int blk, int c, float (&v)[2][8]) {
+	constexpr int rb = t == XALM_Q8_0 ? 544 : t == XALM_Q8 ? 512 : t == XALM_Q4_0 ? 288 : t == XALM_Q4_1 ? 320 : t == XALM_Q5_0 ? 352 : 384;
+	constexpr bool bytes = t == XALM_Q8_0 || t == XALM_Q8, fifth = t == XALM_Q5_0 || t == XALM_Q5_1, has_min = t == XALM_Q4_1 || t == XALM_Q5_1;
+	constexpr int sc = (bytes ? 512 : 256) + (fifth ? 64 : 0), bias = bytes ? 128 : t == XALM_Q4_0 ? 8 : t == XALM_Q5_0 ? 16 : 0;
+	const uint8_t* rec = w.p0 + ((size_t) tile * (w.n / 32) + blk) * rb;
+	const int half = c >> 1, lane0 = g * 4 + (c & 1) * 2;
+	float2 d = make_float2(0.01f, 0.01f), mn = make_float2(0.f, 0.f); // Q8: fixed scale 1/100
+	if (has_min) {
+		const uint2 s = *reinterpret_cast<const uint2*>(rec + sc + g * 8);
+		d = __half22float2(*reinterpret_cast<const __half2*>(&s.x));
+		mn = __half22float2(*reinterpret_cast<const __half2*>(&s.y));
+	} else if (t != XALM_Q8) d = __half22float2(*reinterpret_cast<const __half2*>(rec + sc + g * 4));
 #pragma unroll
-	for (int i = 0; i < 8; i++) {
-		const int kk = kk0 + i, tig = (kk % 16) / 4, e = kk % 4, lane = g * 4 + tig;
-		if (t == XALM_Q8_0 || t == XALM_Q8) {
-			const int q = (int) rec[lane * 16 + j * 4 + e] - 128;
-			v[i] = __fmul_rn(d, (float) q);
-			continue;
+	for (int p = 0; p < 2; p++) { // two lanes' words: elements 0 .. 3, then 4 .. 7
+		const int lane = lane0 + p;
+		uint32_t wd[2]; // rows g and g + 8
+		if (bytes) {
+			const uint2 q = *reinterpret_cast<const uint2*>(rec + lane * 16 + half * 8);
+			wd[0] = q.x; wd[1] = q.y;
+		} else {
+			const uint32_t q = *reinterpret_cast<const uint32_t*>(rec + lane * 8 + half * 4);
+			wd[0] = q & 0x0F0F0F0Fu; wd[1] = (q >> 4) & 0x0F0F0F0Fu;
 		}
-		const uint8_t byte = rec[lane * 8 + half * 4 + e];
-		int q = hi ? (byte >> 4) : (byte & 15);
-		if (t == XALM_Q5_0 || t == XALM_Q5_1) {
-			const uint32_t hb = *reinterpret_cast<const uint16_t*>(rec + 256 + lane * 2);
-			q |= (int) ((hb >> (4 * j + e)) & 1u) << 4;
+		if (fifth) {
+			const uint32_t hb = (uint32_t) *reinterpret_cast<const uint16_t*>(rec + 256 + lane * 2) >> (8 * half);
+			wd[0] |= (((hb & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
+			wd[1] |= ((((hb >> 4) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
 		}
-		switch (t) {
-			case XALM_Q4_0: v[i] = __fmul_rn(d, (float) (q - 8)); break;
-			case XALM_Q5_0: v[i] = __fmul_rn(d, (float) (q - 16)); break;
-			default: v[i] = __fadd_rn(__fmul_rn(d, (float) q), mn); break; // Q4_1, Q5_1
-		}
+#pragma unroll
+		for (int e = 0; e < 4; e++)
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				const float q = (float) ((int) ((wd[h] >> (8 * e)) & 0xFFu) - bias), x = __fmul_rn(h ? d.y : d.x, q);
+				v[h][4 * p + e] = has_min ? __fadd_rn(x, h ? mn.y : mn.x) : x;
+			}
 	}
 }
 
