@@ -419,6 +419,159 @@ __global__ void __launch_bounds__(256) rows_gemm_kernel(const float* __restrict_
 	}
 }
 
+// ---- the same for bf16 weights and many tokens on the tensor cores in fp32 grade: activations as three bf16 planes (their 24 bits), so that every product is
+// exact; 16 products a sum from zero, small planes first, sums of more in round-to-nearest (the tensor cores' own additions truncate) ------------------
+// Bound: latency.  A pass's products whose shapes the tcgen05 GEMM does not take, or that stay in fp32 grade: a latent's per-head products, low-rank decays.
+// A warp makes 32 x 32 outputs with operands of its own in shared memory (no barrier between the steps), the next 32 channels on their way to registers.
+// WK = 1: 64 x 64 outputs per CTA.  WK = 4: the four warps share the steps of 32 x 32 outputs, where the other form would leave SMs idle.  The epilogue is a loop
+// over the finished tile: unrolled over a thread's 32 outputs it took 26 us whatever the product, the time to fetch its code.  Before (fp32 FMA
+// tiles of 64 x 64, as rows_gemm_kernel) -> now: 1024 tokens of 8 heads 128 -> 256 channels 45.0 -> 16.6 us, 256 tokens of 16 heads 512 -> 128 53.4 -> 16.5, 256 x 32 over 1024
+// channels 88 -> 10.4, 256 x 1024 over 32 12.5 -> 4.4.
+// A CTA whose sums are not all finite does them again in fp32 FMAs: an infinity times a zero plane is no NaN there.
+constexpr int RM_BK = 32, RM_LD = 40; // channels of a step; bf16 between two rows in shared memory (the eight rows of an 8 x 8 matrix on different banks)
+constexpr int RM_WARP_BYTES = 4 * 32 * RM_LD * 2; // a warp's three planes of 32 rows, and 32 rows of weights
+__device__ __forceinline__ void rm_split(float x, float y, uint32_t (&p)[3]) { // two fp32 values as three pairs of bf16 whose sums they are
+#pragma unroll
+	for (int i = 0; i < 3; i++) {
+		const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+		p[i] = *reinterpret_cast<const uint32_t*>(&h);
+		x -= __low2float(h);
+		y -= __high2float(h);
+	}
+}
+__device__ __forceinline__ void rm_ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t) __cvta_generic_to_shared(p)) : "memory");
+}
+template <int WK>
+__global__ void __launch_bounds__(128, 4) rows_mma_kernel(const float* A, int lda, const __nv_bfloat16* __restrict__ W, int T, int N, int K, RowsEpi e) {
+	constexpr int BT = WK == 1 ? 64 : 32, OLD = BT + 2; // outputs of a CTA: BT x BT; floats between two rows of them in shared memory
+	if (blockIdx.z) { // one product of a batch
+		A += (size_t) blockIdx.z * e.batch_a;
+		W += (size_t) blockIdx.z * e.batch_w;
+		e.out += (size_t) blockIdx.z * e.batch_o;
+		if (e.mul) e.mul += (size_t) blockIdx.z * e.batch_o;
+	}
+	__shared__ __align__(16) uint8_t sm[4 * RM_WARP_BYTES];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
+	const int wm = WK == 1 ? (warp >> 1) * 32 : 0, wn = WK == 1 ? (warp & 1) * 32 : 0, kw = WK == 1 ? 0 : warp * RM_BK;
+	__nv_bfloat16 *as = reinterpret_cast<__nv_bfloat16*>(sm + warp * RM_WARP_BYTES), *ws = as + 3 * 32 * RM_LD;
+	float4 an[8]; // the next 32 channels: rows lane / 8 + 4 i, four channels; rows lane / 4 + 8 i, eight
+	uint4 wx[4];
+	auto request = [&](int k0) {
+#pragma unroll
+		for (int i = 0; i < 8; i++) {
+			const int r = m0 + wm + lane / 8 + 4 * i, k = k0 + lane % 8 * 4;
+			an[i] = r < T && k < K ? *reinterpret_cast<const float4*>(A + (size_t) r * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+		}
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			const int r = n0 + wn + lane / 4 + 8 * i, k = k0 + lane % 4 * 8;
+			wx[i] = r < N && k < K ? *reinterpret_cast<const uint4*>(W + (size_t) r * K + k) : make_uint4(0, 0, 0, 0);
+		}
+	};
+	float acc[2][4][4] = {};
+	request(kw);
+#pragma unroll 1
+	for (int k0 = kw; k0 < K; k0 += WK * RM_BK) {
+		__syncwarp(); // the channels before are read
+#pragma unroll
+		for (int i = 0; i < 8; i++) {
+			uint32_t lo[3], hi[3];
+			rm_split(an[i].x, an[i].y, lo);
+			rm_split(an[i].z, an[i].w, hi);
+#pragma unroll
+			for (int p = 0; p < 3; p++) *reinterpret_cast<uint2*>(&as[(p * 32 + lane / 8 + 4 * i) * RM_LD + lane % 8 * 4]) = make_uint2(lo[p], hi[p]);
+		}
+#pragma unroll
+		for (int i = 0; i < 4; i++) *reinterpret_cast<uint4*>(&ws[(lane / 4 + 8 * i) * RM_LD + lane % 4 * 8]) = wx[i];
+		__syncwarp();
+		if (k0 + WK * RM_BK < K) request(k0 + WK * RM_BK);
+#pragma unroll
+		for (int ks = 0; ks < RM_BK / 16; ks++) {
+			uint32_t a[3][2][4], b[2][4]; // b: two pairs of 8-column fragments
+			const int mr = lane & 7, mid = lane >> 3;
+#pragma unroll
+			for (int p = 0; p < 3; p++)
+#pragma unroll
+				for (int i = 0; i < 2; i++) rm_ldsm4(a[p][i], &as[(p * 32 + 16 * i + (mid & 1) * 8 + mr) * RM_LD + ks * 16 + (mid >> 1) * 8]);
+#pragma unroll
+			for (int j = 0; j < 2; j++) rm_ldsm4(b[j], &ws[(16 * j + (mid >> 1) * 8 + mr) * RM_LD + ks * 16 + (mid & 1) * 8]);
+#pragma unroll
+			for (int i = 0; i < 2; i++) {
+				float d[4][4] = {};
+#pragma unroll
+				for (int p = 2; p >= 0; p--)
+#pragma unroll
+					for (int j = 0; j < 4; j++)
+						asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+						    : "+f"(d[j][0]), "+f"(d[j][1]), "+f"(d[j][2]), "+f"(d[j][3])
+						    : "r"(a[p][i][0]), "r"(a[p][i][1]), "r"(a[p][i][2]), "r"(a[p][i][3]), "r"(b[j >> 1][2 * (j & 1)]), "r"(b[j >> 1][2 * (j & 1) + 1]));
+#pragma unroll
+				for (int j = 0; j < 4; j++)
+#pragma unroll
+					for (int x = 0; x < 4; x++) acc[i][j][x] += d[j][x];
+			}
+		}
+	}
+	// ---- the tile in shared memory (WK: as many parts of it), then output by output ----
+	__syncthreads();
+	float* o = reinterpret_cast<float*>(sm) + (WK == 1 ? 0 : warp * 32 * OLD);
+	bool bad = false;
+#pragma unroll
+	for (int i = 0; i < 2; i++)
+#pragma unroll
+		for (int j = 0; j < 4; j++)
+#pragma unroll
+			for (int x = 0; x < 4; x += 2) {
+				bad |= !(fabsf(acc[i][j][x]) < INFINITY) || !(fabsf(acc[i][j][x + 1]) < INFINITY);
+				*reinterpret_cast<float2*>(o + (wm + 16 * i + lane / 4 + 4 * x) * OLD + wn + 8 * j + lane % 4 * 2) = make_float2(acc[i][j][x], acc[i][j][x + 1]);
+			}
+	bad = __syncthreads_or(bad);
+	const float* all = reinterpret_cast<const float*>(sm);
+	if (!bad && e.kind == EPI_STORE && !(e.cap > 0.f) && !e.mul && !e.add && ((e.ldo | N) & 1) == 0 && (reinterpret_cast<uintptr_t>(e.out) & 7) == 0) { // plain rows: two columns a store
+#pragma unroll 4
+		for (int i = tid; i < BT * BT / 2; i += 128) {
+			const int r = i / (BT / 2), c = i % (BT / 2) * 2;
+			if (m0 + r >= T || n0 + c >= N) continue;
+			float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+			for (int w = 0; w < WK; w++) {
+				const float2 part = *reinterpret_cast<const float2*>(all + w * 32 * OLD + r * OLD + c);
+				v.x += part.x;
+				v.y += part.y;
+			}
+			*reinterpret_cast<float2*>(e.out + (size_t) (m0 + r) * e.ldo + n0 + c) = v;
+		}
+		return;
+	}
+#pragma unroll 1
+	for (int i = tid; i < BT * BT / 2; i += 128) {
+		const int r = i / (BT / 2), c = i % (BT / 2) * 2, row = m0 + r, col = n0 + c;
+		if (row >= T || col >= N) continue;
+		float2 v = make_float2(0.f, 0.f);
+		if (!bad) {
+#pragma unroll
+			for (int w = 0; w < WK; w++) {
+				const float2 part = *reinterpret_cast<const float2*>(all + w * 32 * OLD + r * OLD + c);
+				v.x += part.x;
+				v.y += part.y;
+			}
+		} else
+#pragma unroll 1
+			for (int k = 0; k < K; k++) {
+				const float x = A[(size_t) row * lda + k];
+				v.x = fmaf(x, ldf(W + (size_t) col * K + k), v.x);
+				if (col + 1 < N) v.y = fmaf(x, ldf(W + (size_t) (col + 1) * K + k), v.y);
+			}
+		if (e.kind == EPI_GLU) {
+			if (col + 1 < N) epi_apply(e, row, col, N, v.x, v.y);
+		} else {
+#pragma unroll 1
+			for (int k = 0; k < 2 && col + k < N; k++) epi_apply(e, row, col + k, N, k ? v.y : v.x, 0.f);
+		}
+	}
+}
+
 // ---- the epilogues alone, on a product that another kernel left in memory (the tensor-core GEMM stores plain fp32 rows) --------------
 static __global__ void rows_epilogue_kernel(const float* __restrict__ src, int lds, int T, int N, RowsEpi e) {
 	const int step = e.kind == EPI_GLU ? 2 : 1, per_row = (N + step - 1) / step;
@@ -1793,6 +1946,10 @@ static inline int launch_rows(const float* A, int lda, const void* W, bool w_bf1
 			else XALM_ROWS_MATVEC(float, 4);
 		}
 #undef XALM_ROWS_MATVEC
+	} else if (wide && lda % 4 == 0) {
+		const int tiles = (N + 63) / 64 * ((T + 63) / 64) * batch;
+		if (tiles < 148 && K > RM_BK) rows_mma_kernel<4><<<dim3((N + 31) / 32, (T + 31) / 32, batch), 128, 0, s>>>(A, lda, (const __nv_bfloat16*) W, T, N, K, e);
+		else rows_mma_kernel<1><<<dim3((N + 63) / 64, (T + 63) / 64, batch), 128, 0, s>>>(A, lda, (const __nv_bfloat16*) W, T, N, K, e);
 	} else {
 		const dim3 grid((N + 63) / 64, (T + 63) / 64, batch);
 		if (w_bf16) rows_gemm_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(A, lda, (const __nv_bfloat16*) W, T, N, K, e);
