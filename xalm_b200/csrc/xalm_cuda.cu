@@ -470,7 +470,7 @@ __global__ void embed_kernel(int type, const uint8_t* __restrict__ table, size_t
 // a token's parameters from pinned host memory, before the kernels that read them ahead of their dependency waits
 __global__ void step_in_kernel(const int* in, int* out) { out[threadIdx.x] = in[threadIdx.x]; }
 __global__ void logits_out_kernel(const float* logits, float* host, int n) {
-	pdl_wait();
+	pdl_enter();
 	pinned_out(logits, host, n);
 }
 
