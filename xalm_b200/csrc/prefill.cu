@@ -429,6 +429,7 @@ struct GemmArgs {
 	const uint8_t* b_lo; // residual plane of the weights (NB = 2)
 	int MT, NT, KT;     // tile counts; M tiles are [mt0, mt0 + MT)
 	int mt0;
+	int tile_lo, tile_hi; // the tiles of this launch among MT x NT, M tiles fastest (launch_gemm_planes; a grouped launch makes all)
 	int M;              // valid rows
 	int N;              // valid outputs (GLU: hidden units; else columns)
 	int epi;
@@ -769,13 +770,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmArgs
 	const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
 	const int MT = FOR == GF_GROUP ? *g.gn_tiles : g.MT;
-	const int n_tiles = MT * g.NT;
+	const int n_tiles = FOR == GF_GROUP ? MT * g.NT : g.tile_hi;
 	const int KT = g.KT;
 	struct { int rank, ks, tile0, tiles, k_lo, k_hi; } cl; // of SPLIT: this CTA's place in its cluster, the cluster's tiles, this CTA's K steps of each
 	if constexpr (SPLIT) {
 		asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cl.rank));
 		asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cl.ks));
-		cl.tile0 = (int) blockIdx.x / cl.ks; cl.tiles = (int) gridDim.x / cl.ks;
+		cl.tile0 = g.tile_lo + (int) blockIdx.x / cl.ks; cl.tiles = (int) gridDim.x / cl.ks;
 		cl.k_lo = cl.rank * KT / cl.ks; cl.k_hi = (cl.rank + 1) * KT / cl.ks;
 	}
 
@@ -1583,6 +1584,7 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 	cfg->attrs = at;
 	cfg->numAttrs = 1;
 }
+template <int NA, int NB> constexpr float gemm_step_us() { return NA == 1 ? 0.36f : NB == 1 ? 0.58f : 1.08f; }
 // How many CTAs, one cluster, share a tile's K steps.  Few tiles (short prompts, narrow matrices) leave SMs idle while a CTA's time is its K steps, each
 // of which waits for the 48 to 96 KB that one SM draws in.  (Splitting the columns instead would read the activations once per part.)  Each CTA sums its
 // share of the steps, the sums are joined through distributed shared memory and every CTA finishes its share of the columns: there is no workspace,
@@ -1598,7 +1600,7 @@ static void gemm_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at
 // K steps with 8 tiles and more.  Two planes take longer per step and share more often: 16 steps up to 36 tiles (2/1 256 x 4096 x 1024 18.5 -> 15.3, 2/2
 // 22.6 -> 16.8), 64 steps at 80 tiles with 2/2 (640 x 4096 x 4096 76 -> 68).  A twentieth less is asked for, since 2/1 lost there (45.8 -> 47.2 in three shares).
 template <int NA, int NB, int FOR>
-static int gemm_split(int tiles, int KT) {
+static int gemm_split(int tiles, int KT, float* est = nullptr) { // est: the time that the rule expects
 	static std::atomic<int> fits[GEMM_MAX_SPLIT + 1]; // clusters of this size that run at a time, 0: not asked yet
 	static std::atomic<bool> attr{false};
 	if (!attr.load()) {
@@ -1608,7 +1610,7 @@ static int gemm_split(int tiles, int KT) {
 		}
 		attr.store(true);
 	}
-	constexpr float STEP = NA == 1 ? 0.36f : NB == 1 ? 0.58f : 1.08f; // us
+	constexpr float STEP = gemm_step_us<NA, NB>();
 	const float whole = (float) cdiv(tiles, sm_count()) * (float) KT * STEP;
 	int best = 1;
 	float best_us = 0.95f * whole;
@@ -1628,20 +1630,38 @@ static int gemm_split(int tiles, int KT) {
 		const float us = (float) cdiv(tiles, n) * ((float) cdiv(KT, ks) * STEP + 4.f + 0.5f * (float) ks);
 		if (us < best_us) { best_us = us; best = ks; }
 	}
+	if (est) *est = best > 1 ? best_us : whole;
 	return best;
 }
+// Where a CTA per tile is the better split of the whole, the tiles behind the last full wave (one per SM) still leave SMs idle for a tile's whole time: 336 tiles
+// of 333 tokens x W1|W3 (7B) are two waves and 40 tiles, 512 of 4096 tokens x 4096 columns three and 68.  They are a launch of their own, in clusters by the same
+// rule, where that rule expects to save more than TAIL_US: no tile of the second launch starts before the last of the first is stored, and waves that were not in step
+// come into step.  Back to back, us in one launch -> two (planes; tokens x columns x K):
+//   2/2: 4096 x 4096 x 14336 931 -> 845, 4096 x 6144 x 4096 420 -> 391, 1024 x 6144 x 4096 152 -> 120, 333 x 28672 x 4096 222 -> 190, 1200 x 4096 x 1536 55.6 -> 50.3
+//   2/1: 4096 x 4096 x 14336 533 -> 487, 1024 x 28672 x 4096 286 -> 271, 4096 x 4096 x 4096 170 -> 164;  1/1: 4096 x 4096 x 14336 320 -> 302
+// TAIL_US is where the sides part: with 5 us, 1/1 lost at 64 K steps and many waves (expected 12 less, 4096 x 28672 x 4096 597 -> 609) and 2/2 at 16 (expected 7 less,
+// 700 x 8192 x 1024 41.3 -> 43.3).
 template <int NA, int NB, int FOR>
-static int launch_gemm_planes(const GemmArgs& g, const GemmMap<FOR>& map, int tiles, cudaStream_t s) {
-	const int ks = gemm_split<NA, NB, FOR>(tiles, g.KT);
-	cudaError_t e;
-	if (ks > 1) {
+static int launch_gemm_planes(GemmArgs g, const GemmMap<FOR>& map, int tiles, cudaStream_t s) {
+	constexpr float TAIL_US = 12.5f;
+	int ks = gemm_split<NA, NB, FOR>(tiles, g.KT), head = ks > 1 ? 0 : tiles;
+	if (const int rest = tiles % sm_count(); ks == 1 && rest && rest < tiles) {
+		float us;
+		ks = gemm_split<NA, NB, FOR>(rest, g.KT, &us);
+		if (ks > 1 && us + TAIL_US < (float) g.KT * gemm_step_us<NA, NB>()) head = tiles - rest;
+	}
+	cudaError_t e = cudaSuccess;
+	if (head) {
+		g.tile_lo = 0; g.tile_hi = head;
+		XALM_TRY((launch_gemm_inst<NA, NB, FOR>(g, map, std::min(head, sm_count()), s)));
+		e = cudaGetLastError();
+	}
+	if (head < tiles && e == cudaSuccess) {
+		g.tile_lo = head; g.tile_hi = tiles;
 		cudaLaunchConfig_t cfg = {};
 		cudaLaunchAttribute at[1];
-		gemm_cluster_config<NA, NB>(&cfg, at, std::min(tiles, sm_count() / ks) * ks, ks, s);
-		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, FOR, true>, g, map);
-	} else {
-		XALM_TRY((launch_gemm_inst<NA, NB, FOR>(g, map, std::min(tiles, sm_count()), s)));
-		e = cudaGetLastError();
+		gemm_cluster_config<NA, NB>(&cfg, at, std::min(tiles - head, sm_count() / ks) * ks, ks, s);
+		e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NA, NB, FOR, true>, (const GemmArgs) g, map);
 	}
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "gemm_tc launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
