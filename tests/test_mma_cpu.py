@@ -1,9 +1,9 @@
 """numpy model of the tensor-core decode matvec (xalm_b200/csrc/matvec_mma.cuh) and of its weight layout
 (xalm_b200/csrc/frag_layout.cuh), run on the CPU.
 
-The kernel feeds mma.sync.m16n8k32.u8.u8.s32 with the STORED weight bytes (quant + bias) as A and, as B, the three unsigned
-limbs of the OFFSET activations X' = X + 2^23 plus a column of ones; the accumulators start at -bias * (limb sums).  This file
-restates that arithmetic in integers and checks the claims of the kernel's header:
+The kernel feeds mma.sync.m16n8k32.s8.u8.s32 with signed quants as A and, as B, the three unsigned limbs of the OFFSET activations
+X' = X + 2^23 plus a column of ones, accumulators from zero (tests/test_gpu_mma_stages.py).  This file restates the form with biased
+bytes u = quant + bias, whose accumulators start at -bias * (limb sums); the integers are the same:
   * 65536 * v(l0', ones) + v(l1', l2') == sum_k (u_k - bias) * X_k exactly, for every bias the formats use;
   * every intermediate fits the int32 accumulators of the mma;
   * a one-hot x gives back d * q (+ m) bit for bit;

@@ -1,5 +1,5 @@
 // matvec_mma.cuh — the decode matvec for the integer weight formats on the TENSOR cores' integer path
-// (mma.sync.m16n8k32.s32.u8.u8), weights in fragment tiles (frag_layout.cuh).
+// (mma.sync.m16n8k32.s32.s8.u8), weights in fragment tiles (frag_layout.cuh).
 //
 // Why.  The dp4a core (matvec_idp.cuh) spends 24 IDP.4A plus ~30 unpack / convert / scale instructions per 32-weight block and
 // lane: 0.112 (q8_0) - 0.124 (q4_0) warp instructions per weight.  ncu: q4_0 W1|W3 runs at
