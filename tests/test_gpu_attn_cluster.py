@@ -53,3 +53,25 @@ def test_what_is_not_finite_goes_where_the_split_kernel_sends_it(what):
         assert np.array_equal(f(a), f(b))
     fin = np.isfinite(a)
     assert np.max(np.abs(a[fin] - b[fin])) < 64 * 10 * 2.0 ** -24
+
+
+# the first slot of all, of a warp's unit (16, 64), inside a unit, the last; alone, and as the only key of its warp (n = 17)
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 32, 8), (64, 32, 4)])
+@pytest.mark.parametrize("n,slot", [(1, 0), (17, 0), (17, 16), (300, 0), (300, 16), (300, 64), (300, 77), (300, 299)])
+@pytest.mark.parametrize("what", ["key nan", "key inf", "key -inf", "value nan", "value inf"])
+def test_what_is_not_finite_at_any_slot(what, n, slot, hd, nh, nkv):
+    """Against IEEE arithmetic in float64: a score that is NaN or +inf makes its head NaN, one that is -inf weighs nothing, a value reaches its own channel."""
+    q, k, v = inputs(hd, n, nh, nkv, 11)
+    kind, val = what.split()
+    (k if kind == "key" else v)[slot, 3 * hd + 9] = float(val)
+    got = both(q, k, v, hd, n, nh, nkv)[1].reshape(nh, hd)
+    K, V = (a[:n].astype(np.float64).reshape(n, nkv, hd) for a in (k, v))
+    with np.errstate(invalid="ignore"):
+        for h in range(nh):
+            s = K[:, h // (nh // nkv)] @ q[h * hd:(h + 1) * hd].astype(np.float64) / np.sqrt(hd)
+            p = np.exp(s - s.max())
+            want = p / p.sum() @ V[:, h // (nh // nkv)]
+            for f in (np.isnan, np.isposinf, np.isneginf):
+                assert np.array_equal(f(got[h]), f(want))
+            fin = np.isfinite(want)
+            assert not fin.any() or np.max(np.abs(got[h][fin] - want[fin])) < 64 * 10 * 2.0 ** -24  # as above

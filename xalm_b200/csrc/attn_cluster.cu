@@ -8,7 +8,7 @@
 // Queries and probabilities are fp32 values: each enters as three fp16 planes, scaled by powers of two, whose products with the cache's fp16 are exact.  Sums
 // of 16 products start from zero and are added in round-to-nearest as a tree, since the tensor cores' own additions truncate.  Distance from float64 over
 // 20 to 3002 keys and queries of deviation 0.3, 1 and 3: 0.99 times the split kernel's (0.86 to 1.13).  A warp that meets a score or a sum that is not finite
-// does its keys again in fp32 FMAs, so that an infinity or a NaN goes where it goes there (its zero planes would spread it).
+// does its keys again in fp32 FMAs, so that an infinity goes where it goes there (its zero planes would spread it); a NaN score, wherever its key lies, makes its head NaN.
 // A step's attention in the graph, split kernel before: 7B at position 3001 12.3 -> 9.5 us; per token, with it and without: 7B q8_0 1938 -> 1870 us, 8 layers of
 // q4_0 at 700 458 -> 428, 6 layers of bf16 at width 2048 and position 1777 275 -> 256.  Tried and not faster: rings of the neighbouring products cut
 // so that this kernel's CTAs fit beside them (no difference).
@@ -278,9 +278,8 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 					for (int e = 0; e < E; e++)
 						x += __ldcg(a.q + (size_t) (kvh * GP + h) * HD + lane + 32 * e) * __half2float(__ldcg(kbase + (size_t) slot * kv_stride + lane + 32 * e));
 					x = warp_sum(x) * inv_sqrt;
-					const float mn = fmaxf(mh, x);
-					if (mn == -CUDART_INF_F) continue;
-					const float corr = expf(mh - mn), pr = expf(x - mn);
+					const float mn = fmaxf(mh, x); // (-inf also where the first score is a NaN)
+					const float corr = mh == mn ? 1.f : expf(mh - mn), pr = x == -CUDART_INF_F ? 0.f : expf(x - mn);
 					lh = lh * corr + pr;
 					mh = mn;
 #pragma unroll
