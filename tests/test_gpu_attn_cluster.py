@@ -75,3 +75,10 @@ def test_what_is_not_finite_at_any_slot(what, n, slot, hd, nh, nkv):
                 assert np.array_equal(f(got[h]), f(want))
             fin = np.isfinite(want)
             assert not fin.any() or np.max(np.abs(got[h][fin] - want[fin])) < 64 * 10 * 2.0 ** -24  # as above
+
+
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 160, 40), (64, 320, 80), (32, 304, 38), (256, 640, 80)])
+def test_many_kv_heads_are_the_split_kernels(hd, nh, nkv):
+    """Fewer than four CTAs per kv head: slower than the split kernel on short contexts.  The kernels add in another order, so equal bits are the same kernel."""
+    assert np.array_equal(*both(*inputs(hd, 100, nh, nkv, 2), hd, 100, nh, nkv))
+    assert not np.array_equal(*both(*inputs(hd, 100, nh // nkv * 8, 8, 2), hd, 100, nh // nkv * 8, 8))

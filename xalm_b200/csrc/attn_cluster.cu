@@ -382,8 +382,8 @@ template <int HD, int GP>
 static int ac_size(int n_kv) {
 	int sms = 148, dev = 0;
 	if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	for (int C = AC_MAX_CTAS; C >= 1; C /= 2) {
-		if (C > 1 && C * n_kv > sms) continue;
+	for (int C = AC_MAX_CTAS; C >= 4 && n_kv > 0; C /= 2) {
+		if (C * n_kv > sms) continue;
 		cudaLaunchConfig_t cfg;
 		cudaLaunchAttribute at[2];
 		int n = 0;
@@ -391,7 +391,7 @@ static int ac_size(int n_kv) {
 			cudaGetLastError();
 			continue;
 		}
-		if (n >= n_kv || C == 1) return C;
+		if (n >= n_kv) return C;
 	}
 	return 0;
 }
@@ -408,7 +408,10 @@ static int ac_size(int n_kv) {
 // CTAs per kv head so that all clusters run at once on the current device; 0: the split kernel is the faster one for these heads.  Alone, back to back, buffers
 // beyond L2 (split kernel / this one, us): four heads of 128 over 8 kv heads 10.3 / 8.2 at 500 keys, 14.4 / 12.4 at 4096, 28.7 / 28.7 at 16384, 47 / 51 at 32768;
 // eight heads 14.4 / 10.3, 20.5 / 16.1, 49 / 35, 84 / 59; two heads 8.3 / 8.3, 12.4 / 12.3, 22.6 / 28.7; one head 10.1 / 10.3, 22.6 / 22.6.  Of 256 channels: eight
-// heads 26.6 / 14.4, 41 / 29, four 14.4 / 11.4, 20.5 / 22.6.
+// heads 26.6 / 14.4, 41 / 29, four 14.4 / 11.4, 20.5 / 22.6.  Operands in L2, 1 to 32 kv heads of 32 and 64 channels: four heads 0.55 to 0.95 of the split kernel's
+// time up to 4096 keys, 0.88 to 1.1 at 16384; eight heads 0.4 to 0.9.  The line for four heads is one of capacity, since a captured step serves every position.
+// From 38 kv heads on a cluster has one or two CTAs, 4 or 8 warps, and short contexts lose (100 keys, 128 channels, four heads: 74 kv heads 7.0 / 8.2, 80 7.0 / 12.2;
+// eight heads 10.6 / 12.5, 10.4 / 19.9): the split kernel's.
 int attn_cluster_size(int head_dim, int G, int n_kv_heads, int max_kv_len) {
 	if (G == 4 && max_kv_len > 16384) return 0;
 #define XALM_AC_SIZE(HD_, GP_) return ac_size<HD_, GP_>(n_kv_heads)
