@@ -197,17 +197,29 @@ struct MmaFmt<XALM_Q5_1> { // d * (ql | qh << 4) + m
 };
 
 __host__ __device__ inline bool mma_supported(int t) { return frag_record_bytes(t) != 0; }
-// records (32-element block columns) per ring stage: about 36 KB
-__host__ __device__ constexpr int mma_sb(int record_bytes) { return record_bytes > 400 ? 64 : 128; }
+// records (32-element block columns) per ring stage, 32 to 48 KB; half as many for rows that leave no room for three such stages (mma_stages)
+__host__ __device__ constexpr int mma_sb(int record_bytes, bool half = false) { return (record_bytes > 400 ? 64 : 128) / (half ? 2 : 1); }
 __host__ __device__ inline int mma_pb(int NS) { return NS + 2 < 8 ? 8 : NS + 2; } // partial-sum buffers (tiles in flight), as idp_pb
 
-__host__ __device__ inline size_t mma_smem_bytes(int type, int n, int NS) {
+__host__ __device__ inline size_t mma_smem_bytes(int type, int n, int NS, bool half) {
 	size_t s = xm_bytes(n);
-	s += (size_t) NS * mma_sb(frag_record_bytes(type)) * frag_record_bytes(type);
+	s += (size_t) NS * mma_sb(frag_record_bytes(type), half) * frag_record_bytes(type);
 	s += (size_t) mma_pb(NS) * MMA_NCW * MMA_RC * sizeof(float);
 	s += (2 * (size_t) NS + 2 * mma_pb(NS)) * sizeof(uint64_t);
 	s += MMA_NCW * sizeof(float);
 	return s + 128;
+}
+// Ring stages for rows of n elements (8 at most), and their size; 0: the rows' activations leave no room for a ring.  Two full stages keep too little in flight:
+// 8192 rows of 28672, two full -> four or five of half the size: q8_0 49.3 -> 43.7 us, q4_0 32.2 -> 28.9, q4_1 34.0 -> 32.7, q5_1 39.5 -> 39.0 (q5_0 38.9 -> 39.7).
+// The longest rows are of 44192 (q8_0), 43712 (q4_0) to 40832 (q5_1) elements.
+inline int mma_stages(int type, int n, bool* half) {
+	for (const bool h : {false, true})
+		for (int ns = 8; ns >= (h ? 2 : 3); ns--)
+			if (mma_smem_bytes(type, n, ns, h) <= 226 * 1024) {
+				*half = h;
+				return ns;
+			}
+	return 0;
 }
 
 struct MmaArgs {
@@ -216,10 +228,10 @@ struct MmaArgs {
 	int n_tiles;  // virtual rows / 16
 };
 
-template <int TYPE, bool NORM>
+template <int TYPE, bool NORM, bool HALF> // HALF: stages of half the records
 __global__ void __maxnreg__(80) matvec_mma_kernel(const MmaArgs ta) {
 	using F = MmaFmt<TYPE>;
-	constexpr int RC = MMA_RC, NCW = MMA_NCW, NT = MMA_NT, RB = F::RB, SB = mma_sb(RB), MP = MMA_MP, QB = 4 * NCW; // QB: records that are unrolled
+	constexpr int RC = MMA_RC, NCW = MMA_NCW, NT = MMA_NT, RB = F::RB, SB = mma_sb(RB, HALF), MP = MMA_MP, QB = SB < 4 * NCW ? SB : 4 * NCW; // QB: records that are unrolled
 	constexpr int STAGE = SB * RB;
 	auto cbar = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
 	const MatvecArgs& a = ta.a;
@@ -507,7 +519,7 @@ __global__ void __maxnreg__(80) matvec_mma_kernel(const MmaArgs ta) {
 			const int left = nb - kr * SB;
 #pragma unroll
 			for (int q = 0; q < SB; q += QB) {
-				if (left >= q + QB) { // this warp's four records sit at fixed offsets (every address = base + immediate)
+				if (left >= q + QB) { // this warp's records sit at fixed offsets (every address = base + immediate)
 #pragma unroll
 					for (int i = q / NCW; i < (q + QB) / NCW; i++) record(rec + (size_t) i * NCW * RB, bq + (size_t) i * NCW * 32, tq + i * NCW * TW);
 				} else {

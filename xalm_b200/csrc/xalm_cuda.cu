@@ -351,9 +351,9 @@ static int launch_matvec_idp(const MatvecArgs& a, cudaStream_t s, bool pdl) {
 // ---------------------------------------------------------------------------------------------------------
 // tensor-core matvec dispatch (matvec_mma.cuh): the integer weight formats in fragment tiles
 // ---------------------------------------------------------------------------------------------------------
-template <int TYPE, bool NORM>
+template <int TYPE, bool NORM, bool HALF>
 static cudaError_t launch_mma_inst(const MmaArgs& ta, size_t smem, cudaStream_t s, bool pdl) {
-	auto kern = matvec_mma_kernel<TYPE, NORM>;
+	auto kern = matvec_mma_kernel<TYPE, NORM, HALF>;
 	cudaError_t e = ensure_smem_attr(kern, 227 * 1024);
 	if (e != cudaSuccess) return e;
 	int grid = num_sms(); // persistent: one CTA per SM
@@ -368,17 +368,20 @@ static int launch_matvec_mma(const MatvecArgs& a, cudaStream_t s, bool pdl) {
 	if ((a.epi == EPI_GLU) != (a.w.glu_half != 0))
 		return set_error(XALM_ERR_STATE, "fragment layout: gate|up interleave (%d) does not match the epilogue (%d)", a.w.glu_half, a.epi);
 	const bool norm = a.norm_w != nullptr;
-	int NS = 0;
-	for (int ns = 8; ns >= 2; ns--)
-		if (mma_smem_bytes(t, a.n, ns) <= 226 * 1024) { NS = ns; break; }
+	bool half = false;
+	const int NS = mma_stages(t, a.n, &half);
 	if (!NS) return set_error(XALM_ERR_UNSUPPORTED, "matmul: rows of %d elements do not fit the tensor-core matvec's shared memory", a.n);
 	MmaArgs ta;
 	ta.a = a;
 	ta.NS = NS;
 	ta.n_tiles = vrows / MMA_RC;
-	const size_t smem = mma_smem_bytes(t, a.n, NS);
+	const size_t smem = mma_smem_bytes(t, a.n, NS, half);
 	cudaError_t e;
-#define XALM_MMA_CASE(T) case T: e = norm ? launch_mma_inst<T, true>(ta, smem, s, pdl) : launch_mma_inst<T, false>(ta, smem, s, pdl); break;
+#define XALM_MMA_CASE(T)                                                                                                                         \
+	case T:                                                                                                                                      \
+		if (half) e = norm ? launch_mma_inst<T, true, true>(ta, smem, s, pdl) : launch_mma_inst<T, false, true>(ta, smem, s, pdl);              \
+		else e = norm ? launch_mma_inst<T, true, false>(ta, smem, s, pdl) : launch_mma_inst<T, false, false>(ta, smem, s, pdl);                 \
+		break;
 	switch (t) {
 		XALM_MMA_CASE(XALM_Q8_0)
 		XALM_MMA_CASE(XALM_Q8)
@@ -689,8 +692,8 @@ static int alloc_wmat(DevAlloc& da, WMat& m, int type, int rows, int n, int glu_
 	// 1 (default): all of them.  2: the 4/5-bit formats; the 8-bit ones under tensor parallelism, where the per-rank rows are short (the dp4a kernel
 	// maps one 32-element block to a lane: rows of 512 elements keep 16 of its 256 lanes busy)
 	const bool mma_on = tune("mma") == 1 || (tune("mma") == 2 && (sharded || (type != XALM_Q8_0 && type != XALM_Q8)));
-	if (mma_supported(type) && n % 32 == 0 && rows % MMA_RC == 0 && glu_half % 8 == 0 && mma_on && tune("tma") && !tune("mega") &&
-	    mma_smem_bytes(type, n, 2) <= 226 * 1024) {
+	bool half;
+	if (mma_supported(type) && n % 32 == 0 && rows % MMA_RC == 0 && glu_half % 8 == 0 && mma_on && tune("tma") && !tune("mega") && mma_stages(type, n, &half)) {
 		// integer formats on the tensor-core path: fragment tiles (frag_layout.cuh); same byte count as on disk
 		m.layout_frag = 1;
 		m.glu_half = glu_half;
