@@ -1698,14 +1698,15 @@ int xalm_cuda_sync(xalm_cuda_model* m) {
 // took 20 us more: pieces of 4 to 64 bytes over PCIe.
 int xalm_cuda_forward(xalm_cuda_model* m, int token, int pos, int mode, float* logits_host) {
 	XALM_TRY(check_token(m, token, pos, mode));
-	if (m->tp_size == 1 && !m->mega && tune("graph")) {
+	const bool leaves = mode == XALM_OUTPUT_LOGITS && !logits_host; // the logits stay on the device, h_logits keeps what it held
+	if (m->tp_size == 1 && !m->mega && !leaves && tune("graph")) {
 		XALM_CUDA_CHECK(cudaSetDevice(m->device));
 		XALM_TRY(ensure_graph(m, mode, true));
 		*m->h_step_io = step_params(m, token, pos, mode);
 		XALM_CUDA_CHECK(cudaGraphLaunch(m->graph_io[mode], m->stream));
 		m->last_launches = m->launches_per_token[mode];
 		XALM_CUDA_CHECK(cudaStreamSynchronize(m->stream));
-		if (mode == XALM_OUTPUT_LOGITS && logits_host && logits_host != m->h_logits) memcpy(logits_host, m->h_logits, (size_t) m->c.vocab_size * sizeof(float));
+		if (mode == XALM_OUTPUT_LOGITS && logits_host != m->h_logits) memcpy(logits_host, m->h_logits, (size_t) m->c.vocab_size * sizeof(float));
 		return XALM_OK;
 	}
 	XALM_TRY(xalm_cuda_forward_async(m, token, pos, mode));
