@@ -3,6 +3,9 @@ import numpy as np
 import pytest
 
 from xalm_b200 import capi
+from xalm_b200.model import InferenceState
+
+from gpu_util import synth_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -82,3 +85,20 @@ def test_many_kv_heads_are_the_split_kernels(hd, nh, nkv):
     """Fewer than four CTAs per kv head: slower than the split kernel on short contexts.  The kernels add in another order, so equal bits are the same kernel."""
     assert np.array_equal(*both(*inputs(hd, 100, nh, nkv, 2), hd, 100, nh, nkv))
     assert not np.array_equal(*both(*inputs(hd, 100, nh // nkv * 8, 8, 2), hd, 100, nh // nkv * 8, 8))
+
+
+@pytest.mark.parametrize("cluster", [1, 0])
+def test_the_timeline_has_every_layers_attention(cluster):
+    capi.tune("attn_cluster", cluster)
+    config, om, gm = synth_pair("small", "q8_0", seed=1, std=0.03)   # four query heads per kv head
+    capi.tune("attn_cluster", 1)
+    state = InferenceState(config)
+    gm.forward(state, 5, 0, 1)
+    capi.timeline_start(200)
+    gm.forward(state, 6, 1, 1)
+    rec = capi.timeline_stop(200)
+    at = rec[rec[:, 0] == 300].astype(np.int64)
+    assert len(at) == config["n_layers"]
+    assert np.all(at[:, 1] <= at[:, 2]) and np.all(at[:, 2] <= at[:, 3]) and np.all(at[1:, 1] > at[:-1, 1])
+    capi.timeline_start(0)
+    gm.close(); om.close()

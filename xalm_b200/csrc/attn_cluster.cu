@@ -80,6 +80,11 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 	ac_cluster_arrive(); // (1) every CTA of the cluster runs
 	const int C = gridDim.x, rank = blockIdx.x, kvh = blockIdx.y; // one cluster per kv head
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+	// The in-kernel timeline, as the split kernel's: its buffer (asked for here, looked at when the first keys are on their way), the time of the start and of the wait's
+	// end.  In shared memory: no registers are left, and the timer is read only while it records (read always, a layer took 0.2 us more).
+	__shared__ unsigned long long tl_sm[3];
+	const bool stamps = a.tl && (tid | rank | kvh) == 0;
+	const unsigned long long tl_buf = stamps ? __ldcg(reinterpret_cast<const unsigned long long*>(&a.tl->buf)) : 0ull;
 	if (tid == 0) l2_prefetch_slice(a.pf_ptr, a.pf_bytes, kvh * C + rank, C * (int) gridDim.y);
 
 	const bool fixed = a.kv_len_fixed >= 0;
@@ -106,7 +111,10 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		if (u0 + j * du < nu) fetch(u0 + j * du, j, AC_EARLY);
 	commit();
 
+	if (stamps) tl_sm[0] = tl_buf;
+	if (tl_buf) tl_sm[1] = gtime();
 	pdl_wait();
+	if (tl_buf) tl_sm[2] = gtime();
 #pragma unroll
 	for (int j = 0; j < NST; j++) {
 		const int u = u0 + j * du;
@@ -357,6 +365,11 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		num += __shfl_xor_sync(0xffffffffu, num, 2);
 		den += __shfl_xor_sync(0xffffffffu, den, 2);
 		if (in && part == 0) a.out[(size_t) (kvh * GP + h) * HD + rank * own + x / GP] = num * (1.f / AC_PSCALE) / den;
+	}
+	if (a.tl && (tid | rank | kvh) == 0 && tl_sm[0]) {
+		const unsigned int slot = atomicAdd(&a.tl->count, 1u);
+		unsigned long long* r = reinterpret_cast<unsigned long long*>(tl_sm[0]) + 4 * (size_t) slot;
+		if (slot < a.tl->cap) { r[0] = 300; r[1] = tl_sm[1]; r[2] = tl_sm[2]; r[3] = gtime(); }
 	}
 }
 

@@ -632,6 +632,14 @@ static cudaError_t launch_attn_hd(const AttnArgs& a, int G, cudaStream_t s, bool
 	}
 	return cudaErrorInvalidValue;
 }
+static Timeline* timeline_dev() { // of the current device
+	void* p = nullptr;
+	if (cudaGetSymbolAddress(&p, d_timeline) != cudaSuccess) {
+		cudaGetLastError();
+		return nullptr;
+	}
+	return (Timeline*) p;
+}
 static int launch_attn(const AttnArgs& a, int head_dim, int G, cudaStream_t s, bool pdl) {
 	cudaError_t e;
 	switch (head_dim) {
@@ -851,6 +859,7 @@ struct xalm_cuda_model {
 	unsigned int* tickets = nullptr;
 	int attn_splits = 0;
 	int attn_cluster = 0; // CTAs per kv head of attn_cluster.cu; 0: the split kernel of attention.cuh
+	Timeline* timeline = nullptr;
 	StepParams* d_step = nullptr;
 	StepParams* h_step = nullptr; // pinned ring
 	StepParams* h_step_io = nullptr; // pinned: the token of a call that waits for it
@@ -1520,7 +1529,7 @@ static void fill_layer_args(xalm_cuda_model* m, int l, MatvecArgs* qkv, AttnArgs
 		AttnArgs a = {};
 		a.q = m->q; a.k_cache = L.k_cache; a.v_cache = L.v_cache; a.out = m->xb2; a.step = m->d_step; a.kv_len_fixed = -1;
 		a.n_kv_heads = m->n_kv_heads_l; a.n_splits = m->attn_splits; a.min_split = tune("attn_min_split");
-		a.part_acc = m->attn_acc; a.part_ml = m->attn_ml; a.tickets = m->tickets;
+		a.part_acc = m->attn_acc; a.part_ml = m->attn_ml; a.tickets = m->tickets; a.tl = m->timeline;
 		*at = a;
 	}
 	{ // Wo + residual
@@ -1596,6 +1605,7 @@ int xalm_cuda_finalize(xalm_cuda_model* m) {
 	XALM_CUDA_CHECK(cudaMemcpy(m->rope_freq, freq.data(), freq.size() * sizeof(float), cudaMemcpyHostToDevice));
 	const int G = c.n_heads / c.n_kv_heads;
 	m->attn_splits = attn_auto_splits(m->n_kv_heads_l);
+	m->timeline = timeline_dev();
 	m->attn_cluster = tune("attn_cluster") ? attn_cluster_size(c.head_dim, G, m->n_kv_heads_l, c.max_seq_len) : 0;
 	// the last-CTA merge parks 3 floats per (split, head) in the 8 x G x head_dim floats of the per-warp partial area (attention.cuh)
 	if (m->attn_splits > 8 * c.head_dim / 3) m->attn_splits = 8 * c.head_dim / 3;
@@ -1913,6 +1923,7 @@ int xalm_cuda_mha(float* xout, float* att, const uint16_t* kb, const uint16_t* v
 	a.q = (const float*) dq; a.k_cache = (const __half*) dk; a.v_cache = (const __half*) dv; a.out = (float*) dout;
 	a.kv_len_fixed = kv_len; a.n_kv_heads = n_kv_heads; a.n_splits = splits; a.min_split = tune("attn_min_split");
 	a.part_acc = (float*) dacc; a.part_ml = (float*) dml; a.tickets = (unsigned int*) dtick;
+	a.tl = timeline_dev();
 	const int C = tune("attn_cluster") ? attn_cluster_size(head_dim, G, n_kv_heads, kv_len) : 0;
 	XALM_TRY(C ? launch_attn_cluster(a, head_dim, G, C, 0, false) : launch_attn(a, head_dim, G, 0, false));
 	if (att) {
