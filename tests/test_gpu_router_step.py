@@ -52,3 +52,60 @@ def test_groups_and_scores(E, top, n_groups, keep, score, group, renorm):
         assert np.array_equal(idx[0], want)   # (random scores: no two within fp32 rounding)
         w = s[want] / s[want].sum() if renorm else s[want]
         assert np.abs(wgt[0] - w).max() < 1e-5
+
+
+# What is not finite, against the kernel of longer passes (two equal tokens): NaN rows (which have no place in an order: that kernel's choice is the rule), infinite
+# scores of either sign and infinities in the token, whose sigmoids are ties
+@pytest.mark.parametrize("E,top", [(4, 2), (16, 4), (31, 5), (32, 32)])
+@pytest.mark.parametrize("what", ["nan row 0", "nan row 3", "nan row last", "nan rows", "all nan", "inf row", "inf token", "huge token"])
+@pytest.mark.parametrize("score,groups", [("sigmoid", 0), ("softmax", 0), ("softmax", 4)])
+def test_what_is_not_finite_as_in_longer_passes(E, top, what, score, groups):
+    if groups and E % groups:
+        pytest.skip("experts do not form that many groups")
+    K, ff = 128, 8
+    rng = np.random.default_rng(E)
+    h, wr = rng.standard_normal((1, K)).astype(np.float32), bf16(3 * rng.standard_normal((E, K)) / K ** 0.5)
+    if what == "all nan":
+        h[0, 3] = np.nan
+    elif what == "nan rows":
+        wr[1::3, 5] = np.nan
+    elif what.startswith("nan row"):
+        wr[{"0": 0, "3": 3, "last": E - 1}[what.split()[-1]], 7] = np.nan
+    elif what == "inf row":
+        wr[2, 7], wr[1, 7] = np.inf, -np.inf
+    elif what == "inf token":
+        h[0, 9] = np.inf
+    else:
+        h *= 1e30
+    wg, wu, wd = (bf16(rng.standard_normal(s)) for s in ((E, ff, K), (E, ff, K), (E, K, ff)))
+    # (two groups of two experts hold too few for the largest choices)
+    kw = dict(n_groups=groups, keep_groups=max(2, -(-top * groups // E)) if groups else 0, score=score, group="max", renormalise=True, w_bf16=True)
+    one = capi.moe_ffn_routed(h, wr, wg, wu, wd, top, **kw)
+    two = capi.moe_ffn_routed(np.repeat(h, 2, axis=0), wr, wg, wu, wd, top, **kw)
+    assert np.array_equal(one[0][0], two[0][0]) and np.array_equal(np.isnan(one[1][0]), np.isnan(two[1][0]))
+    fin = np.isfinite(two[1][0])
+    assert np.abs(one[1][0][fin] - two[1][0][fin]).max(initial=0) < 1e-5
+
+
+@pytest.mark.parametrize("E,top,K", [(32, 4, 2480), (32, 32, 64), (1, 1, 40000), (8, 3, 8192)])   # the first two: as many rows, and as many bytes, as it takes
+@pytest.mark.parametrize("bad", [None, "nan", "inf"])
+def test_plain_logits_with_bias_and_gate(E, top, K, bad):
+    rng = np.random.default_rng(K + E)
+    h, wr, gate = rng.standard_normal((1, K)).astype(np.float32), bf16(3 * rng.standard_normal((E, K)) / K ** 0.5), bf16(rng.standard_normal(K) / K ** 0.5)
+    bias = rng.standard_normal(E).astype(np.float32)
+    if bad:
+        bias[E // 2] = float(bad)
+    ff = 8
+    wg, wu, wd = (bf16(rng.standard_normal(s) / K ** 0.5) for s in ((E, ff, K), (E, ff, K), (E, K, ff)))
+    x, base = np.zeros((1, K), np.float32), np.ones((1, K), np.float32)
+    one = capi.moe_chosen(x, h, wr, wg, wu, wd, top, bias=bias, base=base, gate_row=gate, w_bf16=True)
+    r2 = lambda a: np.repeat(a, 2, axis=0)
+    two = capi.moe_chosen(r2(x), r2(h), wr, wg, wu, wd, top, bias=bias, base=r2(base), gate_row=gate, w_bf16=True)
+    assert np.array_equal(one[1][0], two[1][0]) and np.array_equal(np.isnan(one[2][0]), np.isnan(two[2][0]))
+    if bad:
+        return
+    z = (h.astype(np.float64) @ wr.T.astype(np.float64))[0] + bias
+    want = np.argsort(-z, kind="stable")[:top]
+    w = np.exp(z[want] - z[want[0]])
+    assert np.array_equal(one[1][0], want) and np.abs(one[2][0] - w / w.sum()).max() < 1e-5
+    assert np.abs(one[0] - two[0][:1]).max() < 1e-4   # sums of up to 32 rows of order one, and the gate's

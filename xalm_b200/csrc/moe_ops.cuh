@@ -168,12 +168,14 @@ __global__ void __launch_bounds__(256) moe_router_kernel(MoeRouteArgs a) {
 // 16 experts of 2048 channels with four chosen: the kernel above 9.7 us in a step (a row after another from memory, a choice through ten shuffles
 // with two results each, the weights through memory); this one 6.7 us alone: 0.3 until the copy is under way, 0.6 for the token's channels, 2.2 for the
 // rows, 0.9 for the choice.  A chat of 48 steps of Pavitar 2048, two such layers: 11.72 -> 11.40 ms.
+// Up to its limits it stays ahead (us, this kernel / the one above): 32 experts of 64 channels 6.6 / 7.1, of 2560 12.0 / 17.8; 16 of 5120 10.8 / 14.3; one of 16384 6.7 / 19.4.
 constexpr int MOE_STEP_BYTES = 160 * 1024;
+static inline size_t moe_router_smem(int K, int E, int n_groups) { return (size_t) (K + 2 * E + std::max(n_groups, 1)) * 4; } // of moe_router_kernel
 static inline bool moe_step_fits(const MoeRouteArgs& a) {
-	return a.w_bf16 && a.E <= 32 && a.K % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.h)) & 15) == 0 &&
+	return moe_router_smem(a.K, a.E, a.n_groups) <= 200 * 1024 && a.w_bf16 && a.E <= 32 && a.K % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.h)) & 15) == 0 &&
 	       (size_t) (a.E + (a.gate_out ? 1 : 0)) * a.K * 2 <= MOE_STEP_BYTES;
 }
-// the lane with the largest of the values of the lanes that are live, the lowest on ties, NaN last; -1: none
+// the lane with the largest of the values of the lanes that are live, the lowest on ties; -1: none
 __device__ __forceinline__ int moe_best(float v, bool live) {
 	const uint32_t u = __float_as_uint(v + 0.f), key = !live ? 0u : v != v ? 1u : u ^ (u >> 31 ? 0xffffffffu : 0x80000000u);
 	const uint32_t top = __reduce_max_sync(0xffffffffu, key), who = __ballot_sync(0xffffffffu, key == top);
@@ -245,8 +247,15 @@ static __global__ void __launch_bounds__(256) moe_router_step_kernel(MoeRouteArg
 	float w = 0.f; // lane r keeps choice r
 	int idx = 0;
 	const float cmp = a.correction ? s + correction : s;
+	const bool unordered = __any_sync(0xffffffffu, live && cmp != cmp); // a NaN has no place in an order: chosen as in moe_router_kernel
 	for (int r = 0; r < a.top; r++) {
-		const int best = moe_best(cmp, live);
+		int best;
+		if (unordered) {
+			float bv = live ? cmp : -INFINITY;
+			best = live ? lane : -1;
+			warp_argmax(bv, best);
+			best = __shfl_sync(0xffffffffu, best, 0);
+		} else best = moe_best(cmp, live);
 		const float v = __shfl_sync(0xffffffffu, s, max(best, 0));
 		if (lane == r) { idx = max(best, 0); w = best < 0 ? 0.f : v; }
 		live = live && lane != best;
@@ -527,7 +536,6 @@ __global__ void __launch_bounds__(256, 2) moe_few_kernel(MoeGemmArgs a) {
 }
 
 // ---- launchers ------------------------------------------------------------------------------------------------------------------
-static inline size_t moe_router_smem(int K, int E, int n_groups) { return (size_t) (K + 2 * E + std::max(n_groups, 1)) * 4; }
 static inline int moe_prepare(int K, int E, int n_groups) { // outside a stream capture
 	XALM_CUDA_CHECK(cudaFuncSetAttribute(moe_router_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_STEP_BYTES));
 	if (moe_router_smem(K, E, n_groups) > 48 * 1024) {
