@@ -23,7 +23,7 @@ def kernels():
     out = {}
     for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
         text = re.sub(r"//[^\n]*", "", open(path).read())
-        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\s*(?=\())?", text):
+        for m in re.finditer(r"__global__\s+void\s+(?:(?:__launch_bounds__|__maxnreg__)\s*(?=\())?", text):
             at = m.end()
             if text[at] == "(":
                 at = closed(text, at)
@@ -52,3 +52,10 @@ def test_every_kernel_of_a_one_token_step_waits_for_the_one_before():
     assert len(found) > 15
     for name in found:
         assert "pdl_enter()" in ks[name][1], name
+
+
+def test_no_two_kernels_share_a_name():
+    """The checks above look kernels up by name."""
+    names = [n for path in glob.glob(os.path.join(CSRC, "*.cu*")) for n in
+             re.findall(r"__global__\s+void\s+(?:__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)|__maxnreg__\s*\(\d+\))?\s*(\w+)\s*\((?=[^;{]*\)\s*\{)", open(path).read())]
+    assert len(names) > 70 and sorted(names) == sorted(set(names))

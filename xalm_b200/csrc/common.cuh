@@ -94,15 +94,6 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size
 	return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// ---- a step's inputs and logits in pinned host memory, read and written by kernels: a copy's node in the graph, and the change from it to a kernel and back,
-//      take longer than a kernel more (the engine's copies of 16 bytes and 128 KB: about 4 and 10 us of a step, these two 2 and 4) ----
-__device__ __forceinline__ void pinned_out(const float* src, float* dst, int n) { // every thread of the grid
-	const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-	if (i + 4 <= n) *reinterpret_cast<float4*>(dst + i) = __ldcg(reinterpret_cast<const float4*>(src + i));
-	else
-		for (int k = i; k < n; k++) dst[k] = __ldcg(src + k);
-}
-
 // ---- L2 prefetch of a slice of the NEXT kernel's first bytes (cp.async.bulk.prefetch.L2): CTA `cta` of `n_ctas` takes its share ----
 __device__ __forceinline__ void l2_prefetch_slice(const uint8_t* ptr, unsigned long long bytes, int cta, int n_ctas) {
 	if (!ptr || !bytes) return;

@@ -36,6 +36,7 @@
 #include "host/json.h"
 #include "mix_ops.cuh"
 #include "prefill.h"
+#include "step_io.cuh"
 #include "target_prob.cuh"
 
 namespace xalm {
@@ -333,13 +334,6 @@ int check_ready(SeqModel* m) {
 	if (!m->finalized) return set_error(XALM_ERR_STATE, "the model is not finalized");
 	XALM_CUDA_CHECK(cudaSetDevice(m->device));
 	return XALM_OK;
-}
-
-// the first and the last kernel of a step whose inputs and logits lie in pinned host memory
-__global__ void step_in_kernel(const int* in, int* out) { out[threadIdx.x] = in[threadIdx.x]; }
-__global__ void logits_out_kernel(const float* logits, float* host, int n) {
-	pdl_enter();
-	pinned_out(logits, host, n);
 }
 
 int ensure_graph(SeqModel* m, int mode, bool io) {

@@ -34,6 +34,7 @@
 #include "decode_mega.h"
 #include "prefill.h"
 #include "family.h"
+#include "step_io.cuh"
 
 namespace xalm {
 
@@ -468,13 +469,6 @@ __global__ void embed_kernel(int type, const uint8_t* __restrict__ table, size_t
 	pdl_wait();
 	const uint8_t* row = table + (size_t) step->token * row_bytes;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += gridDim.x * blockDim.x) x[i] = decode_disk_elem(type, row, i);
-}
-
-// a token's parameters from pinned host memory, before the kernels that read them ahead of their dependency waits
-__global__ void step_in_kernel(const int* in, int* out) { out[threadIdx.x] = in[threadIdx.x]; }
-__global__ void logits_out_kernel(const float* logits, float* host, int n) {
-	pdl_enter();
-	pinned_out(logits, host, n);
 }
 
 __global__ void dequant_kernel(int type, const uint8_t* __restrict__ src, size_t n, float* __restrict__ dst) {
@@ -1704,7 +1698,7 @@ int xalm_cuda_sync(xalm_cuda_model* m) {
 }
 
 // The caller waits for the token, so its parameters can lie in pinned memory that a kernel reads, and a kernel leaves the logits in pinned memory: one graph
-// launch without copies (pinned_out in common.cuh; four q8_0 layers of width 1024: 114.4 -> 105.7 us).  The classifier writing its rows there itself
+// launch without copies (step_io.cuh; four q8_0 layers of width 1024: 114.4 -> 105.7 us).  The classifier writing its rows there itself
 // took 20 us more: pieces of 4 to 64 bytes over PCIe.
 int xalm_cuda_forward(xalm_cuda_model* m, int token, int pos, int mode, float* logits_host) {
 	XALM_TRY(check_token(m, token, pos, mode));
