@@ -1,12 +1,12 @@
 """numpy model of the tensor-core decode matvec (xalm_b200/csrc/matvec_mma.cuh) and of its weight layout
 (xalm_b200/csrc/frag_layout.cuh), run on the CPU.
 
-The kernel feeds mma.sync.m16n8k32.s8.u8.s32 with signed quants as A and, as B, the three unsigned limbs of the OFFSET activations
-X' = X + 2^23 plus a column of ones, accumulators from zero (tests/test_gpu_mma_stages.py).  This file restates the form with biased
-bytes u = quant + bias, whose accumulators start at -bias * (limb sums); the integers are the same:
-  * 65536 * v(l0', ones) + v(l1', l2') == sum_k (u_k - bias) * X_k exactly, for every bias the formats use;
-  * every intermediate fits the int32 accumulators of the mma;
-  * a one-hot x gives back d * q (+ m) bit for bit;
+The kernel feeds mma.sync.m16n8k32.s8.u8.s32 (u8.u8 for the formats with a minimum) with quants times MUL as A and, as B, the three unsigned limbs of the
+OFFSET activations X' = X + 2^23 plus a column of ones; the accumulators start at zero.  This file restates that arithmetic and checks the claims of the kernel's header:
+  * the bytes that a record's stored quant becomes are MUL * quant, signed, for every code;
+  * 65536 * v(l0', ones) + v(l1', l2') == MUL * sum_k q_k * X_k exactly;
+  * every intermediate fits int32;
+  * a one-hot x gives back d * q (+ m) bit for bit, with the factors 65536 and 1 / MUL applied at a tile's end;
 and for the layout: the (row, element) -> byte map of a record is a bijection that puts the mma's A fragment of lane t at
 bytes [16 t, 16 t + 16) (8-bit) / [8 t, 8 t + 8) (4-bit), with the two rows of a GLU pair in the same lane.
 The GPU side of the same checks is tests/test_gpu_formats.py (one-hot bit exactness, random x against the oracle).
@@ -17,8 +17,35 @@ import pytest
 F32 = np.float32
 
 
+# format -> (MUL, has a minimum, what the kernel makes of a stored code as the byte fed to the mma, the code's quant)
+def nibble_up(u):
+    return ((u << 4) & 0xF0) ^ 0x80           # Q4_0: a nibble in the byte's upper half, its top bit turned
+
+
+FORMATS = {
+    "q8_0": (1, False, lambda u: u ^ 0x80, lambda u: u - 128, 256),
+    "q4_0": (16, False, nibble_up, lambda u: u - 8, 16),
+    "q5_0": (8, False, lambda u: ((u << 3) & 0xFF) ^ 0x80, lambda u: u - 16, 32),
+    "q4_1": (1, True, lambda u: u, lambda u: u, 16),
+    "q5_1": (1, True, lambda u: u, lambda u: u, 32),
+}
+
+
+def operand(fmt, u):
+    """The bytes that codes u become, as the mma reads them: signed, or unsigned where there is a minimum."""
+    b = FORMATS[fmt][2](np.asarray(u, dtype=np.int64)) & 0xFF
+    return b if FORMATS[fmt][1] else np.where(b >= 128, b - 256, b)
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+def test_the_byte_of_every_code_is_its_quant_times_mul(fmt):
+    mul, _, _, quant, n = FORMATS[fmt]
+    u = np.arange(n)
+    assert np.array_equal(operand(fmt, u), mul * quant(u))
+
+
 def stage_block(x):
-    """xm_store_group8 over one 32-element block: offset limbs l0' l1' l2' (each 0..255), their sums, dx."""
+    """xm_store_group8 over one 32-element block: X, the offset limbs l0' l1' l2' (each 0..255), dx."""
     x = np.asarray(x, dtype=F32)
     mb = int(np.max(x.view(np.uint32) & 0x7FFFFFFF))
     eb = mb >> 23
@@ -30,73 +57,66 @@ def stage_block(x):
     X = np.minimum(np.rint(prod).astype(np.int64), 8388607)
     Xo = X + 8388608
     assert Xo.min() >= 0 and Xo.max() < 1 << 24
-    limbs = np.stack([(Xo >> 16) & 255, (Xo >> 8) & 255, Xo & 255])
-    return X, limbs, limbs.sum(axis=1), dx
+    return X, np.stack([(Xo >> 16) & 255, (Xo >> 8) & 255, Xo & 255]), dx
 
 
-def mma_block(u, bias, limbs, sums):
-    """One record column of the mma for one row: accumulators of the four used B columns -> (v01, v23)."""
-    u = u.astype(np.int64)
-    c_l2 = -bias * sums[2] + int(np.dot(u, limbs[2]))
-    c_l1 = -bias * sums[1] + int(np.dot(u, limbs[1]))
-    c_l0 = -bias * (sums[0] - 4096) + int(np.dot(u, limbs[0]))
-    c_one = int(u.sum())
+def mma_block(a, limbs):
+    """One record column of the mma for one row: the accumulators of the four used B columns, from zero -> (v01, v23)."""
+    c_l2, c_l1, c_l0, c_one = (int(np.dot(a, limbs[2])), int(np.dot(a, limbs[1])), int(np.dot(a, limbs[0])), int(a.sum()))
     for c in (c_l2, c_l1, c_l0, c_one):
         assert abs(c) < 2 ** 31
-    v01 = 256 * c_l1 + c_l2          # lane tig = 0: columns (l2', l1')
-    v23 = c_l0 - 128 * c_one         # lane tig = 1: columns (l0', ones); 128 * 65536 = 2^23 removes the offset
-    assert abs(v01) < 2 ** 31 and abs(v23) < 2 ** 31
+    v01 = 256 * c_l1 + c_l2          # lane position 0: columns (l2', l1')
+    v23 = c_l0 - 128 * c_one         # lane position 1: columns (l0', ones); 128 * 65536 = 2^23 removes the offset
+    assert abs(256 * c_l1) < 2 ** 31 and abs(128 * c_one) < 2 ** 31 and abs(v01) < 2 ** 31 and abs(v23) < 2 ** 31
     return v01, v23
 
 
-@pytest.mark.parametrize("bias,qmax", [(128, 255), (8, 15), (16, 31), (0, 15), (0, 31)])
+@pytest.mark.parametrize("fmt", FORMATS)
 @pytest.mark.parametrize("scale", [1e-12, 1.0, 250.0])
-def test_offset_limb_mma_is_the_exact_integer_dot_product(bias, qmax, scale):
-    rng = np.random.default_rng(bias * 7 + qmax)
+def test_offset_limb_mma_is_the_exact_integer_dot_product(fmt, scale):
+    mul, _, _, quant, n = FORMATS[fmt]
+    rng = np.random.default_rng(n * 7 + mul)
     for trial in range(40):
         x = (rng.standard_normal(32) * scale).astype(F32)
-        if trial == 0:
-            x[:] = np.abs(x).max()                      # every element at the block maximum: the largest sums
-        if trial == 1:
-            x[:] = -np.abs(x).max()
-        X, limbs, sums, dx = stage_block(x)
-        u = rng.integers(0, qmax + 1, 32)
-        if trial < 2:
-            u[:] = qmax
-        v01, v23 = mma_block(u, bias, limbs, sums)
-        assert 65536 * v23 + v01 == int(np.dot(u.astype(np.int64) - bias, X))
+        u = rng.integers(0, n, 32)
+        if trial < 4:                                   # the largest sums: every element at the block's maximum, the quants at either end
+            x[:] = (1 if trial & 1 else -1) * np.abs(x).max()
+            u[:] = n - 1 if trial & 2 else 0
+        X, limbs, dx = stage_block(x)
+        v01, v23 = mma_block(operand(fmt, u), limbs)
+        assert 65536 * v23 + v01 == mul * int(np.dot(quant(u), X))
 
 
 def test_dead_and_nonfinite_blocks_contribute_nothing():
     for x in (np.zeros(32, F32), np.full(32, 1e-30, F32), np.array([np.inf] + [1.0] * 31, F32)):
-        X, limbs, sums, dx = stage_block(x)
+        X, limbs, dx = stage_block(x)
         assert dx == 0 and np.all(X == 0)
-        v01, v23 = mma_block(np.full(32, 200), 128, limbs, sums)
-        assert v01 == 0 and v23 == 0                    # and dx = 0 multiplies whatever is left
+        v01, v23 = mma_block(operand("q8_0", np.full(32, 200)), limbs)
+        assert 65536 * v23 + v01 == 0                   # and dx = 0 multiplies either lane's part
 
 
-@pytest.mark.parametrize("bias,qmax,has_min", [(128, 255, False), (8, 15, False), (16, 31, False), (0, 15, True), (0, 31, True)])
-def test_one_hot_returns_the_dequantised_weight_bit_for_bit(bias, qmax, has_min):
+@pytest.mark.parametrize("fmt", FORMATS)
+def test_one_hot_returns_the_dequantised_weight_bit_for_bit(fmt):
+    mul, has_min, _, quant, n = FORMATS[fmt]
     rng = np.random.default_rng(3)
     for _ in range(200):
         j = int(rng.integers(0, 32))
         x = np.zeros(32, F32)
         x[j] = 1.0
-        X, limbs, sums, dx = stage_block(x)
-        u = rng.integers(0, qmax + 1, 32)
+        X, limbs, dx = stage_block(x)
+        u = rng.integers(0, n, 32)
         d = F32(np.float16(rng.standard_normal() * 0.1))
         m = F32(np.float16(rng.standard_normal())) if has_min else None
-        v01, v23 = mma_block(u, bias, limbs, sums)
-        # the two lanes accumulate float(v) * (d * dx [* 65536]) separately, the quad reduction adds them
-        y1 = F32(np.float64(F32(v23)) * np.float64(F32(d * F32(dx * F32(65536.0)))))
-        y0 = F32(np.float64(F32(v01)) * np.float64(F32(d * dx)))
+        v01, v23 = mma_block(operand(fmt, u), limbs)
+        # either lane adds float(v) * (d * dx); at the tile's end lane position 0 is multiplied by 1 / MUL, 1 by 65536 / MUL, and the two are added
+        y0 = F32(F32(v01) * F32(d * dx))
+        y1 = F32(F32(v23) * F32(d * dx))
         if has_min:
-            tot = (int(sums[0]) - 4096) * 65536 + int(sums[1]) * 256 + int(sums[2])
-            sx = F32(F32(tot) * dx)
+            sx = F32(F32(int(X.sum())) * dx)
             assert sx == 1.0
             y0 = F32(np.float64(m) * np.float64(sx) + np.float64(y0))
-        y = F32(y0 + y1)
-        want = F32(F32(d * F32(int(u[j]) - bias)) + (m if has_min else F32(0)))   # quants.py: d * q (+ m), one rounding
+        y = F32(F32(y0 * F32(1.0 / mul)) + F32(y1 * F32(65536.0 / mul)))
+        want = F32(F32(d * F32(int(quant(u[j])))) + (m if has_min else F32(0)))   # quants.py: d * q (+ m), one rounding
         assert y.view(np.uint32) == want.view(np.uint32) or (y == 0 and want == 0)
 
 
