@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""bench.py — Mistral-7B batch-1 decode throughput on N B200s (BASELINE.json metric), with roofline and CPU baseline.
+"""bench.py — Mistral-7B batch-1 decode throughput on N B200s (the reference's headline metric), with roofline and CPU baseline.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--shape m7] [--wtype q8_0] [--ctx 4096]
 
 A "step" is one decoded token: one pass of the hot path (embed -> 32 x [norm+QKV+rope+KV, attention, Wo+residual,
-norm+W1|W3+GLU, W2+residual] -> norm+classifier).  The workload is BASELINE config[1]: Mistral-7B-v0.2 architecture,
+norm+W1|W3+GLU, W2+residual] -> norm+classifier).  The workload: Mistral-7B-v0.2 architecture,
 random-init weights N(0, 0.02^2) quantised to q8_0 with the reference's own quantiser rules, batch 1, 4k context; the K
 timed tokens sit at positions spread uniformly over [0, ctx) (the fp16 KV ring is fully allocated, so attention streams
 kv_len rows of it exactly as a hydrated cache would).  Weights (7.5 GB) are far larger than L2 (126 MB), so every step
@@ -14,7 +14,7 @@ streams them from HBM; no L2 flush is needed between steps.
 `e2e`    : the same loop through the public API (Model.forward + Sampler.sample_argmax on HOST logits): every step
            copies the step's inputs (token, position: one 32-byte StepParams from pinned memory) host->device and the
            logits (vocab * 4 bytes) device->host, and is timed by the wall clock around the synchronous calls.
-`--impl reference` : the reference's CPU path (oracle/ restatement; the reference C++ does not build on x86, DESIGN.md)
+`--impl reference` : the reference's CPU path (oracle/ restatement; the reference C++ does not build on x86)
            on all host cores, same model, one token per step.
 N > 1    : tensor parallel over N GPUs (one process per GPU, strong scaling: same model, sharded).
 """
@@ -93,7 +93,7 @@ def measured_peak_gbs() -> tuple:
             return float(json.load(open(p))["hbm_gbs"]), "measured (MEASURED_PEAKS.json)"
         except Exception:
             pass
-    return 6650.0, "fallback (B200_PROFILING.md)"
+    return 6650.0, "fallback (measured earlier on a B200)"
 
 
 def positions_for(steps: int, ctx: int) -> list:
@@ -144,7 +144,7 @@ def build_model_streaming(cfg_full: dict, cfg: dict, wtype, seed: int, keep_host
 
 
 def run_reference(args):
-    """The reference's CPU implementation of the path (oracle port; DESIGN.md explains why the C++ cannot be built
+    """The reference's CPU implementation of the path (oracle port: the C++ needs ARM NEON and cannot be built
     here) on all host cores.  Under torchrun only rank 0 works."""
     if int(os.environ.get("RANK", "0")) != 0:
         return
@@ -203,18 +203,18 @@ def measured_peak_tflops() -> tuple:
             return float(d["bf16_tflops"]), float(d["bf16_tflops_sustained"]), "measured (MEASURED_PEAKS.json)"
         except Exception:
             pass
-    return 1590.0, 1400.0, "fallback (B200_PROFILING.md)"
+    return 1590.0, 1400.0, "fallback (measured earlier on a B200)"
 
 
 def gemm_flops(cfg: dict, T: int, with_cls: bool = True) -> float:
-    """2*T*(weights that enter a GEMM): the seven per-layer contractions + the classifier (SURVEY.md 8d: 2*T*7.11e9 for m7)."""
+    """2*T*(weights that enter a GEMM): the seven per-layer contractions + the classifier (2*T*7.11e9 for m7)."""
     q_dim, kv_dim = cfg["n_heads"] * cfg["head_dim"], cfg["n_kv_heads"] * cfg["head_dim"]
     per_layer = cfg["dim"] * (q_dim + 2 * kv_dim) + q_dim * cfg["dim"] + 3 * cfg["dim"] * cfg["hidden_dim"]
     return 2.0 * T * (cfg["n_layers"] * per_layer + (cfg["vocab_size"] * cfg["dim"] if with_cls else 0))
 
 
 def perplexity_summary(model, cfg, capi, n_tok: int) -> dict:
-    """Device-timed tok/s of the batched perplexity pass (BASELINE config[2]) in both operand modes + its accuracy against
+    """Device-timed tok/s of the batched perplexity pass in both operand modes + its accuracy against
     the decode kernels, on the model bench.py already holds.  Full line: `bench.py --workload perplexity`."""
     import torch
     from xalm_b200.model import InferenceState
@@ -255,7 +255,7 @@ def gemm_traffic(args, n_tok):
 
 
 def run_perplexity_workload(args):
-    """perplexity mode on a 4k-token synthetic input.  A step = one batched pass over `--tokens` positions
+    """Perplexity mode on a 4k-token synthetic input.  A step = one batched pass over `--tokens` positions
     (every position's logits + softmax-at-target), weights resident.  `value` device-timed; `e2e` through Model.prefill with
     host tokens in and host probabilities out.  --impl reference: the oracle's token-at-a-time loop on a bounded sample."""
     from xalm_b200 import synth, types as T, xalm_file as X
@@ -754,7 +754,7 @@ def main():
                     help="also time steps at positions >= ctx: the KV ring is full (kv_len = ctx), 2 attention sinks active (infer.cpp:608-613)")
     ap.add_argument("--no-prefill", action="store_true", help="skip the perplexity-mode summary appended to the decode line at N=1")
     ap.add_argument("--workload", default="decode", choices=["decode", "perplexity", "families", "bolovik", "duletar", "kubolorn", "mizerax", "pavitar"],
-                    help="decode = BASELINE config[1] (the headline metric); perplexity = config[2]: batched prefill of a 4k-token input; "
+                    help="decode = the headline metric; perplexity: batched prefill of a 4k-token input; "
                          "families = prefill and one-token-step throughput of the Nabalix family beside the Llama family at equal layer sizes; "
                          "bolovik = the same for the Bolovik family beside the Nabalix and Llama families; "
                          "duletar = the same for the Duletar family beside the Bolovik family; "
@@ -998,7 +998,7 @@ def main():
     if parity is not None:
         line["parity"] = parity
 
-    # ---- BASELINE config[2] beside it (N = 1): the batched prefill / perplexity pass on the same resident model ----
+    # ---- beside it (N = 1): the batched prefill / perplexity pass on the same resident model ----
     if world == 1 and not args.no_prefill and cfg["head_dim"] in (64, 128):
         try:
             line["perplexity_mode"] = perplexity_summary(model, cfg, capi, min(4096, ctx))

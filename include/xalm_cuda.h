@@ -2,7 +2,7 @@
  * xalm_cuda.h — C ABI of the B200 (sm_100a) `-d cuda` backend for Xalm's transformer forward pass.
  *
  * The reference has no plugin/FFI interface; its only device seam is three C++ call sites
- * (SURVEY.md §8b).  Each entry point below names the reference interface it stands in for.
+ * Each entry point below names the reference interface it stands in for.
  * Paths are relative to the reference tree (jubruckne/Xalm).
  *
  *   - nothing but POD, raw pointers and sizes crosses this boundary; no exceptions: every call
@@ -24,7 +24,7 @@ extern "C" {
 
 /* Tensor element types.  0..9: `Type` ids, src/types.h:505-514.  1007..1012: the gguf-style block
  * formats convert.py writes (XType values, convert.py:56-61; layouts quants.py:281-464,638-683) which
- * the reference runtime never learned to load (SURVEY.md §0.4).  2007: convert.py's qi8 (:538-551). */
+ * the reference runtime never learned to load.  2007: convert.py's qi8 (:538-551). */
 enum xalm_type {
 	XALM_UNKNOWN = 0,
 	XALM_F32 = 1, XALM_F16 = 2, XALM_BF16 = 3,
@@ -79,7 +79,7 @@ int xalm_cuda_type_info(int type_id, int* block_elems, int* block_bytes);
 
 /* ---- model lifecycle: Model::from_xalm (model.cpp:48-118) + the commented-out
  *      `model.cuda(); state.cuda();` (main.cpp:211-212, :283-284) ------------------------------ */
-/* tp_rank/tp_size: tensor-parallel shard this handle holds (1 GPU: 0/1).  Sharding per SURVEY.md §8e. */
+/* tp_rank/tp_size: tensor-parallel shard this handle holds (1 GPU: 0/1). */
 int xalm_cuda_create(const xalm_config* cfg, int device, int tp_rank, int tp_size, xalm_cuda_model** out);
 /* One call per tensor of model.cpp:83-114 ("embed.weight", "l.{i}.attn.{norm,q,k,v,down}.weight",
  * "l.{i}.mlp.{norm,gate,down,up}.weight", "output.norm.weight", "output.weight").  `shape` is the ELEMENT
@@ -280,7 +280,7 @@ int xalm_cuda_latent_window(float* out, const float* q, const float* cache, cons
 int xalm_cuda_moe_chosen(float* x_io, float* out_pairs, int* idx, float* wgt, const float* h, const float* w_router, const float* bias, const float* w_gate,
                          const float* w_up, const float* w_down, const float* base, int base_gated, int T, int K, int E, int top, int ff, int w_bf16);
 
-/* Tensor parallel plumbing (no reference analogue; north star).  Rank 0 makes an id, the host side ships it to
+/* Tensor parallel plumbing (no reference analogue).  Rank 0 makes an id, the host side ships it to
  * the other ranks (torch.distributed / MPI / a file), every rank calls comm_init before finalize. */
 #define XALM_COMM_ID_BYTES 128
 int xalm_cuda_comm_unique_id(void* id128);
@@ -318,7 +318,7 @@ int xalm_cuda_sync(xalm_cuda_model* m);
  * xalm_cuda_logits_host then keeps what it held.  Synchronous.  Tensor-core operands are fp16 with fp32 accumulation; the "prefill_split"
  * knob (xalm_cuda_tune) picks how fp32 values enter them: 3 (default) = hi+lo fp16 pairs for activations, weights and the
  * attention operands (3 MMAs per product; 32-layer 4k-token logits within ~1e-3 of the token-at-a-time path), 2 = pairs
- * for activations only, 1 = plain fp16 (fastest; ~4e-2 at that depth).  1e-2. */
+ * for activations only, 1 = plain fp16 (fastest; ~4e-2 at that depth).  Tolerance: 1e-2. */
 int xalm_cuda_prefill(xalm_cuda_model* m, const int* tokens, int n, int pos0, int want_logits, float* logits_host,
                       const int* targets, float* probs_host);
 /* Enqueue only (no read-back, no host sync) — bench.py's device-timed leg. */
@@ -327,7 +327,8 @@ int xalm_cuda_prefill_async(xalm_cuda_model* m, const int* tokens, int n, int po
 float* xalm_cuda_logits_host(xalm_cuda_model* m);
 /* Model::active_bytes(pos) (model.cpp:12-35), 64-bit, per-format bytes; this rank's shard only. */
 int xalm_cuda_active_bytes(xalm_cuda_model* m, long long pos, long long* bytes);
-/* Kernels launched by the last forward (bench.py's gpu_launches). */
+/* Kernels launched by the last forward (bench.py's gpu_launches): the token's own.  The two kernels around a waited step that take its parameters in and its logits
+ * out, where copies would be, are not counted. */
 int xalm_cuda_last_launch_count(xalm_cuda_model* m, int* n);
 
 /* ---- state read-back for parity tests (InferenceState accessors model.h:124-139, Block KV model.h:222-223) -- */
@@ -359,7 +360,7 @@ int xalm_cuda_ffn(float* xout, const float* x, const void* w1, const void* w2, c
  * "tail_prefetch_mb", "attn_cluster", ...); an XALM_<KEY> environment variable overrides the stored value.  Takes effect for graphs captured
  * afterwards; "mma" (which matvec kernel and device layout the integer formats take: 0 = dp4a + unit layout, 1 = tensor-core mma +
  * fragment tiles (the default), 2 = mma for the 4/5-bit formats and, under tensor parallelism, the 8-bit ones, dp4a for the rest) and
- * "mega" are read when a matrix is uploaded; "attn_cluster" = 0 gives every step's attention to the split-K kernel. */
+ * "mega" are read when a matrix is uploaded; "attn_cluster" (0 gives every step's attention to the split-K kernel) when a model is finalized. */
 int xalm_cuda_tune(const char* key, int value);
 
 /* In-kernel timeline (there is no nsys here): with out == NULL start recording up to n_records kernels; with out != NULL

@@ -5,20 +5,20 @@
 // __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs may
 // load this library.  Nothing under xalm_b200/ links, imports or calls it.
 //
-// Parity status: PINNED TO THE REFERENCE ITSELF.  The reference ships no tests / golden vectors (SURVEY.md §0.10), but
+// Parity status: PINNED TO THE REFERENCE ITSELF.  The reference ships no tests / golden vectors, but
 // its own C++ forward pass (src/infer.cpp, model.cpp, tensor.cpp, sampler.cpp, tokenizer.cpp) compiles untouched behind
-// the NEON / <print> shims of oracle/ref_shim/ (recipe: oracle/Makefile.ref -> oracle/_ref/libxalm_ref.so, dev container
-// only).  tests/golden/ref_fwd_*.npz are logits, greedy tokens, sampler probabilities and KV-cache bits produced by that
+// the NEON / <print> shims of oracle/ref_shim/ (recipe: oracle/Makefile.ref -> oracle/_ref/libxalm_ref.so, where the
+// reference's tree is).  tests/golden/ref_fwd_*.npz are logits, greedy tokens, sampler probabilities and KV-cache bits produced by that
 // library (generator: tests/golden/make_ref_forward.py); tests/test_reference_forward.py requires this restatement to
 // reproduce them, and compares it with the live library when it is present.  Also pinned (tests/test_oracle_*.py):
-//   * block-quant dequant  == /root/reference/quants.py  (bit-exact, golden vectors)
+//   * block-quant dequant  == quants.py  (bit-exact, golden vectors)
 //   * fp8 decode           == torch float8 casts except the NaN/Inf codes the
 //                             reference treats as finite (types.h:302-314)
 //   * .xalm layout         == files written by /root/reference/convert.py
 //
 // Every function cites the reference file:line it restates.  All paths are
 // relative to /root/reference/.  Arithmetic is fp32 unless stated, fp16 KV cache,
-// exactly as the reference (SURVEY.md §0.5).
+// exactly as the reference.
 // =============================================================================
 #include <algorithm>
 #include <cfloat>
@@ -96,7 +96,7 @@ static inline float get_float(int t, const void* data, size_t i) {
 
 // ---- block formats: one block -> block_size floats -------------------------------
 // quants.py:302-313 (Q4_0), :337-350 (Q4_1), :376-393 (Q5_0), :419-438 (Q5_1),
-// :458-464 (Q8_0), :664-683 (TQ1_0).  Layouts: SURVEY.md Appendix B.
+// :458-464 (Q8_0), :664-683 (TQ1_0).
 static void dequant_block(int t, const uint8_t* b, float* y) {
 	switch (t) {
 		case T_Q8_0: {
@@ -454,7 +454,7 @@ int orc_forward(orc_model* m, int token, int pos, int mode) {
 		if (!type_block(m->embed.type, &bs, &ts)) return 3;
 		if (bs == 1) {
 			for (int i = 0; i < c.dim; ++i) m->x[i] = get_float(m->embed.type, m->embed.data, (size_t) token * c.dim + i);
-		} else { // block formats: extension (the reference cannot load them, SURVEY.md §0.4)
+		} else { // block formats: extension (the reference cannot load them)
 			const uint8_t* row = (const uint8_t*) m->embed.data + (size_t) token * (c.dim / bs * ts);
 			row_dequant(m->embed.type, row, c.dim, m->x.data());
 		}
@@ -487,7 +487,7 @@ uint16_t* orc_kv(orc_model* m, int layer, int which) {
 	return which == 0 ? m->blocks[layer].key_cache.data() : m->blocks[layer].value_cache.data();
 }
 
-// ---- Sampler: sampler.cpp:3-30 — note the FLT_MIN (not lowest) seed, SURVEY.md §0.8 -----------
+// ---- Sampler: sampler.cpp:3-30 — note the FLT_MIN (not lowest) seed -----------
 float orc_sample_prob(const float* logits, int vocab_size, int index) {
 	float max_val = std::numeric_limits<float>::min();
 	for (int i = 0; i < vocab_size; ++i) if (logits[i] > max_val) max_val = logits[i];

@@ -1,11 +1,11 @@
 #!/usr/bin/env python
 """Generate the golden fixtures under tests/golden/ from the REFERENCE's own executable Python.
 
-Run in the dev container only (it needs /root/reference, which does not exist on the GPU box):
+Needs the reference's tree in /root/reference:
 
     python tests/golden/make_golden.py
 
-What it pins (SURVEY.md §8c — the reference has no tests of its own, so these are the only
+What it pins (the reference has no tests of its own, so these are the only
 executable pins there are):
 
   blocks_<fmt>.npz   /root/reference/quants.py quantize() and dequantize() for the six block formats

@@ -2,7 +2,7 @@
 """Golden vectors of the REFERENCE's own forward pass (jubruckne/Xalm src/infer.cpp, model.cpp, sampler.cpp), generated by
 running the unmodified reference C++ — compiled by oracle/Makefile.ref behind the NEON / <print> shims — on small checkpoints.
 
-Run in the dev container only (needs /root/reference):
+Needs the reference's tree in /root/reference:
 
     make -f oracle/Makefile.ref && python tests/golden/make_ref_forward.py
 

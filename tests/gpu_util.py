@@ -9,7 +9,7 @@ from xalm_b200 import types as T
 from xalm_b200 import xalm_file as X
 from xalm_b200.model import InferenceState, Model, Sampler
 
-LOGIT_TOL = 1e-2      # north star: logits within max-abs 1e-2 of the reference CPU path
+LOGIT_TOL = 1e-2      # logits within max-abs 1e-2 of the reference CPU path
 
 
 def bits(a):

@@ -1,4 +1,4 @@
-"""Dequantised weight values must be BIT-EXACT (north star): the dequant entry point, and the weights the hot
+"""Dequantised weight values must be BIT-EXACT: the dequant entry point, and the weights the hot
 matvec kernel effectively multiplies by (extracted with one-hot activations), against the CPU oracle / quants.py."""
 import os
 

@@ -213,7 +213,7 @@ def test_sampler_quirk_on_device_logits():
 
 @pytest.mark.parametrize("shape,wtype,layers", [("l70", "q8_0", 1), ("l8", "q4_0", 2)])
 def test_baseline_shapes_depth_reduced(shape, wtype, layers):
-    """BASELINE configs 4/5 at reduced depth (SURVEY.md §7 '70B parity'): Llama-70B dims (8192/28672, 64 q heads on 8 kv heads,
+    """Large shapes at reduced depth: Llama-70B dims (8192/28672, 64 q heads on 8 kv heads,
     128k vocab) and Llama-8B dims, full width — exercises GQA 8:1, 28672-long rows (activations read through L1), big vocab."""
     config, om, gm = synth_pair(shape, wtype, seed=3, std=0.02, n_layers=layers)
     prompt = [int(t) for t in np.random.default_rng(1).integers(3, config["vocab_size"], size=6)]
@@ -224,7 +224,7 @@ def test_baseline_shapes_depth_reduced(shape, wtype, layers):
 
 
 def test_full_size_mistral_7b_q8_0_parity():
-    """BASELINE config 2 at FULL size (32 layers, 7.2 B weights, q8_0): the CPU oracle manages ~8 tok/s on the GPU box's
+    """Mistral-7B at FULL size (32 layers, 7.2 B weights, q8_0): the CPU oracle manages ~8 tok/s on 16 host
     cores, so direct parity is affordable: 4 prompt tokens + 12 greedy steps, token-exact, logits within 1e-2, and the
     ring/sink path exercised right after (-T is not needed: positions stay < 4096)."""
     config, om, gm = synth_pair("m7", "q8_0", seed=0, std=0.02)
@@ -232,7 +232,7 @@ def test_full_size_mistral_7b_q8_0_parity():
     otoks, gtoks, maxdiff, margin = greedy_compare(config, om, gm, [1, 415, 28747, 1824], 12)
     assert maxdiff <= LOGIT_TOL, f"logits differ by {maxdiff}"
     assert otoks == gtoks, f"greedy tokens diverge (min margin {margin})"
-    # algorithmic bytes: Model::active_bytes == SURVEY.md §8d formula (7.555 GB + 0.131 MB per cached position)
+    # algorithmic bytes: Model::active_bytes == the formula of model.cpp:12-35 (7.555 GB + 0.131 MB per cached position)
     from xalm_b200.model import active_bytes_formula
     assert gm.active_bytes(0) == active_bytes_formula(config, 34 / 32, 0) == om.active_bytes(0)
     assert abs(gm.active_bytes(0) / 1e9 - 7.555) < 0.01

@@ -1,8 +1,8 @@
-"""Batched prefill / perplexity on the tcgen05 path (BASELINE config 3) against the oracle and the token-at-a-time path.
+"""Batched prefill / perplexity on the tcgen05 path against the oracle and the token-at-a-time path.
 
 * the GEMM alone, every weight format: out = a . W^T with W bit-exactly dequantised (capi.dequant is pinned to the oracle
   in test_gpu_formats.py) and both operands rounded to fp16 exactly as the kernel rounds them -> tight tolerance;
-* the whole forward: logits of every position vs the CPU oracle run token by token (north star: max-abs 1e-2),
+* the whole forward: logits of every position vs the CPU oracle run token by token (max-abs 1e-2),
   KV cache contents, perplexity probabilities (Sampler::sample_prob), chunked prefill, prefill followed by decode.
 """
 import numpy as np
@@ -186,7 +186,7 @@ def test_prefill_single_token_and_full_cache():
 
 
 def test_prefill_4096_tokens_vs_oracle():
-    """BASELINE config 3 at its full length: 4096 positions in one pass through attn_tc_kernel (head_dim 128, GQA 8:2) and the
+    """The full length: 4096 positions in one pass through attn_tc_kernel (head_dim 128, GQA 8:2) and the
     tcgen05 GEMMs, against the ORACLE run token by token (not against the repo's own decode kernels): logits at 40 positions
     spread over the sequence plus the last 8, max-abs 1e-2, and Sampler::sample_prob at every position."""
     config, om, gm = synth_pair("small", "q8_0", seed=3, std=0.03, n_layers=2, max_seq_len=4096)

@@ -51,7 +51,7 @@ def test_tp_shard_aware_upload(world, wtype, shape):
 
 
 def test_tp2_long_hydrate_prompt():
-    """120 HYDRATE tokens before the first logits: 120 drained exchanges in a row (the protocol hole of round 1 was here)."""
+    """120 HYDRATE tokens before the first logits: 120 drained exchanges in a row (a protocol without the drain hangs or overwrites here)."""
     if _ngpu() < 2:
         pytest.skip("needs 2 GPUs")
     env = dict(os.environ, XALM_TP_PROMPT="120")

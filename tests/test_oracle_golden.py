@@ -52,7 +52,7 @@ def test_scalar_formats():
     bf = (x.view(np.uint32) >> 16).astype(np.uint16)
     assert np.array_equal(oracle.dequant(T.BF16.id, bf.view(np.uint8), 512), (bf.astype(np.uint32) << 16).view(np.float32))
     q = np.arange(-128, 128, dtype=np.int8)
-    # types.h:423-424: (1.f/100.f) * q — NOT q / 100 (70 of 256 codes differ, SURVEY.md §7)
+    # types.h:423-424: (1.f/100.f) * q — NOT q / 100 (70 of 256 codes differ)
     want = np.float32(1.0) / np.float32(100.0) * q.astype(np.float32)
     assert np.array_equal(oracle.dequant(T.Q8.id, q.view(np.uint8), 256), want)
     assert (want != q.astype(np.float32) / np.float32(100.0)).sum() > 0

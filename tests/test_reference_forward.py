@@ -5,8 +5,8 @@ reference C++ (src/infer.cpp, model.cpp, sampler.cpp compiled by oracle/Makefile
 
   * CPU: the oracle restatement (oracle/xalm_oracle.cpp) must reproduce them — same greedy tokens, logits within fp32
     reassociation noise, identical KV bits up to libm/accumulation-order rounding of single entries.
-  * GPU: the CUDA path must reproduce them — token-exact, logits within the north star's 1e-2.
-  * when oracle/_ref/libxalm_ref.so is present (dev container), the oracle is also compared with the live reference on a
+  * GPU: the CUDA path must reproduce them — token-exact, logits within 1e-2.
+  * when oracle/_ref/libxalm_ref.so is present, the oracle is also compared with the live reference on a
     checkpoint no fixture covers.
 """
 import ctypes as C
@@ -111,7 +111,7 @@ def test_cuda_reproduces_the_reference(name, tmp_path):
         nxt = sampler.sample_argmax(state)
         assert nxt == toks[n_prompt + step], f"{name}: greedy token {step} differs from the reference CPU path"
         model.forward(state, nxt, n_prompt + step, 1)
-    assert worst <= 1e-2, f"{name}: logits differ from the reference by {worst}"
+    assert worst <= 1e-2, f"{name}: logits differ from the reference by {worst}"                            
     for l in range(config["n_layers"]):
         for which, nm in ((0, "k"), (1, "v")):
             ref_bits = g[f"{nm}_{l}"]

@@ -1,4 +1,4 @@
-"""The fused tensor-parallel exchange (matvec_tma.cuh, DESIGN.md §7) as a protocol, checked on the CPU.
+"""The fused tensor-parallel exchange (matvec_tma.cuh) as a protocol, checked on the CPU.
 
 Every rank runs   push(0), recv(0), push(1), recv(1), ...   where push(i) writes {value, tag = base + i + 1} words into slot i & 1
 of EVERY rank's receive area (posted NVLink stores, no flag, no fence) and recv(i) polls its own slot until all P sources carry

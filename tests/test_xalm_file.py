@@ -80,7 +80,7 @@ def _oracle_from_file(path, context=0, acc_mode=1):
 def test_oracle_runs_convert_py_checkpoints_through_ring_buffer(golden_dir):
     """10 greedy steps with max_seq_len=6: ring buffer + 2 attention sinks + per-step sink re-rotation are
     all active from pos 6 on (infer.cpp:416-431, 608-613).  f16 / q8_0 / f8 checkpoints of the same source
-    weights must give finite logits and start with the same greedy tokens (SURVEY.md §8c probe)."""
+    weights must give finite logits and start with the same greedy tokens."""
     seqs = {}
     for t in ("f16", "q8_0", "f8_e4m3"):
         f, c, m = _oracle_from_file(os.path.join(golden_dir, f"tiny_{t}.xalm"), context=6)
@@ -106,7 +106,7 @@ def test_oracle_accumulation_modes_bound_the_noise(golden_dir):
         out[mode] = lg
         m.close(); f.close()
     # fp32 reassociation noise is ~1e-6, but one fp16 KV element rounding the other way (1 fp16 ulp) feeds
-    # back at the 1e-4 level (SURVEY.md §7 "token-exact greedy"): the 1e-2 logit tolerance covers both.
+    # back at the 1e-4 level: the 1e-2 logit tolerance covers both.
     assert np.max(np.abs(out[0] - out[2])) < 2e-3 and np.max(np.abs(out[1] - out[2])) < 2e-3
 
 

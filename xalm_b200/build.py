@@ -1,7 +1,7 @@
 """Build recipes: the CUDA C-ABI library (sm_100a only) and the C++ host executable.
 
-Everything is built IN-TREE (xalm_b200/libxalm_cuda.so, xalm_b200/xalm_main) so the artefacts travel to the
-GPU box with the repo snapshot.  nvcc cross-compiles without a GPU.
+Everything is built IN-TREE (xalm_b200/libxalm_cuda.so, xalm_b200/xalm_main) so the artefacts travel with
+a copy of the tree.  nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 

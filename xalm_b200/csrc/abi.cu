@@ -62,8 +62,8 @@ static std::map<std::string, int>& tuning() {
 	    {"tp_fused", 1},     // tensor parallel: fuse the two per-layer exchanges into the matvec kernels (push over NVLink + receive in the next prologue)
 	    {"idp_per_sm", 2},
 	    {"mma", 1},         // integer formats on the tensor-core matvec (fragment tiles + mma.sync int8, matvec_mma.cuh): 0 = never (unit layout + dp4a), 1 = all six,
-	                        // 2 = the 4/5-bit formats, and the 8-bit ones under tensor parallelism.  q8_0 per token, 2 -> 1: 7B at position 3001 1872 -> 1816 us, four
-	                        // layers of width 1024 138 -> 114, of width 2048 165 -> 143 (the dp4a kernel gives a lane a whole block: rows of 1024 keep a quarter of its lanes busy)
+	                        // 2 = the 4/5-bit formats, and the 8-bit ones under tensor parallelism.  q8_0 per token, 2 -> 1: 7B at position 3001 1864 -> 1800 us, four
+	                        // layers of width 1024 129 -> 108, of width 2048 132 -> 120 (the dp4a kernel gives a lane a whole block: rows of 1024 keep a quarter of its lanes busy)
     {"idp_ng", 0},      // consumer groups per CTA of the integer-dot matvec: 0 = by format, 2 = one 17-warp CTA per SM, 1 = two 9-warp CTAs
 	    {"tail_prefetch_mb", 8}, // each decode kernel pulls this many MB of the NEXT kernel's first weights into L2 once its own loads are issued
 	    {"prefill_split", 3}, // batched prefill operand precision: 1 = fp16 x fp16 (fastest; logits drift ~4e-2 over 32 layers), 2 = hi+lo fp16

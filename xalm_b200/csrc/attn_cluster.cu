@@ -9,9 +9,9 @@
 // of 16 products start from zero and are added in round-to-nearest as a tree, since the tensor cores' own additions truncate.  Distance from float64 over
 // 20 to 3002 keys and queries of deviation 0.3, 1 and 3: 0.99 times the split kernel's (0.86 to 1.13).  A warp that meets a score or a sum that is not finite
 // does its keys again in fp32 FMAs, so that an infinity goes where it goes there (its zero planes would spread it); a NaN score, wherever its key lies, makes its head NaN.
-// A step's attention in the graph, split kernel before: 7B at position 3001 12.3 -> 9.5 us; per token, with it and without: 7B q8_0 1938 -> 1870 us, 8 layers of
-// q4_0 at 700 458 -> 428, 6 layers of bf16 at width 2048 and position 1777 275 -> 256.  Tried and not faster: rings of the neighbouring products cut
-// so that this kernel's CTAs fit beside them (no difference).
+// Per token, with the split kernel and with this one: 32 layers of q8_0 of width 4096 at position 3001 1854 -> 1800 us, 8 of q4_0 at 700 398 -> 374, 6 of bf16 at width 2048
+// and position 1777 267 -> 249, 4 of q8_0 at width 1024 116 -> 108.  Tried and not faster: rings of the neighbouring products cut so that this kernel's CTAs fit beside
+// them (no difference).
 #define XALM_SECONDARY_TU
 #include "attention.cuh"
 #include "family.h"

@@ -7,7 +7,7 @@
 //     16-byte-aligned planes, same byte count as on disk) and, per format, the 16-byte "chunk" a lane loads
 //     with one 128-bit request plus the fused dequant·x arithmetic the matvec kernel runs on it.
 //
-// Bit-exactness notes (SURVEY.md §7): an f16 scale (11 significant bits) times a <=8-bit integer is exact in
+// Bit-exactness notes: an f16 scale (11 significant bits) times a <=8-bit integer is exact in
 // fp32, so d*q never rounds and d*q+m rounds once whether or not it is fused; Q8 multiplies by fp32(1/100);
 // fp8 codes that IEEE-style decoders call NaN/Inf are ordinary finite numbers in the reference.
 #pragma once
@@ -88,7 +88,7 @@ __device__ __forceinline__ float decode_scalar(int t, const uint8_t* p, size_t i
 
 __device__ __forceinline__ float ld_f16_unaligned(const uint8_t* p) { return f16_bits_to_f32((uint16_t) (p[0] | (p[1] << 8))); }
 
-// element j of an on-disk block (quants.py:302-313, 337-350, 376-393, 419-438, 458-464, 664-683; SURVEY App. B)
+// element j of an on-disk block (quants.py:302-313, 337-350, 376-393, 419-438, 458-464, 664-683)
 __device__ inline float decode_block_elem(int t, const uint8_t* b, int j) {
 	switch (t) {
 		case XALM_Q8_0: return __fmul_rn((float) (int8_t) b[2 + j], ld_f16_unaligned(b));

@@ -52,7 +52,7 @@ namespace {
 double now_s() { return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count(); }
 
 double hbm_peak_gbs() {
-	// measured on this pool (MEASURED_PEAKS.json); XALM_HBM_PEAK_GBS overrides
+	// a measured copy on a B200; XALM_HBM_PEAK_GBS overrides
 	if (const char* e = getenv("XALM_HBM_PEAK_GBS")) return atof(e);
 	return 6538.3;
 }

@@ -3,11 +3,11 @@
 // error behaviour as /root/reference/src/{types,tensor,xalm,model,sampler,tokenizer}.h) with the compute behind the
 // C ABI of include/xalm_cuda.h.  Portable C++20 (g++ 13, x86-64): no NEON, no <print>.
 //
-// What changes relative to the reference, by design (SURVEY.md §8b):
+// What changes relative to the reference, by design:
 //   * Device gains CUDA (model.h:21-23); Model::cuda() / InferenceState::cuda() exist (main.cpp:211-212 has them
 //     commented out); Model::forward on a model that is not on the device throws — there is no CPU path here.
 //   * Type::parse also accepts the block formats convert.py writes (q4_0 q4_1 q5_0 q5_1 q8_0 tq1_0, qi8) and the
-//     loader maps their byte-shaped headers back to element shapes (SURVEY.md §0.4).
+//     loader maps their byte-shaped headers back to element shapes.
 #pragma once
 #include <cfloat>
 #include <cstdint>
@@ -201,7 +201,7 @@ private:
 	int tp_size_ = 1;
 };
 
-// ---- Sampler (sampler.h / sampler.cpp): host-side, unchanged semantics incl. the FLT_MIN seed (SURVEY.md §0.8) ---
+// ---- Sampler (sampler.h / sampler.cpp): host-side, unchanged semantics incl. the FLT_MIN seed ---
 struct Sampler {
 	int vocab_size;
 	explicit Sampler(const Config& config) noexcept : vocab_size(config.vocab_size) {}

@@ -1,8 +1,8 @@
 // quantize.cpp — host-side writers for the weight formats: fp32 rows -> on-disk bytes.
 //
-// Needed by the synthetic-checkpoint generator (BASELINE configs are random-init models that must be produced on
-// the GPU box, where the reference's Python is not available) and by Tensor::convert_to on the C++ host side.
-// Each quantiser reproduces /root/reference/quants.py *byte for byte* (tests/test_quantize.py checks that against
+// Needed by the synthetic-checkpoint generator (the benchmark's are random-init models that must be produced
+// where the reference's Python is not available) and by Tensor::convert_to on the C++ host side.
+// Each quantiser reproduces quants.py *byte for byte* (tests/test_quantize.py checks that against
 // fixtures generated by quants.py itself):
 //   Q8_0  quants.py:444-456   d = max|x|/127, round half away from zero (np_roundf, :108-112)
 //   Q4_0  quants.py:283-300   d = x[argmax|x|] / -8, trunc(float32(double(x)*double(1/d) + 8.5)), clip 0..15

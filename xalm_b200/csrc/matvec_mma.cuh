@@ -20,11 +20,14 @@
 // kernel returns the dequantised weight bit for bit (d*q exact, d*q+m rounds once).
 //
 // Bound: the 8-bit formats HBM (28672 x 4096 21.2 us, 19.7 with the multiplication left out), the 4-bit ones the consumers' issue slots and what they read
-// from shared memory (16.2 us, 12.0).  A record used to take biased weights, accumulator inits of 16 bytes and a branch around the limbs of unused
-// columns, 30 instructions of which 22 are left; 128 records a stage instead of 64 take the per-stage work off the 4-bit formats.  Back to back, buffers
-// beyond L2, before -> after: q4_0 28672 x 4096 17.6 -> 16.2 us, 4096 x 14336 11.4 -> 9.3, 4096 x 4096 5.0 -> 4.4; q8_0 28672 x 4096
-// 21.5 -> 21.2, 4096 x 14336 13.6 -> 12.5 (dp4a 22.9, 13.2).  Tried and not faster: the same in fp16 mma (twice the tensor instructions and wider
-// activations: 21.0 us), a warp's activations held in registers for two or four tiles (17.9, 19.1), 8 or 24 multiplying warps (16.6, 18.4).
+// from shared memory (16.4 us, 12.0).  A record used to take biased weights, accumulator inits of 16 bytes and a branch around the limbs of unused
+// columns, 30 instructions of which 22 are left; stages of 36 to 48 KB instead of 18 to 24 take the per-stage work off the 4- and 5-bit formats.  Back to back, buffers
+// beyond L2, us, before -> after (the 8-bit formats: the dp4a kernel, which they took on one GPU): norm + gate|up + GLU of 28672 x 4096 q4_0 18.7 -> 16.4, q4_1 19.8 -> 17.4,
+// q5_0 23.0 -> 21.6, q5_1 23.5 -> 21.0, q8_0 22.7 -> 21.3, q8 22.3 -> 20.0; residual of 4096 x 14336 11.6 -> 9.7, 12.1 -> 10.2, 13.3 -> 12.3, 14.1 -> 12.5, 12.7 -> 12.7,
+// 12.2 -> 11.8; of 4096 x 4096 5.1 -> 4.4, 5.4 -> 4.6, 5.7 -> 5.3, 5.9 -> 5.5, 5.7 -> 5.4, 5.7 -> 5.3.  Alone, fewer than 74 tiles of long 8-bit rows are the dp4a kernel's (1024 x 8192
+// 1.25 times as fast: twice the CTAs), but not in a step, where the next product's first stages are on their way (two layers of 8192 and 28672: 339 us with either, four
+// of 1024 and 4096 98 against 111).  Tried and not faster: the same in fp16 mma (twice the tensor instructions and wider activations), a warp's activations held in
+// registers for two or four tiles, 8 or 24 multiplying warps.
 //
 // Skeleton: as matvec_idp.cuh — persistent CTAs (one per SM), a producer warp streaming records into an mbarrier ring with ONE
 // cp.async.bulk per stage (a tile's records are contiguous), 16 consumer warps, rmsnorm prologue (1/rms applied to the row

@@ -369,8 +369,7 @@ int ensure_graph(SeqModel* m, int mode, bool io) {
 
 // one pass of n <= chunk tokens at the sequence's position; the logits (want) stay on the device
 // waits: the caller waits for the pass before it returns, so that a one-token step may take its inputs from pinned memory and leave its logits in
-// h_logits, one graph launch in all.  (Two copies from pageable memory before the graph and one behind it cost a step 10 us, copies inside it 4 us:
-// 48 steps of Bolovik 4096 13.00 -> 12.78 ms, of Pavitar 2048 12.07 -> 11.84.)
+// h_logits, one graph launch in all.  (Two copies from pageable memory before the graph and one behind it cost a step 10 us, copies inside it 4 us.)
 int run_pass(SeqModel* m, const int* tokens, int n, int want, bool waits = false) {
 	for (int i = 0; i < n; i++)
 		if (tokens[i] < 0 || tokens[i] >= m->vocab) return set_error(XALM_ERR_INVALID, "token %d out of range", tokens[i]);

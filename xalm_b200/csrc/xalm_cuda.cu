@@ -1068,7 +1068,7 @@ int xalm_cuda_comm_init(xalm_cuda_model* m, const void* id128) {
 	return XALM_OK;
 }
 
-// the rows / columns of tensor `piece` (full element shape er x ec) that rank R of P keeps (SURVEY.md 8e)
+// the rows / columns of tensor `piece` (full element shape er x ec) that rank R of P keeps
 static void shard_range_of(const xalm_cuda_model* m, int piece, int er, int ec, int* r0, int* r1, int* c0, int* c1) {
 	const int R = m->tp_rank;
 	*r0 = 0; *r1 = er; *c0 = 0; *c1 = ec;

@@ -321,7 +321,7 @@ def generate(model: "Model", state: "InferenceState", sampler: "Sampler", prompt
 
 
 def active_bytes_formula(c: dict, bytes_per_weight: float, pos: int, emb_bpw: float | None = None, norm_bytes: int = 4) -> int:
-    """SURVEY.md §8d: B(pos) = dim*b_emb + dim*b_norm + vocab*dim*b_cls + L*[2*dim*b_norm + (2*q_dim*dim + 2*kv_dim*dim +
+    """B(pos) = dim*b_emb + dim*b_norm + vocab*dim*b_cls + L*[2*dim*b_norm + (2*q_dim*dim + 2*kv_dim*dim +
     3*dim*hidden)*b_w + 2*min(max_seq_len,pos+1)*kv_dim*2]."""
     emb_bpw = bytes_per_weight if emb_bpw is None else emb_bpw
     q_dim, kv_dim = c["n_heads"] * c["head_dim"], c["n_kv_heads"] * c["head_dim"]

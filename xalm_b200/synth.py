@@ -1,9 +1,9 @@
-"""Synthetic random-init checkpoints for the BASELINE configs.
+"""Synthetic random-init checkpoints of the benchmark's model shapes.
 
 Weights ~ N(0, 0.02^2) from a counter-based generator (seeded, thread-count independent), norm weights 1.0,
 a byte-fallback tokenizer, cast/quantised to the requested format by the host library's writers
 (csrc/host/quantize.cpp — byte-identical to the reference's quants.py, see tests/test_quantize.py).
-Must run on the GPU box, which has neither the reference tree nor room to ship 7B-70B files.
+Needs neither the reference tree nor files of 7B to 70B weights.
 """
 from __future__ import annotations
 
@@ -21,13 +21,13 @@ from . import xalm_file as X
 _HOST = None
 
 SHAPES = {
-    # Mistral-7B-v0.2 (BASELINE configs 1-3)
+    # Mistral-7B-v0.2
     "m7": dict(dim=4096, hidden_dim=14336, head_dim=128, n_layers=32, n_heads=32, n_kv_heads=8, vocab_size=32000,
                max_seq_len=32768, rope_theta=1000000.0, arch="MistralForCausalLM"),
-    # Llama-3-8B style (config 4)
+    # Llama-3-8B style
     "l8": dict(dim=4096, hidden_dim=14336, head_dim=128, n_layers=32, n_heads=32, n_kv_heads=8, vocab_size=128256,
                max_seq_len=8192, rope_theta=500000.0, arch="LlamaForCausalLM"),
-    # Llama-3-70B style (config 5)
+    # Llama-3-70B style
     "l70": dict(dim=8192, hidden_dim=28672, head_dim=128, n_layers=80, n_heads=64, n_kv_heads=8, vocab_size=128256,
                 max_seq_len=8192, rope_theta=500000.0, arch="LlamaForCausalLM"),
     # small shapes for tests / smoke

@@ -1,4 +1,4 @@
-"""Tensor-parallel plan and plumbing (host side of SURVEY.md §8e; the reference has no parallelism at all).
+"""Tensor-parallel plan and plumbing (host side; the reference has no parallelism at all).
 
 The C ABI takes FULL tensors and keeps this rank's shard; `shard_ranges` states which (rows, element columns) that is so
 tests can check the plan and emulate it on the CPU.  `init_model_parallel` does the one exchange the backend needs from

@@ -2,7 +2,7 @@
 
 Ids 0..9 are the reference's `Type` ids (/root/reference/src/types.h:505-514); the block
 formats take the values convert.py gives them in `XType` (/root/reference/convert.py:56-61),
-since the reference C++ never assigned them an id (SURVEY.md §0.4).  `block`/`bytes` are
+since the reference C++ never assigned them an id.  `block`/`bytes` are
 quants.py's GGML_QUANT_SIZES (/root/reference/quants.py:45-77).
 """
 from __future__ import annotations

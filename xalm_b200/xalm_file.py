@@ -11,8 +11,7 @@ Layout (reader: /root/reference/src/xalm.h:90-192; writer: /root/reference/conve
                          (convert.py:1057-1108); "tokenizer.tokens" (U8, NUL-separated) last.
 
 Block-quantised tensors are stored as uint8 rows and carry their BYTE shape in the header
-(`[rows, cols/32*34]` for q8_0; quants.py:79-83).  The reference reader cannot load those
-(SURVEY.md §0.4); this one maps them back to element shapes through `types.XType.elem_shape`.
+(`[rows, cols/32*34]` for q8_0; quants.py:79-83).  The reference reader cannot load those; this one maps them back to element shapes through `types.XType.elem_shape`.
 """
 from __future__ import annotations
 
@@ -149,7 +148,7 @@ class XalmFile:
                 if size < 0:
                     raise ValueError("bad size")
                 if size == 0 or h + off + size > file_size:
-                    raise ValueError("offset out of range")  # stricter than xalm.h:112,173 (SURVEY App. C)
+                    raise ValueError("offset out of range")  # stricter than xalm.h:112,173
                 eshape = typ.elem_shape(shape)
                 n = 1
                 for s in eshape:
