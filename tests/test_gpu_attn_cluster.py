@@ -87,18 +87,30 @@ def test_many_kv_heads_are_the_split_kernels(hd, nh, nkv):
     assert not np.array_equal(*both(*inputs(hd, 100, nh // nkv * 8, 8, 2), hd, 100, nh // nkv * 8, 8))
 
 
+@pytest.mark.parametrize("graph", [1, 0])
 @pytest.mark.parametrize("cluster", [1, 0])
-def test_the_timeline_has_every_layers_attention(cluster):
+def test_the_timeline_has_every_layers_attention(cluster, graph):
+    """Of steps that were captured before it began to record as of others; and no step afterwards is another one."""
     capi.tune("attn_cluster", cluster)
     config, om, gm = synth_pair("small", "q8_0", seed=1, std=0.03)   # four query heads per kv head
     capi.tune("attn_cluster", 1)
-    state = InferenceState(config)
-    gm.forward(state, 5, 0, 1)
-    capi.timeline_start(200)
-    gm.forward(state, 6, 1, 1)
-    rec = capi.timeline_stop(200)
-    at = rec[rec[:, 0] == 300].astype(np.int64)
-    assert len(at) == config["n_layers"]
-    assert np.all(at[:, 1] <= at[:, 2]) and np.all(at[:, 2] <= at[:, 3]) and np.all(at[1:, 1] > at[:-1, 1])
-    capi.timeline_start(0)
+    capi.tune("graph", graph)
+    try:
+        state, logits = InferenceState(config), []
+        for again in range(2):
+            gm.forward(state, 5, 0, 1)
+            capi.timeline_start(400)
+            for call in (lambda: gm.forward(state, 6, 1, 1), lambda: (gm.forward_async(6, 1, 1), gm.sync())):
+                call()
+                logits.append(gm.read_state(capi.S_LOGITS, config["vocab_size"]))
+            rec = capi.timeline_stop(400)
+            at = rec[rec[:, 0] == 300].astype(np.int64)
+            assert len(at) == 2 * config["n_layers"]
+            assert np.all(at[:, 1] <= at[:, 2]) and np.all(at[:, 2] <= at[:, 3]) and np.all(at[1:, 1] > at[:-1, 1])
+        gm.forward(state, 6, 1, 1)
+        logits.append(state.logits().copy())
+        assert all(np.array_equal(a, logits[0]) for a in logits)
+    finally:
+        capi.tune("graph", 1)
+        capi.timeline_start(0)
     gm.close(); om.close()

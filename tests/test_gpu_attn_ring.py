@@ -53,3 +53,23 @@ def test_steps_in_flight(nh, nkv):
         kv.append([gm.read_kv(layer, which).copy() for layer in range(4) for which in (0, 1)] + [gm.read_state(capi.S_LOGITS, config["vocab_size"])])
     assert all(np.array_equal(a, b) for a, b in zip(*kv))
     gm.close(); om.close()
+
+
+@pytest.mark.parametrize("nh,nkv", [(8, 2), (8, 1)])
+def test_graph_and_programmatic_launches_change_no_bit(nh, nkv):
+    outs = []
+    try:
+        for graph, pdl in ((1, 1), (0, 1), (1, 0), (0, 0)):
+            capi.tune("graph", graph)
+            capi.tune("pdl", pdl)
+            config, om, gm = synth_pair("tiny", "q8_0", seed=6, std=0.06, context=20, n_heads=nh, n_kv_heads=nkv, head_dim=32, n_layers=3)
+            state, seq = InferenceState(config), []
+            for pos, tok in enumerate([1, 84, 61, 35, 90, 107, 100, 119, 7, 9, 300, 2] * 3):
+                gm.forward(state, tok, pos, 1)
+                seq.append(state.logits().copy())
+            outs.append(np.stack(seq))
+            gm.close(); om.close()
+    finally:
+        capi.tune("graph", 1)
+        capi.tune("pdl", 1)
+    assert all(np.array_equal(outs[0], o) for o in outs[1:])

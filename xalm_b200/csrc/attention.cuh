@@ -35,7 +35,7 @@ struct AttnArgs {
 	unsigned int* tickets; // (n_kv_heads,) zero-initialised, self-resetting
 	const uint8_t* pf_ptr; // first bytes of the next kernel's weights (Wo), pulled into L2 before this kernel waits for q
 	unsigned long long pf_bytes;
-	Timeline* tl;          // attn_cluster.cu, which cannot name xalm_cuda.cu's: where it stamps its start, its wait's end and its end (NULL: nowhere)
+	Timeline* tl;          // attn_cluster.cu, which cannot name xalm_cuda.cu's: where it stamps its start, its wait's end and its end (NULL: nothing records)
 };
 
 // K/V rows: coherent L2 loads (ld.global.cg).  NOT the read-only path: row kv_pos and the sink rows are written by the QKV

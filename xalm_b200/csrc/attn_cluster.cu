@@ -65,7 +65,7 @@ __device__ __forceinline__ void ac_cp_wait() { asm volatile("cp.async.wait_group
 
 enum { AC_EARLY = 0, AC_LATE = 1, AC_ALL = 2 }; // rows that this step's QKV kernel does not write | those it does | all
 
-template <int HD, int GP> // GP: query heads of a kv head
+template <int HD, int GP, bool TL> // GP: query heads of a kv head; TL: with stamps of the in-kernel timeline, as the split kernel's (code of their own: looked up at every launch they took 0.2 us a layer)
 __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnArgs a) {
 	constexpr int NW = AC_NW, NST = ac_stages(HD), KEYS = AC_KEYS, NTH = NW * 32, PIECES = HD / 8, TILE = KEYS * HD; // TILE: halves of a unit's keys
 	extern __shared__ __align__(128) uint8_t smem[];
@@ -80,11 +80,8 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 	ac_cluster_arrive(); // (1) every CTA of the cluster runs
 	const int C = gridDim.x, rank = blockIdx.x, kvh = blockIdx.y; // one cluster per kv head
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-	// The in-kernel timeline, as the split kernel's: its buffer (asked for here, looked at when the first keys are on their way), the time of the start and of the wait's
-	// end.  In shared memory: no registers are left, and the timer is read only while it records (read always, a layer took 0.2 us more).
-	__shared__ unsigned long long tl_sm[3];
-	const bool stamps = a.tl && (tid | rank | kvh) == 0;
-	const unsigned long long tl_buf = stamps ? __ldcg(reinterpret_cast<const unsigned long long*>(&a.tl->buf)) : 0ull;
+	__shared__ unsigned long long tl_sm[TL ? 2 : 1]; // the start, the wait's end (no registers are left)
+	if (TL && (tid | rank | kvh) == 0) tl_sm[0] = gtime();
 	if (tid == 0) l2_prefetch_slice(a.pf_ptr, a.pf_bytes, kvh * C + rank, C * (int) gridDim.y);
 
 	const bool fixed = a.kv_len_fixed >= 0;
@@ -111,10 +108,8 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		if (u0 + j * du < nu) fetch(u0 + j * du, j, AC_EARLY);
 	commit();
 
-	if (stamps) tl_sm[0] = tl_buf;
-	if (tl_buf) tl_sm[1] = gtime();
 	pdl_wait();
-	if (tl_buf) tl_sm[2] = gtime();
+	if (TL && (tid | rank | kvh) == 0) tl_sm[1] = gtime();
 #pragma unroll
 	for (int j = 0; j < NST; j++) {
 		const int u = u0 + j * du;
@@ -366,16 +361,16 @@ __global__ void __launch_bounds__(AC_NW * 32, 4) attn_cluster_kernel(const AttnA
 		den += __shfl_xor_sync(0xffffffffu, den, 2);
 		if (in && part == 0) a.out[(size_t) (kvh * GP + h) * HD + rank * own + x / GP] = num * (1.f / AC_PSCALE) / den;
 	}
-	if (a.tl && (tid | rank | kvh) == 0 && tl_sm[0]) {
+	if (TL && (tid | rank | kvh) == 0 && a.tl->buf) {
 		const unsigned int slot = atomicAdd(&a.tl->count, 1u);
-		unsigned long long* r = reinterpret_cast<unsigned long long*>(tl_sm[0]) + 4 * (size_t) slot;
-		if (slot < a.tl->cap) { r[0] = 300; r[1] = tl_sm[1]; r[2] = tl_sm[2]; r[3] = gtime(); }
+		unsigned long long* r = a.tl->buf + 4 * (size_t) slot;
+		if (slot < a.tl->cap) { r[0] = 300; r[1] = tl_sm[0]; r[2] = tl_sm[1]; r[3] = gtime(); }
 	}
 }
 
-template <int HD, int GP>
+template <int HD, int GP, bool TL = false>
 static cudaError_t ac_config(int n_kv, int C, cudaStream_t s, bool pdl, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
-	auto kern = attn_cluster_kernel<HD, GP>;
+	auto kern = attn_cluster_kernel<HD, GP, TL>;
 	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) ac_smem_bytes(HD, GP));
 	if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 	*cfg = {};
@@ -400,7 +395,7 @@ static int ac_size(int n_kv) {
 		cudaLaunchConfig_t cfg;
 		cudaLaunchAttribute at[2];
 		int n = 0;
-		if (ac_config<HD, GP>(n_kv, C, 0, false, &cfg, at) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, attn_cluster_kernel<HD, GP>, &cfg) != cudaSuccess) {
+		if (ac_config<HD, GP>(n_kv, C, 0, false, &cfg, at) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, attn_cluster_kernel<HD, GP, false>, &cfg) != cudaSuccess) {
 			cudaGetLastError();
 			continue;
 		}
@@ -438,11 +433,15 @@ int launch_attn_cluster(const AttnArgs& a, int head_dim, int G, int C, cudaStrea
 	cudaError_t e = cudaErrorInvalidValue;
 	cudaLaunchConfig_t cfg;
 	cudaLaunchAttribute at[2];
+#define XALM_AC_LAUNCH_TL(HD_, GP_, TL_)                                                \
+	e = ac_config<HD_, GP_, TL_>(a.n_kv_heads, C, s, pdl, &cfg, at);                    \
+	if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD_, GP_, TL_>, a);
 #define XALM_AC_LAUNCH(HD_, GP_)                                                        \
-	e = ac_config<HD_, GP_>(a.n_kv_heads, C, s, pdl, &cfg, at);                         \
-	if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD_, GP_>, a);
+	if (a.tl) { XALM_AC_LAUNCH_TL(HD_, GP_, true) }                                     \
+	else { XALM_AC_LAUNCH_TL(HD_, GP_, false) }
 	XALM_AC_CASES(XALM_AC_LAUNCH)
 #undef XALM_AC_LAUNCH
+#undef XALM_AC_LAUNCH_TL
 	if (e != cudaSuccess) return set_error(XALM_ERR_CUDA, "attention launch failed: %s", cudaGetErrorString(e));
 	return XALM_OK;
 }

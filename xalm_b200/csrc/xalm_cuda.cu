@@ -22,6 +22,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <string>
 #include <vector>
@@ -626,8 +627,10 @@ static cudaError_t launch_attn_hd(const AttnArgs& a, int G, cudaStream_t s, bool
 	}
 	return cudaErrorInvalidValue;
 }
-static Timeline* timeline_dev() { // of the current device
+static std::atomic<bool> g_timeline_on{false};
+static Timeline* timeline_dev() { // the current device's, while it records
 	void* p = nullptr;
+	if (!g_timeline_on.load()) return nullptr;
 	if (cudaGetSymbolAddress(&p, d_timeline) != cudaSuccess) {
 		cudaGetLastError();
 		return nullptr;
@@ -853,7 +856,7 @@ struct xalm_cuda_model {
 	unsigned int* tickets = nullptr;
 	int attn_splits = 0;
 	int attn_cluster = 0; // CTAs per kv head of attn_cluster.cu; 0: the split kernel of attention.cuh
-	Timeline* timeline = nullptr;
+	Timeline* timeline = nullptr; // what the steps' attention stamps (follow_timeline)
 	StepParams* d_step = nullptr;
 	StepParams* h_step = nullptr; // pinned ring
 	StepParams* h_step_io = nullptr; // pinned: the token of a call that waits for it
@@ -1599,7 +1602,6 @@ int xalm_cuda_finalize(xalm_cuda_model* m) {
 	XALM_CUDA_CHECK(cudaMemcpy(m->rope_freq, freq.data(), freq.size() * sizeof(float), cudaMemcpyHostToDevice));
 	const int G = c.n_heads / c.n_kv_heads;
 	m->attn_splits = attn_auto_splits(m->n_kv_heads_l);
-	m->timeline = timeline_dev();
 	m->attn_cluster = tune("attn_cluster") ? attn_cluster_size(c.head_dim, G, m->n_kv_heads_l, c.max_seq_len) : 0;
 	// the last-CTA merge parks 3 floats per (split, head) in the 8 x G x head_dim floats of the per-warp partial area (attention.cuh)
 	if (m->attn_splits > 8 * c.head_dim / 3) m->attn_splits = 8 * c.head_dim / 3;
@@ -1622,10 +1624,25 @@ int xalm_cuda_finalize(xalm_cuda_model* m) {
 	return XALM_OK;
 }
 
+// when recording began or ended since the last step, steps are captured again
+static int follow_timeline(xalm_cuda_model* m) {
+	Timeline* tl = timeline_dev();
+	if (tl == m->timeline) return XALM_OK;
+	XALM_CUDA_CHECK(cudaStreamSynchronize(m->stream));
+	for (cudaGraphExec_t* e : {&m->graph[0], &m->graph[1], &m->graph_io[0], &m->graph_io[1]})
+		if (*e) {
+			XALM_CUDA_CHECK(cudaGraphExecDestroy(*e));
+			*e = nullptr;
+		}
+	m->timeline = tl;
+	return XALM_OK;
+}
+
 static int ensure_graph(xalm_cuda_model* m, int mode, bool io = false) {
 	cudaGraphExec_t* exec = io ? &m->graph_io[mode] : &m->graph[mode];
-	if (*exec) return XALM_OK;
 	cudaStream_t s = m->stream;
+	XALM_TRY(follow_timeline(m));
+	if (*exec) return XALM_OK;
 	cudaGraph_t g = nullptr;
 	XALM_CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
 	int nl = 0;
@@ -1679,6 +1696,7 @@ int xalm_cuda_forward_async(xalm_cuda_model* m, int token, int pos, int mode) {
 		XALM_CUDA_CHECK(cudaGraphLaunch(m->graph[mode], s));
 		m->last_launches = m->launches_per_token[mode];
 	} else {
+		XALM_TRY(follow_timeline(m));
 		XALM_TRY(enqueue_token(m, mode, s, &m->last_launches));
 	}
 	return XALM_OK;
@@ -2085,9 +2103,11 @@ int xalm_cuda_timeline(int n_records, unsigned long long* out, int* n_out) {
 			t.buf = dbuf; t.cap = (unsigned) n_records;
 		}
 		XALM_CUDA_CHECK(cudaMemcpyToSymbol(d_timeline, &t, sizeof t));
+		g_timeline_on = n_records > 0;
 		return XALM_OK;
 	}
 	Timeline t;
+	g_timeline_on = false;
 	XALM_CUDA_CHECK(cudaMemcpyFromSymbol(&t, d_timeline, sizeof t));
 	int n = (int) (t.count < (unsigned) cap ? t.count : (unsigned) cap);
 	if (n > n_records) n = n_records;
